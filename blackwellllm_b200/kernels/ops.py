@@ -514,6 +514,40 @@ def attention_simt(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor
     return out
 
 
+def attention_f32_supports(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, nh: int) -> bool:
+    """Whether the tiled float32 kernel takes this geometry: head sizes in fours up to 256, at most 64 query heads per kv
+    head (a tile stacks 64 rows), rows that begin on 16 bytes.  A mask (causal, window, blocks) is all it knows of options."""
+    nkv, hd = k_pages.shape[1], k_pages.shape[3]
+    return (hd % 4 == 0 and hd <= 256 and nh % nkv == 0 and nh // nkv <= 64
+            and not any(t.data_ptr() % 16 for t in (q, k_pages, v_pages)))
+
+
+def attention_f32(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, batch, block_table: torch.Tensor, nh: int,
+                  window: Optional[int], scale: float, chunk: Optional[int] = None) -> torch.Tensor:
+    """Causal attention in float32 over tiles of stacked rows (prompt portions) and slices of keys (decoding requests)."""
+    _dev(q, "q", torch.float32); _dev(k_pages, "k_pages", torch.float32); _dev(v_pages, "v_pages", torch.float32)
+    _dev(block_table, "block_table", torch.int32)
+    num_pages, nkv, page_size, hd = k_pages.shape
+    if q.shape[1] != nh * hd:
+        raise KernelError("attention: q must be [T, nh * head_dim]")
+    out = torch.empty_like(q)
+    rows_w, n_rows, keys_w, n_keys, merge_w, n_merge, slices, _ = attention_work(
+        batch, nh // nkv, nkv, window, hd, rows_tile=64, page_size=page_size, chunk=chunk)
+    part_o = part_ml = None
+    if n_merge:
+        part_o = torch.empty((slices * nkv * 16, hd), dtype=torch.float32, device=out.device)
+        part_ml = torch.empty((slices * nkv * 16, 2), dtype=torch.float32, device=out.device)
+    fn = _fn("attention_f32", "bw_attention_f32", _ATTN_F32_ARGS)
+    _check(fn(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(batch.cu_q), _ptr(batch.q_start), _ptr(block_table),
+              block_table.shape[1], _ptr(rows_w), n_rows, _ptr(keys_w), n_keys, _ptr(merge_w), n_merge, _ptr(part_o),
+              _ptr(part_ml), nh, nkv, hd, page_size, num_pages, int(window or 0), int(chunk or 0), float(scale), _stream()),
+           "attention_f32")
+    return out
+
+
+_ATTN_F32_ARGS = [c_void_p] * 7 + [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p] + [c_int] * 7 + [c_float, c_void_p]
+
+
 def _gate_args(gate: Optional[tuple], T: int, nh: int, hd: int):
     """``gate`` = (float32 tensor [T, nh * dv], possibly a column range of a wider one; dv): what the attention
     kernels take as pointer, row stride and value size.  (g [T, nh], dv, "head"): one number per head; the kernels
@@ -891,6 +925,9 @@ def paged_attention(q, k_pages: torch.Tensor, v_pages: torch.Tensor, batch,
         if batch.T == batch.R and attention_takes_unrotated(k_pages.shape[3], k_pages.shape[2]):
             return attention_mma(q, k_pages, v_pages, batch, block_table, nh, window, scale, chunk, sink, gate)
         q = q.materialise()
+    if q.dtype == torch.float32 and not (sink is not None or gate is not None or dist is not None or softcap or rel is not None
+                                         or (keep_first and window)) and attention_f32_supports(q, k_pages, v_pages, nh):
+        return attention_f32(q, k_pages, v_pages, batch, block_table, nh, window, scale, chunk)
     if q.dtype == torch.float32:
         return attention_simt(q, k_pages, v_pages, batch.positions, batch.req_of_token, block_table, nh,
                               window, scale, chunk=chunk, sink=sink, gate=gate, dist=dist, keep_first=keep_first,

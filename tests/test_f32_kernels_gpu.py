@@ -1,8 +1,11 @@
-"""The 32-bit path's products for a few tokens, at the edges of their tiles, against 64 bits."""
+"""The 32-bit path's products for a few tokens and its tiled attention, at the edges of their tiles, against 64 bits and against the
+general kernels that take every other form."""
 import math
 
 import pytest
 import torch
+
+from test_kernels_gpu import FakeBatch, paged_case, plain_rows
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -43,3 +46,34 @@ def test_few_tokens(ops, M, N, K):
     assert product_error(ops.gemm_simt(wide[:, 4:4 + K], w), wide[:, 4:4 + K], w) <= bound      # rows further apart
     # rows that do not begin on 16 bytes: the general kernel
     assert product_error(ops.gemm_simt(wide[:, 3:3 + K], w), wide[:, 3:3 + K], w) <= 2 ** -24 * K
+
+
+@pytest.mark.parametrize("nh,nkv,hd,page", [(4, 2, 16, 16), (3, 1, 20, 8), (8, 8, 64, 16), (32, 8, 128, 16), (14, 2, 132, 4),
+                                            (6, 2, 256, 32), (17, 1, 32, 16), (64, 1, 8, 16), (5, 5, 80, 24)])
+@pytest.mark.parametrize("window,chunk", [(None, None), (1, None), (50, None), (None, 96), (40, 64)])
+def test_tiled_attention(ops, nh, nkv, hd, page, window, chunk):
+    # prompt portions (from position 0, continuing, ragged), single tokens at 1 and at many keys, a two-token portion
+    q_lens, kv_lens = [70, 1, 33, 2, 1, 130], [70, 900, 97, 64, 1, 400]
+    q, kp, vp, table, refs = paged_case(q_lens, kv_lens, nh, nkv, hd, page, torch.float32, seed=hd)
+    batch = FakeBatch(q_lens, kv_lens)
+    assert ops.attention_f32_supports(q, kp, vp, nh)
+    out = ops.attention_f32(q, kp, vp, batch, table, nh, window, hd ** -0.5, chunk)
+    general = ops.attention_simt(q, kp, vp, batch.positions, batch.req_of_token, table, nh, window, hd ** -0.5, chunk=chunk)
+    assert not torch.isnan(out).any()
+    # both are float32 softmaxes over at most 900 keys: scores up to |s| < 8 off by 2^-22 |s| sqrt(hd) move a weight by 2e-5 at most
+    assert float((out - general).abs().max()) <= 2e-5 * float(general.abs().max())
+    if chunk is None:
+        ref = plain_rows(refs, window, nh, hd)
+        assert float((out.double().cpu() - ref).abs().max()) <= 2e-5 * float(ref.abs().max())
+    # a table entry without a page hides its keys in both kernels
+    table[1, 3] = -1
+    out = ops.attention_f32(q, kp, vp, batch, table, nh, window, hd ** -0.5, chunk)
+    general = ops.attention_simt(q, kp, vp, batch.positions, batch.req_of_token, table, nh, window, hd ** -0.5, chunk=chunk)
+    assert float((out - general).abs().max()) <= 2e-5 * float(general.abs().max())
+
+
+def test_rows_off_16_bytes_go_to_the_general_kernel(ops):
+    q, kp, vp, table, refs = paged_case([5, 1], [5, 40], 4, 2, 18, 16, torch.float32, seed=3)
+    assert not ops.attention_f32_supports(q, kp, vp, 4)                   # a head size that is no multiple of four
+    out = ops.paged_attention(q, kp, vp, FakeBatch([5, 1], [5, 40]), table, 4, None, 18 ** -0.5)
+    assert float((out.double().cpu() - plain_rows(refs, None, 4, 18)).abs().max()) <= 2e-5
