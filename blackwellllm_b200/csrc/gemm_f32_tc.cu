@@ -1,0 +1,352 @@
+// out[M, N] (=|+=) x[M, K] . w[N, K]^T (+ bias), float32 in and out, on the tensor cores without losing float32's precision.
+//
+// Every operand is split into two TF32 numbers, hi = x rounded to 11 bits and lo = x - hi, which is exact and has at most 12 bits, of
+// which the tensor cores read 11 (what they drop is below 2^-23 |x|), and three products are summed, hi hi apart from hi lo + lo hi (lo lo is below 2^-22 of the product).  The
+// tensor cores' own sums are kept short: an accumulator takes 64 channels and is then added into float32 registers, rounded to
+// nearest, so no long chain runs through the tensor cores' accumulation.  Measured against 64 bits over the products of an 8B
+// decoder (K 4096 and 14336): relative error 2.2e-7 to 2.6e-7, where one chain of float32 FMAs (gemm_simt.cu) has 1.2e-6 to 2.2e-6.
+// A value that is not finite, or within 2^-12 of float32's largest, makes the results it enters NaN (inf - inf in the split).
+//
+// Weights are the 128-row operand (from tensor memory), tokens the other (from shared memory).  The tokens are split beforehand by a
+// small kernel (they are read again by every block of features); the weights, which are read once, on the way: a warp a quarter
+// of the rows, a lane a row, from the TMA tile into tensor memory.
+// An MMA of up to 128 columns takes 65 to 72 ns whatever its width, also where accumulators alternate, so there are few and wide
+// ones: hi of the weights times hi and lo of the tokens side by side (2 BN columns), and lo times hi into the second half: 8 for a
+// stage of 32 channels.  (Three products into one accumulator, 12 MMAs: 0.8 us a stage.)
+// Roles (896 threads): warp 0 TMA; warp 1 TMEM owner and MMAs; warps 4..11 split the weights, two groups that take stages in turn;
+// warps 12..27 add the accumulators up, 32 tokens each group of four, and write the result.  Every wait is bounded; a timeout sets
+// the status word and all roles fall through to the exit.
+// What bounds it: the MMAs' time (tensor pipe 41 % busy); for few tokens, with it, the bytes of the weights.  Measured, x 28672 x 4096:
+// 16 tokens 166 us (2.8 TB/s), 64 tokens 188 us, 301 tokens 524 us (135 TFLOP/s).  The products of 301 tokens in eight layers of the
+// 8B shape and its head: 9.9 ms, on gemm_simt.cu's tiles 65.0 ms.
+#include "tcgen05.cuh"
+
+using bf16 = __nv_bfloat16;
+
+namespace {
+
+constexpr int BM = 128, BK = 32, MAX_BN = 128;
+constexpr int A_BYTES = BM * BK * 4;
+constexpr int SUM_STAGES = 2;      // stages of an accumulator before it is added up
+constexpr int SPLIT_GROUPS = 2, SUM_GROUPS = 4;     // of four warps each, from warps 4 and 12 on
+constexpr int THREADS = 32 * (4 + 4 * SPLIT_GROUPS + 4 * SUM_GROUPS);
+constexpr int SMEM_BUDGET = 224 * 1024;
+constexpr int MAX_STAGES = 7;
+
+__device__ int g_status = 0;
+
+// Columns of tensor memory: one accumulator of 2 BN columns or (up to 64 tokens) two, then 64 (hi, lo) of every stage.
+__host__ __device__ constexpr int acc_cols(int bn) { return bn <= 32 ? 64 : bn <= 64 ? 128 : 256; }
+__host__ __device__ constexpr int acc_count(int bn) { return bn <= 64 ? 2 : 1; }
+__host__ __device__ constexpr int stage_bytes(int bn) { return A_BYTES + 2 * bn * BK * 4; }
+__host__ __device__ constexpr int stages_for(int bn) {
+    const int tmem = (512 - acc_count(bn) * acc_cols(bn)) / 64, smem = SMEM_BUDGET / stage_bytes(bn);
+    const int s = tmem < smem ? tmem : smem;
+    return s < MAX_STAGES ? s : MAX_STAGES;
+}
+
+// x rounded to TF32, halves away from zero (three integer instructions fewer than the conversion instruction takes; a NaN whose
+// bits overflow here stays one in x - hi)
+__device__ __forceinline__ float tf32_hi(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u); }
+// D[tmem] (+)= A[tmem] * B[smem]^T, TF32 inputs, float32 accumulators; one thread issues
+__device__ __forceinline__ void umma_tf32_ts(uint32_t d, uint32_t a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+                 "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n}"
+                 ::"r"(d), "r"(a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+// float32 accumulator, TF32 A and B (format 2), both K-major
+__device__ __forceinline__ uint32_t idesc_tf32(int n) {
+    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+}
+
+struct Out {
+    float* out; const void* bias; float* part;   // part: [splits][M][N], or null
+    long long ldo;
+    int bias_type, accumulate, M, N;
+};
+
+__device__ __forceinline__ float bias_at(const Out& o, int n) {
+    if (!o.bias) return 0.f;
+    return o.bias_type == BW_F32 ? ((const float*)o.bias)[n] : __bfloat162float(((const bf16*)o.bias)[n]);
+}
+
+// hi and lo parts of x, [2][M][K]; K % 4 == 0
+__global__ void __launch_bounds__(256)
+split_kernel(const float* __restrict__ x, float* __restrict__ xs, int M, int K, long long ldx) {
+    BW_PDL_TRIGGER();
+    BW_PDL_WAIT();
+    const int k4 = K / 4;
+    const long long total = (long long)M * k4;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const int row = (int)(i / k4), c = (int)(i - (long long)row * k4) * 4;
+        const float4 v = *reinterpret_cast<const float4*>(x + row * ldx + c);
+        const float in[4] = {v.x, v.y, v.z, v.w};
+        float hi[4], lo[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            hi[j] = tf32_hi(in[j]);
+            lo[j] = in[j] - hi[j];
+        }
+        *reinterpret_cast<float4*>(xs + (size_t)row * K + c) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<float4*>(xs + ((size_t)M + row) * K + c) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+    }
+}
+
+// block: (tile of features, tile of tokens, K split)
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, Out o, int bn, int kb_total,
+                   int kb_per_split) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t bars[3 * MAX_STAGES + 4];
+    __shared__ uint32_t tmem_slot[2];
+    BW_PDL_TRIGGER();
+    const int stages = stages_for(bn), per_stage = stage_bytes(bn);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t full0 = bw::smem_u32(bars), ready0 = full0 + 8 * MAX_STAGES, empty0 = ready0 + 8 * MAX_STAGES;
+    const uint32_t tfull0 = empty0 + 8 * MAX_STAGES, tempty0 = tfull0 + 16;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < stages; ++s) {
+            bw::mbar_init(full0 + 8 * s, 1);
+            bw::mbar_init(ready0 + 8 * s, 4);
+            bw::mbar_init(empty0 + 8 * s, 1);
+        }
+        for (int a = 0; a < 2; ++a) { bw::mbar_init(tfull0 + 8 * a, 1); bw::mbar_init(tempty0 + 8 * a, 4 * SUM_GROUPS); }
+        bw::fence_barrier_init();
+        bw::tma_prefetch_desc(&tm_w);
+        bw::tma_prefetch_desc(&tm_x);
+        tmem_slot[1] = (uint32_t)g_status;      // an earlier timeout: later launches do no work
+    }
+    if (warp == 1) bw::tmem_alloc(bw::smem_u32(tmem_slot), 512);
+    bw::tc_fence_before();
+    __syncthreads();
+    bw::tc_fence_after();
+    const uint32_t tmem = tmem_slot[0], tmem_a = tmem + acc_count(bn) * acc_cols(bn);
+    const bool dead = tmem_slot[1] != 0;
+    const int n0 = blockIdx.x * BM, m0 = blockIdx.y * bn, split = blockIdx.z;
+    const int kb0 = split * kb_per_split, nkb = min(kb_total, kb0 + kb_per_split) - kb0;
+
+    if (dead) {
+        // fall through to the exit
+    } else if (warp == 0) {
+        if (lane == 0) {
+            // the weights of the first stages are nobody's output: requested before the wait for the earlier kernels
+            const int ahead = min(nkb, stages);
+            for (int i = 0; i < ahead; ++i) {
+                bw::mbar_expect_tx(full0 + 8 * i, per_stage);
+                bw::tma_load_2d(bw::smem_u32(smem + i * per_stage), &tm_w, full0 + 8 * i, (kb0 + i) * BK, n0);
+            }
+            BW_PDL_WAIT();
+            for (int i = 0; i < nkb; ++i) {
+                const int s = i % stages;
+                const uint32_t dst = bw::smem_u32(smem + s * per_stage);
+                if (i >= ahead) {
+                    if (!bw::mbar_wait(empty0 + 8 * s, (i / stages - 1) & 1, &g_status, 1)) break;
+                    bw::mbar_expect_tx(full0 + 8 * s, per_stage);
+                    bw::tma_load_2d(dst, &tm_w, full0 + 8 * s, (kb0 + i) * BK, n0);
+                }
+                bw::tma_load_2d(dst + A_BYTES, &tm_x, full0 + 8 * s, (kb0 + i) * BK, m0);
+                bw::tma_load_2d(dst + A_BYTES + bn * BK * 4, &tm_x, full0 + 8 * s, (kb0 + i) * BK, o.M + m0);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = idesc_tf32(bn), idesc2 = idesc_tf32(2 * bn);
+            const int accs = acc_count(bn);
+            bool ok = true;
+            for (int i = 0; i < nkb; ++i) {
+                const int s = i % stages, p = i / SUM_STAGES, buf = p % accs;
+                const bool fresh = i % SUM_STAGES == 0;
+                ok = bw::mbar_wait(full0 + 8 * s, (i / stages) & 1, &g_status, 2) && bw::mbar_wait(ready0 + 8 * s, (i / stages) & 1, &g_status, 3);
+                if (ok && fresh) ok = bw::mbar_wait(tempty0 + 8 * buf, ((p / accs) & 1) ^ 1, &g_status, 4);
+                if (!ok) break;
+                bw::tc_fence_after();
+                const uint32_t d = tmem + buf * acc_cols(bn), hi = tmem_a + s * 64;
+                const uint64_t b = bw::umma_smem_desc_sw128(bw::smem_u32(smem + s * per_stage + A_BYTES));
+                // 8 channels an MMA: 8 columns of A, 32 bytes (2 units of 16) of B's rows; B's lo rows lie behind its hi rows
+#pragma unroll
+                for (int k = 0; k < 4; ++k) umma_tf32_ts(d, hi + 8 * k, b + 2 * k, idesc2, !fresh || k != 0);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) umma_tf32_ts(d + bn, hi + 32 + 8 * k, b + 2 * k, idesc, 1);
+                bw::umma_commit(empty0 + 8 * s);
+                if (i % SUM_STAGES == SUM_STAGES - 1 || i == nkb - 1) bw::umma_commit(tfull0 + 8 * buf);
+            }
+        }
+    } else if (warp >= 4 && warp < 4 + 4 * SPLIT_GROUPS) {
+        const int quarter = warp & 3, row = quarter * 32 + lane;
+        for (int i = (warp - 4) / 4; i < nkb; i += SPLIT_GROUPS) {
+            const int s = i % stages;
+            if (!bw::mbar_wait(full0 + 8 * s, (i / stages) & 1, &g_status, 5)) break;
+            bw::tc_fence_after();      // (the MMAs that read this stage's columns before are complete: the tile was loaded after them)
+            const uint8_t* src = smem + s * per_stage + row * 128;
+            const uint32_t dst = tmem_a + s * 64 + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {           // 16 channels at a time
+                uint32_t hi[16], lo[16];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {       // 16-byte pieces of the row where the 128-byte swizzle put them
+                    const float4 v = *reinterpret_cast<const float4*>(src + (((4 * h + j) ^ (row & 7)) << 4));
+                    const float in[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float h32 = tf32_hi(in[c]);
+                        hi[4 * j + c] = __float_as_uint(h32);
+                        lo[4 * j + c] = __float_as_uint(in[c] - h32);
+                    }
+                }
+                bw::tmem_st_32x16(dst + 16 * h, hi);
+                bw::tmem_st_32x16(dst + 32 + 16 * h, lo);
+            }
+            bw::tmem_st_wait();
+            bw::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) bw::mbar_arrive(ready0 + 8 * s);
+        }
+    } else if (warp >= 4 + 4 * SPLIT_GROUPS) {
+        constexpr int COLS = MAX_BN / SUM_GROUPS;
+        const int quarter = warp & 3, first = ((warp - 4 - 4 * SPLIT_GROUPS) / 4) * COLS, cols = min(bn - first, COLS);
+        float sum[COLS];
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) sum[c] = 0.f;
+        bool ok = true;
+        const int accs = acc_count(bn);
+        for (int p = 0; p * SUM_STAGES < nkb; ++p) {
+            const int buf = p % accs;
+            if (!bw::mbar_wait(tfull0 + 8 * buf, (p / accs) & 1, &g_status, 6)) { ok = false; break; }
+            bw::tc_fence_after();
+            const uint32_t from = tmem + buf * acc_cols(bn) + first + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll
+            for (int c0 = 0; c0 < COLS; c0 += 16) {
+                if (c0 >= cols) continue;
+                uint32_t big[16], small[16];
+                bw::tmem_ld_32x16(from + c0, big);
+                bw::tmem_ld_32x16(from + bn + c0, small);
+                bw::tmem_ld_wait();
+#pragma unroll
+                for (int c = 0; c < 16; ++c) sum[c0 + c] += __uint_as_float(big[c]) + __uint_as_float(small[c]);
+            }
+            bw::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) bw::mbar_arrive(tempty0 + 8 * buf);
+        }
+        BW_PDL_WAIT();      // the result belongs to earlier kernels until here
+        const int n = n0 + quarter * 32 + lane, t0 = m0 + first;
+        if (ok && n < o.N) {
+            const bool whole = !o.part;
+            const long long ld = whole ? o.ldo : o.N;
+            const float b = whole ? bias_at(o, n) : 0.f;
+            const bool add = whole && o.accumulate;
+            float* dst = whole ? o.out + (size_t)t0 * ld + n : o.part + ((size_t)split * o.M + t0) * o.N + n;
+#pragma unroll
+            for (int c0 = 0; c0 < COLS; c0 += 16) {       // sixteen tokens' old values in flight
+                if (c0 >= cols) continue;
+                float old[16];
+#pragma unroll
+                for (int c = 0; c < 16; ++c) old[c] = add && t0 + c0 + c < o.M ? dst[(size_t)(c0 + c) * ld] : 0.f;
+#pragma unroll
+                for (int c = 0; c < 16; ++c)
+                    if (t0 + c0 + c < o.M) dst[(size_t)(c0 + c) * ld] = add ? sum[c0 + c] + b + old[c] : sum[c0 + c] + b;
+                asm volatile("" ::: "memory");
+            }
+        }
+    }
+    bw::tc_fence_before();
+    __syncthreads();
+    bw::tc_fence_after();
+    if (warp == 1) bw::tmem_dealloc(tmem, 512);
+}
+
+// the K splits' planes, in split order
+__global__ void __launch_bounds__(256)
+sum_kernel(Out o, int splits) {
+    BW_PDL_TRIGGER();
+    BW_PDL_WAIT();
+    const int n = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
+    if (n >= o.N) return;
+    const size_t plane = (size_t)o.M * o.N;
+    const float* p = o.part + (size_t)m * o.N + n;
+    float s = p[0];
+    for (int i = 1; i < splits; ++i) s += p[i * plane];
+    s += bias_at(o, n);
+    float* dst = o.out + m * o.ldo + n;
+    *dst = o.accumulate ? s + *dst : s;
+}
+
+bool encode(CUtensorMap* m, const void* base, long long rows, long long cols, int box_rows) {
+    typedef CUresult (*Fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                           const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static Fn fn = nullptr;
+    if (!fn) {
+        void* ptr = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+            return false;
+        fn = (Fn)ptr;
+    }
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)cols * 4};
+    const cuuint32_t box[2] = {BK, (cuuint32_t)box_rows}, estr[2] = {1, 1};
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+}  // namespace
+
+// How the product is cut: tokens of a tile (a multiple of 16, at most 128: the tiles as even as they can be) and K splits.  A split costs
+// a round of the SMs a part of its stages, about eight stages' time of its own (filling and draining the pipeline), and its plane a
+// pass through memory (a stage of one SM takes 0.55 us, with more than 64 tokens 0.7 us; the planes 8 bytes a value at 5 TB/s).
+BW_EXPORT int bw_gemm_f32_tc_plan(int M, int N, int K, int sms, int* bn_out, int* splits_out) {
+    if (M <= 0 || N <= 0 || K <= 0 || sms <= 0) return BW_ERR_BAD_ARG;
+    const int tiles_m = (M + MAX_BN - 1) / MAX_BN;
+    const int bn = (((M + tiles_m - 1) / tiles_m) + 15) / 16 * 16;
+    const long long tiles = (long long)((M + bn - 1) / bn) * ((N + BM - 1) / BM);
+    const int kb = (K + BK - 1) / BK;
+    int best = 1;
+    double best_us = 0;
+    for (int s = 1; s <= 16 && (s == 1 || (kb / s >= 8 && M <= 65535)); ++s) {
+        const int per = (kb + s - 1) / s, used = (kb + per - 1) / per;
+        if (used != s) continue;
+        const long long rounds = (tiles * s + sms - 1) / sms;
+        double us = (bn <= 64 ? 0.55 : 0.7) * rounds * (per + 8);
+        if (s > 1) us += 3.0 + 8e-12 * 1e6 / 5.0 * s * (double)M * N;
+        if (s == 1 || us < best_us) { best = s; best_us = us; }
+    }
+    *bn_out = bn;
+    *splits_out = best;
+    return 0;
+}
+
+// xs: float32 [2 * M * K] for the tokens' parts; part: float32 [splits * M * N], not read or written with one split (may be null).
+// K % 4 == 0, rows of x and w begin on 16 bytes; bn and splits from bw_gemm_f32_tc_plan.
+BW_EXPORT int bw_gemm_f32_tc(const float* x, const float* w, const void* bias, int bias_type, float* out, int M, int N, int K, long long ldx,
+                             long long ldo, int accumulate, float* xs, float* part, int bn, int splits, void* stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (K <= 0 || K % 4 || ldx % 4 || ldx < K || ldo < N || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)xs) & 15)) return BW_ERR_BAD_ARG;
+    if (bn < 16 || bn > MAX_BN || bn % 16 || splits < 1 || (splits > 1 && !part)) return BW_ERR_BAD_ARG;
+    const int kb = (K + BK - 1) / BK, per = (kb + splits - 1) / splits;
+    if ((kb + per - 1) / per != splits || (M + bn - 1) / bn > 65535 || (splits > 1 && M > 65535)) return BW_ERR_BAD_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    CUtensorMap tm_w, tm_x;
+    if (!encode(&tm_w, w, N, K, BM) || !encode(&tm_x, xs, 2ll * M, K, bn)) return BW_ERR_DRIVER;
+    const long long pieces = ((long long)M * (K / 4) + 255) / 256;
+    bw::launch(split_kernel, dim3((unsigned)(pieces < 4 * bw::num_sms() ? pieces : 4 * bw::num_sms())), dim3(256), 0, s, x, xs, M, K, ldx);
+    BW_LAUNCH_CHECK();
+    static bool done[bw::MAX_DEVICES] = {};
+    const cudaError_t e = bw::allow_dynamic_smem(gemm_f32_tc_kernel, SMEM_BUDGET + 1024, done);
+    if (e != cudaSuccess) return (int)e;
+    const Out o = {out, bias, splits > 1 ? part : nullptr, ldo, bias_type, accumulate, M, N};
+    bw::launch(gemm_f32_tc_kernel, dim3((N + BM - 1) / BM, (M + bn - 1) / bn, splits), dim3(THREADS),
+               (size_t)stages_for(bn) * stage_bytes(bn) + 1024, s, tm_w, tm_x, o, bn, kb, per);
+    BW_LAUNCH_CHECK();
+    if (splits > 1) {
+        bw::launch(sum_kernel, dim3((N + 255) / 256, M), dim3(256), 0, s, o, splits);
+        BW_LAUNCH_CHECK();
+    }
+    return 0;
+}
+
+// 0 if no bounded wait ever gave up (synchronises the device)
+BW_EXPORT int bw_gemm_f32_tc_status() {
+    int v = 0;
+    if (cudaMemcpyFromSymbol(&v, g_status, sizeof(int)) != cudaSuccess) return -1;
+    return v;
+}

@@ -483,6 +483,60 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = N
 
 # ------------------------------------------------------------------ attention
 
+GEMM_F32_FEW_TOKENS = 8      # up to here a product's weights go straight into registers (the CUDA-core library's kernel for few tokens)
+_GEMM_F32_TC_ARGS = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_void_p, c_void_p, c_int,
+                     c_int, c_void_p]
+_f32_plans = {}
+
+
+def gemm_f32_tc_supports(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether the tensor-core product of split float32 operands takes these: channels in fours, rows that begin on 16 bytes, and a
+    weight of at least one tile's rows and eight stages' channels (a smaller one is all latency there, and its chains too short to err more)."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and w.shape[0] >= 128 and w.shape[1] >= 256 and w.shape[1] % 4 == 0
+            and x.dim() == 2 and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
+             accumulate: bool = False) -> torch.Tensor:
+    """out (=|+=) x @ w.T (+ bias) in float32: above ``GEMM_F32_FEW_TOKENS`` rows on the tensor cores from operands split into two
+    TF32 parts, whose error is no larger than that of float32 FMAs; else, and for forms that kernel does not take, on the CUDA cores."""
+    M = x.shape[0]
+    if M <= GEMM_F32_FEW_TOKENS or not gemm_f32_tc_supports(x, w):
+        return gemm_simt(x, w, bias, out=out, accumulate=accumulate)
+    _dev(x, "x", torch.float32, contiguous=False); _dev(w, "w", torch.float32)
+    N, K = w.shape
+    if x.shape[1] != K:
+        raise KernelError(f"gemm: x has {x.shape[1]} columns, w has {K}")
+    if out is None:
+        if accumulate:
+            raise KernelError("gemm: accumulate needs an output tensor")
+        out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    _dev(out, "out", torch.float32, contiguous=False)
+    if out.shape != (M, N) or out.stride(1) != 1:
+        raise KernelError("gemm: out must be [M, N] with contiguous rows")
+    if bias is not None:
+        _dev(bias, "bias")
+        if bias.numel() != N:
+            raise KernelError("gemm: bias must have N entries")
+    plan = _f32_plans.get((M, N, K))
+    if plan is None:
+        bn, splits = c_int(), c_int()
+        _check_plan = _fn("gemm_f32_tc", "bw_gemm_f32_tc_plan", [c_int, c_int, c_int, c_int, c_void_p, c_void_p])(
+            M, N, K, num_sms(x.device), ctypes.addressof(bn), ctypes.addressof(splits))
+        if _check_plan != 0:
+            raise KernelError(f"gemm_f32_tc: no plan for {M} x {N} x {K}")
+        if len(_f32_plans) > 4096:
+            _f32_plans.clear()
+        plan = _f32_plans[(M, N, K)] = (bn.value, splits.value)
+    bn, splits = plan
+    parts = torch.empty((2 * M * K,), dtype=torch.float32, device=x.device)
+    planes = torch.empty((splits * M * N,), dtype=torch.float32, device=x.device) if splits > 1 else None
+    fn = _fn("gemm_f32_tc", "bw_gemm_f32_tc", _GEMM_F32_TC_ARGS, tag=f"{M}x{N}x{K}")
+    _check(fn(_ptr(x), _ptr(w), _ptr(bias), _code(bias, "bias") if bias is not None else 0, _ptr(out), M, N, K, x.stride(0),
+              out.stride(0), int(accumulate), _ptr(parts), _ptr(planes), bn, splits, _stream()), "gemm_f32_tc")
+    return out
+
+
 def attention_simt(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, positions: torch.Tensor,
                    req_of_token: torch.Tensor, block_table: torch.Tensor, nh: int, window: Optional[int],
                    scale: float, out: Optional[torch.Tensor] = None, chunk: Optional[int] = None,

@@ -1,7 +1,9 @@
 """A weight matrix [out, in] with an optional bias, and the one place that picks
 the matrix-product kernel for it.
 
-float32 weights run on the CUDA cores with float32 FMAs (the true 32-bit path).
+float32 weights are multiplied in float32 (the true 32-bit path): on the CUDA cores for a few
+tokens and for small weights, else on the tensor cores from operands split in two, with an
+error no larger than that of a chain of float32 FMAs.
 bfloat16 weights run on the tcgen05 tensor-core kernel; a shape that kernel
 refuses (an inner size that is no multiple of 8, which a TMA row stride cannot
 express) runs on the CUDA-core kernel with bfloat16 operands and float32 sums.
@@ -31,6 +33,8 @@ class Linear:
             raise ops.KernelError(f"Linear: input is {x.dtype}, weight is {w.dtype}")
         if w.dtype == torch.bfloat16 and ops.gemm_tc_supports(x, w):
             return ops.gemm_tc(x, w, self.bias, out=out, out_dtype=out_dtype, accumulate=accumulate)
+        if w.dtype == torch.float32 and out_dtype in (None, torch.float32) and (out is None or out.dtype == torch.float32):
+            return ops.gemm_f32(x, w, self.bias, out=out, accumulate=accumulate)
         return ops.gemm_simt(x, w, self.bias, out=out, out_dtype=out_dtype, accumulate=accumulate)
 
     def _may_defer(self, x: torch.Tensor, out: torch.Tensor) -> bool:

@@ -48,6 +48,38 @@ def test_few_tokens(ops, M, N, K):
     assert product_error(ops.gemm_simt(wide[:, 3:3 + K], w), wide[:, 3:3 + K], w) <= 2 ** -24 * K
 
 
+# tokens on both sides of the widths of a tile and of its columns in tensor memory; ragged features; channels that leave the last
+# stage ragged, and enough of them for K splits
+@pytest.mark.parametrize("M", [9, 16, 17, 33, 65, 128, 129, 200, 257])
+@pytest.mark.parametrize("N,K", [(128, 256), (130, 260), (200, 1028), (1024, 4100), (4096, 2048)])
+def test_split_products(ops, M, N, K):
+    x, w, b, base = rand(M, K + 4, seed=1)[:, 4:], rand(N, K, seed=2), rand(N, seed=3), rand(M, N + 1, seed=4)
+    assert ops.gemm_f32_tc_supports(x, w)
+    want = x.double() @ w.double().T
+    size = float(want.pow(2).mean().sqrt())
+    err = lambda out, ref: float((out.double() - ref).pow(2).mean().sqrt()) / size
+    plain = ops.gemm_f32(x, w)
+    # no further off than one chain of float32 FMAs, whose error grows with the root of K (from 17 tokens on gemm_simt is that chain;
+    # up to 1,028 channels both are at a few roundings of the result, 2^-24 each)
+    chain = ops.gemm_simt(x.repeat(2, 1), w)[:M]
+    assert err(plain, want) <= max(err(chain, want), 1.5e-7)
+    # products off by up to 2^-22 each add up like their root: at most 2^-22 of the result's size, and the largest of 1e6 is five times that
+    assert float((plain.double() - want).abs().max()) / size <= 2 ** -22 * 8 + 2 ** -24 * math.sqrt(K)
+    out = base.clone()
+    ops.gemm_f32(x, w, b.bfloat16(), out=out[:, :N], accumulate=True)
+    assert err(out[:, :N], want + b.bfloat16().double() + base[:, :N].double()) <= 3e-7 * max(1.0, 1.0 / size)
+    assert torch.equal(out[:, N], base[:, N])
+    assert torch.equal(ops.gemm_f32(x, w), plain)
+
+
+def test_split_products_over_the_range_of_float32(ops):
+    """Magnitudes from the smallest normal products to large ones, in one product each: the split is relative to each value."""
+    for scale_x, scale_w in ((1e-15, 1e-15), (1e15, 1e15), (1e-18, 1e18)):
+        x, w = rand(40, 512, seed=1) * scale_x, rand(256, 512, seed=2) * scale_w
+        want = x.double() @ w.double().T
+        assert float((ops.gemm_f32(x, w).double() - want).abs().max()) <= 1e-6 * float(want.abs().max())
+
+
 @pytest.mark.parametrize("nh,nkv,hd,page", [(4, 2, 16, 16), (3, 1, 20, 8), (8, 8, 64, 16), (32, 8, 128, 16), (14, 2, 132, 4),
                                             (6, 2, 256, 32), (17, 1, 32, 16), (64, 1, 8, 16), (5, 5, 80, 24)])
 @pytest.mark.parametrize("window,chunk", [(None, None), (1, None), (50, None), (None, 96), (40, 64)])
