@@ -60,7 +60,8 @@ def native():
                 "bwh_free_request": (ci, [vp, ci]), "bwh_num_blocks": (ci, [vp, ci, ci]),
                 "bwh_blocks": (ci, [vp, ci, ci, vp, ci]), "bwh_check": (ci, [vp]),
                 "bwh_pack_step": (ll, [vp, ci, vp, vp, vp, vp, vp, ci, ci, ll, vp, ll, vp, vp]),
-                "bwh_release_passed_many": (ci, [vp, ci, vp]), "bwh_set_keep_first": (ci, [vp, ci, ci])}
+                "bwh_release_passed_many": (ci, [vp, ci, vp]), "bwh_set_keep_first": (ci, [vp, ci, ci]),
+                "bwh_uniform": (None, [ci, vp, vp, vp])}
         for name, (res, args) in sigs.items():
             fn = getattr(lib, name)
             fn.restype, fn.argtypes = res, args

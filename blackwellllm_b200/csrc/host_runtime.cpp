@@ -391,3 +391,19 @@ BWH_EXPORT int bwh_release_passed_many(void* cache, int R, const int* handles) {
     }
     return freed;
 }
+
+// One number in [0, 1) with 24 bits per row: the draws[i]-th of the stream of seeds[i] (Philox 4x32-10, as sampling/params.py has
+// it: 4 us a number there, 25 ns here, where a step of 32 sampled rows waits for them).
+BWH_EXPORT void bwh_uniform(int n, const uint64_t* seeds, const uint64_t* draws, float* out) {
+    for (int i = 0; i < n; ++i) {
+        uint32_t c0 = (uint32_t)draws[i], c1 = (uint32_t)(draws[i] >> 32), c2 = 0, c3 = 0;
+        uint32_t k0 = (uint32_t)seeds[i], k1 = (uint32_t)(seeds[i] >> 32);
+        for (int round = 0; round < 10; ++round) {
+            const uint64_t p0 = 0xD2511F53ull * c0, p1 = 0xCD9E8D57ull * c2;
+            const uint32_t n0 = (uint32_t)(p1 >> 32) ^ c1 ^ k0, n2 = (uint32_t)(p0 >> 32) ^ c3 ^ k1;
+            c1 = (uint32_t)p1; c3 = (uint32_t)p0; c0 = n0; c2 = n2;
+            k0 += 0x9E3779B9u; k1 += 0xBB67AE85u;
+        }
+        out[i] = (float)(c0 >> 8) * (1.0f / 16777216.0f);
+    }
+}

@@ -16,6 +16,8 @@ from __future__ import annotations
 from dataclasses import dataclass
 from typing import Optional, Sequence, Tuple
 
+import numpy as np
+
 _M0, _M1 = 0xD2511F53, 0xCD9E8D57
 _W0, _W1 = 0x9E3779B9, 0xBB67AE85
 _MASK = 0xFFFFFFFF
@@ -37,6 +39,15 @@ def uniform(seed: int, index: int) -> float:
     """The ``index``-th number of the stream of ``seed``: uniform in [0, 1) with 24 bits."""
     r = philox4x32((index & _MASK, (index >> 32) & _MASK, 0, 0), (seed & _MASK, (seed >> 32) & _MASK))
     return (r[0] >> 8) * (1.0 / (1 << 24))
+
+
+def uniform_many(seeds: Sequence[int], indices: Sequence[int]) -> np.ndarray:
+    """:func:`uniform` of every (seed, index), float32, in the host runtime."""
+    from ..cache.manager import native
+    out = np.empty(len(seeds), dtype=np.float32)
+    s, i = (np.array([int(v) & 0xFFFFFFFFFFFFFFFF for v in vals], dtype=np.uint64) for vals in (seeds, indices))
+    native().bwh_uniform(len(out), s.ctypes.data, i.ctypes.data, out.ctypes.data)
+    return out
 
 
 @dataclass

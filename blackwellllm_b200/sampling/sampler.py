@@ -14,7 +14,7 @@ from typing import List, Optional, Sequence
 import torch
 
 from ..kernels import ops
-from .params import SamplingParams, uniform
+from .params import SamplingParams, uniform_many
 
 
 class Sampler:
@@ -61,8 +61,11 @@ class Sampler:
             return ops.sample(logits, None, None, None)
         host = torch.empty((3, R), dtype=torch.float32, pin_memory=True)
         rows = host.numpy()   # filled row by row: one assignment each instead of one per request
-        rows[0] = [0.0 if p.greedy else p.temperature for p in params]
+        temps = [0.0 if p.greedy else p.temperature for p in params]
+        rows[0] = temps
         rows[1] = [p.top_p for p in params]
-        rows[2] = [0.0 if p.greedy else uniform(seeds[r], draw_index[r]) for r, p in enumerate(params)]
+        rows[2] = uniform_many(seeds, draw_index)
+        if 0.0 in temps:
+            rows[2][rows[0] == 0.0] = 0.0      # greedy rows draw nothing
         dev = host.to(self.device, non_blocking=True)
         return ops.sample(logits, dev[0], dev[1], dev[2])
