@@ -5,8 +5,10 @@
 // A block of eight warps takes a tile of ROWS stacked query rows (token-major, then the heads of the group) of one request and
 // kv head and walks 32 keys at a time (two stages, cp.async).  Scores: each thread a few rows times a few keys.  Softmax and
 // values: warp w owns rows w ROWS / 8 on, a lane four channels (twice that for heads above 128), so probabilities pass through
-// shared memory inside the warp only.  ROWS = 64 for prompt portions, 16 for the few rows of a decoding request, whose keys are
-// dealt out in slices to fill the GPU; a second kernel merges the slices.
+// shared memory inside the warp only.  ROWS = 64 for prompt portions, 16 for the few rows of a decoding request, whose slices of
+// SLICE keys have blocks of their own; a second kernel adds them up.
+// A row's result is the same bits whatever else is in the batch: both forms make a softmax per slice of SLICE keys, counted from
+// position 0, in the same order of operations, and fold the slices in their order (fold()).
 // What bounds it: decode, the bytes of keys and values; prompts, shared-memory reads (six 16-byte reads per 32 FMAs).  Measured at
 // head size 128, groups of 4, 8 kv heads, against attention_simt.cu (a block per token and head, a lane a key): 4 requests at
 // 1,000 keys 45 us with the merge against 347, 301 prompt tokens 84 us against 827.
@@ -14,7 +16,7 @@
 
 namespace {
 
-constexpr int THREADS = 256, WARPS = 8, KEYS = 32, SLICE_ROWS = 16;
+constexpr int THREADS = 256, WARPS = 8, KEYS = 32, SLICE_ROWS = 16, SLICE = 128;
 
 struct Params {
     const float *q, *k_pages, *v_pages;
@@ -34,13 +36,26 @@ __host__ __device__ constexpr int smem_floats(int rows, int hd) {
     return rows * (hd + 4) + 2 * KEYS * (hd + 4) + 2 * KEYS * hd + rows * (KEYS + 4) + 2 * KEYS;
 }
 
+// One more slice (maximum m, sum l) of a row: the factors of what was there (M, L) and of the slice; M and L are updated.  A slice in
+// which the row sees no key changes nothing.
+__device__ __forceinline__ float2 fold(float& M, float& L, float m, float l) {
+    if (m == -INFINITY) return make_float2(1.f, 0.f);
+    const float to = fmaxf(M, m), a = M == -INFINITY ? 0.f : expf(M - to), b = expf(m - to);
+    L = fmaf(L, a, __fmul_rn(l, b));
+    M = to;
+    return make_float2(a, b);
+}
+__device__ __forceinline__ float folded(float O, float o, float2 f) { return fmaf(O, f.x, __fmul_rn(o, f.y)); }
+// The slices that the rows at positions pos0 .. end - 1 see: from this key on, and so many.
+__device__ __forceinline__ int slices_from(const Params& p, int pos0) { return bw::first_visible(pos0, p.window, p.chunk) / SLICE * SLICE; }
+__device__ __forceinline__ int slices_of(int base, int end) { return (end - base + SLICE - 1) / SLICE; }
+
 // SLICES: work items (request, slice, slices, first slot), all tokens of the request's segment; else (request, first token).
 // CH: groups of four channels of a lane.
 template <int ROWS, int CH, bool SLICES>
 __global__ void __launch_bounds__(THREADS)
 attention_f32_kernel(Params p, const int4* __restrict__ work) {
     BW_PDL_TRIGGER();
-    BW_PDL_WAIT();
     extern __shared__ float4 smem4[];
     const int hd = p.hd, ldk = hd + 4, G = p.nh / p.nkv;
     float* qs = reinterpret_cast<float*>(smem4);          // [ROWS][ldk]
@@ -48,7 +63,7 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
     float* vs = ks + 2 * KEYS * ldk;                      // [2][KEYS][hd]
     float* ps = vs + 2 * KEYS * hd;                       // [ROWS][KEYS + 4]
     int* known = reinterpret_cast<int*>(ps + ROWS * (KEYS + 4));   // [2][KEYS]: the key has a page
-    constexpr int LDP = KEYS + 4;
+    constexpr int LDP = KEYS + 4, PER = SLICE / KEYS;     // tiles of a slice
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kvh = blockIdx.y;
     const int4 item = work[blockIdx.x];
     const int r = item.x;
@@ -57,10 +72,11 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
     const int tokens = min(ROWS / G, q_len - t0), rows = tokens * G;
     const int pos0 = p.q_start[r] + t0, end = pos0 + tokens;
     const int* bt = p.block_table + (size_t)r * p.max_blocks;
-    const int base = bw::first_visible(pos0, p.window, p.chunk) & ~(KEYS - 1);
+    const int base = slices_from(p, pos0), slices = slices_of(base, end);
+    if (SLICES && item.y >= slices) return;               // (the list is as long as the longest context may get)
     const int all = (end - base + KEYS - 1) / KEYS;
-    const int first = SLICES ? (int)((long long)all * item.y / item.z) : 0;
-    const int last = SLICES ? (int)((long long)all * (item.y + 1) / item.z) : all;
+    const int first = SLICES ? item.y * PER : 0, last = SLICES ? min(first + PER, all) : all;
+    BW_PDL_WAIT();
 
     for (int i = warp; i < ROWS; i += WARPS) {      // rows beyond the tile's are zeros
         const float* src = p.q + ((size_t)(row0 + t0 + i / G) * p.nh + (size_t)kvh * G + i % G) * hd;
@@ -91,6 +107,14 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
         m[i] = -INFINITY; l[i] = 0.f;
 #pragma unroll
         for (int c = 0; c < CH * 4; ++c) o[i][c] = 0.f;
+    }
+    constexpr int FOLDED = SLICES ? 1 : RW;         // rows of a portion fold their slices here
+    float O[FOLDED][CH * 4], M[FOLDED], L[FOLDED];
+#pragma unroll
+    for (int i = 0; i < FOLDED; ++i) {
+        M[i] = -INFINITY; L[i] = 0.f;
+#pragma unroll
+        for (int c = 0; c < CH * 4; ++c) O[i][c] = 0.f;
     }
     constexpr int TX = ROWS == 64 ? 8 : 16, RPT = ROWS == 64 ? 2 : 1, KPT = KEYS / TX, TY = THREADS / TX;
     const int tx = tid % TX, ty = tid / TX;
@@ -171,56 +195,79 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
                     }
                 }
         }
+        if constexpr (!SLICES) {
+            if ((tile + 1) % PER == 0 || tile + 1 == last) {
+#pragma unroll
+                for (int i = 0; i < RW; ++i) {
+                    const float2 f = fold(M[i], L[i], m[i], l[i]);
+#pragma unroll
+                    for (int c = 0; c < CH * 4; ++c) { O[i][c] = folded(O[i][c], o[i][c], f); o[i][c] = 0.f; }
+                    m[i] = -INFINITY; l[i] = 0.f;
+                }
+            }
+        }
         __syncthreads();        // (the next fetch overwrites this stage, the next scores the probabilities)
     }
 #pragma unroll
     for (int i = 0; i < RW; ++i) {
         const int row = warp * RW + i;
         if (row >= rows) continue;
-        const bool partial = SLICES && item.z > 1;
-        const float f = partial ? 1.f : (l[i] > 0.f ? 1.f / l[i] : 0.f);
+        float f = 1.f;
         float* dst;
-        if (partial) {
+        if (SLICES && item.z > 1) {
             const size_t slot = ((size_t)(item.w + item.y) * p.nkv + kvh) * SLICE_ROWS + row;
             dst = p.part_o + slot * hd;
             if (lane == 0) { p.part_ml[2 * slot] = m[i]; p.part_ml[2 * slot + 1] = l[i]; }
         } else {
+            const float sum = SLICES ? l[i] : L[i];
+            f = sum > 0.f ? 1.f / sum : 0.f;
             dst = p.out + ((size_t)(row0 + t0 + row / G) * p.nh + (size_t)kvh * G + row % G) * hd;
+        }
+        float res[CH * 4];
+#pragma unroll
+        for (int c = 0; c < CH * 4; ++c) {
+            if constexpr (SLICES) res[c] = o[i][c] * f;
+            else res[c] = O[i][c] * f;
         }
 #pragma unroll
         for (int h = 0; h < CH; ++h) {
             const int c = lane * 4 + 128 * h;
-            if (c < hd) *reinterpret_cast<float4*>(dst + c) = make_float4(o[i][4 * h] * f, o[i][4 * h + 1] * f, o[i][4 * h + 2] * f, o[i][4 * h + 3] * f);
+            if (c < hd) *reinterpret_cast<float4*>(dst + c) = make_float4(res[4 * h], res[4 * h + 1], res[4 * h + 2], res[4 * h + 3]);
         }
     }
 }
 
-// Slices of one (request, kv head, row), in slice order; a thread a channel.
-__global__ void __launch_bounds__(128)
+// Slices of one (request, kv head, row), in slice order; a thread four channels.
+__global__ void __launch_bounds__(64)
 attention_f32_merge_kernel(Params p, const int4* __restrict__ work) {
     BW_PDL_TRIGGER();
-    BW_PDL_WAIT();
     const int4 item = work[blockIdx.x];
-    const int r = item.x, kvh = blockIdx.y, row = blockIdx.z, G = p.nh / p.nkv, hd = p.hd;
-    const int row0 = p.cu_q[r], q_len = p.cu_q[r + 1] - row0;
-    if (row >= q_len * G) return;
-    auto slot = [&](int s) { return ((size_t)(item.w + s) * p.nkv + kvh) * SLICE_ROWS + row; };
-    float M = -INFINITY;
-    for (int s = 0; s < item.z; ++s) M = fmaxf(M, p.part_ml[2 * slot(s)]);
-    float L = 0.f;
-    for (int s = 0; s < item.z; ++s) {
-        const float m = p.part_ml[2 * slot(s)];
-        L += m == -INFINITY ? 0.f : p.part_ml[2 * slot(s) + 1] * expf(m - M);
+    const int r = item.x, kvh = blockIdx.y, row = blockIdx.z, G = p.nh / p.nkv, hd = p.hd, c = threadIdx.x * 4;
+    const int row0 = p.cu_q[r], q_len = p.cu_q[r + 1] - row0, pos0 = p.q_start[r];
+    if (row >= q_len * G || c >= hd) return;
+    const int slices = slices_of(slices_from(p, pos0), pos0 + q_len);
+    BW_PDL_WAIT();
+    float M = -INFINITY, L = 0.f, O[4] = {0.f, 0.f, 0.f, 0.f};
+    constexpr int AHEAD = 8;             // slices whose loads are in flight together
+    for (int s0 = 0; s0 < slices; s0 += AHEAD) {
+        float4 v[AHEAD];
+        float2 ml[AHEAD];
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            const size_t slot = ((size_t)(item.w + min(s0 + i, slices - 1)) * p.nkv + kvh) * SLICE_ROWS + row;
+            ml[i] = *reinterpret_cast<const float2*>(p.part_ml + 2 * slot);
+            v[i] = *reinterpret_cast<const float4*>(p.part_o + slot * hd + c);
+        }
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            if (s0 + i >= slices) break;
+            const float2 f = fold(M, L, ml[i].x, ml[i].y);
+            O[0] = folded(O[0], v[i].x, f); O[1] = folded(O[1], v[i].y, f); O[2] = folded(O[2], v[i].z, f); O[3] = folded(O[3], v[i].w, f);
+        }
     }
     const float inv = L > 0.f ? 1.f / L : 0.f;
-    for (int c = threadIdx.x; c < hd; c += blockDim.x) {
-        float o = 0.f;
-        for (int s = 0; s < item.z; ++s) {
-            const float m = p.part_ml[2 * slot(s)];
-            if (m != -INFINITY) o += p.part_o[slot(s) * hd + c] * expf(m - M);
-        }
-        p.out[((size_t)(row0 + row / G) * p.nh + (size_t)kvh * G + row % G) * hd + c] = o * inv;
-    }
+    *reinterpret_cast<float4*>(p.out + ((size_t)(row0 + row / G) * p.nh + (size_t)kvh * G + row % G) * hd + c) =
+        make_float4(O[0] * inv, O[1] * inv, O[2] * inv, O[3] * inv);
 }
 
 template <int ROWS, int CH, bool SLICES>
@@ -235,8 +282,11 @@ int go(const Params& p, const int* work, int n, cudaStream_t s) {
 
 }  // namespace
 
+// The keys of a slice (the work lists count with it).
+BW_EXPORT int bw_attention_f32_slice() { return SLICE; }
+
 // rows_w: int32 [n_rows][4] (request, first token, 0, 0), tiles of 64 / (nh / nkv) tokens; keys_w: [n_keys][4] (request, slice,
-// slices, first slot) for segments of at most 16 stacked rows; merge_w: [n_merge][4] (request, 0, slices, first slot).  part_o,
+// slices, first slot) for segments of at most 16 stacked rows, at least as many slices as the segment's rows see; merge_w: [n_merge][4] (request, 0, slices, first slot).  part_o,
 // part_ml: float32 [slots][nkv][16][hd] and [..][2] (null without merge items).  hd % 4 == 0, hd <= 256, nh / nkv <= 64.
 BW_EXPORT int bw_attention_f32(const float* q, const float* k_pages, const float* v_pages, float* out, const int* cu_q,
                                const int* q_start, const int* block_table, int max_blocks, const int* rows_w, int n_rows,
@@ -251,7 +301,7 @@ BW_EXPORT int bw_attention_f32(const float* q, const float* k_pages, const float
     if (n_rows) rc = hd <= 128 ? go<64, 1, false>(p, rows_w, n_rows, s) : go<64, 2, false>(p, rows_w, n_rows, s);
     if (rc == 0 && n_keys) rc = hd <= 128 ? go<SLICE_ROWS, 1, true>(p, keys_w, n_keys, s) : go<SLICE_ROWS, 2, true>(p, keys_w, n_keys, s);
     if (rc == 0 && n_merge) {
-        bw::launch(attention_f32_merge_kernel, dim3(n_merge, nkv, SLICE_ROWS), dim3(128), 0, s, p, (const int4*)merge_w);
+        bw::launch(attention_f32_merge_kernel, dim3(n_merge, nkv, SLICE_ROWS), dim3(64), 0, s, p, (const int4*)merge_w);
         BW_LAUNCH_CHECK();
     }
     return rc;

@@ -10,15 +10,17 @@
 // Weights are the 128-row operand (from tensor memory), tokens the other (from shared memory).  The tokens are split beforehand by a
 // small kernel (they are read again by every block of features); the weights, which are read once, on the way: a warp a quarter
 // of the rows, a lane a row, from the TMA tile into tensor memory.
-// An MMA of up to 128 columns takes 65 to 72 ns whatever its width, also where accumulators alternate, so there are few and wide
-// ones: hi of the weights times hi and lo of the tokens side by side (2 BN columns), and lo times hi into the second half: 8 for a
-// stage of 32 channels.  (Three products into one accumulator, 12 MMAs: 0.8 us a stage.)
+// Few and wide MMAs: hi of the weights times hi and lo of the tokens side by side (2 BN columns), and lo times hi into the second
+// half: 8 for a stage of 32 channels.
+// A token's result is the same whatever else is in the batch: the channels of all tiles of features, laid end to end, are cut into one
+// range per SM, whatever the number of tokens; a range's part of a tile is summed as above, and a tile's parts are added in their
+// order by a second kernel.  (So every SM also streams the same number of bytes, and no round of blocks ends half empty.)
 // Roles (896 threads): warp 0 TMA; warp 1 TMEM owner and MMAs; warps 4..11 split the weights, two groups that take stages in turn;
 // warps 12..27 add the accumulators up, 32 tokens each group of four, and write the result.  Every wait is bounded; a timeout sets
 // the status word and all roles fall through to the exit.
-// What bounds it: the MMAs' time (tensor pipe 41 % busy); for few tokens, with it, the bytes of the weights.  Measured, x 28672 x 4096:
-// 16 tokens 166 us (2.8 TB/s), 64 tokens 188 us, 301 tokens 524 us (135 TFLOP/s).  The products of 301 tokens in eight layers of the
-// 8B shape and its head: 9.9 ms, on gemm_simt.cu's tiles 65.0 ms.
+// What bounds it: up to 16 tokens the bytes of the weights, above 64 the MMAs and shared memory.  Measured, x 28672 x 4096: 1 to 16
+// tokens 111 us (4.2 TB/s), 64 tokens 141 us, 128 tokens 191 us (157 TFLOP/s), 301 tokens 511 us.  301 tokens scored in eight layers of
+// the 8B shape, logits at each: 72.2 ms on gemm_simt.cu's tiles (65.0 of them products), 12.8 ms so.
 #include "tcgen05.cuh"
 
 using bf16 = __nv_bfloat16;
@@ -60,9 +62,38 @@ __device__ __forceinline__ uint32_t idesc_tf32(int n) {
 }
 
 struct Out {
-    float* out; const void* bias; float* part;   // part: [splits][M][N], or null
+    float* out; const void* bias; float* part;   // part: [parts][M][N]
     long long ldo;
     int bias_type, accumulate, M, N;
+};
+
+// The stages (32 channels of a tile of features) of all tiles, dealt out to `ctas` ranges.
+struct Cut {
+    int kb_total, tiles_n, ctas;
+    __host__ __device__ long long total() const { return (long long)tiles_n * kb_total; }
+    __host__ __device__ long long begin(int c) const { return c * total() / ctas; }
+    __host__ __device__ int owner(long long kb) const { return (int)(((kb + 1) * ctas + total() - 1) / total()) - 1; }
+    __host__ __device__ int first_part(int tile) const { return owner((long long)tile * kb_total); }
+    __host__ __device__ int parts(int tile) const { return owner((long long)(tile + 1) * kb_total - 1) - first_part(tile) + 1; }
+};
+// One CTA's items: for every tile of tokens, its range's piece of every tile of features.
+struct Items {
+    Cut cut;
+    int tiles_m, mt;
+    int lo, hi, at;
+    int tile, kb0, n;        // the item: tile of features, first stage, stages (tile of tokens: mt)
+    __device__ Items(const Cut& c, int tiles_m_) : cut(c), tiles_m(tiles_m_), mt(0) {
+        lo = (int)cut.begin(blockIdx.x); hi = (int)cut.begin(blockIdx.x + 1); at = lo;
+    }
+    __device__ bool next() {
+        if (at >= hi) { at = lo; ++mt; }
+        if (mt >= tiles_m || lo >= hi) return false;
+        tile = at / cut.kb_total;
+        kb0 = at - tile * cut.kb_total;
+        n = min(cut.kb_total - kb0, hi - at);
+        at += n;
+        return true;
+    }
 };
 
 __device__ __forceinline__ float bias_at(const Out& o, int n) {
@@ -92,10 +123,9 @@ split_kernel(const float* __restrict__ x, float* __restrict__ xs, int M, int K, 
     }
 }
 
-// block: (tile of features, tile of tokens, K split)
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, Out o, int bn, int kb_total,
-                   int kb_per_split) {
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, Out o, int bn, Cut cut,
+                   int tiles_m) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t bars[3 * MAX_STAGES + 4];
@@ -123,60 +153,78 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     bw::tc_fence_after();
     const uint32_t tmem = tmem_slot[0], tmem_a = tmem + acc_count(bn) * acc_cols(bn);
     const bool dead = tmem_slot[1] != 0;
-    const int n0 = blockIdx.x * BM, m0 = blockIdx.y * bn, split = blockIdx.z;
-    const int kb0 = split * kb_per_split, nkb = min(kb_total, kb0 + kb_per_split) - kb0;
+    Items it(cut, tiles_m);
 
     if (dead) {
         // fall through to the exit
     } else if (warp == 0) {
         if (lane == 0) {
             // the weights of the first stages are nobody's output: requested before the wait for the earlier kernels
-            const int ahead = min(nkb, stages);
-            for (int i = 0; i < ahead; ++i) {
-                bw::mbar_expect_tx(full0 + 8 * i, per_stage);
-                bw::tma_load_2d(bw::smem_u32(smem + i * per_stage), &tm_w, full0 + 8 * i, (kb0 + i) * BK, n0);
+            int ahead = 0, s = 0;
+            uint32_t round = 0;
+            Items peek = it;
+            if (peek.next()) {
+                ahead = min(peek.n, stages);
+                for (int i = 0; i < ahead; ++i) {
+                    bw::mbar_expect_tx(full0 + 8 * i, per_stage);
+                    bw::tma_load_2d(bw::smem_u32(smem + i * per_stage), &tm_w, full0 + 8 * i, (peek.kb0 + i) * BK, peek.tile * BM);
+                }
             }
             BW_PDL_WAIT();
-            for (int i = 0; i < nkb; ++i) {
-                const int s = i % stages;
-                const uint32_t dst = bw::smem_u32(smem + s * per_stage);
-                if (i >= ahead) {
-                    if (!bw::mbar_wait(empty0 + 8 * s, (i / stages - 1) & 1, &g_status, 1)) break;
-                    bw::mbar_expect_tx(full0 + 8 * s, per_stage);
-                    bw::tma_load_2d(dst, &tm_w, full0 + 8 * s, (kb0 + i) * BK, n0);
+            bool ok = true;
+            while (ok && it.next()) {
+                for (int i = 0; i < it.n; ++i) {
+                    const uint32_t dst = bw::smem_u32(smem + s * per_stage);
+                    if (ahead > 0) --ahead;
+                    else {
+                        if (round > 0 && !bw::mbar_wait(empty0 + 8 * s, (round - 1) & 1, &g_status, 1)) { ok = false; break; }
+                        bw::mbar_expect_tx(full0 + 8 * s, per_stage);
+                        bw::tma_load_2d(dst, &tm_w, full0 + 8 * s, (it.kb0 + i) * BK, it.tile * BM);
+                    }
+                    bw::tma_load_2d(dst + A_BYTES, &tm_x, full0 + 8 * s, (it.kb0 + i) * BK, it.mt * bn);
+                    bw::tma_load_2d(dst + A_BYTES + bn * BK * 4, &tm_x, full0 + 8 * s, (it.kb0 + i) * BK, o.M + it.mt * bn);
+                    if (++s == stages) { s = 0; ++round; }
                 }
-                bw::tma_load_2d(dst + A_BYTES, &tm_x, full0 + 8 * s, (kb0 + i) * BK, m0);
-                bw::tma_load_2d(dst + A_BYTES + bn * BK * 4, &tm_x, full0 + 8 * s, (kb0 + i) * BK, o.M + m0);
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = idesc_tf32(bn), idesc2 = idesc_tf32(2 * bn);
-            const int accs = acc_count(bn);
-            bool ok = true;
-            for (int i = 0; i < nkb; ++i) {
-                const int s = i % stages, p = i / SUM_STAGES, buf = p % accs;
-                const bool fresh = i % SUM_STAGES == 0;
-                ok = bw::mbar_wait(full0 + 8 * s, (i / stages) & 1, &g_status, 2) && bw::mbar_wait(ready0 + 8 * s, (i / stages) & 1, &g_status, 3);
-                if (ok && fresh) ok = bw::mbar_wait(tempty0 + 8 * buf, ((p / accs) & 1) ^ 1, &g_status, 4);
-                if (!ok) break;
+        // the whole warp walks the stages, one elected lane issues: operands the compiler knows to be the same in all lanes (in a branch
+        // of one lane an MMA took 100 to 150 cycles to issue, whatever its size; so 9, or what the tensor pipe needs)
+        const uint32_t base = __shfl_sync(0xffffffffu, tmem, 0), cols_a = base + acc_count(bn) * acc_cols(bn);
+        const uint32_t idesc = idesc_tf32(bn), idesc2 = idesc_tf32(2 * bn), smem0 = bw::smem_u32(smem);
+        const int accs = acc_count(bn);
+        int s = 0, ph = 0, p = 0;
+        bool ok = true;
+        while (ok && it.next()) {
+            for (int i = 0; i < it.n; ++i) {
+                const int buf = p % accs;
+                const bool fresh = i % SUM_STAGES == 0, last = i % SUM_STAGES == SUM_STAGES - 1 || i == it.n - 1;
+                ok = bw::mbar_wait(full0 + 8 * s, ph, &g_status, 2) && bw::mbar_wait(ready0 + 8 * s, ph, &g_status, 3);
+                if (fresh) ok = ok && bw::mbar_wait(tempty0 + 8 * buf, ((p / accs) & 1) ^ 1, &g_status, 4);
+                if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
                 bw::tc_fence_after();
-                const uint32_t d = tmem + buf * acc_cols(bn), hi = tmem_a + s * 64;
-                const uint64_t b = bw::umma_smem_desc_sw128(bw::smem_u32(smem + s * per_stage + A_BYTES));
-                // 8 channels an MMA: 8 columns of A, 32 bytes (2 units of 16) of B's rows; B's lo rows lie behind its hi rows
+                const uint32_t d = base + buf * acc_cols(bn), hi = cols_a + s * 64;
+                const uint64_t b = bw::umma_smem_desc_sw128(smem0 + s * per_stage + A_BYTES);
+                if (bw::elect_one()) {
+                    // 8 channels an MMA: 8 columns of A, 32 bytes (2 units of 16) of B's rows; B's lo rows lie behind its hi rows
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma_tf32_ts(d, hi + 8 * k, b + 2 * k, idesc2, !fresh || k != 0);
+                    for (int k = 0; k < 4; ++k) umma_tf32_ts(d, hi + 8 * k, b + 2 * k, idesc2, !fresh || k != 0);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma_tf32_ts(d + bn, hi + 32 + 8 * k, b + 2 * k, idesc, 1);
-                bw::umma_commit(empty0 + 8 * s);
-                if (i % SUM_STAGES == SUM_STAGES - 1 || i == nkb - 1) bw::umma_commit(tfull0 + 8 * buf);
+                    for (int k = 0; k < 4; ++k) umma_tf32_ts(d + bn, hi + 32 + 8 * k, b + 2 * k, idesc, 1);
+                    bw::umma_commit(empty0 + 8 * s);
+                    if (last) bw::umma_commit(tfull0 + 8 * buf);
+                }
+                __syncwarp();
+                if (last) ++p;
+                if (++s == stages) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp >= 4 && warp < 4 + 4 * SPLIT_GROUPS) {
         const int quarter = warp & 3, row = quarter * 32 + lane;
-        for (int i = (warp - 4) / 4; i < nkb; i += SPLIT_GROUPS) {
-            const int s = i % stages;
-            if (!bw::mbar_wait(full0 + 8 * s, (i / stages) & 1, &g_status, 5)) break;
+        const long long all = (cut.begin(blockIdx.x + 1) - cut.begin(blockIdx.x)) * tiles_m;      // stages of all items
+        int s = (warp - 4) / 4, ph = 0;
+        for (long long i = s; i < all; i += SPLIT_GROUPS) {
+            if (!bw::mbar_wait(full0 + 8 * s, ph, &g_status, 5)) break;
             bw::tc_fence_after();      // (the MMAs that read this stage's columns before are complete: the tile was loaded after them)
             const uint8_t* src = smem + s * per_stage + row * 128;
             const uint32_t dst = tmem_a + s * 64 + ((uint32_t)(quarter * 32) << 16);
@@ -201,42 +249,47 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             bw::tc_fence_before();
             __syncwarp();
             if (lane == 0) bw::mbar_arrive(ready0 + 8 * s);
+            s += SPLIT_GROUPS;
+            if (s >= stages) { s -= stages; ph ^= 1; }
         }
     } else if (warp >= 4 + 4 * SPLIT_GROUPS) {
         constexpr int COLS = MAX_BN / SUM_GROUPS;
         const int quarter = warp & 3, first = ((warp - 4 - 4 * SPLIT_GROUPS) / 4) * COLS, cols = min(bn - first, COLS);
-        float sum[COLS];
-#pragma unroll
-        for (int c = 0; c < COLS; ++c) sum[c] = 0.f;
-        bool ok = true;
         const int accs = acc_count(bn);
-        for (int p = 0; p * SUM_STAGES < nkb; ++p) {
-            const int buf = p % accs;
-            if (!bw::mbar_wait(tfull0 + 8 * buf, (p / accs) & 1, &g_status, 6)) { ok = false; break; }
-            bw::tc_fence_after();
-            const uint32_t from = tmem + buf * acc_cols(bn) + first + ((uint32_t)(quarter * 32) << 16);
+        bool ok = true, waited = false;
+        int p = 0;
+        while (ok && it.next()) {
+            float sum[COLS];
 #pragma unroll
-            for (int c0 = 0; c0 < COLS; c0 += 16) {
-                if (c0 >= cols) continue;
-                uint32_t big[16], small[16];
-                bw::tmem_ld_32x16(from + c0, big);
-                bw::tmem_ld_32x16(from + bn + c0, small);
-                bw::tmem_ld_wait();
+            for (int c = 0; c < COLS; ++c) sum[c] = 0.f;
+            for (int i = 0; i < it.n; i += SUM_STAGES, ++p) {
+                const int buf = p % accs;
+                if (!bw::mbar_wait(tfull0 + 8 * buf, (p / accs) & 1, &g_status, 6)) { ok = false; break; }
+                bw::tc_fence_after();
+                const uint32_t from = tmem + buf * acc_cols(bn) + first + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll
-                for (int c = 0; c < 16; ++c) sum[c0 + c] += __uint_as_float(big[c]) + __uint_as_float(small[c]);
+                for (int c0 = 0; c0 < COLS; c0 += 16) {
+                    if (c0 >= cols) continue;
+                    uint32_t big[16], small[16];
+                    bw::tmem_ld_32x16(from + c0, big);
+                    bw::tmem_ld_32x16(from + bn + c0, small);
+                    bw::tmem_ld_wait();
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) sum[c0 + c] += __uint_as_float(big[c]) + __uint_as_float(small[c]);
+                }
+                bw::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) bw::mbar_arrive(tempty0 + 8 * buf);
             }
-            bw::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) bw::mbar_arrive(tempty0 + 8 * buf);
-        }
-        BW_PDL_WAIT();      // the result belongs to earlier kernels until here
-        const int n = n0 + quarter * 32 + lane, t0 = m0 + first;
-        if (ok && n < o.N) {
-            const bool whole = !o.part;
+            if (!waited) { BW_PDL_WAIT(); waited = true; }      // the result belongs to earlier kernels until here
+            const int n = it.tile * BM + quarter * 32 + lane, t0 = it.mt * bn + first;
+            if (!ok || n >= o.N) continue;
+            const bool whole = it.n == cut.kb_total;
             const long long ld = whole ? o.ldo : o.N;
             const float b = whole ? bias_at(o, n) : 0.f;
             const bool add = whole && o.accumulate;
-            float* dst = whole ? o.out + (size_t)t0 * ld + n : o.part + ((size_t)split * o.M + t0) * o.N + n;
+            float* dst = whole ? o.out + (size_t)t0 * ld + n
+                               : o.part + ((size_t)((int)blockIdx.x - cut.first_part(it.tile)) * o.M + t0) * o.N + n;
 #pragma unroll
             for (int c0 = 0; c0 < COLS; c0 += 16) {       // sixteen tokens' old values in flight
                 if (c0 >= cols) continue;
@@ -256,20 +309,34 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     if (warp == 1) bw::tmem_dealloc(tmem, 512);
 }
 
-// the K splits' planes, in split order
+// The parts of the tiles that several ranges share, in their order; four features a thread where V is 4.
+template <int V>
 __global__ void __launch_bounds__(256)
-sum_kernel(Out o, int splits) {
+sum_kernel(Out o, Cut cut) {
     BW_PDL_TRIGGER();
     BW_PDL_WAIT();
-    const int n = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
+    const int n = (blockIdx.x * blockDim.x + threadIdx.x) * V, m = blockIdx.y;
     if (n >= o.N) return;
+    const int parts = cut.parts(n / BM);
+    if (parts == 1) return;
     const size_t plane = (size_t)o.M * o.N;
     const float* p = o.part + (size_t)m * o.N + n;
-    float s = p[0];
-    for (int i = 1; i < splits; ++i) s += p[i * plane];
-    s += bias_at(o, n);
+    float s[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) s[e] = 0.f;
+    for (int i = 0; i < parts; ++i) {
+        float v[V];
+        if constexpr (V == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p + i * plane);
+        else v[0] = p[i * plane];
+#pragma unroll
+        for (int e = 0; e < V; ++e) s[e] = i ? s[e] + v[e] : v[e];
+    }
     float* dst = o.out + m * o.ldo + n;
-    *dst = o.accumulate ? s + *dst : s;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+        s[e] += bias_at(o, n + e);
+        dst[e] = o.accumulate ? s[e] + dst[e] : s[e];
+    }
 }
 
 bool encode(CUtensorMap* m, const void* base, long long rows, long long cols, int box_rows) {
@@ -291,39 +358,34 @@ bool encode(CUtensorMap* m, const void* base, long long rows, long long cols, in
 
 }  // namespace
 
-// How the product is cut: tokens of a tile (a multiple of 16, at most 128: the tiles as even as they can be) and K splits.  A split costs
-// a round of the SMs a part of its stages, about eight stages' time of its own (filling and draining the pipeline), and its plane a
-// pass through memory (a stage of one SM takes 0.55 us, with more than 64 tokens 0.7 us; the planes 8 bytes a value at 5 TB/s).
-BW_EXPORT int bw_gemm_f32_tc_plan(int M, int N, int K, int sms, int* bn_out, int* splits_out) {
-    if (M <= 0 || N <= 0 || K <= 0 || sms <= 0) return BW_ERR_BAD_ARG;
-    const int tiles_m = (M + MAX_BN - 1) / MAX_BN;
-    const int bn = (((M + tiles_m - 1) / tiles_m) + 15) / 16 * 16;
-    const long long tiles = (long long)((M + bn - 1) / bn) * ((N + BM - 1) / BM);
-    const int kb = (K + BK - 1) / BK;
-    int best = 1;
-    double best_us = 0;
-    for (int s = 1; s <= 16 && (s == 1 || (kb / s >= 8 && M <= 65535)); ++s) {
-        const int per = (kb + s - 1) / s, used = (kb + per - 1) / per;
-        if (used != s) continue;
-        const long long rounds = (tiles * s + sms - 1) / sms;
-        double us = (bn <= 64 ? 0.55 : 0.7) * rounds * (per + 8);
-        if (s > 1) us += 3.0 + 8e-12 * 1e6 / 5.0 * s * (double)M * N;
-        if (s == 1 || us < best_us) { best = s; best_us = us; }
-    }
-    *bn_out = bn;
-    *splits_out = best;
-    return 0;
+static Cut cut_of(int N, int K) {
+    Cut c = {(K + BK - 1) / BK, (N + BM - 1) / BM, 1};
+    const long long most = c.total() / 8;        // eight stages or more each: less would be all filling and draining
+    c.ctas = most < 1 ? 1 : most < bw::num_sms() ? (int)most : bw::num_sms();
+    return c;
 }
 
-// xs: float32 [2 * M * K] for the tokens' parts; part: float32 [splits * M * N], not read or written with one split (may be null).
-// K % 4 == 0, rows of x and w begin on 16 bytes; bn and splits from bw_gemm_f32_tc_plan.
+// The parts that a tile of features comes in at most (their planes are the scratch of bw_gemm_f32_tc).
+BW_EXPORT int bw_gemm_f32_tc_parts(int N, int K) {
+    if (N <= 0 || K <= 0) return BW_ERR_BAD_ARG;
+    const Cut c = cut_of(N, K);
+    int most = 1;
+    for (int t = 0; t < c.tiles_n; ++t) if (c.parts(t) > most) most = c.parts(t);
+    return most;
+}
+
+// xs: float32 [2 * M * K] for the tokens' parts; part: float32 [parts * M * N] (bw_gemm_f32_tc_parts), not used where that is 1.
+// K % 4 == 0, rows of x and w begin on 16 bytes; at most 65,535 tokens.
 BW_EXPORT int bw_gemm_f32_tc(const float* x, const float* w, const void* bias, int bias_type, float* out, int M, int N, int K, long long ldx,
-                             long long ldo, int accumulate, float* xs, float* part, int bn, int splits, void* stream) {
+                             long long ldo, int accumulate, float* xs, float* part, void* stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (K <= 0 || K % 4 || ldx % 4 || ldx < K || ldo < N || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)xs) & 15)) return BW_ERR_BAD_ARG;
-    if (bn < 16 || bn > MAX_BN || bn % 16 || splits < 1 || (splits > 1 && !part)) return BW_ERR_BAD_ARG;
-    const int kb = (K + BK - 1) / BK, per = (kb + splits - 1) / splits;
-    if ((kb + per - 1) / per != splits || (M + bn - 1) / bn > 65535 || (splits > 1 && M > 65535)) return BW_ERR_BAD_ARG;
+    if (K <= 0 || K % 4 || ldx % 4 || ldx < K || ldo < N || M > 65535 || cut_of(N, K).total() > 0x7fffffff || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)xs) & 15)) return BW_ERR_BAD_ARG;
+    const Cut cut = cut_of(N, K);
+    bool shared = false;
+    for (int t = 0; t < cut.tiles_n && !shared; ++t) shared = cut.parts(t) > 1;
+    if (shared && (!part || ((uintptr_t)part & 15))) return BW_ERR_BAD_ARG;
+    // tiles of tokens as even as they can be, a multiple of 16
+    const int tiles = (M + MAX_BN - 1) / MAX_BN, bn = ((M + tiles - 1) / tiles + 15) / 16 * 16, tiles_m = (M + bn - 1) / bn;
     cudaStream_t s = (cudaStream_t)stream;
     CUtensorMap tm_w, tm_x;
     if (!encode(&tm_w, w, N, K, BM) || !encode(&tm_x, xs, 2ll * M, K, bn)) return BW_ERR_DRIVER;
@@ -333,12 +395,13 @@ BW_EXPORT int bw_gemm_f32_tc(const float* x, const float* w, const void* bias, i
     static bool done[bw::MAX_DEVICES] = {};
     const cudaError_t e = bw::allow_dynamic_smem(gemm_f32_tc_kernel, SMEM_BUDGET + 1024, done);
     if (e != cudaSuccess) return (int)e;
-    const Out o = {out, bias, splits > 1 ? part : nullptr, ldo, bias_type, accumulate, M, N};
-    bw::launch(gemm_f32_tc_kernel, dim3((N + BM - 1) / BM, (M + bn - 1) / bn, splits), dim3(THREADS),
-               (size_t)stages_for(bn) * stage_bytes(bn) + 1024, s, tm_w, tm_x, o, bn, kb, per);
+    const Out o = {out, bias, part, ldo, bias_type, accumulate, M, N};
+    bw::launch(gemm_f32_tc_kernel, dim3(cut.ctas), dim3(THREADS), (size_t)stages_for(bn) * stage_bytes(bn) + 1024, s, tm_w, tm_x, o, bn, cut,
+               tiles_m);
     BW_LAUNCH_CHECK();
-    if (splits > 1) {
-        bw::launch(sum_kernel, dim3((N + 255) / 256, M), dim3(256), 0, s, o, splits);
+    if (shared) {
+        if (N % 4 == 0) bw::launch(sum_kernel<4>, dim3((N / 4 + 255) / 256, M), dim3(256), 0, s, o, cut);
+        else bw::launch(sum_kernel<1>, dim3((N + 255) / 256, M), dim3(256), 0, s, o, cut);
         BW_LAUNCH_CHECK();
     }
     return 0;

@@ -483,10 +483,9 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = N
 
 # ------------------------------------------------------------------ attention
 
-GEMM_F32_FEW_TOKENS = 8      # up to here a product's weights go straight into registers (the CUDA-core library's kernel for few tokens)
-_GEMM_F32_TC_ARGS = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_void_p, c_void_p, c_int,
-                     c_int, c_void_p]
-_f32_plans = {}
+_GEMM_F32_TC_ARGS = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_void_p, c_void_p, c_void_p]
+_GEMM_F32_TOKENS = 512       # tokens of one launch: the planes of the tiles' parts stay below 200 MB at the largest layer sizes
+_f32_parts = {}
 
 
 def gemm_f32_tc_supports(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -498,13 +497,12 @@ def gemm_f32_tc_supports(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
              accumulate: bool = False) -> torch.Tensor:
-    """out (=|+=) x @ w.T (+ bias) in float32: above ``GEMM_F32_FEW_TOKENS`` rows on the tensor cores from operands split into two
-    TF32 parts, whose error is no larger than that of float32 FMAs; else, and for forms that kernel does not take, on the CUDA cores."""
-    M = x.shape[0]
-    if M <= GEMM_F32_FEW_TOKENS or not gemm_f32_tc_supports(x, w):
+    """out (=|+=) x @ w.T (+ bias) in float32, a row's result independent of the other rows: on the tensor cores from operands split
+    into two TF32 parts, whose error is no larger than that of float32 FMAs; forms that kernel does not take on the CUDA cores."""
+    if not gemm_f32_tc_supports(x, w):
         return gemm_simt(x, w, bias, out=out, accumulate=accumulate)
     _dev(x, "x", torch.float32, contiguous=False); _dev(w, "w", torch.float32)
-    N, K = w.shape
+    M, (N, K) = x.shape[0], w.shape
     if x.shape[1] != K:
         raise KernelError(f"gemm: x has {x.shape[1]} columns, w has {K}")
     if out is None:
@@ -518,22 +516,17 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = No
         _dev(bias, "bias")
         if bias.numel() != N:
             raise KernelError("gemm: bias must have N entries")
-    plan = _f32_plans.get((M, N, K))
-    if plan is None:
-        bn, splits = c_int(), c_int()
-        _check_plan = _fn("gemm_f32_tc", "bw_gemm_f32_tc_plan", [c_int, c_int, c_int, c_int, c_void_p, c_void_p])(
-            M, N, K, num_sms(x.device), ctypes.addressof(bn), ctypes.addressof(splits))
-        if _check_plan != 0:
-            raise KernelError(f"gemm_f32_tc: no plan for {M} x {N} x {K}")
-        if len(_f32_plans) > 4096:
-            _f32_plans.clear()
-        plan = _f32_plans[(M, N, K)] = (bn.value, splits.value)
-    bn, splits = plan
-    parts = torch.empty((2 * M * K,), dtype=torch.float32, device=x.device)
-    planes = torch.empty((splits * M * N,), dtype=torch.float32, device=x.device) if splits > 1 else None
+    parts = _f32_parts.get((N, K))
+    if parts is None:
+        parts = _f32_parts[(N, K)] = _fn("gemm_f32_tc", "bw_gemm_f32_tc_parts", [c_int, c_int])(N, K)
+    most = min(M, _GEMM_F32_TOKENS)
+    split = torch.empty((2 * most * K,), dtype=torch.float32, device=x.device)
+    planes = torch.empty((parts * most * N,), dtype=torch.float32, device=x.device) if parts > 1 else None
     fn = _fn("gemm_f32_tc", "bw_gemm_f32_tc", _GEMM_F32_TC_ARGS, tag=f"{M}x{N}x{K}")
-    _check(fn(_ptr(x), _ptr(w), _ptr(bias), _code(bias, "bias") if bias is not None else 0, _ptr(out), M, N, K, x.stride(0),
-              out.stride(0), int(accumulate), _ptr(parts), _ptr(planes), bn, splits, _stream()), "gemm_f32_tc")
+    for at in range(0, M, _GEMM_F32_TOKENS):
+        n = min(_GEMM_F32_TOKENS, M - at)
+        _check(fn(_ptr(x[at:]), _ptr(w), _ptr(bias), _code(bias, "bias") if bias is not None else 0, _ptr(out[at:]), n, N, K, x.stride(0),
+                  out.stride(0), int(accumulate), _ptr(split), _ptr(planes), _stream()), "gemm_f32_tc")
     return out
 
 
@@ -585,8 +578,7 @@ def attention_f32(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
     if q.shape[1] != nh * hd:
         raise KernelError("attention: q must be [T, nh * head_dim]")
     out = torch.empty_like(q)
-    rows_w, n_rows, keys_w, n_keys, merge_w, n_merge, slices, _ = attention_work(
-        batch, nh // nkv, nkv, window, hd, rows_tile=64, page_size=page_size, chunk=chunk)
+    rows_w, n_rows, keys_w, n_keys, merge_w, n_merge, slices = _attention_f32_work(batch, nh // nkv, window, chunk)
     part_o = part_ml = None
     if n_merge:
         part_o = torch.empty((slices * nkv * 16, hd), dtype=torch.float32, device=out.device)
@@ -597,6 +589,42 @@ def attention_f32(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
               _ptr(part_ml), nh, nkv, hd, page_size, num_pages, int(window or 0), int(chunk or 0), float(scale), _stream()),
            "attention_f32")
     return out
+
+
+def plan_attention_f32(q_len, q_start, kv_len, G: int, window: Optional[int], chunk: Optional[int], slice_keys: int,
+                       static_bound: Optional[int] = None):
+    """The work lists of the tiled float32 attention as plain lists, of the form of :func:`plan_attention_work`; a segment of at most
+    16 stacked rows has a block for every slice of ``slice_keys`` keys, counted from position 0, that its rows may see."""
+    rows, keys, merge, slots = [], [], [], 0
+    for r, n_q in enumerate(q_len):
+        if n_q * G > 16:
+            rows += [(r, t0, 0, 0) for t0 in range(0, n_q, 64 // G)]
+            continue
+        n = -(-(static_bound or kv_len[r]) // slice_keys)
+        for reach in (window, chunk):     # the keys before its first row that a segment reaches back to, from a slice's start
+            if reach:
+                n = min(n, -(-(reach + n_q + slice_keys - 1) // slice_keys))
+        keys += [(r, s, n, slots) for s in range(n)]
+        if n > 1:
+            merge.append((r, 0, n, slots))
+        slots += n
+    rows.sort(key=lambda it: -(q_start[it[0]] + it[1]))     # the tiles with the most keys first
+    return rows, keys, merge, slots
+
+
+def _attention_f32_work(batch, G: int, window: Optional[int], chunk: Optional[int]):
+    """:func:`plan_attention_f32` for this batch on the device, made once per step and shared by its layers."""
+    key = ("attn_f32_work", G, window, chunk)
+    work = batch.static_extras.get(key)
+    if work is None:
+        R, dev = batch.R, batch.token_ids.device
+        rows, keys, merge, slots = plan_attention_f32(batch.h_q_len[:R], batch.h_q_start[:R], batch.h_kv_len[:R], G, window, chunk,
+                                                      _fn("attention_f32", "bw_attention_f32_slice", [])(), batch.static_bound)
+
+        def up(items):
+            return torch.tensor(items, dtype=torch.int32).pin_memory().to(dev, non_blocking=True) if items else None
+        work = batch.static_extras[key] = (up(rows), len(rows), up(keys), len(keys), up(merge), len(merge), slots)
+    return work
 
 
 _ATTN_F32_ARGS = [c_void_p] * 7 + [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p] + [c_int] * 7 + [c_float, c_void_p]
