@@ -194,50 +194,57 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             load(&tmV, v_s, v_full, i, pv);
         }
     } else if (warp == 4) {
-        if (lane == 0) {
-            auto issue_qk = [&](int s) {   // keys of stage s -> S buffer s
+        // the whole warp walks the tiles and one elected lane issues (see tcgen05.cuh, elect_one)
+        const uint32_t tmem0 = __shfl_sync(0xffffffffu, tmem_base, 0), q0 = bw::smem_u32(q_s), k0 = bw::smem_u32(k_s), v0 = bw::smem_u32(v_s);
+        auto issue_qk = [&](int s) {   // keys of stage s -> S buffer s
+            if (bw::elect_one()) {
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ++ks) {
-                    const uint64_t da = bw::umma_smem_desc_sw128(bw::smem_u32(q_s + (ks >> 2) * Q_SLICE)) + 2 * (ks & 3);
-                    const uint64_t db = bw::umma_smem_desc_sw128(bw::smem_u32(k_s + s * KV_BYTES + (ks >> 2) * KV_SLICE)) + 2 * (ks & 3);
-                    bw::umma_bf16(tmem_S + 64 * s, da, db, IDESC_QK, ks != 0);
+                    const uint64_t da = bw::umma_smem_desc_sw128(q0 + (ks >> 2) * Q_SLICE) + 2 * (ks & 3);
+                    const uint64_t db = bw::umma_smem_desc_sw128(k0 + s * KV_BYTES + (ks >> 2) * KV_SLICE) + 2 * (ks & 3);
+                    bw::umma_bf16(tmem0 + 64 * s, da, db, IDESC_QK, ks != 0);
                 }
                 bw::umma_commit(s_full + 8 * s);
                 bw::umma_commit(k_empty + 8 * s);
-            };
-            auto issue_pv = [&](int s, bool first) {   // P in the first 32 columns of S buffer s, values of stage s
-                // one product per 16 keys over all HD channels: the operand's 64-channel slices lie
-                // KV_SLICE bytes apart (the descriptor's leading byte offset)
+            }
+            __syncwarp();
+        };
+        auto issue_pv = [&](int s, bool first) {   // P in the first 32 columns of S buffer s, values of stage s
+            // one product per 16 keys over all HD channels: the operand's 64-channel slices lie
+            // KV_SLICE bytes apart (the descriptor's leading byte offset)
+            if (bw::elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < BN / 16; ++kk) {
-                    const uint64_t db = bw::umma_smem_desc_mn_sw128(bw::smem_u32(v_s + s * KV_BYTES), KV_SLICE)
+                    const uint64_t db = bw::umma_smem_desc_mn_sw128(v0 + s * KV_BYTES, KV_SLICE)
                                         + (uint64_t)kk * (2048 >> 4);   // 16 keys = two 8-row groups
-                    bw::umma_bf16_ts(tmem_O, tmem_S + 64 * s + 8 * kk, db, IDESC_PV, !(first && kk == 0));
+                    bw::umma_bf16_ts(tmem0 + 128, tmem0 + 64 * s + 8 * kk, db, IDESC_PV, !(first && kk == 0));
                 }
                 bw::umma_commit(pv_done + 8 * s);
                 bw::umma_commit(v_empty + 8 * s);
-            };
-            bool ok = bw::mbar_wait(q_full, 0, &g_status, 11) && bw::mbar_wait(k_full, 0, &g_status, 12);
-            if (ok) { bw::tc_fence_after(); issue_qk(0); }
-            for (int i = 0; i < n_tiles && ok; ++i) {
-                const int s = i & 1;
-                if (i + 1 < n_tiles) {
-                    // S of the next tile, while the softmax warps work on this one.  Its buffer holds
-                    // P of tile i - 1, which the P V issued before still reads as its operand: that
-                    // product must be complete before this one may overwrite the buffer (the order of
-                    // two tensor instructions is promised only when they write the same accumulator).
-                    if (!bw::mbar_wait(k_full + 8 * (s ^ 1), ((i + 1) >> 1) & 1, &g_status, 14)) break;
-#if ATTN_STRICT_ORDER
-                    if (i >= 1 && !bw::mbar_wait(pv_done + 8 * (s ^ 1), ((i - 1) >> 1) & 1, &g_status, 22)) break;
-#endif
-                    bw::tc_fence_after();
-                    issue_qk(s ^ 1);
-                }
-                if (!bw::mbar_wait(p_full + 8 * s, (i >> 1) & 1, &g_status, 13)) break;   // P(i) written, O rescaled
-                if (!bw::mbar_wait(v_full + 8 * s, (i >> 1) & 1, &g_status, 20)) break;
-                bw::tc_fence_after();
-                issue_pv(s, i == 0);
             }
+            __syncwarp();
+        };
+        auto all = [](bool ok) { return __all_sync(0xffffffffu, ok) != 0; };
+        bool ok = all(bw::mbar_wait(q_full, 0, &g_status, 11) && bw::mbar_wait(k_full, 0, &g_status, 12));
+        if (ok) { bw::tc_fence_after(); issue_qk(0); }
+        for (int i = 0; i < n_tiles && ok; ++i) {
+            const int s = i & 1;
+            if (i + 1 < n_tiles) {
+                // S of the next tile, while the softmax warps work on this one.  Its buffer holds
+                // P of tile i - 1, which the P V issued before still reads as its operand: that
+                // product must be complete before this one may overwrite the buffer (the order of
+                // two tensor instructions is promised only when they write the same accumulator).
+                if (!all(bw::mbar_wait(k_full + 8 * (s ^ 1), ((i + 1) >> 1) & 1, &g_status, 14))) break;
+#if ATTN_STRICT_ORDER
+                if (i >= 1 && !all(bw::mbar_wait(pv_done + 8 * (s ^ 1), ((i - 1) >> 1) & 1, &g_status, 22))) break;
+#endif
+                bw::tc_fence_after();
+                issue_qk(s ^ 1);
+            }
+            if (!all(bw::mbar_wait(p_full + 8 * s, (i >> 1) & 1, &g_status, 13))) break;   // P(i) written, O rescaled
+            if (!all(bw::mbar_wait(v_full + 8 * s, (i >> 1) & 1, &g_status, 20))) break;
+            bw::tc_fence_after();
+            issue_pv(s, i == 0);
         }
     } else {
         const int row = warp * 32 + lane;

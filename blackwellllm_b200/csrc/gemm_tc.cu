@@ -575,25 +575,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            uint32_t it = 0, n = 0;
-            bool ok = true;
-            Items items(ep, kb_total, kb_per_split, tiles, num_work);
-            Item im;
-            for (; ok && items.next(im); ++n) {
-                const int nkb = im.nkb;
-                const uint32_t acc = n & 1, accph = (n >> 1) & 1;
-                if (!bw::mbar_wait(tempty0 + 8 * acc, accph ^ 1, &g_status, 4)) break;   // epilogue drained it
+        // the whole warp walks the k-blocks and one elected lane issues (see tcgen05.cuh, elect_one)
+        uint32_t it = 0, n = 0;
+        bool ok = true;
+        const uint32_t tmem0 = __shfl_sync(0xffffffffu, tmem_base, 0), smem0 = bw::smem_u32(smem);
+        Items items(ep, kb_total, kb_per_split, tiles, num_work);
+        Item im;
+        for (; ok && items.next(im); ++n) {
+            const int nkb = im.nkb;
+            const uint32_t acc = n & 1, accph = (n >> 1) & 1;
+            if (!__all_sync(0xffffffffu, bw::mbar_wait(tempty0 + 8 * acc, accph ^ 1, &g_status, 4))) break;   // epilogue drained it
+            bw::tc_fence_after();
+            const uint32_t tmem_acc = tmem0 + acc * NSUB * ACC_COLS;
+            for (int i = 0; i < nkb; ++i, ++it) {
+                const int s = it % STAGES;
+                const uint32_t ph = (it / STAGES) & 1;
+                if (!__all_sync(0xffffffffu, bw::mbar_wait(full0 + 8 * s, ph, &g_status, 2))) { ok = false; break; }
                 bw::tc_fence_after();
-                const uint32_t tmem_acc = tmem_base + acc * NSUB * ACC_COLS;
-                for (int i = 0; i < nkb; ++i, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1;
-                    if (!bw::mbar_wait(full0 + 8 * s, ph, &g_status, 2)) { ok = false; break; }
-                    bw::tc_fence_after();
-                    const uint32_t a_addr = bw::smem_u32(smem + s * STAGE_BYTES);
-                    const uint64_t da = bw::umma_smem_desc_sw128(a_addr);
-                    const uint64_t db = bw::umma_smem_desc_sw128(a_addr + A_BYTES);
+                const uint32_t a_addr = smem0 + s * STAGE_BYTES;
+                const uint64_t da = bw::umma_smem_desc_sw128(a_addr);
+                const uint64_t db = bw::umma_smem_desc_sw128(a_addr + A_BYTES);
+                if (bw::elect_one()) {
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k) {
                         // advance 32 bytes (2 units of 16 B) along K inside the swizzle row
@@ -601,8 +603,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         else bw::umma_bf16(tmem_acc, da + 2 * k, db + 2 * k, IDESC, (i | k) != 0);
                     }
                     bw::umma_commit(empty0 + 8 * s);   // the stage is free once these MMAs are done
+                    if (i == nkb - 1) bw::umma_commit(tfull0 + 8 * acc);     // this accumulator is complete
                 }
-                bw::umma_commit(tfull0 + 8 * acc);     // this accumulator is complete
+                __syncwarp();
             }
         }
     } else {
@@ -848,30 +851,34 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {      // the whole warp walks the k-blocks and one elected lane issues (see tcgen05.cuh, elect_one)
             uint32_t it = 0, n = 0;
             bool ok = true;
+            const uint32_t tmem0 = __shfl_sync(0xffffffffu, tmem_base, 0), smem0 = bw::smem_u32(smem);
             Items items(ep, kb_total, kb_per_split, tiles, num_work, pair, n_pairs);
             Item im;
             for (; ok && items.next(im); ++n) {
                 const uint32_t acc = n & 1, accph = (n >> 1) & 1;
-                if (!bw::mbar_wait_cluster(tempty0 + 8 * acc, accph ^ 1, &g_status, 34)) break;   // both epilogues drained it
+                if (!__all_sync(0xffffffffu, bw::mbar_wait_cluster(tempty0 + 8 * acc, accph ^ 1, &g_status, 34))) break;   // both epilogues drained it
                 bw::tc_fence_after();
-                const uint32_t tmem_acc = tmem_base + acc * 256;
+                const uint32_t tmem_acc = tmem0 + acc * 256;
                 for (int i = 0; i < im.nkb; ++i, ++it) {
                     const int s = it % STAGES;
                     const uint32_t ph = (it / STAGES) & 1;
-                    if (!bw::mbar_wait_cluster(full0 + 8 * s, ph, &g_status, 32)) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, bw::mbar_wait_cluster(full0 + 8 * s, ph, &g_status, 32))) { ok = false; break; }
                     bw::tc_fence_after();
-                    const uint32_t a_addr = bw::smem_u32(smem + s * STAGE_BYTES);
+                    const uint32_t a_addr = smem0 + s * STAGE_BYTES;
                     const uint64_t da = bw::umma_smem_desc_sw128(a_addr);
                     const uint64_t db = bw::umma_smem_desc_sw128(a_addr + A_BYTES);
+                    if (bw::elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; ++k)
-                        bw::umma_bf16_pair(tmem_acc, da + 2 * k, db + 2 * k, IDESC, (i | k) != 0);
-                    bw::umma_commit_pair(empty0 + 8 * s, 3);   // the stage is free in both CTAs
+                        for (int k = 0; k < BK / UMMA_K; ++k)
+                            bw::umma_bf16_pair(tmem_acc, da + 2 * k, db + 2 * k, IDESC, (i | k) != 0);
+                        bw::umma_commit_pair(empty0 + 8 * s, 3);   // the stage is free in both CTAs
+                        if (i == im.nkb - 1) bw::umma_commit_pair(tfull0 + 8 * acc, 3);     // both CTAs' rows of the accumulator are complete
+                    }
+                    __syncwarp();
                 }
-                bw::umma_commit_pair(tfull0 + 8 * acc, 3);     // both CTAs' rows of the accumulator are complete
             }
         }
     } else {

@@ -68,22 +68,24 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            bool ok = true;
-            for (int i = 0; i < nkb; ++i) {
-                const int s = i % STAGES;
-                const uint32_t ph = (i / STAGES) & 1;
-                if (!bw::mbar_wait(full0 + 8 * s, ph, &g_status, 2)) { ok = false; break; }
-                bw::tc_fence_after();
-                const uint32_t a_addr = bw::smem_u32(smem + s * STAGE_BYTES);
-                const uint64_t da = bw::umma_smem_desc_sw128(a_addr);
-                const uint64_t db = bw::umma_smem_desc_sw128(a_addr + A_BYTES);
+        // the whole warp walks the k-blocks and one elected lane issues (see tcgen05.cuh, elect_one)
+        const uint32_t tmem0 = __shfl_sync(0xffffffffu, tmem_base, 0), smem0 = bw::smem_u32(smem);
+        for (int i = 0; i < nkb; ++i) {
+            const int s = i % STAGES;
+            const uint32_t ph = (i / STAGES) & 1;
+            if (!__all_sync(0xffffffffu, bw::mbar_wait(full0 + 8 * s, ph, &g_status, 2))) break;
+            bw::tc_fence_after();
+            const uint32_t a_addr = smem0 + s * STAGE_BYTES;
+            const uint64_t da = bw::umma_smem_desc_sw128(a_addr);
+            const uint64_t db = bw::umma_smem_desc_sw128(a_addr + A_BYTES);
+            if (bw::elect_one()) {
 #pragma unroll
                 for (int k = 0; k < BK / UMMA_K; ++k)   // 32 bytes (2 units of 16) further along K inside the swizzle row
-                    bw::umma_bf16(tmem_base, da + 2 * k, db + 2 * k, IDESC, (i | k) != 0);
+                    bw::umma_bf16(tmem0, da + 2 * k, db + 2 * k, IDESC, (i | k) != 0);
                 bw::umma_commit(empty0 + 8 * s);
+                if (i == nkb - 1) bw::umma_commit(done);
             }
-            if (ok) bw::umma_commit(done);
+            __syncwarp();
         }
     } else {
         const int quarter = warp & 3;
