@@ -91,6 +91,17 @@ row_step_kernel(RowParams p) {
     __shared__ float2 scratch[32];
     const int H = p.H, step = blockDim.x * W;
     const float inv_h = 1.f / (float)H;
+    // a row of one access per thread (few rows: all latency) has its gains, which no kernel writes, before the wait
+    constexpr bool EARLY = NV == 1;
+    float g_y[W], g_z[W], g_p[W], g_n[W];
+    if constexpr (EARLY) {
+        const int c = threadIdx.x * W;
+        if (c < H) {
+            if (p.pair) { ld<W>(p.gy + c, g_y); ld<W>(p.gz + c, g_z); }
+            if (p.gp) ld<W>(p.gp + c, g_p);
+            if (p.gn) ld<W>(p.gn + c, g_n);
+        }
+    }
     BW_PDL_WAIT();
     const size_t row = (size_t)(p.rows ? p.rows[blockIdx.x] : (int)blockIdx.x) * H;
     float x[NV][W];
@@ -134,10 +145,9 @@ row_step_kernel(RowParams p) {
             for (int i = 0; i < NV; ++i) {
                 const int c = i * step + threadIdx.x * W;
                 if (c < H) {
-                    float gy[W], gz[W];
-                    ld<W>(p.gy + c, gy); ld<W>(p.gz + c, gz);
+                    if constexpr (!EARLY) { ld<W>(p.gy + c, g_y); ld<W>(p.gz + c, g_z); }
 #pragma unroll
-                    for (int e = 0; e < W; ++e) y[i][e] = 0.5f * (y[i][e] * ry * gy[e] + z[i][e] * rz * gz[e]);
+                    for (int e = 0; e < W; ++e) y[i][e] = 0.5f * (y[i][e] * ry * g_y[e] + z[i][e] * rz * g_z[e]);
                 }
             }
         }
@@ -164,12 +174,11 @@ row_step_kernel(RowParams p) {
         for (int i = 0; i < NV; ++i) {
             const int c = i * step + threadIdx.x * W;
             if (c < H) {
-                float g[W];
-                if (p.gp) ld<W>(p.gp + c, g);
+                if constexpr (!EARLY) { if (p.gp) ld<W>(p.gp + c, g_p); }
 #pragma unroll
                 for (int e = 0; e < W; ++e) {
                     float v = (y[i][e] - mean) * r;
-                    if (p.gp) v *= g[e];
+                    if (p.gp) v *= g_p[e];
                     x[i][e] += v;
                 }
                 if (!p.rows) {
@@ -204,18 +213,18 @@ row_step_kernel(RowParams p) {
     for (int i = 0; i < NV; ++i) {
         const int c = i * step + threadIdx.x * W;
         if (c < H) {
-            float g[W], o[W];
-            if (p.gn) ld<W>(p.gn + c, g);
+            float o[W];
+            if constexpr (!EARLY) { if (p.gn) ld<W>(p.gn + c, g_n); }
             if (p.next == NORM_TANH) {
                 float b[W];
 #pragma unroll
                 for (int e = 0; e < W; ++e) b[e] = 0.f;
                 if (p.bn) ld<W>(p.bn + c, b);
 #pragma unroll
-                for (int e = 0; e < W; ++e) o[e] = fmaf(tanhf(p.alpha * x[i][e]), p.gn ? g[e] : 1.f, b[e]);
+                for (int e = 0; e < W; ++e) o[e] = fmaf(tanhf(p.alpha * x[i][e]), p.gn ? g_n[e] : 1.f, b[e]);
             } else {
 #pragma unroll
-                for (int e = 0; e < W; ++e) { o[e] = (x[i][e] - mean) * r; if (p.gn) o[e] *= g[e]; }
+                for (int e = 0; e < W; ++e) { o[e] = (x[i][e] - mean) * r; if (p.gn) o[e] *= g_n[e]; }
             }
             if constexpr (W == 4) st4(out + c, o);
             else st(out + c, o[0]);
