@@ -50,20 +50,23 @@ __device__ __forceinline__ void hist_add(Hist& h, unsigned bin, u64 q) {
 }
 
 // One row per cluster.  The weights e = exp((x - max) / T) are made once and stay in registers (NV a thread; NV = 0: a row too
-// long for that is read again for every pass).  Masses are integers, e * 2^shift rounded (`scale` = 2^shift, shift at most 45 and
+// long for that is read again for every pass) or, with more rows than clusters that fit at one block an SM, in shared memory (IN_SMEM:
+// two blocks an SM at 32 registers a thread).  Masses are integers, e * 2^shift rounded (`scale` = 2^shift, shift at most 45 and
 // such that a row's mass fits 62 bits): their sums are exact in any order, so the blocks of a row may add them as they come.
 // The nucleus threshold, the largest weight whose mass together with all larger ones reaches the target, is found ten bits of the
 // float pattern at a time (30 bits: e <= 1) from histograms that the blocks read from one another's shared memory: three passes
 // over registers, in place of the 30 passes over the row that a bisection takes.
 // What bounds it: latency (five cluster barriers, three histogram passes); a row of 128,256 is 0.5 MB.  Measured, temperature 0.6,
-// top_p 0.9: a row of 128,256 in 26 us, 32 rows of 152,064 in 79 us (one block per row and the bisection: 728 and 1,162 us).
-template <int NV>
-__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(THREADS)
+// top_p 0.9: a row of 128,256 in 26 us, 32 rows of 152,064 in 63 us (79 in registers; one block per row and the bisection: 728 and
+// 1,162 us).
+template <int NV, bool IN_SMEM = false>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(THREADS, IN_SMEM ? 2 : 1)
 sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
               const float* __restrict__ top_p, const float* __restrict__ u, int* __restrict__ out,
               int V, size_t ld, float scale) {
     BW_PDL_TRIGGER();
     BW_PDL_WAIT();
+    extern __shared__ float kept_smem[];        // IN_SMEM: [WARPS][per_warp]
     __shared__ Hist hist[3];
     __shared__ float sv[WARPS], all_max[CLUSTER];
     __shared__ int si[WARPS], all_arg[CLUSTER];
@@ -98,8 +101,12 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
         for (int i = 0; i < NV; ++i)
             if (32 * i < left) argmax_pair(mx, arg, e[i], first + 32 * i);
     } else {
-        for (int i = 0; i < iters; ++i)
-            if (32 * i < left) argmax_pair(mx, arg, row[first + 32 * i], first + 32 * i);
+#pragma unroll 4
+        for (int i = 0; i < iters; ++i) {
+            const float x = 32 * i < left ? row[first + 32 * i] : -INFINITY;
+            if constexpr (IN_SMEM) kept_smem[warp * per_warp + 32 * i + lane] = x;
+            if (32 * i < left) argmax_pair(mx, arg, x, first + 32 * i);
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -137,6 +144,7 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     const float invT = 1.f / T;
     auto weight = [&](int i) {     // of this thread's i-th token; -1: there is none
         if constexpr (NV > 0) return e[i];
+        else if constexpr (IN_SMEM) return kept_smem[warp * per_warp + 32 * i + lane];
         else return 32 * i < left ? expf((row[first + 32 * i] - mx) * invT) : -1.f;
     };
     auto mass = [&](float w) { return __float2ull_rn(w * scale); };
@@ -144,6 +152,12 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     if constexpr (NV > 0) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) e[i] = 32 * i < left ? expf((e[i] - mx) * invT) : -1.f;
+    }
+    if constexpr (IN_SMEM) {       // (each thread its own)
+        for (int i = 0; i < iters; ++i) {
+            float& k = kept_smem[warp * per_warp + 32 * i + lane];
+            k = 32 * i < left ? expf((k - mx) * invT) : -1.f;
+        }
     }
     float tau = 0.f;
     if (tp < 1.f) {
@@ -315,6 +329,16 @@ BW_EXPORT int bw_sample(const float* logits, const float* temperature, const flo
     const int per_block = (V + CLUSTER - 1) / CLUSTER;
     const int iters = ((per_block + WARPS - 1) / WARPS + 31) / 32;
     const dim3 grid((unsigned)R * CLUSTER), block(THREADS);
+    // more rows than clusters at one block an SM: two blocks an SM, weights in shared memory (19 rows of 152,064 61 us, 32 63 us; in registers 79)
+    const int at_once = bw::num_sms() / CLUSTER;
+    const size_t kept = (size_t)iters * 32 * WARPS * sizeof(float);
+    if (temperature && R > at_once && kept <= 80 * 1024) {      // (two blocks and their histograms in an SM's shared memory)
+        static bool done[bw::MAX_DEVICES] = {};
+        if (const cudaError_t e = bw::allow_dynamic_smem(sample_kernel<0, true>, 80 * 1024, done); e != cudaSuccess) return (int)e;
+        bw::launch(sample_kernel<0, true>, grid, block, kept, (cudaStream_t)stream, logits, temperature, top_p, u, out, V, (size_t)ld, scale);
+        BW_LAUNCH_CHECK();
+        return 0;
+    }
 #define BW_SAMPLE(NV) bw::launch(sample_kernel<NV>, grid, block, 0, (cudaStream_t)stream, logits, temperature, top_p, u, out, V, (size_t)ld, scale)
     // registers for 8 tokens a thread (rows up to 65,536) or 20 (up to 163,840: 64 registers a thread allow no more)
     if (iters <= 8) BW_SAMPLE(8);
