@@ -236,11 +236,32 @@ __global__ void __launch_bounds__(128)
 gla_gate_kernel(const float* __restrict__ o, const float* __restrict__ g, long long g_ld, int g_off,
                 const float* __restrict__ gain, OT* __restrict__ out, int T, int heads, int dv, float eps, int ready) {
     BW_PDL_TRIGGER();
-    BW_PDL_WAIT();
     const int item = blockIdx.x * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (item >= T * heads) return;
     const int t = item / heads, h = item - t * heads;
+    if (dv <= 128) {      // the head in registers: one round of loads, the gain, which no kernel writes, before the wait
+        float x[4], z[4], w[4], ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = lane + 32 * i < dv ? gain[lane + 32 * i] : 0.f;
+        BW_PDL_WAIT();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int c = lane + 32 * i;
+            x[i] = c < dv ? o[((size_t)t * heads + h) * dv + c] : 0.f;
+            z[i] = c < dv ? g[(size_t)t * g_ld + g_off + (size_t)h * dv + c] : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ss = fmaf(x[i], x[i], ss);
+        const float r = rsqrtf(bw::warp_sum(ss) / (float)dv + eps);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int c = lane + 32 * i;
+            if (c < dv) out[((size_t)t * heads + h) * dv + c] = bw::from_f32<OT>(x[i] * r * w[i] * (ready ? z[i] : z[i] / (1.f + expf(-z[i]))));
+        }
+        return;
+    }
+    BW_PDL_WAIT();
     const float* orow = o + (size_t)t * heads * dv + (size_t)h * dv;
     const float* grow = g + (size_t)t * g_ld + g_off + (size_t)h * dv;
     float ss = 0.f;

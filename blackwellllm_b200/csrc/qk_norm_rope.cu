@@ -138,7 +138,9 @@ head_norm_rope_kernel(const float* __restrict__ qkv, long long ld, const int* __
     const int half = rotary_dim >> 1;
     const float* tab = rotary_dim ? table + (size_t)t * rotary_dim : nullptr;
     const int n_heads = nh + (has_kv ? nkv : 0);
-    for (int h = warp; h < n_heads; h += nwarps) {
+    // blocks of a token (blockIdx.y) take its heads in turn
+    const int warp0 = blockIdx.y * nwarps + warp, all_warps = gridDim.y * nwarps;
+    for (int h = warp0; h < n_heads; h += all_warps) {
         const bool is_q = h < nh;
         if (!is_q && page < 0) continue;
         const float* src = is_q ? row + (size_t)h * dq : row + nq + (size_t)(h - nh) * dq;
@@ -168,12 +170,17 @@ head_norm_rope_kernel(const float* __restrict__ qkv, long long ld, const int* __
         if (vec2) {
             // rotation of halves, even sizes up to 256, aligned rows: a lane keeps pairs of neighbouring channels and their
             // partners in registers, so a head is read once
-            float2 a[2], b[2], q[4];
+            float2 a[2], b[2], q[4], ga[2], gb[2], cs[2], sn[2];
             float ss = 0.f;
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
+            for (int i = 0; i < 2; ++i) {      // (gains and angles with them: one round of loads)
                 const int c = i * 64 + lane * 2;
-                a[i] = b[i] = make_float2(0.f, 0.f);
+                a[i] = b[i] = cs[i] = sn[i] = make_float2(0.f, 0.f);
+                ga[i] = gb[i] = make_float2(1.f, 1.f);
+                if (c < half) {
+                    cs[i] = *reinterpret_cast<const float2*>(tab + c); sn[i] = *reinterpret_cast<const float2*>(tab + half + c);
+                    if (gain) { ga[i] = *reinterpret_cast<const float2*>(gain + c); gb[i] = *reinterpret_cast<const float2*>(gain + half + c); }
+                }
                 if (c < half) { a[i] = *reinterpret_cast<const float2*>(src + c); b[i] = *reinterpret_cast<const float2*>(src + half + c); }
                 ss = fmaf(a[i].x, a[i].x, ss); ss = fmaf(a[i].y, a[i].y, ss); ss = fmaf(b[i].x, b[i].x, ss); ss = fmaf(b[i].y, b[i].y, ss);
             }
@@ -188,12 +195,9 @@ head_norm_rope_kernel(const float* __restrict__ qkv, long long ld, const int* __
             for (int i = 0; i < 2; ++i) {
                 const int c = i * 64 + lane * 2;
                 if (c < half) {
-                    const float2 ga = gain ? *reinterpret_cast<const float2*>(gain + c) : make_float2(1.f, 1.f);
-                    const float2 gb = gain ? *reinterpret_cast<const float2*>(gain + half + c) : make_float2(1.f, 1.f);
-                    const float2 cs = *reinterpret_cast<const float2*>(tab + c), sn = *reinterpret_cast<const float2*>(tab + half + c);
-                    const float x0 = a[i].x * r2 * ga.x, x1 = a[i].y * r2 * ga.y, y0 = b[i].x * r2 * gb.x, y1 = b[i].y * r2 * gb.y;
-                    put2(dst + c, x0 * cs.x - y0 * sn.x, x1 * cs.y - y1 * sn.y);
-                    put2(dst + half + c, y0 * cs.x + x0 * sn.x, y1 * cs.y + x1 * sn.y);
+                    const float x0 = a[i].x * r2 * ga[i].x, x1 = a[i].y * r2 * ga[i].y, y0 = b[i].x * r2 * gb[i].x, y1 = b[i].y * r2 * gb[i].y;
+                    put2(dst + c, x0 * cs[i].x - y0 * sn[i].x, x1 * cs[i].y - y1 * sn[i].y);
+                    put2(dst + half + c, y0 * cs[i].x + x0 * sn[i].x, y1 * cs[i].y + x1 * sn[i].y);
                 }
             }
 #pragma unroll
@@ -255,7 +259,7 @@ head_norm_rope_kernel(const float* __restrict__ qkv, long long ld, const int* __
     auto value = [&](size_t i) { const float v = vsrc[i]; return vf ? (1.f - lam) * v + lam * vf[i] : v; };
     if (page >= 0 && v_eps > 0.f) {
         // every value head divided by its own root mean square (no gain): a warp per head
-        for (int h = warp; h < nkv; h += nwarps) {
+        for (int h = warp0; h < nkv; h += all_warps) {
             float ss = 0.f;
             for (int c = lane; c < dv; c += 32) { const float v = value((size_t)h * dv + c); ss = fmaf(v, v, ss); }
             const float r = rsqrtf(bw::warp_sum(ss) / (float)dv + v_eps);
@@ -266,7 +270,7 @@ head_norm_rope_kernel(const float* __restrict__ qkv, long long ld, const int* __
     }
     if (page >= 0) {
         if (vec_v && !vf) {
-            for (int idx = threadIdx.x * 4; idx < nkv * dpad; idx += blockDim.x * 4) {
+            for (int idx = (blockIdx.y * blockDim.x + threadIdx.x) * 4; idx < nkv * dpad; idx += gridDim.y * blockDim.x * 4) {
                 const int h = idx / dpad, c = idx - h * dpad;
                 float4 o = c < dv ? *reinterpret_cast<const float4*>(vsrc + (size_t)h * dv + c) : make_float4(0.f, 0.f, 0.f, 0.f);
                 o.x *= v_scale; o.y *= v_scale; o.z *= v_scale; o.w *= v_scale;
@@ -274,7 +278,7 @@ head_norm_rope_kernel(const float* __restrict__ qkv, long long ld, const int* __
             }
             return;
         }
-        for (int idx = threadIdx.x; idx < nkv * dpad; idx += blockDim.x) {
+        for (int idx = blockIdx.y * blockDim.x + threadIdx.x; idx < nkv * dpad; idx += gridDim.y * blockDim.x) {
             const int h = idx / dpad, c = idx - h * dpad;
             const float o = c < dv ? value((size_t)h * dv + c) * v_scale : 0.f;
             v_pages[(((size_t)page * nkv + h) * page_size + slot) * dpad + c] = bw::from_f32<OT>(o);
@@ -316,7 +320,10 @@ BW_EXPORT int bw_head_norm_rope_append(const float* qkv, long long ld, const int
                       (((uintptr_t)qkv | (uintptr_t)q_gain | (uintptr_t)k_gain | (uintptr_t)q_out | (uintptr_t)k_pages) & 7) == 0;
     const int vec_v = (dv & 3) == 0 && (dpad & 3) == 0 && (ld & 3) == 0 && (v_col & 3) == 0 &&
                       (((uintptr_t)qkv | (uintptr_t)v_pages) & 15) == 0;
-#define BW_HN(OT) bw::launch((head_norm_rope_kernel<OT>), dim3(T), dim3(256), 0, s, qkv, ld, positions, req_of_token, block_table, \
+    // few tokens: a warp per head where the SMs allow it (8 tokens of 24 heads: 7 us with one block a token, three rounds of heads)
+    const int heads = nh + (has_kv ? nkv : 0), spare = 2 * bw::num_sms() / T, rounds = (heads + 7) / 8;
+    const int per_token = spare < 1 ? 1 : spare < rounds ? spare : rounds;
+#define BW_HN(OT) bw::launch((head_norm_rope_kernel<OT>), dim3(T, per_token), dim3(256), 0, s, qkv, ld, positions, req_of_token, block_table, \
         max_blocks, table, rotary_dim, interleaved, q_gain, k_gain, eps, q_coef, q_every, (OT*)q_out, (OT*)k_pages, (OT*)v_pages, \
         nh, nkv, dq, dv, dpad, page_size, num_pages, has_kv, vec, vec2, pairs, vec_v, v_eps, v_first, v_first_ld, v_lam, \
         q_head_mult, v_col, v_scale)

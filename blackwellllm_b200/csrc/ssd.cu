@@ -47,11 +47,17 @@ ssd_out_vec_kernel(const float* __restrict__ y, const float* __restrict__ x, lon
                    long long z_ld, const float* __restrict__ D, const float* __restrict__ gain, OT* __restrict__ out, int inner,
                    int vdim, int part, float eps) {
     BW_PDL_TRIGGER();
-    BW_PDL_WAIT();
     __shared__ float scratch[32];
     const size_t t = blockIdx.x;
     const int c0 = blockIdx.y * part, c1 = c0 + part;
-    float4 u[NV];
+    float4 u[NV], w[NV];
+    float Dh[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {      // what no kernel writes, before the wait
+        const int c = c0 + (i * blockDim.x + threadIdx.x) * 4;
+        if (c < c1) { w[i] = *reinterpret_cast<const float4*>(gain + c); Dh[i] = D[c / vdim]; }
+    }
+    BW_PDL_WAIT();
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -60,7 +66,7 @@ ssd_out_vec_kernel(const float* __restrict__ y, const float* __restrict__ x, lon
         if (c < c1) {
             const float4 a = *reinterpret_cast<const float4*>(y + t * inner + c), b = *reinterpret_cast<const float4*>(x + t * x_ld + c),
                          g = *reinterpret_cast<const float4*>(z + t * z_ld + c);
-            const float d = D[c / vdim];
+            const float d = Dh[i];
             u[i].x = (a.x + d * b.x) * (g.x / (1.f + expf(-g.x))); u[i].y = (a.y + d * b.y) * (g.y / (1.f + expf(-g.y)));
             u[i].z = (a.z + d * b.z) * (g.z / (1.f + expf(-g.z))); u[i].w = (a.w + d * b.w) * (g.w / (1.f + expf(-g.w)));
         }
@@ -71,8 +77,7 @@ ssd_out_vec_kernel(const float* __restrict__ y, const float* __restrict__ x, lon
     for (int i = 0; i < NV; ++i) {
         const int c = c0 + (i * blockDim.x + threadIdx.x) * 4;
         if (c < c1) {
-            const float4 g = *reinterpret_cast<const float4*>(gain + c);
-            put4(out + t * inner + c, make_float4(u[i].x * r * g.x, u[i].y * r * g.y, u[i].z * r * g.z, u[i].w * r * g.w));
+            put4(out + t * inner + c, make_float4(u[i].x * r * w[i].x, u[i].y * r * w[i].y, u[i].z * r * w[i].z, u[i].w * r * w[i].w));
         }
     }
 }
