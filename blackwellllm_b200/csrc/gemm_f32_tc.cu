@@ -10,17 +10,21 @@
 // Weights are the 128-row operand (from tensor memory), tokens the other (from shared memory).  The tokens are split beforehand by a
 // small kernel (they are read again by every block of features); the weights, which are read once, on the way: a warp a quarter
 // of the rows, a lane a row, from the TMA tile into tensor memory.
-// Few and wide MMAs: hi of the weights times hi and lo of the tokens side by side (2 BN columns), and lo times hi into the second
-// half: 8 for a stage of 32 channels.
+// hi hi goes into two accumulators in turn; the small products have one of their own over a whole piece (their sums are 2^-11 of the
+// others', and so is what the accumulation drops).
+// Three rings: the weights' tiles, which are free again once they are split; the split weights in tensor memory; the tokens' tiles.
+// With one ring for all three (a stage held from its load to its MMAs' end) four stages of loads were in flight, and every
+// accumulator was drained while nothing ran: 64 tokens took 138 us, 128 tokens 188 us, 301 tokens 508 us at the sizes below.
 // A token's result is the same whatever else is in the batch: the channels of all tiles of features, laid end to end, are cut into one
 // range per SM, whatever the number of tokens; a range's part of a tile is summed as above, and a tile's parts are added in their
 // order by a second kernel.  (So every SM also streams the same number of bytes, and no round of blocks ends half empty.)
-// Roles (896 threads): warp 0 TMA; warp 1 TMEM owner and MMAs; warps 4..11 split the weights, two groups that take stages in turn;
-// warps 12..27 add the accumulators up, 32 tokens each group of four, and write the result.  Every wait is bounded; a timeout sets
-// the status word and all roles fall through to the exit.
-// What bounds it: up to 16 tokens the bytes of the weights, above 64 the MMAs and shared memory.  Measured, x 28672 x 4096: 1 to 16
-// tokens 111 us (4.2 TB/s), 64 tokens 141 us, 128 tokens 191 us (157 TFLOP/s), 301 tokens 511 us.  301 tokens scored in eight layers of
-// the 8B shape, logits at each: 72.2 ms on gemm_simt.cu's tiles (65.0 of them products), 12.8 ms so.
+// Roles (896 threads): warp 0 loads weights; warp 1 TMEM owner and MMAs; warp 2 loads tokens; warps 4..11 split the weights, two
+// groups that take stages in turn; warps 12..27 add the accumulators up, 32 tokens each group of four, and write the result.  Every
+// wait is bounded; a timeout sets the status word and all roles fall through to the exit.
+// What bounds it: the MMA warp.  Of 857 cycles a stage of 32 channels at 16 tokens 550 are its issue of 12 MMAs (the tensor pipe needs
+// 120) and 300 its waits; at 128 tokens 768 of 1,369 are MMAs.  Measured, x 28672 x 4096: 1 to 16 tokens 91 us (5.1 TB/s), 64 tokens
+// 127 us, 128 tokens 173 us (174 TFLOP/s), 301 tokens 476 us; gemm_simt.cu's tiles: eight layers of the 8B shape with logits at each of
+// 301 tokens 72.2 ms, of which 65.0 were products.
 #include "tcgen05.cuh"
 
 using bf16 = __nv_bfloat16;
@@ -33,19 +37,22 @@ constexpr int SUM_STAGES = 2;      // stages of an accumulator before it is adde
 constexpr int SPLIT_GROUPS = 2, SUM_GROUPS = 4;     // of four warps each, from warps 4 and 12 on
 constexpr int THREADS = 32 * (4 + 4 * SPLIT_GROUPS + 4 * SUM_GROUPS);
 constexpr int SMEM_BUDGET = 224 * 1024;
-constexpr int MAX_STAGES = 7;
+constexpr int MAX_W = 12, MAX_T = 4, MAX_X = 6;     // stages of the rings: weights' tiles, split weights, tokens' tiles
 
 __device__ int g_status = 0;
 
-// Columns of tensor memory: one accumulator of 2 BN columns or (up to 64 tokens) two, then 64 (hi, lo) of every stage.
-__host__ __device__ constexpr int acc_cols(int bn) { return bn <= 32 ? 64 : bn <= 64 ? 128 : 256; }
-__host__ __device__ constexpr int acc_count(int bn) { return bn <= 64 ? 2 : 1; }
-__host__ __device__ constexpr int stage_bytes(int bn) { return A_BYTES + 2 * bn * BK * 4; }
-__host__ __device__ constexpr int stages_for(int bn) {
-    const int tmem = (512 - acc_count(bn) * acc_cols(bn)) / 64, smem = SMEM_BUDGET / stage_bytes(bn);
-    const int s = tmem < smem ? tmem : smem;
-    return s < MAX_STAGES ? s : MAX_STAGES;
+// Tensor memory: the small products' accumulator, two of hi hi, then the split weights, 64 columns (hi, lo) a stage.
+__host__ __device__ constexpr int acc_cols(int bn) { return (bn + 31) / 32 * 32; }
+__host__ __device__ constexpr int t_stages(int bn) { return (512 - 3 * acc_cols(bn)) / 64 < MAX_T ? (512 - 3 * acc_cols(bn)) / 64 : MAX_T; }
+static_assert(t_stages(MAX_BN) == 2, "two stages of split weights beside the accumulators");
+// Shared memory: what the tokens' ring leaves goes to the weights.
+__host__ __device__ constexpr int x_bytes(int bn) { return 2 * bn * BK * 4; }
+__host__ __device__ constexpr int x_stages(int bn) { return bn > 64 ? 4 : MAX_X; }
+__host__ __device__ constexpr int w_stages(int bn) {
+    const int n = (SMEM_BUDGET - x_stages(bn) * x_bytes(bn)) / A_BYTES;
+    return n < MAX_W ? n : MAX_W;
 }
+__host__ __device__ constexpr int ring_bytes(int bn) { return w_stages(bn) * A_BYTES + x_stages(bn) * x_bytes(bn); }
 
 // x rounded to TF32, halves away from zero (three integer instructions fewer than the conversion instruction takes; a NaN whose
 // bits overflow here stays one in x - hi)
@@ -128,20 +135,21 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                    int tiles_m) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t bars[3 * MAX_STAGES + 4];
+    __shared__ uint64_t bars[2 * (MAX_W + MAX_T + MAX_X) + 5];
     __shared__ uint32_t tmem_slot[2];
     BW_PDL_TRIGGER();
-    const int stages = stages_for(bn), per_stage = stage_bytes(bn);
+    const int ws = w_stages(bn), ts = t_stages(bn), xs = x_stages(bn);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t full0 = bw::smem_u32(bars), ready0 = full0 + 8 * MAX_STAGES, empty0 = ready0 + 8 * MAX_STAGES;
-    const uint32_t tfull0 = empty0 + 8 * MAX_STAGES, tempty0 = tfull0 + 16;
+    const uint32_t wfull0 = bw::smem_u32(bars), wfree0 = wfull0 + 8 * MAX_W, ready0 = wfree0 + 8 * MAX_W, tfree0 = ready0 + 8 * MAX_T;
+    const uint32_t xfull0 = tfree0 + 8 * MAX_T, xfree0 = xfull0 + 8 * MAX_X;
+    const uint32_t sum_full0 = xfree0 + 8 * MAX_X, sum_free0 = sum_full0 + 16, small_free = sum_free0 + 16;
+    uint8_t* smem_x = smem + ws * A_BYTES;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < stages; ++s) {
-            bw::mbar_init(full0 + 8 * s, 1);
-            bw::mbar_init(ready0 + 8 * s, 4);
-            bw::mbar_init(empty0 + 8 * s, 1);
-        }
-        for (int a = 0; a < 2; ++a) { bw::mbar_init(tfull0 + 8 * a, 1); bw::mbar_init(tempty0 + 8 * a, 4 * SUM_GROUPS); }
+        for (int s = 0; s < ws; ++s) { bw::mbar_init(wfull0 + 8 * s, 1); bw::mbar_init(wfree0 + 8 * s, 4); }
+        for (int s = 0; s < ts; ++s) { bw::mbar_init(ready0 + 8 * s, 4); bw::mbar_init(tfree0 + 8 * s, 1); }
+        for (int s = 0; s < xs; ++s) { bw::mbar_init(xfull0 + 8 * s, 1); bw::mbar_init(xfree0 + 8 * s, 1); }
+        for (int a = 0; a < 2; ++a) { bw::mbar_init(sum_full0 + 8 * a, 1); bw::mbar_init(sum_free0 + 8 * a, 4 * SUM_GROUPS); }
+        bw::mbar_init(small_free, 4 * SUM_GROUPS);
         bw::fence_barrier_init();
         bw::tma_prefetch_desc(&tm_w);
         bw::tma_prefetch_desc(&tm_x);
@@ -151,139 +159,157 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     bw::tc_fence_before();
     __syncthreads();
     bw::tc_fence_after();
-    const uint32_t tmem = tmem_slot[0], tmem_a = tmem + acc_count(bn) * acc_cols(bn);
+    const uint32_t tmem = tmem_slot[0];
     const bool dead = tmem_slot[1] != 0;
     Items it(cut, tiles_m);
 
     if (dead) {
         // fall through to the exit
     } else if (warp == 0) {
-        if (lane == 0) {
-            // the weights of the first stages are nobody's output: requested before the wait for the earlier kernels
-            int ahead = 0, s = 0;
-            uint32_t round = 0;
-            Items peek = it;
-            if (peek.next()) {
-                ahead = min(peek.n, stages);
-                for (int i = 0; i < ahead; ++i) {
-                    bw::mbar_expect_tx(full0 + 8 * i, per_stage);
-                    bw::tma_load_2d(bw::smem_u32(smem + i * per_stage), &tm_w, full0 + 8 * i, (peek.kb0 + i) * BK, peek.tile * BM);
-                }
-            }
-            BW_PDL_WAIT();
+        if (lane == 0) {       // the weights are nobody's output: no wait for the earlier kernels
+            int s = 0, ph = 1;
             bool ok = true;
             while (ok && it.next()) {
                 for (int i = 0; i < it.n; ++i) {
-                    const uint32_t dst = bw::smem_u32(smem + s * per_stage);
-                    if (ahead > 0) --ahead;
-                    else {
-                        if (round > 0 && !bw::mbar_wait(empty0 + 8 * s, (round - 1) & 1, &g_status, 1)) { ok = false; break; }
-                        bw::mbar_expect_tx(full0 + 8 * s, per_stage);
-                        bw::tma_load_2d(dst, &tm_w, full0 + 8 * s, (it.kb0 + i) * BK, it.tile * BM);
-                    }
-                    bw::tma_load_2d(dst + A_BYTES, &tm_x, full0 + 8 * s, (it.kb0 + i) * BK, it.mt * bn);
-                    bw::tma_load_2d(dst + A_BYTES + bn * BK * 4, &tm_x, full0 + 8 * s, (it.kb0 + i) * BK, o.M + it.mt * bn);
-                    if (++s == stages) { s = 0; ++round; }
+                    if (!bw::mbar_wait(wfree0 + 8 * s, ph, &g_status, 1)) { ok = false; break; }
+                    bw::mbar_expect_tx(wfull0 + 8 * s, A_BYTES);
+                    bw::tma_load_2d(bw::smem_u32(smem + s * A_BYTES), &tm_w, wfull0 + 8 * s, (it.kb0 + i) * BK, it.tile * BM);
+                    if (++s == ws) { s = 0; ph ^= 1; }
+                }
+            }
+        }
+    } else if (warp == 2) {
+        if (lane == 0) {
+            const int bytes = x_bytes(bn);
+            int s = 0, ph = 1;
+            bool ok = true;
+            BW_PDL_WAIT();
+            while (ok && it.next()) {
+                for (int i = 0; i < it.n; ++i) {
+                    if (!bw::mbar_wait(xfree0 + 8 * s, ph, &g_status, 2)) { ok = false; break; }
+                    const uint32_t dst = bw::smem_u32(smem_x + s * bytes);
+                    bw::mbar_expect_tx(xfull0 + 8 * s, bytes);
+                    bw::tma_load_2d(dst, &tm_x, xfull0 + 8 * s, (it.kb0 + i) * BK, it.mt * bn);
+                    bw::tma_load_2d(dst + bytes / 2, &tm_x, xfull0 + 8 * s, (it.kb0 + i) * BK, o.M + it.mt * bn);
+                    if (++s == xs) { s = 0; ph ^= 1; }
                 }
             }
         }
     } else if (warp == 1) {
         // the whole warp walks the stages, one elected lane issues: operands the compiler knows to be the same in all lanes (in a branch
         // of one lane an MMA took 100 to 150 cycles to issue, whatever its size; so 9, or what the tensor pipe needs)
-        const uint32_t base = __shfl_sync(0xffffffffu, tmem, 0), cols_a = base + acc_count(bn) * acc_cols(bn);
-        const uint32_t idesc = idesc_tf32(bn), idesc2 = idesc_tf32(2 * bn), smem0 = bw::smem_u32(smem);
-        const int accs = acc_count(bn);
-        int s = 0, ph = 0, p = 0;
+        const uint32_t small = __shfl_sync(0xffffffffu, tmem, 0), cols_a = small + 3 * acc_cols(bn);
+        const uint32_t idesc = idesc_tf32(bn), smem0 = bw::smem_u32(smem_x), lo_units = (uint32_t)bn * BK * 4 / 16;
+        int xst = 0, xph = 0, tst = 0, tph = 0, p = 0, items = 0;
         bool ok = true;
         while (ok && it.next()) {
-            for (int i = 0; i < it.n; ++i) {
-                const int buf = p % accs;
+            ok = __all_sync(0xffffffffu, bw::mbar_wait(small_free, (items++ & 1) ^ 1, &g_status, 3));
+            for (int i = 0; ok && i < it.n; ++i) {
+                const int buf = p & 1;
                 const bool fresh = i % SUM_STAGES == 0, last = i % SUM_STAGES == SUM_STAGES - 1 || i == it.n - 1;
-                ok = bw::mbar_wait(full0 + 8 * s, ph, &g_status, 2) && bw::mbar_wait(ready0 + 8 * s, ph, &g_status, 3);
-                if (fresh) ok = ok && bw::mbar_wait(tempty0 + 8 * buf, ((p / accs) & 1) ^ 1, &g_status, 4);
+                ok = bw::mbar_wait(xfull0 + 8 * xst, xph, &g_status, 4) && bw::mbar_wait(ready0 + 8 * tst, tph, &g_status, 5);
+                if (fresh) ok = ok && bw::mbar_wait(sum_free0 + 8 * buf, ((p >> 1) & 1) ^ 1, &g_status, 6);
                 if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
                 bw::tc_fence_after();
-                const uint32_t d = base + buf * acc_cols(bn), hi = cols_a + s * 64;
-                const uint64_t b = bw::umma_smem_desc_sw128(smem0 + s * per_stage + A_BYTES);
+                const uint32_t d = small + (1 + buf) * acc_cols(bn), hi = cols_a + tst * 64;
+                const uint64_t b = bw::umma_smem_desc_sw128(smem0 + xst * x_bytes(bn));
                 if (bw::elect_one()) {
                     // 8 channels an MMA: 8 columns of A, 32 bytes (2 units of 16) of B's rows; B's lo rows lie behind its hi rows
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) umma_tf32_ts(d, hi + 8 * k, b + 2 * k, idesc2, !fresh || k != 0);
+                    for (int k = 0; k < 4; ++k) umma_tf32_ts(d, hi + 8 * k, b + 2 * k, idesc, !fresh || k != 0);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) umma_tf32_ts(d + bn, hi + 32 + 8 * k, b + 2 * k, idesc, 1);
-                    bw::umma_commit(empty0 + 8 * s);
-                    if (last) bw::umma_commit(tfull0 + 8 * buf);
+                    for (int k = 0; k < 4; ++k) umma_tf32_ts(small, hi + 8 * k, b + lo_units + 2 * k, idesc, i != 0 || k != 0);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) umma_tf32_ts(small, hi + 32 + 8 * k, b + 2 * k, idesc, 1);
+                    bw::umma_commit(tfree0 + 8 * tst);
+                    bw::umma_commit(xfree0 + 8 * xst);
+                    if (last) bw::umma_commit(sum_full0 + 8 * buf);
                 }
                 __syncwarp();
                 if (last) ++p;
-                if (++s == stages) { s = 0; ph ^= 1; }
+                if (++tst == ts) { tst = 0; tph ^= 1; }
+                if (++xst == xs) { xst = 0; xph ^= 1; }
             }
         }
     } else if (warp >= 4 && warp < 4 + 4 * SPLIT_GROUPS) {
         const int quarter = warp & 3, row = quarter * 32 + lane;
         const long long all = (cut.begin(blockIdx.x + 1) - cut.begin(blockIdx.x)) * tiles_m;      // stages of all items
-        int s = (warp - 4) / 4, ph = 0;
-        for (long long i = s; i < all; i += SPLIT_GROUPS) {
-            if (!bw::mbar_wait(full0 + 8 * s, ph, &g_status, 5)) break;
-            bw::tc_fence_after();      // (the MMAs that read this stage's columns before are complete: the tile was loaded after them)
-            const uint8_t* src = smem + s * per_stage + row * 128;
-            const uint32_t dst = tmem_a + s * 64 + ((uint32_t)(quarter * 32) << 16);
+        const uint32_t tmem_a = tmem + 3 * acc_cols(bn) + ((uint32_t)(quarter * 32) << 16);
+        const int group = (warp - 4) / 4;
+        int s = group, ph = 0, slot = group, tph = 1;
+        for (long long i = group; i < all; i += SPLIT_GROUPS) {
+            if (!__all_sync(0xffffffffu, bw::mbar_wait(wfull0 + 8 * s, ph, &g_status, 7))) break;
+            const uint8_t* src = smem + s * A_BYTES + row * 128;
+            uint32_t hi[2][16];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {           // 16-byte pieces of the row where the 128-byte swizzle put them
+                const uint4 v = *reinterpret_cast<const uint4*>(src + ((j ^ (row & 7)) << 4));
+                uint32_t* to = &hi[j >> 2][4 * (j & 3)];
+                to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w;
+            }
+            __syncwarp();
+            if (lane == 0) bw::mbar_arrive(wfree0 + 8 * s);
+            if (!__all_sync(0xffffffffu, bw::mbar_wait(tfree0 + 8 * slot, tph, &g_status, 8))) break;
+            bw::tc_fence_after();
+            const uint32_t dst = tmem_a + slot * 64;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {           // 16 channels at a time
-                uint32_t hi[16], lo[16];
+                uint32_t lo[16];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {       // 16-byte pieces of the row where the 128-byte swizzle put them
-                    const float4 v = *reinterpret_cast<const float4*>(src + (((4 * h + j) ^ (row & 7)) << 4));
-                    const float in[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const float h32 = tf32_hi(in[c]);
-                        hi[4 * j + c] = __float_as_uint(h32);
-                        lo[4 * j + c] = __float_as_uint(in[c] - h32);
-                    }
+                for (int c = 0; c < 16; ++c) {
+                    const float x = __uint_as_float(hi[h][c]), h32 = tf32_hi(x);
+                    lo[c] = __float_as_uint(x - h32);
+                    hi[h][c] = __float_as_uint(h32);
                 }
-                bw::tmem_st_32x16(dst + 16 * h, hi);
+                bw::tmem_st_32x16(dst + 16 * h, hi[h]);
                 bw::tmem_st_32x16(dst + 32 + 16 * h, lo);
             }
             bw::tmem_st_wait();
             bw::tc_fence_before();
             __syncwarp();
-            if (lane == 0) bw::mbar_arrive(ready0 + 8 * s);
+            if (lane == 0) bw::mbar_arrive(ready0 + 8 * slot);
             s += SPLIT_GROUPS;
-            if (s >= stages) { s -= stages; ph ^= 1; }
+            if (s >= ws) { s -= ws; ph ^= 1; }
+            slot += SPLIT_GROUPS;
+            if (slot >= ts) { slot -= ts; tph ^= 1; }
         }
     } else if (warp >= 4 + 4 * SPLIT_GROUPS) {
         constexpr int COLS = MAX_BN / SUM_GROUPS;
         const int quarter = warp & 3, first = ((warp - 4 - 4 * SPLIT_GROUPS) / 4) * COLS, cols = min(bn - first, COLS);
-        const int accs = acc_count(bn);
+        const uint32_t mine = tmem + first + ((uint32_t)(quarter * 32) << 16);
         bool ok = true, waited = false;
         int p = 0;
         while (ok && it.next()) {
             float sum[COLS];
 #pragma unroll
             for (int c = 0; c < COLS; ++c) sum[c] = 0.f;
-            for (int i = 0; i < it.n; i += SUM_STAGES, ++p) {
-                const int buf = p % accs;
-                if (!bw::mbar_wait(tfull0 + 8 * buf, (p / accs) & 1, &g_status, 6)) { ok = false; break; }
-                bw::tc_fence_after();
-                const uint32_t from = tmem + buf * acc_cols(bn) + first + ((uint32_t)(quarter * 32) << 16);
+            auto add_up = [&](uint32_t from) {
 #pragma unroll
                 for (int c0 = 0; c0 < COLS; c0 += 16) {
                     if (c0 >= cols) continue;
-                    uint32_t big[16], small[16];
-                    bw::tmem_ld_32x16(from + c0, big);
-                    bw::tmem_ld_32x16(from + bn + c0, small);
+                    uint32_t v[16];
+                    bw::tmem_ld_32x16(from + c0, v);
                     bw::tmem_ld_wait();
 #pragma unroll
-                    for (int c = 0; c < 16; ++c) sum[c0 + c] += __uint_as_float(big[c]) + __uint_as_float(small[c]);
+                    for (int c = 0; c < 16; ++c) sum[c0 + c] += __uint_as_float(v[c]);
                 }
                 bw::tc_fence_before();
                 __syncwarp();
-                if (lane == 0) bw::mbar_arrive(tempty0 + 8 * buf);
+            };
+            for (int i = 0; i < it.n; i += SUM_STAGES, ++p) {
+                const int buf = p & 1;
+                ok = __all_sync(0xffffffffu, bw::mbar_wait(sum_full0 + 8 * buf, (p >> 1) & 1, &g_status, 9));
+                if (!ok) break;
+                bw::tc_fence_after();
+                add_up(mine + (1 + buf) * acc_cols(bn));
+                if (lane == 0) bw::mbar_arrive(sum_free0 + 8 * buf);
             }
+            if (!ok) break;
+            add_up(mine);              // the small products: complete with the piece's last stage
+            if (lane == 0) bw::mbar_arrive(small_free);
             if (!waited) { BW_PDL_WAIT(); waited = true; }      // the result belongs to earlier kernels until here
             const int n = it.tile * BM + quarter * 32 + lane, t0 = it.mt * bn + first;
-            if (!ok || n >= o.N) continue;
+            if (n >= o.N) continue;
             const bool whole = it.n == cut.kb_total;
             const long long ld = whole ? o.ldo : o.N;
             const float b = whole ? bias_at(o, n) : 0.f;
@@ -396,7 +422,7 @@ BW_EXPORT int bw_gemm_f32_tc(const float* x, const float* w, const void* bias, i
     const cudaError_t e = bw::allow_dynamic_smem(gemm_f32_tc_kernel, SMEM_BUDGET + 1024, done);
     if (e != cudaSuccess) return (int)e;
     const Out o = {out, bias, part, ldo, bias_type, accumulate, M, N};
-    bw::launch(gemm_f32_tc_kernel, dim3(cut.ctas), dim3(THREADS), (size_t)stages_for(bn) * stage_bytes(bn) + 1024, s, tm_w, tm_x, o, bn, cut,
+    bw::launch(gemm_f32_tc_kernel, dim3(cut.ctas), dim3(THREADS), (size_t)ring_bytes(bn) + 1024, s, tm_w, tm_x, o, bn, cut,
                tiles_m);
     BW_LAUNCH_CHECK();
     if (shared) {
