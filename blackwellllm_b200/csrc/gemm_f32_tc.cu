@@ -21,10 +21,10 @@
 // Roles (896 threads): warp 0 loads weights; warp 1 TMEM owner and MMAs; warp 2 loads tokens; warps 4..11 split the weights, two
 // groups that take stages in turn; warps 12..27 add the accumulators up, 32 tokens each group of four, and write the result.  Every
 // wait is bounded; a timeout sets the status word and all roles fall through to the exit.
-// What bounds it: the MMA warp.  Of 857 cycles a stage of 32 channels at 16 tokens 550 are its issue of 12 MMAs (the tensor pipe needs
-// 120) and 300 its waits; at 128 tokens 768 of 1,369 are MMAs.  Measured, x 28672 x 4096: 1 to 16 tokens 91 us (5.1 TB/s), 64 tokens
-// 127 us, 128 tokens 173 us (174 TFLOP/s), 301 tokens 476 us; gemm_simt.cu's tiles: eight layers of the 8B shape with logits at each of
-// 301 tokens 72.2 ms, of which 65.0 were products.
+// What bounds it: the MMA warp, in its waits (about 300 cycles a stage of 32 channels, of 1,369 at 128 tokens; 768 are MMAs) and its
+// issue.  Measured, x 28672 x 4096: 1 to 16 tokens 84 to 88 us (5.6 TB/s), 64 tokens 122 us, 128 tokens 167 us (180 TFLOP/s), 301 tokens
+// 454 us; with loop bounds that the compiler could not know to be the same in all lanes 91, 127, 173 and 476 us.  gemm_simt.cu's tiles:
+// eight layers of the 8B shape with logits at each of 301 tokens 72.2 ms, of which 65.0 were products.
 #include "tcgen05.cuh"
 
 using bf16 = __nv_bfloat16;
@@ -139,7 +139,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     __shared__ uint32_t tmem_slot[2];
     BW_PDL_TRIGGER();
     const int ws = w_stages(bn), ts = t_stages(bn), xs = x_stages(bn);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t wfull0 = bw::smem_u32(bars), wfree0 = wfull0 + 8 * MAX_W, ready0 = wfree0 + 8 * MAX_W, tfree0 = ready0 + 8 * MAX_T;
     const uint32_t xfull0 = tfree0 + 8 * MAX_T, xfree0 = xfull0 + 8 * MAX_X;
     const uint32_t sum_full0 = xfree0 + 8 * MAX_X, sum_free0 = sum_full0 + 16, small_free = sum_free0 + 16;
@@ -202,11 +202,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         const uint32_t idesc = idesc_tf32(bn), smem0 = bw::smem_u32(smem_x), lo_units = (uint32_t)bn * BK * 4 / 16;
         int xst = 0, xph = 0, tst = 0, tph = 0, p = 0, items = 0;
         bool ok = true;
-        while (ok && it.next()) {
+        while (ok && __shfl_sync(0xffffffffu, (int)it.next(), 0)) {
+            const int n = __shfl_sync(0xffffffffu, it.n, 0);      // (known to be the same in all lanes, like all that the loop changes)
             ok = __all_sync(0xffffffffu, bw::mbar_wait(small_free, (items++ & 1) ^ 1, &g_status, 3));
-            for (int i = 0; ok && i < it.n; ++i) {
+            for (int i = 0; ok && i < n; ++i) {
                 const int buf = p & 1;
-                const bool fresh = i % SUM_STAGES == 0, last = i % SUM_STAGES == SUM_STAGES - 1 || i == it.n - 1;
+                const bool fresh = i % SUM_STAGES == 0, last = i % SUM_STAGES == SUM_STAGES - 1 || i == n - 1;
                 ok = bw::mbar_wait(xfull0 + 8 * xst, xph, &g_status, 4) && bw::mbar_wait(ready0 + 8 * tst, tph, &g_status, 5);
                 if (fresh) ok = ok && bw::mbar_wait(sum_free0 + 8 * buf, ((p >> 1) & 1) ^ 1, &g_status, 6);
                 if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
