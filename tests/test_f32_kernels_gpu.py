@@ -46,6 +46,51 @@ def test_split_products(ops, M, N, K):
         assert torch.equal(ops.gemm_f32(x[rows], w), plain[rows])
 
 
+@pytest.mark.parametrize("M,N,K", [(301, 6144, 4096), (301, 4096, 4096), (128, 4096, 2048), (17, 6144, 4096)])
+def test_queued_products_repeat_themselves(ops, M, N, K):
+    """Products right behind other kernels, nothing waited for in between: every one the bits of the same product by itself.  (The
+    product's blocks start beside those of the kernels before, whose memory traffic holds up their reads of shared memory.)"""
+    gain, xs, w = torch.ones(K, device=DEV), [rand(M, K, seed=s) for s in (1, 2)], rand(N, K, seed=3)
+    alone = []
+    for x in xs:
+        torch.cuda.synchronize()
+        y = ops.rmsnorm(x, gain, 1e-5, torch.float32)
+        torch.cuda.synchronize()
+        alone.append(ops.gemm_f32(y, w))
+    for _ in range(8):
+        queued = [ops.gemm_f32(ops.rmsnorm(xs[i % 2], gain, 1e-5, torch.float32), w) for i in range(300)]
+        assert all(torch.equal(out, alone[i % 2]) for i, out in enumerate(queued))
+
+
+def test_queued_steps_repeat_themselves():
+    """Whole float32 steps of two engines in turn, queued: the logits of a step that was waited for.  (A step's prompt gets its pages
+    in another order each time, and everything it reads was written by the steps right before it.)"""
+    from blackwellllm_b200 import Engine, StepEntry
+    raw = {"architectures": ["LlamaForCausalLM"], "model_type": "llama", "hidden_size": 4096, "num_attention_heads": 32,
+           "num_key_value_heads": 8, "head_dim": 128, "intermediate_size": 14336, "num_hidden_layers": 2, "vocab_size": 32064,
+           "rope_theta": 500000.0, "rms_norm_eps": 1e-5, "tie_word_embeddings": False}
+    n = 301
+    engines = [Engine.from_config(raw, seed=s, dtype="float32", num_pages=24, max_requests=2, max_batch_tokens=512, max_context=384)
+               for s in (0, 1)]
+    entry = StepEntry("p", torch.randint(0, 32064, (n,), generator=torch.Generator().manual_seed(5)).tolist(), list(range(n)))
+
+    def step(e):
+        logits = e.step([entry])
+        e.end_request("p")
+        return logits
+
+    alone = []
+    for e in engines:
+        for _ in range(2):
+            torch.cuda.synchronize()
+            logits = step(e)
+            torch.cuda.synchronize()
+        alone.append(logits)
+    for _ in range(10):
+        queued = [step(engines[i % 2]) for i in range(60)]
+        assert all(torch.equal(out, alone[i % 2]) for i, out in enumerate(queued))
+
+
 def test_split_products_over_the_range_of_float32(ops):
     """Magnitudes from the smallest normal products to large ones, in one product each: the split is relative to each value."""
     for scale_x, scale_w in ((1e-15, 1e-15), (1e15, 1e15), (1e-18, 1e18)):
