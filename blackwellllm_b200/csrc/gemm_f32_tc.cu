@@ -52,6 +52,15 @@ __host__ __device__ constexpr int w_stages(int bn) {
     const int n = (SMEM_BUDGET - x_stages(bn) * x_bytes(bn)) / A_BYTES;
     return n < MAX_W ? n : MAX_W;
 }
+// A warp that waits for a phase by its parity must not be two phases ahead of it.  The split groups take stages in turn, and what holds
+// a group back is its own slot among the split weights: behind it at most t_stages stages are unfinished.  So no slot may have two
+// groups waiting for it, and a stage of the weights' ring may come round again only after the group that had it before is done.
+constexpr bool rings_hold() {
+    for (int bn = 16; bn <= MAX_BN; bn += 16)
+        if (t_stages(bn) < SPLIT_GROUPS || w_stages(bn) < t_stages(bn) + SPLIT_GROUPS) return false;
+    return true;
+}
+static_assert(rings_hold(), "a split group could pass a wait two phases early");
 __host__ __device__ constexpr int ring_bytes(int bn) { return w_stages(bn) * A_BYTES + x_stages(bn) * x_bytes(bn); }
 
 // x rounded to TF32, halves away from zero (three integer instructions fewer than the conversion instruction takes; a NaN whose
