@@ -13,6 +13,7 @@ multiplied when not, before temperature, nucleus or argmax) is a parameter too.
 """
 from __future__ import annotations
 
+import operator
 from dataclasses import dataclass
 from typing import Optional, Sequence, Tuple
 
@@ -44,9 +45,19 @@ def uniform(seed: int, index: int) -> float:
 def uniform_many(seeds: Sequence[int], indices: Sequence[int]) -> np.ndarray:
     """:func:`uniform` of every (seed, index), float32, in the host runtime."""
     from ..cache.manager import native
+    if len(seeds) != len(indices):
+        raise ValueError(f"one index per seed: {len(seeds)} seeds, {len(indices)} indices")
     out = np.empty(len(seeds), dtype=np.float32)
-    s, i = (np.array([int(v) & 0xFFFFFFFFFFFFFFFF for v in vals], dtype=np.uint64) for vals in (seeds, indices))
+    s, i = (np.array([operator.index(v) & 0xFFFFFFFFFFFFFFFF for v in vals], dtype=np.uint64) for vals in (seeds, indices))
     native().bwh_uniform(len(out), s.ctypes.data, i.ctypes.data, out.ctypes.data)
+    return out
+
+
+def row_draws(params: Sequence["SamplingParams"], seeds: Sequence[int], draw_index: Sequence[int]) -> np.ndarray:
+    """The random number of every row, float32.  Greedy rows draw nothing (0) and theirs are not looked at."""
+    rows = [r for r, p in enumerate(params) if not p.greedy]
+    out = np.zeros(len(params), dtype=np.float32)
+    out[rows] = uniform_many([seeds[r] for r in rows], [draw_index[r] for r in rows])
     return out
 
 

@@ -14,7 +14,7 @@ from typing import List, Optional, Sequence
 import torch
 
 from ..kernels import ops
-from .params import SamplingParams, uniform_many
+from .params import SamplingParams, row_draws
 
 
 class Sampler:
@@ -61,11 +61,8 @@ class Sampler:
             return ops.sample(logits, None, None, None)
         host = torch.empty((3, R), dtype=torch.float32, pin_memory=True)
         rows = host.numpy()   # filled row by row: one assignment each instead of one per request
-        temps = [0.0 if p.greedy else p.temperature for p in params]
-        rows[0] = temps
+        rows[0] = [0.0 if p.greedy else p.temperature for p in params]
         rows[1] = [p.top_p for p in params]
-        rows[2] = uniform_many(seeds, draw_index)
-        if 0.0 in temps:
-            rows[2][rows[0] == 0.0] = 0.0      # greedy rows draw nothing
+        rows[2] = row_draws(params, seeds, draw_index)
         dev = host.to(self.device, non_blocking=True)
         return ops.sample(logits, dev[0], dev[1], dev[2])
