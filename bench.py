@@ -791,7 +791,7 @@ def main():
         kernels["decode"] = renamed(kernel_shares(ops, lambda: eng.step([StepEntry(("seq", b), [toks[b]], [0]) for b in range(B)])))
     finally:
         eng.options.cuda_graphs = graphs_on
-    status = ops.gemm_tc_status() | ops.attention_tc_status()
+    status = ops.gemm_tc_status() | ops.attention_tc_status() | ops.gemm_f32_tc_status()
 
     bytes_step = weight_elems * 2 + B * args.context * kv_per_token * 2
     achieved = bytes_step / (ms_step / 1e3) / 1e9

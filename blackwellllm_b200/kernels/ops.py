@@ -530,6 +530,11 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = No
     return out
 
 
+def gemm_f32_tc_status() -> int:
+    """0 if no bounded wait of the split float32 products ever gave up (synchronises the device)."""
+    return int(_fn("gemm_f32_tc", "bw_gemm_f32_tc_status", [])())
+
+
 def attention_simt(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, positions: torch.Tensor,
                    req_of_token: torch.Tensor, block_table: torch.Tensor, nh: int, window: Optional[int],
                    scale: float, out: Optional[torch.Tensor] = None, chunk: Optional[int] = None,

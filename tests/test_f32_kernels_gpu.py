@@ -17,14 +17,20 @@ def ops():
     return o
 
 
+@pytest.fixture(autouse=True)
+def no_wait_gave_up(ops):
+    yield
+    assert ops.gemm_f32_tc_status() == 0
+
+
 def rand(*shape, seed=0):
     return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(DEV)
 
 
 # tokens on both sides of the widths of a tile and of its columns in tensor memory; ragged features; channels that leave the last
-# stage ragged; tiles in one part and in several; tokens in one launch and in two
+# stage ragged; tiles in one part, in several and both in one launch; tokens in one launch and in two
 @pytest.mark.parametrize("M", [1, 2, 9, 16, 17, 33, 65, 128, 129, 257, 513])
-@pytest.mark.parametrize("N,K", [(128, 256), (130, 260), (200, 1028), (1024, 4100), (4096, 2048)])
+@pytest.mark.parametrize("N,K", [(128, 256), (130, 260), (200, 1028), (1024, 4100), (4096, 2048), (20000, 260)])
 def test_split_products(ops, M, N, K):
     x, w, b, base = rand(M, K + 4, seed=1)[:, 4:], rand(N, K, seed=2), rand(N, seed=3), rand(M, N + 1, seed=4)
     assert ops.gemm_f32_tc_supports(x, w)
