@@ -78,7 +78,7 @@ __device__ __forceinline__ uint32_t idesc_tf32(int n) {
 }
 
 struct Out {
-    float* out; const void* bias; float* part;   // part: [parts][M][N]
+    float* out; const void* bias; float* part;   // part: [piece][M][BM], see Cut
     long long ldo;
     int bias_type, accumulate, M, N;
 };
@@ -91,6 +91,13 @@ struct Cut {
     __host__ __device__ int owner(long long kb) const { return (int)(((kb + 1) * ctas + total() - 1) / total()) - 1; }
     __host__ __device__ int first_part(int tile) const { return owner((long long)tile * kb_total); }
     __host__ __device__ int parts(int tile) const { return owner((long long)(tile + 1) * kb_total - 1) - first_part(tile) + 1; }
+    // The piece that a range has of a tile it shares: a range shares its first tile and its last at most.  (So the scratch is two tiles
+    // a range, 78 MB at 512 tokens, whatever the weight's size: of the 1,002 tiles of a head of 128,256 rows 146 are shared.)
+    __host__ __device__ int piece(int range, int tile) const { return 2 * range + (begin(range) / kb_total != tile); }
+    __host__ bool shared() const {
+        for (int c = 1; c < ctas; ++c) if (begin(c) % kb_total) return true;
+        return false;
+    }
 };
 // One CTA's items: for every tile of tokens, its range's piece of every tile of features.
 struct Items {
@@ -325,11 +332,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             const int n = it.tile * BM + quarter * 32 + lane, t0 = it.mt * bn + first;
             if (n >= o.N) continue;
             const bool whole = it.n == cut.kb_total;
-            const long long ld = whole ? o.ldo : o.N;
+            const long long ld = whole ? o.ldo : BM;
             const float b = whole ? bias_at(o, n) : 0.f;
             const bool add = whole && o.accumulate;
             float* dst = whole ? o.out + (size_t)t0 * ld + n
-                               : o.part + ((size_t)((int)blockIdx.x - cut.first_part(it.tile)) * o.M + t0) * o.N + n;
+                               : o.part + ((size_t)cut.piece(blockIdx.x, it.tile) * o.M + t0) * BM + quarter * 32 + lane;
 #pragma unroll
             for (int c0 = 0; c0 < COLS; c0 += 16) {       // sixteen tokens' old values in flight
                 if (c0 >= cols) continue;
@@ -357,17 +364,16 @@ sum_kernel(Out o, Cut cut) {
     BW_PDL_WAIT();
     const int n = (blockIdx.x * blockDim.x + threadIdx.x) * V, m = blockIdx.y;
     if (n >= o.N) return;
-    const int parts = cut.parts(n / BM);
+    const int tile = n / BM, parts = cut.parts(tile), first = cut.first_part(tile);
     if (parts == 1) return;
-    const size_t plane = (size_t)o.M * o.N;
-    const float* p = o.part + (size_t)m * o.N + n;
     float s[V];
 #pragma unroll
     for (int e = 0; e < V; ++e) s[e] = 0.f;
     for (int i = 0; i < parts; ++i) {
+        const float* p = o.part + ((size_t)cut.piece(first + i, tile) * o.M + m) * BM + (n - tile * BM);
         float v[V];
-        if constexpr (V == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p + i * plane);
-        else v[0] = p[i * plane];
+        if constexpr (V == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+        else v[0] = *p;
 #pragma unroll
         for (int e = 0; e < V; ++e) s[e] = i ? s[e] + v[e] : v[e];
     }
@@ -405,25 +411,22 @@ static Cut cut_of(int N, int K) {
     return c;
 }
 
-// The parts that a tile of features comes in at most (their planes are the scratch of bw_gemm_f32_tc).
-BW_EXPORT int bw_gemm_f32_tc_parts(int N, int K) {
+// The floats of scratch that bw_gemm_f32_tc needs per token for the tiles that several ranges share (0: there are none).
+BW_EXPORT int bw_gemm_f32_tc_part_floats(int N, int K) {
     if (N <= 0 || K <= 0) return BW_ERR_BAD_ARG;
     const Cut c = cut_of(N, K);
-    int most = 1;
-    for (int t = 0; t < c.tiles_n; ++t) if (c.parts(t) > most) most = c.parts(t);
-    return most;
+    return c.shared() ? 2 * c.ctas * BM : 0;
 }
 
-// xs: float32 [2 * M * K] for the tokens' parts; part: float32 [parts * M * N] (bw_gemm_f32_tc_parts), not used where that is 1.
+// xs: float32 [2 * M * K] for the tokens' parts; part: `part_floats` of scratch, M times bw_gemm_f32_tc_part_floats at least.
 // K % 4 == 0, rows of x and w begin on 16 bytes; at most 65,535 tokens.
 BW_EXPORT int bw_gemm_f32_tc(const float* x, const float* w, const void* bias, int bias_type, float* out, int M, int N, int K, long long ldx,
-                             long long ldo, int accumulate, float* xs, float* part, void* stream) {
+                             long long ldo, int accumulate, float* xs, float* part, long long part_floats, void* stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 4 || ldx % 4 || ldx < K || ldo < N || M > 65535 || cut_of(N, K).total() > 0x7fffffff || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)xs) & 15)) return BW_ERR_BAD_ARG;
     const Cut cut = cut_of(N, K);
-    bool shared = false;
-    for (int t = 0; t < cut.tiles_n && !shared; ++t) shared = cut.parts(t) > 1;
-    if (shared && (!part || ((uintptr_t)part & 15))) return BW_ERR_BAD_ARG;
+    const bool shared = cut.shared();
+    if (shared && (!part || ((uintptr_t)part & 15) || part_floats < 2ll * cut.ctas * BM * M)) return BW_ERR_BAD_ARG;
     // tiles of tokens as even as they can be, a multiple of 16
     const int tiles = (M + MAX_BN - 1) / MAX_BN, bn = ((M + tiles - 1) / tiles + 15) / 16 * 16, tiles_m = (M + bn - 1) / bn;
     cudaStream_t s = (cudaStream_t)stream;

@@ -483,9 +483,8 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = N
 
 # ------------------------------------------------------------------ attention
 
-_GEMM_F32_TC_ARGS = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_void_p, c_void_p, c_void_p]
-_GEMM_F32_TOKENS = 512       # tokens of one launch: the planes of the tiles' parts stay below 200 MB at the largest layer sizes
-_f32_parts = {}
+_GEMM_F32_TC_ARGS = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_void_p, c_void_p, c_ll, c_void_p]
+_GEMM_F32_TOKENS = 512       # tokens of one launch: the pieces of shared tiles stay below 80 MB on 148 SMs, whatever the weight's size
 
 
 def gemm_f32_tc_supports(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -493,6 +492,11 @@ def gemm_f32_tc_supports(x: torch.Tensor, w: torch.Tensor) -> bool:
     weight of at least one tile's rows and eight stages' channels (a smaller one is all latency there, and its chains too short to err more)."""
     return (x.dtype == torch.float32 and w.dtype == torch.float32 and w.shape[0] >= 128 and w.shape[1] >= 256 and w.shape[1] % 4 == 0
             and x.dim() == 2 and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_f32_part_floats(N: int, K: int) -> int:
+    """The scratch of a split product per token on the current device, in floats."""
+    return _fn("gemm_f32_tc", "bw_gemm_f32_tc_part_floats", [c_int, c_int])(N, K)
 
 
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
@@ -516,17 +520,15 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = No
         _dev(bias, "bias")
         if bias.numel() != N:
             raise KernelError("gemm: bias must have N entries")
-    parts = _f32_parts.get((N, K))
-    if parts is None:
-        parts = _f32_parts[(N, K)] = _fn("gemm_f32_tc", "bw_gemm_f32_tc_parts", [c_int, c_int])(N, K)
     most = min(M, _GEMM_F32_TOKENS)
     split = torch.empty((2 * most * K,), dtype=torch.float32, device=x.device)
-    planes = torch.empty((parts * most * N,), dtype=torch.float32, device=x.device) if parts > 1 else None
+    floats = most * gemm_f32_part_floats(N, K)
+    part = torch.empty((floats,), dtype=torch.float32, device=x.device) if floats else None
     fn = _fn("gemm_f32_tc", "bw_gemm_f32_tc", _GEMM_F32_TC_ARGS, tag=f"{M}x{N}x{K}")
     for at in range(0, M, _GEMM_F32_TOKENS):
         n = min(_GEMM_F32_TOKENS, M - at)
         _check(fn(_ptr(x[at:]), _ptr(w), _ptr(bias), _code(bias, "bias") if bias is not None else 0, _ptr(out[at:]), n, N, K, x.stride(0),
-                  out.stride(0), int(accumulate), _ptr(split), _ptr(planes), _stream()), "gemm_f32_tc")
+                  out.stride(0), int(accumulate), _ptr(split), _ptr(part), floats, _stream()), "gemm_f32_tc")
     return out
 
 
