@@ -5,7 +5,9 @@
 // tensor cores' own sums are kept short: an accumulator takes 64 channels and is then added into float32 registers, rounded to
 // nearest, so no long chain runs through the tensor cores' accumulation.  Measured against 64 bits over the products of an 8B
 // decoder (K 4096 and 14336): relative error 2.2e-7 to 2.6e-7, where one chain of float32 FMAs (gemm_simt.cu) has 1.2e-6 to 2.2e-6.
-// A value that is not finite, or within 2^-12 of float32's largest, makes the results it enters NaN (inf - inf in the split).
+// What the split drops of an operand is at most 2^-23 of it, one unit of float32's last place: a product by itself (a row of x with one
+// entry) is off by up to 2^-21 where an FMA rounds by 2^-24.  Below 1e-34 an operand's lo is no normal number and keeps multiples of
+// 2^-136 only (relative error at 1e-35 6.6e-7, at 1e-36 6.6e-6).  Results that come out as no number are made again by FMAs: see chain().
 //
 // Weights are the 128-row operand (from tensor memory), tokens the other (from shared memory).  The tokens are split beforehand by a
 // small kernel (they are read again by every block of features); the weights, which are read once, on the way: a warp a quarter
@@ -79,8 +81,9 @@ __device__ __forceinline__ uint32_t idesc_tf32(int n) {
 
 struct Out {
     float* out; const void* bias; float* part;   // part: [piece][M][BM], see Cut
-    long long ldo;
-    int bias_type, accumulate, M, N;
+    const float *x, *w;                           // the operands as they are, for chain()
+    long long ldo, ldx;
+    int bias_type, accumulate, M, N, K;
 };
 
 // The stages (32 channels of a tile of features) of all tiles, dealt out to `ctas` ranges.
@@ -122,6 +125,29 @@ struct Items {
 __device__ __forceinline__ float bias_at(const Out& o, int n) {
     if (!o.bias) return 0.f;
     return o.bias_type == BW_F32 ? ((const float*)o.bias)[n] : __bfloat162float(((const bf16*)o.bias)[n]);
+}
+
+// One result by float32 FMAs, made by a whole warp (the same in all lanes).  An operand that is not finite, or so near float32's largest
+// that hi is not, makes every result it enters a NaN (its lo is one, or the infinity that cancels hi's), and no other operand does unless
+// a sum overflows.  So a result that is a NaN, and only that, is made again here, from the operands as they are: infinities stay
+// infinities.  x 28672 x 4096, 301 tokens of which so many hold a NaN: none 0.49 ms, one 2.0, 16 3.6, all 28 (gemm_simt.cu 3.1).
+__device__ __noinline__ float chain(const float* x, const float* w, int K) {
+    float s = 0.f;
+#pragma unroll 4
+    for (int k = (threadIdx.x & 31) * 4; k < K; k += 128) {
+        const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
+        s = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
+    }
+    return bw::warp_sum(s);
+}
+// chain() for every lane of a converged warp that wants it, for token m and feature n of that lane
+__device__ __forceinline__ float chains(const Out& o, bool wanted, float otherwise, int m, int n) {
+    for (unsigned lanes = __ballot_sync(0xffffffffu, wanted); lanes; lanes &= lanes - 1) {
+        const int from = __ffs(lanes) - 1, mm = __shfl_sync(0xffffffffu, m, from), nn = __shfl_sync(0xffffffffu, n, from);
+        const float v = chain(o.x + (size_t)mm * o.ldx, o.w + (size_t)nn * o.K, o.K);
+        if ((threadIdx.x & 31) == from) otherwise = v;
+    }
+    return otherwise;
 }
 
 // hi and lo parts of x, [2][M][K]; K % 4 == 0
@@ -330,23 +356,34 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             if (lane == 0) bw::mbar_arrive(small_free);
             if (!waited) { BW_PDL_WAIT(); waited = true; }      // the result belongs to earlier kernels until here
             const int n = it.tile * BM + quarter * 32 + lane, t0 = it.mt * bn + first;
-            if (n >= o.N) continue;
+            const bool in = n < o.N;
             const bool whole = it.n == cut.kb_total;
             const long long ld = whole ? o.ldo : BM;
-            const float b = whole ? bias_at(o, n) : 0.f;
+            const float b = whole && in ? bias_at(o, n) : 0.f;
             const bool add = whole && o.accumulate;
             float* dst = whole ? o.out + (size_t)t0 * ld + n
                                : o.part + ((size_t)cut.piece(blockIdx.x, it.tile) * o.M + t0) * BM + quarter * 32 + lane;
+            unsigned again = 0;          // the tokens whose results chain() makes
 #pragma unroll
             for (int c0 = 0; c0 < COLS; c0 += 16) {       // sixteen tokens' old values in flight
                 if (c0 >= cols) continue;
                 float old[16];
 #pragma unroll
-                for (int c = 0; c < 16; ++c) old[c] = add && t0 + c0 + c < o.M ? dst[(size_t)(c0 + c) * ld] : 0.f;
+                for (int c = 0; c < 16; ++c) old[c] = add && in && t0 + c0 + c < o.M ? dst[(size_t)(c0 + c) * ld] : 0.f;
 #pragma unroll
-                for (int c = 0; c < 16; ++c)
-                    if (t0 + c0 + c < o.M) dst[(size_t)(c0 + c) * ld] = add ? sum[c0 + c] + b + old[c] : sum[c0 + c] + b;
+                for (int c = 0; c < 16; ++c) {
+                    if (!in || t0 + c0 + c >= o.M) continue;
+                    if (whole && sum[c0 + c] != sum[c0 + c]) again |= 1u << (c0 + c);
+                    else dst[(size_t)(c0 + c) * ld] = add ? sum[c0 + c] + b + old[c] : sum[c0 + c] + b;
+                }
                 asm volatile("" ::: "memory");
+            }
+            __syncwarp();
+            for (unsigned any = __reduce_or_sync(0xffffffffu, again); any; any &= any - 1) {
+                const int c = __ffs(any) - 1;
+                const bool wanted = again >> c & 1;
+                const float v = chains(o, wanted, 0.f, t0 + c, n) + b;
+                if (wanted) dst[(size_t)c * ld] = add ? v + dst[(size_t)c * ld] : v;
             }
         }
     }
@@ -363,13 +400,13 @@ sum_kernel(Out o, Cut cut) {
     BW_PDL_TRIGGER();
     BW_PDL_WAIT();
     const int n = (blockIdx.x * blockDim.x + threadIdx.x) * V, m = blockIdx.y;
-    if (n >= o.N) return;
-    const int tile = n / BM, parts = cut.parts(tile), first = cut.first_part(tile);
-    if (parts == 1) return;
+    const bool in = n < o.N;
+    const int tile = min(n, o.N - 1) / BM, parts = cut.parts(tile), first = cut.first_part(tile);
+    if (parts == 1) return;          // (a warp's features lie in one tile)
     float s[V];
 #pragma unroll
     for (int e = 0; e < V; ++e) s[e] = 0.f;
-    for (int i = 0; i < parts; ++i) {
+    for (int i = 0; in && i < parts; ++i) {
         const float* p = o.part + ((size_t)cut.piece(first + i, tile) * o.M + m) * BM + (n - tile * BM);
         float v[V];
         if constexpr (V == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
@@ -380,6 +417,8 @@ sum_kernel(Out o, Cut cut) {
     float* dst = o.out + m * o.ldo + n;
 #pragma unroll
     for (int e = 0; e < V; ++e) {
+        s[e] = chains(o, s[e] != s[e], s[e], m, n + e);
+        if (!in) continue;
         s[e] += bias_at(o, n + e);
         dst[e] = o.accumulate ? s[e] + dst[e] : s[e];
     }
@@ -438,7 +477,7 @@ BW_EXPORT int bw_gemm_f32_tc(const float* x, const float* w, const void* bias, i
     static bool done[bw::MAX_DEVICES] = {};
     const cudaError_t e = bw::allow_dynamic_smem(gemm_f32_tc_kernel, SMEM_BUDGET + 1024, done);
     if (e != cudaSuccess) return (int)e;
-    const Out o = {out, bias, part, ldo, bias_type, accumulate, M, N};
+    const Out o = {out, bias, part, x, w, ldo, ldx, bias_type, accumulate, M, N, K};
     bw::launch(gemm_f32_tc_kernel, dim3(cut.ctas), dim3(THREADS), (size_t)ring_bytes(bn) + 1024, s, tm_w, tm_x, o, bn, cut,
                tiles_m);
     BW_LAUNCH_CHECK();

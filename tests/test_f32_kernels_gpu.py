@@ -105,6 +105,59 @@ def test_split_products_over_the_range_of_float32(ops):
         assert float((ops.gemm_f32(x, w).double() - want).abs().max()) <= 1e-6 * float(want.abs().max())
 
 
+# results in tiles of one range, in shared tiles, and both
+@pytest.mark.parametrize("M,N,K", [(3, 130, 260), (40, 1024, 4100), (5, 20000, 260)])
+def test_split_products_of_infinities(ops, M, N, K):
+    """Operands that are not finite, or whose parts would not be, give what a chain of FMAs gives; other rows keep their bits."""
+    x, w, b, base = rand(M, K, seed=1), rand(N, K, seed=2), rand(N, seed=3), rand(M, N, seed=4)
+    plain = ops.gemm_f32(x, w)
+    inf, top = float("inf"), 3.4028e38
+    w[7] = w[7].to(torch.bfloat16).float()                # a weight without a second part, a zero, an infinity, a NaN
+    w[5, 11], w[N - 1, 200], w[64, 30] = 0.0, -inf, float("nan")
+    touched = torch.zeros(M, N, dtype=torch.bool, device=DEV)
+    touched[:, [5, 7, 64, N - 1]] = True
+    for fill in ({(1, 11): inf}, {(1, 11): -inf, (1, 12): inf}, {(2, 5): float("nan")}, {(M - 1, K - 1): top / 2, (M - 1, 3): top},
+                 {(0, 4): -top}):
+        y, rows = x.clone(), sorted({r for r, _ in fill})
+        for at, v in fill.items():
+            y[at] = v
+        hit = touched.clone()
+        hit[rows] = True
+        # near the largest value: what overflows depends on the order of a sum, so the other entries and weights stay small there
+        scale = 1e-4 if any(abs(v) == top for v in fill.values()) else 1.0
+        got, want = ops.gemm_f32(y, w * scale), ops.gemm_simt(y, w * scale)
+        assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+        known = hit & torch.isfinite(want)
+        assert torch.equal(got[torch.isinf(want)], want[torch.isinf(want)])
+        # sums of K products in two orders: each off by 2^-24 K of the largest at most
+        size = want.nan_to_num(0.0, 0.0, 0.0).abs().amax(1, keepdim=True)
+        assert bool(((got - want).abs() <= 2 ** -24 * K * size)[known].all())
+        if scale == 1.0:
+            assert torch.equal(got[~hit], plain[~hit])
+        out = base.clone()
+        ops.gemm_f32(y, w * scale, b, out=out, accumulate=True)
+        assert torch.equal(out.nan_to_num(), (got + b + base).nan_to_num()) and torch.equal(torch.isnan(out), torch.isnan(got))
+
+
+def test_single_products_and_small_magnitudes(ops):
+    """What splitting in two loses where float32 FMAs lose next to nothing: bounds, derived from the parts' 11 bits each."""
+    N, K, M = 256, 512, 40
+    x, w, at = torch.zeros(M, K, device=DEV), rand(N, K, seed=2), torch.arange(M) * 3
+    x[torch.arange(M), at] = 1.0
+    assert bool(((ops.gemm_f32(x, w) - w[:, at].T).abs() <= 2 ** -23 * w[:, at].T.abs()).all())
+    x[torch.arange(M), at] = rand(M, seed=3)
+    want = x.double() @ w.double().T
+    assert bool(((ops.gemm_f32(x, w).double() - want).abs() <= (2 ** -21 + 2 ** -24) * want.abs()).all())
+    x = rand(M, K, seed=4)
+    for scale in (1e-30, 1e-34, 1e-36, 1e-38):
+        for a, b in ((x * scale, w), (x, w * scale)):
+            want, sizes = a.double() @ b.double().T, a.double().abs() @ b.double().abs().T
+            # products of 512 channels as everywhere (see test_split_products), and operands whose lo keeps multiples of 2^-136 only
+            other = w if b is w else x
+            bound = 2 ** -21 * sizes + 2 ** -135 * K * float(other.abs().max())
+            assert bool(((ops.gemm_f32(a, b).double() - want).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("nh,nkv,hd,page", [(4, 2, 16, 16), (3, 1, 20, 8), (8, 8, 64, 16), (32, 8, 128, 16), (14, 2, 132, 4),
                                             (6, 2, 256, 32), (17, 1, 32, 16), (64, 1, 8, 16), (5, 5, 80, 24)])
 @pytest.mark.parametrize("window,chunk", [(None, None), (1, None), (50, None), (None, 96), (40, 64)])
