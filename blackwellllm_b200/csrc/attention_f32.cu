@@ -12,6 +12,7 @@
 // What bounds it: decode, the bytes of keys and values; prompts, shared-memory reads (six 16-byte reads per 32 FMAs).  Measured at
 // head size 128, groups of 4, 8 kv heads, against attention_simt.cu (a block per token and head, a lane a key): 4 requests at
 // 1,000 keys 45 us with the merge against 347, 301 prompt tokens 84 us against 827.
+#include <type_traits>
 #include "common.cuh"
 
 namespace {
@@ -158,6 +159,7 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
             }
         }
         __syncthreads();
+        bool zero = false;
 #pragma unroll
         for (int i = 0; i < RW; ++i) {
             float* pr = ps + (warp * RW + i) * LDP;
@@ -168,33 +170,41 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
             l[i] = l[i] * corr + bw::warp_sum(e);
             m[i] = m_new;
             pr[lane] = e;
+            zero |= e == 0.f && warp * RW + i < rows;
 #pragma unroll
             for (int c = 0; c < CH * 4; ++c) o[i][c] *= corr;
         }
         __syncwarp();
+        // A key without weight (masked, or too far below the largest score) must not add its value, which may be no number: 0 times an
+        // infinity is none.  Rare beside the diagonal and a window's edges, so a warp asks once per tile.
         const float* vt = vs + st * KEYS * hd;
+        auto add_values = [&](auto skip) {
 #pragma unroll 2
-        for (int k4 = 0; k4 < KEYS; k4 += 4) {
-            float4 w[RW];
+            for (int k4 = 0; k4 < KEYS; k4 += 4) {
+                float4 w[RW];
 #pragma unroll
-            for (int i = 0; i < RW; ++i) w[i] = *reinterpret_cast<const float4*>(ps + (warp * RW + i) * LDP + k4);
+                for (int i = 0; i < RW; ++i) w[i] = *reinterpret_cast<const float4*>(ps + (warp * RW + i) * LDP + k4);
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
+                for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-                for (int h = 0; h < CH; ++h) {
-                    const int c = lane * 4 + 128 * h;
-                    if (c >= hd) continue;
-                    const float4 v = *reinterpret_cast<const float4*>(vt + (k4 + kk) * hd + c);
+                    for (int h = 0; h < CH; ++h) {
+                        const int c = lane * 4 + 128 * h;
+                        if (c >= hd) continue;
+                        const float4 v = *reinterpret_cast<const float4*>(vt + (k4 + kk) * hd + c);
 #pragma unroll
-                    for (int i = 0; i < RW; ++i) {
-                        const float e = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
-                        o[i][4 * h] = fmaf(e, v.x, o[i][4 * h]);
-                        o[i][4 * h + 1] = fmaf(e, v.y, o[i][4 * h + 1]);
-                        o[i][4 * h + 2] = fmaf(e, v.z, o[i][4 * h + 2]);
-                        o[i][4 * h + 3] = fmaf(e, v.w, o[i][4 * h + 3]);
+                        for (int i = 0; i < RW; ++i) {
+                            const float e = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
+                            if (decltype(skip)::value && e == 0.f) continue;
+                            o[i][4 * h] = fmaf(e, v.x, o[i][4 * h]);
+                            o[i][4 * h + 1] = fmaf(e, v.y, o[i][4 * h + 1]);
+                            o[i][4 * h + 2] = fmaf(e, v.z, o[i][4 * h + 2]);
+                            o[i][4 * h + 3] = fmaf(e, v.w, o[i][4 * h + 3]);
+                        }
                     }
-                }
-        }
+            }
+        };
+        if (__any_sync(0xffffffffu, zero)) add_values(std::true_type{});
+        else add_values(std::false_type{});
         if constexpr (!SLICES) {
             if ((tile + 1) % PER == 0 || tile + 1 == last) {
 #pragma unroll

@@ -191,6 +191,31 @@ def test_tiled_attention(ops, nh, nkv, hd, page, window, chunk):
     assert float((out - general).abs().max()) <= 2e-5 * float(general.abs().max())
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 16), (8, 2, 128), (3, 1, 132)])
+@pytest.mark.parametrize("window,chunk", [(None, None), (40, None), (None, 64)])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_values_of_hidden_keys_are_not_read_into_a_result(ops, nh, nkv, hd, window, chunk, bad):
+    """A value that is no number reaches the rows that see its key, and leaves the bits of all others."""
+    q_lens, kv_lens, page = [70, 1, 3], [90, 200, 150], 16
+    q, kp, vp, table, _ = paged_case(q_lens, kv_lens, nh, nkv, hd, page, torch.float32, seed=hd)
+    batch = FakeBatch(q_lens, kv_lens)
+    whole = ops.attention_f32(q, kp, vp, batch, table, nh, window, hd ** -0.5, chunk)
+    for r, pos in ((0, 89), (0, 47), (1, 150), (1, 10), (2, 149), (2, 109)):
+        v2 = vp.clone()
+        v2[table[r, pos // page], :, pos % page] = bad
+        out = ops.attention_f32(q, kp, v2, batch, table, nh, window, hd ** -0.5, chunk)
+        general = ops.attention_simt(q, kp, v2, batch.positions, batch.req_of_token, table, nh, window, hd ** -0.5, chunk=chunk)
+        at = batch.positions
+        sees = (batch.req_of_token == r) & (at >= pos)
+        if window:
+            sees &= pos > at - window
+        if chunk:
+            sees &= pos >= at // chunk * chunk
+        assert torch.equal(out[~sees], whole[~sees])
+        assert not torch.isfinite(out[sees]).any()
+        assert torch.equal(torch.isnan(out), torch.isnan(general)) and torch.equal(torch.isinf(out), torch.isinf(general))
+
+
 def test_rows_off_16_bytes_go_to_the_general_kernel(ops):
     q, kp, vp, table, refs = paged_case([5, 1], [5, 40], 4, 2, 18, 16, torch.float32, seed=3)
     assert not ops.attention_f32_supports(q, kp, vp, 4)                   # a head size that is no multiple of four
