@@ -6,9 +6,11 @@
 // kv head and walks 32 keys at a time (two stages, cp.async).  Scores: each thread a few rows times a few keys.  Softmax and
 // values: warp w owns rows w ROWS / 8 on, a lane four channels (twice that for heads above 128), so probabilities pass through
 // shared memory inside the warp only.  ROWS = 64 for prompt portions, 16 for the few rows of a decoding request, whose slices of
-// SLICE keys have blocks of their own; a second kernel adds them up.
-// A row's result is the same bits whatever else is in the batch: both forms make a softmax per slice of SLICE keys, counted from
-// position 0, in the same order of operations, and fold the slices in their order (fold()).
+// keys have blocks of their own; a second kernel adds them up.
+// A row's result is the same bits whatever else is in the batch: both forms make a softmax per slice of keys, counted from position 0,
+// in the same order of operations, and fold the slices in their order (fold()).  A slice has SLICE keys, or as many times SLICE that a
+// row sees MOST slices or hardly more: what a row sees decides, and no batch.  (So a decoding request has at most MOST + 2 blocks and
+// partial results per kv head at any context: 64 requests of 8 kv heads and groups of 4 at 131,072 tokens 69 MB.)
 // What bounds it: decode, the bytes of keys and values; prompts, shared-memory reads (six 16-byte reads per 32 FMAs).  Measured at
 // head size 128, groups of 4, 8 kv heads, against attention_simt.cu (a block per token and head, a lane a key): 4 requests at
 // 1,000 keys 45 us with the merge against 347, 301 prompt tokens 84 us against 827.
@@ -17,7 +19,7 @@
 
 namespace {
 
-constexpr int THREADS = 256, WARPS = 8, KEYS = 32, SLICE_ROWS = 16, SLICE = 128;
+constexpr int THREADS = 256, WARPS = 8, KEYS = 32, SLICE_ROWS = 16, SLICE = 128, MOST = 64;
 
 struct Params {
     const float *q, *k_pages, *v_pages;
@@ -25,7 +27,8 @@ struct Params {
     const int *cu_q, *q_start, *block_table;
     int max_blocks, nh, nkv, hd, page_size, num_pages, window, chunk;
     float scale;
-    float *part_o, *part_ml;      // [slot][kv head][SLICE_ROWS][hd] and [..][2] (maximum, sum)
+    float *part_o, *part_ml;      // [slot][kv head][slot_rows][hd] and [..][2] (maximum, sum)
+    int slot_rows;                // stacked rows of the largest segment that is sliced
 };
 
 __device__ __forceinline__ void copy16(float* dst, const float* src, bool valid) {
@@ -47,11 +50,15 @@ __device__ __forceinline__ float2 fold(float& M, float& L, float m, float l) {
     return make_float2(a, b);
 }
 __device__ __forceinline__ float folded(float O, float o, float2 f) { return fmaf(O, f.x, __fmul_rn(o, f.y)); }
-// The slices that the rows at positions pos0 .. end - 1 see: from this key on, and so many.
-__device__ __forceinline__ int slices_from(const Params& p, int pos0) { return bw::first_visible(pos0, p.window, p.chunk) / SLICE * SLICE; }
-__device__ __forceinline__ int slices_of(int base, int end) { return (end - base + SLICE - 1) / SLICE; }
+// The keys of a slice for the row at a position, and the slices from a key on.
+__device__ __forceinline__ int slice_keys(const Params& p, int pos) {
+    const int sees = pos + 1 - bw::first_visible(pos, p.window, p.chunk);
+    return SLICE * ((sees + SLICE * MOST - 1) / (SLICE * MOST));
+}
+__device__ __forceinline__ int slices_from(const Params& p, int pos, int keys) { return bw::first_visible(pos, p.window, p.chunk) / keys * keys; }
+__device__ __forceinline__ int slices_of(int base, int end, int keys) { return (end - base + keys - 1) / keys; }
 
-// SLICES: work items (request, slice, slices, first slot), all tokens of the request's segment; else (request, first token).
+// SLICES: work items (request, slice, slices, first slot), all tokens of the request's segment, whose slices are of one size; else (request, first token).
 // CH: groups of four channels of a lane.
 template <int ROWS, int CH, bool SLICES>
 __global__ void __launch_bounds__(THREADS)
@@ -64,7 +71,7 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
     float* vs = ks + 2 * KEYS * ldk;                      // [2][KEYS][hd]
     float* ps = vs + 2 * KEYS * hd;                       // [ROWS][KEYS + 4]
     int* known = reinterpret_cast<int*>(ps + ROWS * (KEYS + 4));   // [2][KEYS]: the key has a page
-    constexpr int LDP = KEYS + 4, PER = SLICE / KEYS;     // tiles of a slice
+    constexpr int LDP = KEYS + 4;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kvh = blockIdx.y;
     const int4 item = work[blockIdx.x];
     const int r = item.x;
@@ -73,10 +80,13 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
     const int tokens = min(ROWS / G, q_len - t0), rows = tokens * G;
     const int pos0 = p.q_start[r] + t0, end = pos0 + tokens;
     const int* bt = p.block_table + (size_t)r * p.max_blocks;
-    const int base = slices_from(p, pos0), slices = slices_of(base, end);
-    if (SLICES && item.y >= slices) return;               // (the list is as long as the longest context may get)
+    const int keys = slice_keys(p, pos0), per = keys / KEYS;      // of the first row's slices: keys, tiles
+    const int base = slices_from(p, pos0, SLICES ? keys : SLICE);
+    if (SLICES && item.y >= slices_of(base, end, keys)) return;   // (the list is as long as the longest context may get)
     const int all = (end - base + KEYS - 1) / KEYS;
-    const int first = SLICES ? item.y * PER : 0, last = SLICES ? min(first + PER, all) : all;
+    const int first = SLICES ? item.y * per : 0, last = SLICES ? min(first + per, all) : all;
+    // a portion's rows may differ in the size of their slices (it never shrinks, except where a block of positions begins)
+    const bool same = !SLICES && slice_keys(p, end - 1) == keys && (p.chunk <= 0 || p.chunk <= SLICE * MOST);
     BW_PDL_WAIT();
 
     for (int i = warp; i < ROWS; i += WARPS) {      // rows beyond the tile's are zeros
@@ -206,9 +216,11 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
         if (__any_sync(0xffffffffu, zero)) add_values(std::true_type{});
         else add_values(std::false_type{});
         if constexpr (!SLICES) {
-            if ((tile + 1) % PER == 0 || tile + 1 == last) {
+            const int done = base / KEYS + tile + 1;      // tiles from position 0
+            if (same ? done % per == 0 || tile + 1 == last : done % (SLICE / KEYS) == 0 || tile + 1 == last) {
 #pragma unroll
                 for (int i = 0; i < RW; ++i) {
+                    if (!same && tile + 1 < last && done % (slice_keys(p, pos0 + (warp * RW + i) / G) / KEYS)) continue;
                     const float2 f = fold(M[i], L[i], m[i], l[i]);
 #pragma unroll
                     for (int c = 0; c < CH * 4; ++c) { O[i][c] = folded(O[i][c], o[i][c], f); o[i][c] = 0.f; }
@@ -225,7 +237,7 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
         float f = 1.f;
         float* dst;
         if (SLICES && item.z > 1) {
-            const size_t slot = ((size_t)(item.w + item.y) * p.nkv + kvh) * SLICE_ROWS + row;
+            const size_t slot = ((size_t)(item.w + item.y) * p.nkv + kvh) * p.slot_rows + row;
             dst = p.part_o + slot * hd;
             if (lane == 0) { p.part_ml[2 * slot] = m[i]; p.part_ml[2 * slot + 1] = l[i]; }
         } else {
@@ -255,7 +267,7 @@ attention_f32_merge_kernel(Params p, const int4* __restrict__ work) {
     const int r = item.x, kvh = blockIdx.y, row = blockIdx.z, G = p.nh / p.nkv, hd = p.hd, c = threadIdx.x * 4;
     const int row0 = p.cu_q[r], q_len = p.cu_q[r + 1] - row0, pos0 = p.q_start[r];
     if (row >= q_len * G || c >= hd) return;
-    const int slices = slices_of(slices_from(p, pos0), pos0 + q_len);
+    const int keys = slice_keys(p, pos0), slices = slices_of(slices_from(p, pos0, keys), pos0 + q_len, keys);
     BW_PDL_WAIT();
     float M = -INFINITY, L = 0.f, O[4] = {0.f, 0.f, 0.f, 0.f};
     constexpr int AHEAD = 8;             // slices whose loads are in flight together
@@ -264,7 +276,7 @@ attention_f32_merge_kernel(Params p, const int4* __restrict__ work) {
         float2 ml[AHEAD];
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i) {
-            const size_t slot = ((size_t)(item.w + min(s0 + i, slices - 1)) * p.nkv + kvh) * SLICE_ROWS + row;
+            const size_t slot = ((size_t)(item.w + min(s0 + i, slices - 1)) * p.nkv + kvh) * p.slot_rows + row;
             ml[i] = *reinterpret_cast<const float2*>(p.part_ml + 2 * slot);
             v[i] = *reinterpret_cast<const float4*>(p.part_o + slot * hd + c);
         }
@@ -292,26 +304,28 @@ int go(const Params& p, const int* work, int n, cudaStream_t s) {
 
 }  // namespace
 
-// The keys of a slice (the work lists count with it).
+// The keys of a slice, and the slices that a row sees before its slices grow (the work lists count with them).
 BW_EXPORT int bw_attention_f32_slice() { return SLICE; }
+BW_EXPORT int bw_attention_f32_slices() { return MOST; }
 
 // rows_w: int32 [n_rows][4] (request, first token, 0, 0), tiles of 64 / (nh / nkv) tokens; keys_w: [n_keys][4] (request, slice,
-// slices, first slot) for segments of at most 16 stacked rows, at least as many slices as the segment's rows see; merge_w: [n_merge][4] (request, 0, slices, first slot).  part_o,
-// part_ml: float32 [slots][nkv][16][hd] and [..][2] (null without merge items).  hd % 4 == 0, hd <= 256, nh / nkv <= 64.
+// slices, first slot) for segments of at most slot_rows <= 16 stacked rows whose slices are of one size, at least as many slices as the
+// segment's rows see; merge_w: [n_merge][4] (request, 0, slices, first slot).  part_o,
+// part_ml: float32 [slots][nkv][slot_rows][hd] and [..][2] (null without merge items).  hd % 4 == 0, hd <= 256, nh / nkv <= 64.
 BW_EXPORT int bw_attention_f32(const float* q, const float* k_pages, const float* v_pages, float* out, const int* cu_q,
                                const int* q_start, const int* block_table, int max_blocks, const int* rows_w, int n_rows,
-                               const int* keys_w, int n_keys, const int* merge_w, int n_merge, float* part_o, float* part_ml, int nh,
+                               const int* keys_w, int n_keys, const int* merge_w, int n_merge, float* part_o, float* part_ml, int slot_rows, int nh,
                                int nkv, int hd, int page_size, int num_pages, int window, int chunk, float scale, void* stream) {
     if (nkv <= 0 || nh % nkv || nh / nkv > 64 || hd <= 0 || hd % 4 || hd > 256) return BW_ERR_UNSUPPORTED;
-    if (n_merge && (!part_o || !part_ml)) return BW_ERR_BAD_ARG;
+    if (n_merge && (!part_o || !part_ml || slot_rows <= 0 || slot_rows > SLICE_ROWS)) return BW_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     const Params p = {q, k_pages, v_pages, out, cu_q, q_start, block_table, max_blocks, nh, nkv, hd, page_size, num_pages, window, chunk,
-                      scale, part_o, part_ml};
+                      scale, part_o, part_ml, slot_rows};
     int rc = 0;
     if (n_rows) rc = hd <= 128 ? go<64, 1, false>(p, rows_w, n_rows, s) : go<64, 2, false>(p, rows_w, n_rows, s);
     if (rc == 0 && n_keys) rc = hd <= 128 ? go<SLICE_ROWS, 1, true>(p, keys_w, n_keys, s) : go<SLICE_ROWS, 2, true>(p, keys_w, n_keys, s);
     if (rc == 0 && n_merge) {
-        bw::launch(attention_f32_merge_kernel, dim3(n_merge, nkv, SLICE_ROWS), dim3(64), 0, s, p, (const int4*)merge_w);
+        bw::launch(attention_f32_merge_kernel, dim3(n_merge, nkv, slot_rows), dim3(64), 0, s, p, (const int4*)merge_w);
         BW_LAUNCH_CHECK();
     }
     return rc;

@@ -585,38 +585,43 @@ def attention_f32(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
     if q.shape[1] != nh * hd:
         raise KernelError("attention: q must be [T, nh * head_dim]")
     out = torch.empty_like(q)
-    rows_w, n_rows, keys_w, n_keys, merge_w, n_merge, slices = _attention_f32_work(batch, nh // nkv, window, chunk)
+    rows_w, n_rows, keys_w, n_keys, merge_w, n_merge, slices, slot_rows = _attention_f32_work(batch, nh // nkv, window, chunk)
     part_o = part_ml = None
     if n_merge:
-        part_o = torch.empty((slices * nkv * 16, hd), dtype=torch.float32, device=out.device)
-        part_ml = torch.empty((slices * nkv * 16, 2), dtype=torch.float32, device=out.device)
+        part_o = torch.empty((slices * nkv * slot_rows, hd), dtype=torch.float32, device=out.device)
+        part_ml = torch.empty((slices * nkv * slot_rows, 2), dtype=torch.float32, device=out.device)
     fn = _fn("attention_f32", "bw_attention_f32", _ATTN_F32_ARGS)
     _check(fn(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(batch.cu_q), _ptr(batch.q_start), _ptr(block_table),
               block_table.shape[1], _ptr(rows_w), n_rows, _ptr(keys_w), n_keys, _ptr(merge_w), n_merge, _ptr(part_o),
-              _ptr(part_ml), nh, nkv, hd, page_size, num_pages, int(window or 0), int(chunk or 0), float(scale), _stream()),
+              _ptr(part_ml), slot_rows, nh, nkv, hd, page_size, num_pages, int(window or 0), int(chunk or 0), float(scale), _stream()),
            "attention_f32")
     return out
 
 
 def plan_attention_f32(q_len, q_start, kv_len, G: int, window: Optional[int], chunk: Optional[int], slice_keys: int,
-                       static_bound: Optional[int] = None):
-    """The work lists of the tiled float32 attention as plain lists, of the form of :func:`plan_attention_work`; a segment of at most
-    16 stacked rows has a block for every slice of ``slice_keys`` keys, counted from position 0, that its rows may see."""
-    rows, keys, merge, slots = [], [], [], 0
+                       most: int, static_bound: Optional[int] = None):
+    """The work lists of the tiled float32 attention as plain lists, of the form of :func:`plan_attention_work`, and the stacked rows
+    of the largest sliced segment.  A segment of at most 16 stacked rows whose rows have slices of one size (``slice_keys`` keys, or as
+    many times that as makes ``most`` slices of what a row sees) has a block for every slice that its rows may see."""
+    def of(pos):
+        lo = max(pos - window + 1 if window else 0, pos - pos % chunk if chunk else 0, 0)
+        return -(-(pos + 1 - lo) // (slice_keys * most))
+    rows, keys, merge, slots, slot_rows = [], [], [], 0, 0
     for r, n_q in enumerate(q_len):
-        if n_q * G > 16:
+        if n_q * G > 16 or (n_q > 1 and len({of(q_start[r] + i) for i in range(n_q)}) > 1):
             rows += [(r, t0, 0, 0) for t0 in range(0, n_q, 64 // G)]
             continue
-        n = -(-(static_bound or kv_len[r]) // slice_keys)
-        for reach in (window, chunk):     # the keys before its first row that a segment reaches back to, from a slice's start
-            if reach:
-                n = min(n, -(-(reach + n_q + slice_keys - 1) // slice_keys))
+        n = min(-(-(static_bound or kv_len[r]) // slice_keys), most)
+        if window or chunk:     # the keys before its first row that a segment reaches back to, from a slice's start
+            n = min([-(-(static_bound or kv_len[r]) // slice_keys), most + 2]
+                    + [-(-(reach + n_q + slice_keys - 1) // slice_keys) for reach in (window, chunk) if reach])
         keys += [(r, s, n, slots) for s in range(n)]
         if n > 1:
             merge.append((r, 0, n, slots))
         slots += n
+        slot_rows = max(slot_rows, n_q * G)
     rows.sort(key=lambda it: -(q_start[it[0]] + it[1]))     # the tiles with the most keys first
-    return rows, keys, merge, slots
+    return rows, keys, merge, slots, slot_rows
 
 
 def _attention_f32_work(batch, G: int, window: Optional[int], chunk: Optional[int]):
@@ -625,16 +630,17 @@ def _attention_f32_work(batch, G: int, window: Optional[int], chunk: Optional[in
     work = batch.static_extras.get(key)
     if work is None:
         R, dev = batch.R, batch.token_ids.device
-        rows, keys, merge, slots = plan_attention_f32(batch.h_q_len[:R], batch.h_q_start[:R], batch.h_kv_len[:R], G, window, chunk,
-                                                      _fn("attention_f32", "bw_attention_f32_slice", [])(), batch.static_bound)
+        rows, keys, merge, slots, slot_rows = plan_attention_f32(
+            batch.h_q_len[:R], batch.h_q_start[:R], batch.h_kv_len[:R], G, window, chunk, _fn("attention_f32", "bw_attention_f32_slice", [])(),
+            _fn("attention_f32", "bw_attention_f32_slices", [])(), batch.static_bound)
 
         def up(items):
             return torch.tensor(items, dtype=torch.int32).pin_memory().to(dev, non_blocking=True) if items else None
-        work = batch.static_extras[key] = (up(rows), len(rows), up(keys), len(keys), up(merge), len(merge), slots)
+        work = batch.static_extras[key] = (up(rows), len(rows), up(keys), len(keys), up(merge), len(merge), slots, slot_rows)
     return work
 
 
-_ATTN_F32_ARGS = [c_void_p] * 7 + [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p] + [c_int] * 7 + [c_float, c_void_p]
+_ATTN_F32_ARGS = [c_void_p] * 7 + [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p] + [c_int] * 8 + [c_float, c_void_p]
 
 
 def _gate_args(gate: Optional[tuple], T: int, nh: int, hd: int):

@@ -7,7 +7,7 @@ import random
 
 import pytest
 
-from blackwellllm_b200.kernels.ops import plan_attention_work
+from blackwellllm_b200.kernels.ops import plan_attention_f32, plan_attention_work
 
 
 def random_batch(rng, R, G):
@@ -72,3 +72,49 @@ def test_a_graph_replay_depends_on_the_bound_only():
     alone = plan_attention_work([1], [8191], [8192], 4, 8, None, 128, 128, 16)
     many = plan_attention_work([1] * 64, [8191] * 64, [8192] * 64, 4, 8, None, 128, 128, 16)
     assert alone[3] > many[3] // 64 >= 1   # fewer slices a request when more requests fill the GPU
+
+
+@pytest.mark.parametrize("G", (1, 3, 4, 16, 20))
+@pytest.mark.parametrize("window,chunk", [(None, None), (48, None), (9000, None), (None, 100), (None, 9000), (20000, 30000)])
+def test_float32_slices(G, window, chunk):
+    """The float32 kernel's lists: every token once, and slices for all that a segment's rows may see (counted as the kernel does)."""
+    rng = random.Random(G)
+    first = lambda pos: max(0, pos - window + 1 if window else 0, pos - pos % chunk if chunk else 0)
+    keys_of = lambda pos: 128 * -(-(pos + 1 - first(pos)) // 8192)
+    for trial in range(60):
+        q_len, q_start, kv_len = random_batch(rng, rng.randint(1, 20), G)
+        if trial % 2:
+            q_start = [s + rng.choice((0, 8185, 16380, 40000, 120000)) for s in q_start]
+            kv_len = [s + n for s, n in zip(q_start, q_len)]
+        bound = None
+        if trial % 3 == 0:
+            q_len, kv_len, bound = [1] * len(q_len), [s + 1 for s in q_start], max(q_start) + 1 + rng.randint(0, 100000)
+        rows, keys, merge, slots, slot_rows = plan_attention_f32(q_len, q_start, kv_len, G, window, chunk, 128, 64, bound)
+        tiled, sliced = {}, {}
+        for r, t0, _, _ in rows:
+            tiled.setdefault(r, []).append(t0)
+        for r, s, n, slot in keys:
+            sliced.setdefault(r, []).append((s, n, slot))
+        at = 0
+        for r, n_q in enumerate(q_len):
+            sizes = {keys_of(q_start[r] + i) for i in range(n_q)}
+            if r in tiled:
+                assert r not in sliced and sorted(tiled[r]) == list(range(0, n_q, 64 // G)) and (n_q * G > 16 or len(sizes) > 1)
+                continue
+            n = len(sliced[r])
+            assert sliced[r] == [(s, n, at) for s in range(n)] and len(sizes) == 1 and n_q * G <= slot_rows <= 16
+            size = sizes.pop()
+            base = first(q_start[r]) // size * size
+            assert -(-(kv_len[r] - base) // size) <= n <= 66
+            assert ((r, 0, n, at) in merge) == (n > 1)
+            at += n
+        assert at == slots
+
+
+@pytest.mark.parametrize("bound", (131072, 340000))
+def test_float32_decode_graphs_stay_small(bound):
+    """A decode graph's lists are made for the longest context: blocks and partial results per request are bounded all the same."""
+    R, G, nkv, hd = 64, 4, 8, 128
+    rows, keys, merge, slots, slot_rows = plan_attention_f32([1] * R, [700] * R, [701] * R, G, None, None, 128, 64, bound)
+    assert not rows and len(keys) == slots == 64 * R and slot_rows == G
+    assert 4 * slots * nkv * slot_rows * (hd + 2) <= 70e6

@@ -191,6 +191,28 @@ def test_tiled_attention(ops, nh, nkv, hd, page, window, chunk):
     assert float((out - general).abs().max()) <= 2e-5 * float(general.abs().max())
 
 
+@pytest.mark.parametrize("window,chunk", [(None, None), (9000, None), (None, 8500), (8193, 16500)])
+def test_slices_that_grow_with_the_context(ops, window, chunk):
+    """Beyond 64 slices of 128 keys a row's slices get longer: the same bits in a portion, in a few tokens and by itself, on both sides
+    of the place where they do."""
+    nh, nkv, hd, page = 4, 2, 16, 32
+    q_lens, kv_lens = [40, 3, 1, 90], [8212, 8194, 16385, 17020]
+    q, kp, vp, table, _ = paged_case(q_lens, kv_lens, nh, nkv, hd, page, torch.float32, seed=7)
+    batch = FakeBatch(q_lens, kv_lens)
+    out = ops.attention_f32(q, kp, vp, batch, table, nh, window, hd ** -0.5, chunk)
+    general = ops.attention_simt(q, kp, vp, batch.positions, batch.req_of_token, table, nh, window, hd ** -0.5, chunk=chunk)
+    assert float((out - general).abs().max()) <= 2e-5 * float(general.abs().max())      # (see test_tiled_attention)
+    for r, at, places in ((0, 0, (0, 18, 19, 20, 21, 39)), (1, 40, (0, 1, 2)), (3, 44, (0, 24, 55, 56, 68, 89))):
+        for i in places:
+            for n in (1, 2):
+                if i + n > q_lens[r]:
+                    continue
+                alone = FakeBatch([n], [kv_lens[r] - q_lens[r] + i + n], 131072 if n == 1 else None)
+                rows = slice(at + i, at + i + n)
+                assert torch.equal(ops.attention_f32(q[rows].contiguous(), kp, vp, alone, table[r:r + 1].contiguous(), nh, window, hd ** -0.5,
+                                                     chunk), out[rows])
+
+
 @pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 16), (8, 2, 128), (3, 1, 132)])
 @pytest.mark.parametrize("window,chunk", [(None, None), (40, None), (None, 64)])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
