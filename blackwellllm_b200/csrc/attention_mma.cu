@@ -64,7 +64,6 @@ struct Params {
     // own position writes the rotated key and the value to the cache.  Every request has one token.
     const float* qkv; long long qkv_plane_stride; const float* rope_table;
     int qkv_planes, rd, append;
-    int late_wait;                // attn_keys_tma_kernel: run beside the kernel before (see there)
     bw::DiffHeads diff;           // diff.lam != null: pairs of query heads become one head (G even; the gate has one number per head)
 };
 
@@ -764,10 +763,6 @@ __device__ __forceinline__ void rows_from_qkv(const Params& p, int tok, int g, i
 // Warp 0 issues the boxes of the next tile while all four warps work on the current one.  (A
 // separate producer warp with deeper stages was measured slower: its registers cost the third
 // CTA per SM, and this kernel lives on the number of warps in flight.)
-// late_wait: the kernel before is the prompt portions' attention of the same step (attention_tc.cu, `beside`), which lets this one
-// start only after its own wait for the kernels before it: queries, keys and values are complete then, the two write different rows,
-// and this one waits for it at its end instead, so that whoever waits for this kernel waits for both.  A step of 31 decoding
-// requests at 512 to 4,096 keys beside a portion of 617 tokens (28 heads of 128): 12.31 ms before, 12.15 so.
 __global__ void __launch_bounds__(THREADS)
 attn_keys_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, Params p) {
     BW_PDL_TRIGGER();
@@ -838,7 +833,7 @@ attn_keys_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     // a first tile that holds none of this step's tokens is requested before the wait
     const bool early = t_lo <= t_hi && t_lo * BN + BN <= q_pos0;
     if (early && warp == 0) { lookup(t_lo); issue_tile(0); lookup(t_lo + 1); }
-    if (!p.late_wait) BW_PDL_WAIT();
+    BW_PDL_WAIT();
     // from the unsummed q/k/v product: the slice that holds the token's own position (one per request and
     // kv head, never empty) also makes the token's key and value and puts them into its tile below
     const int t_own = last_pos / BN;
@@ -897,7 +892,6 @@ attn_keys_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     }
     __syncthreads();
     finish_keys(p, st, o, smem, r, g, slice, n_slices, item, n_rows);
-    if (p.late_wait) BW_PDL_WAIT();
 }
 #endif  // HEAD_DIM % 64 == 0
 
@@ -1140,8 +1134,6 @@ BW_EXPORT int bw_attention_head_dim() { return HD; }
 // (bw::DiffHeads: one float32 number on the device, diff_eps, diff_scale, diff_dv; no sink); out is then [tokens, nh / 2 * HD].
 // qkv only where the TMA key-slice kernel runs (head size a multiple of 64, pages of 8 to 64 tokens);
 // BW_ERR_UNSUPPORTED otherwise, and nothing was launched.
-// beside_rows != 0: the launch before on this stream was bw_attention_tc with beside_keys for the same step; the TMA key-slice kernel
-// runs beside it.
 BW_EXPORT int bw_attention_mma(const void* q, const void* k_pages, const void* v_pages, void* out, const int* cu_q,
                                const int* q_start, const int* kv_len, const int* block_table, int max_blocks,
                                const int* rows_work, int n_rows_items, const int* keys_work, int n_keys_items,
@@ -1150,7 +1142,7 @@ BW_EXPORT int bw_attention_mma(const void* q, const void* k_pages, const void* v
                                const float* qkv, int qkv_planes, long long qkv_plane_stride, const float* rope_table,
                                int rd, int append, int merge_max_slices, const float* sink, const float* gate, long long gate_ld,
                                int gate_dv, const float* dist, int keep_first, float softcap, const float* rel, int rel_len,
-                               const float* lam, float diff_eps, float diff_scale, int diff_dv, int beside_rows, void* stream) {
+                               const float* lam, float diff_eps, float diff_scale, int diff_dv, void* stream) {
     if (nkv <= 0 || nh % nkv != 0) return BW_ERR_BAD_ARG;
     if ((rel && rel_len <= 0) || ((rel || softcap > 0.f) && (dist || qkv))) return BW_ERR_UNSUPPORTED;
     const int G = nh / nkv;
@@ -1185,7 +1177,6 @@ BW_EXPORT int bw_attention_mma(const void* q, const void* k_pages, const void* v
     p.gate = gate; p.gate_ld = gate_ld; p.gate_dv = gate_dv;
     p.qkv = qkv; p.qkv_plane_stride = qkv_plane_stride; p.rope_table = rope_table;
     p.qkv_planes = qkv_planes; p.rd = rd; p.append = append;
-    p.late_wait = beside_rows && n_rows_items == 0;
     if (n_rows_items > 0) {
         p.work = rows_work;
         bw::launch((attn_rows_kernel), dim3(dim3(n_rows_items, nkv)), dim3(THREADS), SMEM_ROWS, s, p, 64 / G);

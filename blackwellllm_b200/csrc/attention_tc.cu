@@ -66,7 +66,6 @@ struct Params {
     // softcap > 0: the scaled score s becomes softcap * tanh(s / softcap) before a bias is added.  rel != null: float32
     // [nh][rel_len], rel[query head][min(i - j, rel_len - 1)] is added to the score.  (Not together with dist.)
     float softcap; const float* rel; int rel_len;
-    int beside;           // the next launch may run beside this one (it waits for this one at its end): it may start once the kernels before are done
     bw::DiffHeads diff;   // diff.lam != null: pairs of query heads become one head (G even; the gate has one number per head)
 };
 
@@ -102,7 +101,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 __global__ void __launch_bounds__(HD <= 128 ? 256 : THREADS, HD <= 128 ? 2 : 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, Params p) {
-    if (!p.beside) BW_PDL_TRIGGER();
+    BW_PDL_TRIGGER();
     extern __shared__ __align__(1024) uint8_t smem[];   // the swizzled tiles need 1024-byte alignment
     uint8_t* q_s = smem;
     uint8_t* k_s = q_s + Q_BYTES;                 // [STAGES][KV_BYTES]
@@ -132,7 +131,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     __syncthreads();
     bw::tc_fence_after();
     BW_PDL_WAIT();   // queries, keys and values of this step come from the kernels before
-    if (p.beside) BW_PDL_TRIGGER();
     const uint32_t tmem_base = *tmem_slot;
     const bool dead = tmem_slot[1] != 0;
     const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + 128;   // S buffer b at tmem_S + 64 b
@@ -553,13 +551,12 @@ BW_EXPORT int bw_attention_tc_supported(int nh, int nkv, int page_size) {
 // a tile holds 128 / G tokens.  q, out: [T, nh * HD] bf16; pages: [num_pages, nkv, page_size, HD] bf16.
 // dist: float32 [2][nh] or null; keep_first: see Params.  softcap (> 0: on), rel, rel_len: see Params.  lam != null: pairs of query heads
 // become one (bw::DiffHeads: one float32 number on the device, diff_eps, diff_scale, diff_dv); out is then [T, nh / 2 * HD].
-// beside_keys != 0: the next launch is bw_attention_mma with beside_rows for the same step's decoding requests.
 BW_EXPORT int bw_attention_tc(const void* q, const void* k_pages, const void* v_pages, void* out, const int* cu_q,
                               const int* q_start, const int* kv_len, const int* block_table, int max_blocks,
                               const int* work, int n_items, int T, int nh, int nkv, int page_size, int num_pages,
                               int window, int chunk, float scale, const float* sink, const float* gate, long long gate_ld,
                               int gate_dv, const float* dist, int keep_first, float softcap, const float* rel, int rel_len,
-                              const float* lam, float diff_eps, float diff_scale, int diff_dv, int beside_keys, void* stream) {
+                              const float* lam, float diff_eps, float diff_scale, int diff_dv, void* stream) {
     if (n_items <= 0) return 0;
     if ((rel && rel_len <= 0) || ((rel || softcap > 0.f) && dist)) return BW_ERR_UNSUPPORTED;
     if (!bw_attention_tc_supported(nh, nkv, page_size) || !(scale > 0.f)) return BW_ERR_UNSUPPORTED;
@@ -586,7 +583,6 @@ BW_EXPORT int bw_attention_tc(const void* q, const void* k_pages, const void* v_
     p.window = window > 0 ? window : 0; p.chunk = chunk > 0 ? chunk : 0; p.tpt = tpt;
     p.scale_log2 = scale * 1.4426950408889634f;
     p.sink = sink;
-    p.beside = beside_keys;
     if (lam && (G % 2 || sink || diff_dv <= 0 || diff_dv > HD || (gate && gate_dv >= 0))) return BW_ERR_BAD_ARG;
     p.diff.lam = lam; p.diff.eps = diff_eps; p.diff.scale = diff_scale; p.diff.dv = diff_dv;
     if (gate && gate_dv < 0 ? (-gate_dv > HD || gate_ld < (long long)(lam ? nh / 2 : nh))

@@ -1040,7 +1040,7 @@ def paged_attention(q, k_pages: torch.Tensor, v_pages: torch.Tensor, batch,
 _ATTN_MMA_ARGS = [c_void_p] * 8 + [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,
                                    c_int, c_int, c_int, c_int, c_int, c_int, c_float,
                                    c_void_p, c_int, c_ll, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_ll, c_int,
-                                   c_void_p, c_int, c_float, c_void_p, c_int, c_void_p, c_float, c_float, c_int, c_int, c_void_p]
+                                   c_void_p, c_int, c_float, c_void_p, c_int, c_void_p, c_float, c_float, c_int, c_void_p]
 
 
 _sm_counts = {}
@@ -1180,15 +1180,13 @@ def attention_mma(q, k_pages: torch.Tensor, v_pages: torch.Tensor, batch, block_
         part_ml = torch.empty((slices * nkv * 16, 2), dtype=torch.float32, device=out.device)
     if raw is not None and n_rows:
         raise KernelError("attention: unrotated q/k/v only with one token per request")
-    # decoding requests beside prompt portions: their TMA kernel (which kept first keys do not take) runs beside the portions'
-    beside = int(bool(use_tc and n_rows and n_keys and not keep_first))
     if use_tc and n_rows:
         tc = _fn("attention_tc", "bw_attention_tc", _ATTN_TC_ARGS, macros=attention_tc_macros(hd))
         _check(tc(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(batch.cu_q), _ptr(batch.q_start),
                   _ptr(batch.kv_len), _ptr(block_table), block_table.shape[1], _ptr(rows_w), n_rows, q.shape[0],
                   nh, nkv, page_size, num_pages, int(window or 0), int(chunk or 0), float(scale), _ptr(sink), _ptr(g), g_ld, g_dv,
                   _ptr(dist), keep_first, float(softcap or 0.0), _ptr(rel), rel_len, _ptr(lam), float(d_eps), float(d_scale), int(d_dv),
-                  beside, _stream()), "attention_tc")
+                  _stream()), "attention_tc")
         n_rows = 0
         if not n_keys:
             return out
@@ -1201,13 +1199,13 @@ def attention_mma(q, k_pages: torch.Tensor, v_pages: torch.Tensor, batch, block_
               raw.planes.stride(0) if raw is not None else 0, _ptr(raw.table if raw is not None else None),
               raw.rotary_dim if raw is not None else 0, int(raw.append) if raw is not None else 0, merge_max,
               _ptr(sink), _ptr(g), g_ld, g_dv, _ptr(dist), keep_first, float(softcap or 0.0), _ptr(rel), rel_len,
-              _ptr(lam), float(d_eps), float(d_scale), int(d_dv), beside, _stream()), "attention_mma")
+              _ptr(lam), float(d_eps), float(d_scale), int(d_dv), _stream()), "attention_mma")
     return out
 
 
 _ATTN_TC_ARGS = [c_void_p] * 8 + [c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
                                   c_void_p, c_ll, c_int, c_void_p, c_int, c_float, c_void_p, c_int, c_void_p, c_float, c_float, c_int,
-                                  c_int, c_void_p]
+                                  c_void_p]
 
 
 def attention_tc_supports(hd: int, G: int, page_size: int) -> bool:
