@@ -1,4 +1,4 @@
-// Token choice from float32 logits [R, V], a cluster of 8 blocks per row.
+// Token choice from float32 logits [R, V], a cluster of 8 blocks per row, or one block for short rows and for many.
 //
 //  * temperature <= 0: argmax, the lowest index winning a tie.
 //  * temperature  > 0: softmax(logits / temperature) in float32; optional nucleus
@@ -19,7 +19,7 @@ typedef unsigned long long u64;
 
 constexpr int THREADS = 1024;
 constexpr int WARPS = THREADS / 32;
-constexpr int CLUSTER = 8;          // blocks of a row
+constexpr int ROW_BLOCKS = 8;       // blocks of a row, a cluster
 constexpr int BINS = 1024;          // one per thread: ten bits of a weight's float pattern at a time
 
 __device__ __forceinline__ void argmax_pair(float& v, int& i, float ov, int oi) {
@@ -49,7 +49,7 @@ __device__ __forceinline__ void hist_add(Hist& h, unsigned bin, u64 q) {
     if (up) atomicAdd(&h.hi[bin], up);
 }
 
-// One row per cluster.  The weights e = exp((x - max) / T) are made once and stay in registers (NV a thread; NV = 0: a row too
+// One row per cluster (of CLUSTER blocks).  The weights e = exp((x - max) / T) are made once and stay in registers (NV a thread; NV = 0: a row too
 // long for that is read again for every pass) or, with more rows than clusters that fit at one block an SM, in shared memory (IN_SMEM:
 // two blocks an SM at 32 registers a thread).  Masses are integers, e * 2^shift rounded (`scale` = 2^shift, shift at most 45 and
 // such that a row's mass fits 62 bits): their sums are exact in any order, so the blocks of a row may add them as they come.
@@ -59,8 +59,8 @@ __device__ __forceinline__ void hist_add(Hist& h, unsigned bin, u64 q) {
 // What bounds it: latency (five cluster barriers, three histogram passes); a row of 128,256 is 0.5 MB.  Measured, temperature 0.6,
 // top_p 0.9: a row of 128,256 in 26 us, 32 rows of 152,064 in 63 us (79 in registers; one block per row and the bisection: 728 and
 // 1,162 us).
-template <int NV, bool IN_SMEM = false>
-__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(THREADS, IN_SMEM ? 2 : 1)
+template <int NV, bool IN_SMEM = false, int CLUSTER = ROW_BLOCKS>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(THREADS, IN_SMEM || (NV == 0 && CLUSTER == 1) ? 2 : 1)
 sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
               const float* __restrict__ top_p, const float* __restrict__ u, int* __restrict__ out,
               int V, size_t ld, float scale) {
@@ -325,12 +325,25 @@ BW_EXPORT int bw_sample(const float* logits, const float* temperature, const flo
     int bits = 0;
     while ((1ll << bits) < V) ++bits;
     const float scale = (float)(1ull << (62 - bits < 45 ? 62 - bits : 45));
+    const dim3 block(THREADS);
+    // One block a row where that is faster: a row that fits a block's registers (64 rows of 5,000: nucleus 14 us, 69 on clusters; alone
+    // 13 and 20), or so many rows that their clusters take turns for longer than a block walks its row (greedy / temperature / nucleus,
+    // on clusters and in blocks: 64 rows of 32,000 13 / 19 / 75 and 9 / 27 / 63, 128 of 64,000 24 / 47 / 158 and 16 / 55 / 137, 256 of
+    // 128,256 72 / 168 / 404 and 70 / 157 / 366; of 256,000, which a cluster's registers do not hold, 356 / 479 / 1,180 and
+    // 128 / 323 / 717).
+    const int many = V > 160 * 1024 ? 100 : V / (!temperature && V <= 64 * 1024 ? 870 : 500);
+    if (V <= 8 * THREADS || R > many) {
+        const auto kernel = V <= 8 * THREADS && (temperature || R <= bw::num_sms()) ? sample_kernel<8, false, 1> : sample_kernel<0, false, 1>;
+        bw::launch(kernel, dim3((unsigned)R), block, 0, (cudaStream_t)stream, logits, temperature, top_p, u, out, V, (size_t)ld, scale);
+        BW_LAUNCH_CHECK();
+        return 0;
+    }
     // tokens of a thread: its warp's share of the block's share of the row, in rows of 32
-    const int per_block = (V + CLUSTER - 1) / CLUSTER;
+    const int per_block = (V + ROW_BLOCKS - 1) / ROW_BLOCKS;
     const int iters = ((per_block + WARPS - 1) / WARPS + 31) / 32;
-    const dim3 grid((unsigned)R * CLUSTER), block(THREADS);
+    const dim3 grid((unsigned)R * ROW_BLOCKS);
     // more rows than clusters at one block an SM: two blocks an SM, weights in shared memory (19 rows of 152,064 61 us, 32 63 us; in registers 79)
-    const int at_once = bw::num_sms() / CLUSTER;
+    const int at_once = bw::num_sms() / ROW_BLOCKS;
     const size_t kept = (size_t)iters * 32 * WARPS * sizeof(float);
     if (temperature && R > at_once && kept <= 80 * 1024) {      // (two blocks and their histograms in an SM's shared memory)
         static bool done[bw::MAX_DEVICES] = {};
@@ -340,7 +353,8 @@ BW_EXPORT int bw_sample(const float* logits, const float* temperature, const flo
         return 0;
     }
 #define BW_SAMPLE(NV) bw::launch(sample_kernel<NV>, grid, block, 0, (cudaStream_t)stream, logits, temperature, top_p, u, out, V, (size_t)ld, scale)
-    // registers for 8 tokens a thread (rows up to 65,536) or 20 (up to 163,840: 64 registers a thread allow no more)
+    // registers for 8 tokens a thread (rows up to 65,536) or 20 (up to 163,840: 64 registers a thread allow no more); longer rows are
+    // read again for every pass (a row of 200,000 in 54 us, 32 rows in 146)
     if (iters <= 8) BW_SAMPLE(8);
     else if (iters <= 20) BW_SAMPLE(20);
     else BW_SAMPLE(0);

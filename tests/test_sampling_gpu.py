@@ -74,3 +74,19 @@ def test_ties_masks_and_rows_without_a_weight(V):
     got = ops.sample(rows.to(DEV), torch.ones(2, device=DEV), torch.tensor([0.01, 1.0], device=DEV),
                      torch.tensor([0.9999, 0.9999], device=DEV)).tolist()
     assert all(abs(i - 0.9999 * V) <= 0.0001 * V + 2 for i in got)
+
+
+# rows short enough for one block, and numbers of rows from which one block a row is the faster form, beside the same rows a few at a
+# time on clusters: masses are whole numbers, so both forms choose the same tokens
+@pytest.mark.parametrize("R,V", [(3, 31), (40, 300), (5, 8192), (5, 8193), (45, 16001), (70, 32000), (140, 60000), (260, 128256), (105, 170001)])
+def test_rows_choose_the_same_token_in_every_form(R, V):
+    from blackwellllm_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = torch.randn(R, V, device="cuda", generator=g) * 2
+    x[0], x[1, V // 2:] = 1.0, float("-inf")
+    x[2, V - 1] = 30.0
+    u, one = torch.rand(R, device="cuda", generator=g), torch.ones(R, device="cuda")
+    for args in ((None, None, None), (0.6 * one, None, u), (0.9 * one, 0.9 * one, u), (torch.where(u < 0.5, 0.0, 1.0), 0.3 * one, u)):
+        whole = ops.sample(x, *args)
+        for at in range(0, R, 9):
+            assert torch.equal(ops.sample(x[at:at + 9], *(a[at:at + 9] if a is not None else None for a in args)), whole[at:at + 9])
