@@ -109,7 +109,10 @@ __device__ __forceinline__ void put2(bf16* p, float a, float b) { *reinterpret_c
 // values of this step) and lam = *v_lam a number on the device.  q_head_mult != null: every query head is multiplied by its
 // own number (float32 [nh]).  v_col: the column where the values' heads begin (behind the keys, or the keys' own columns:
 // values that are the key projection before norm and rotation).  v_scale multiplies the values last of all.
-template <typename OT>
+// FEW: a few tokens, all latency: gains and angles are loaded with the rows they scale.  With many tokens their registers cost more
+// warps in flight than the round of loads gains (2,048 tokens of 16 + 4 heads of 128: 27.2 us
+// early, 21.6 late; 296 tokens 4.3 and 4.9).
+template <typename OT, bool FEW>
 __global__ void __launch_bounds__(256)
 head_norm_rope_kernel(const float* __restrict__ qkv, long long ld, const int* __restrict__ positions,
                       const int* __restrict__ req_of_token, const int* __restrict__ block_table, int max_blocks,
@@ -172,15 +175,17 @@ head_norm_rope_kernel(const float* __restrict__ qkv, long long ld, const int* __
             // partners in registers, so a head is read once
             float2 a[2], b[2], q[4], ga[2], gb[2], cs[2], sn[2];
             float ss = 0.f;
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {      // (gains and angles with them: one round of loads)
+            auto scales = [&](int i) {
                 const int c = i * 64 + lane * 2;
-                a[i] = b[i] = cs[i] = sn[i] = make_float2(0.f, 0.f);
-                ga[i] = gb[i] = make_float2(1.f, 1.f);
-                if (c < half) {
-                    cs[i] = *reinterpret_cast<const float2*>(tab + c); sn[i] = *reinterpret_cast<const float2*>(tab + half + c);
-                    if (gain) { ga[i] = *reinterpret_cast<const float2*>(gain + c); gb[i] = *reinterpret_cast<const float2*>(gain + half + c); }
-                }
+                cs[i] = *reinterpret_cast<const float2*>(tab + c); sn[i] = *reinterpret_cast<const float2*>(tab + half + c);
+                ga[i] = gain ? *reinterpret_cast<const float2*>(gain + c) : make_float2(1.f, 1.f);
+                gb[i] = gain ? *reinterpret_cast<const float2*>(gain + half + c) : make_float2(1.f, 1.f);
+            };
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int c = i * 64 + lane * 2;
+                a[i] = b[i] = make_float2(0.f, 0.f);
+                if (FEW && c < half) scales(i);
                 if (c < half) { a[i] = *reinterpret_cast<const float2*>(src + c); b[i] = *reinterpret_cast<const float2*>(src + half + c); }
                 ss = fmaf(a[i].x, a[i].x, ss); ss = fmaf(a[i].y, a[i].y, ss); ss = fmaf(b[i].x, b[i].x, ss); ss = fmaf(b[i].y, b[i].y, ss);
             }
@@ -195,6 +200,7 @@ head_norm_rope_kernel(const float* __restrict__ qkv, long long ld, const int* __
             for (int i = 0; i < 2; ++i) {
                 const int c = i * 64 + lane * 2;
                 if (c < half) {
+                    if (!FEW) scales(i);
                     const float x0 = a[i].x * r2 * ga[i].x, x1 = a[i].y * r2 * ga[i].y, y0 = b[i].x * r2 * gb[i].x, y1 = b[i].y * r2 * gb[i].y;
                     put2(dst + c, x0 * cs[i].x - y0 * sn[i].x, x1 * cs[i].y - y1 * sn[i].y);
                     put2(dst + half + c, y0 * cs[i].x + x0 * sn[i].x, y1 * cs[i].y + x1 * sn[i].y);
@@ -323,7 +329,7 @@ BW_EXPORT int bw_head_norm_rope_append(const float* qkv, long long ld, const int
     // few tokens: a warp per head where the SMs allow it (8 tokens of 24 heads: 7 us with one block a token, three rounds of heads)
     const int heads = nh + (has_kv ? nkv : 0), spare = 2 * bw::num_sms() / T, rounds = (heads + 7) / 8;
     const int per_token = spare < 1 ? 1 : spare < rounds ? spare : rounds;
-#define BW_HN(OT) bw::launch((head_norm_rope_kernel<OT>), dim3(T, per_token), dim3(256), 0, s, qkv, ld, positions, req_of_token, block_table, \
+#define BW_HN(OT) bw::launch((spare ? head_norm_rope_kernel<OT, true> : head_norm_rope_kernel<OT, false>), dim3(T, per_token), dim3(256), 0, s, qkv, ld, positions, req_of_token, block_table, \
         max_blocks, table, rotary_dim, interleaved, q_gain, k_gain, eps, q_coef, q_every, (OT*)q_out, (OT*)k_pages, (OT*)v_pages, \
         nh, nkv, dq, dv, dpad, page_size, num_pages, has_kv, vec, vec2, pairs, vec_v, v_eps, v_first, v_first_ld, v_lam, \
         q_head_mult, v_col, v_scale)
