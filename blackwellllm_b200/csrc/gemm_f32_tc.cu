@@ -102,17 +102,18 @@ struct Cut {
         return false;
     }
 };
-// One CTA's items: for every tile of tokens, its range's piece of every tile of features.
+// One CTA's items: for every tile of tokens that is its own (a weight of fewer ranges than SMs has them dealt out, blockIdx.y), its
+// range's piece of every tile of features.
 struct Items {
     Cut cut;
     int tiles_m, mt;
     int lo, hi, at;
     int tile, kb0, n;        // the item: tile of features, first stage, stages (tile of tokens: mt)
-    __device__ Items(const Cut& c, int tiles_m_) : cut(c), tiles_m(tiles_m_), mt(0) {
+    __device__ Items(const Cut& c, int tiles_m_) : cut(c), tiles_m(tiles_m_), mt(blockIdx.y) {
         lo = (int)cut.begin(blockIdx.x); hi = (int)cut.begin(blockIdx.x + 1); at = lo;
     }
     __device__ bool next() {
-        if (at >= hi) { at = lo; ++mt; }
+        if (at >= hi) { at = lo; mt += gridDim.y; }
         if (mt >= tiles_m || lo >= hi) return false;
         tile = at / cut.kb_total;
         kb0 = at - tile * cut.kb_total;
@@ -276,7 +277,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         }
     } else if (warp >= 4 && warp < 4 + 4 * SPLIT_GROUPS) {
         const int quarter = warp & 3, row = quarter * 32 + lane;
-        const long long all = (cut.begin(blockIdx.x + 1) - cut.begin(blockIdx.x)) * tiles_m;      // stages of all items
+        const int mine = (tiles_m - (int)blockIdx.y + (int)gridDim.y - 1) / (int)gridDim.y;            // tiles of tokens
+        const long long all = (cut.begin(blockIdx.x + 1) - cut.begin(blockIdx.x)) * mine;         // stages of all items
         const uint32_t tmem_a = tmem + 3 * acc_cols(bn) + ((uint32_t)(quarter * 32) << 16);
         const int group = (warp - 4) / 4;
         int s = group, ph = 0, slot = group, tph = 1;
@@ -478,7 +480,10 @@ BW_EXPORT int bw_gemm_f32_tc(const float* x, const float* w, const void* bias, i
     const cudaError_t e = bw::allow_dynamic_smem(gemm_f32_tc_kernel, SMEM_BUDGET + 1024, done);
     if (e != cudaSuccess) return (int)e;
     const Out o = {out, bias, part, x, w, ldo, ldx, bias_type, accumulate, M, N, K};
-    bw::launch(gemm_f32_tc_kernel, dim3(cut.ctas), dim3(THREADS), (size_t)ring_bytes(bn) + 1024, s, tm_w, tm_x, o, bn, cut,
+    // a small weight's ranges leave SMs idle: they take tiles of tokens (300 tokens x 1024 x 256: 23.6 us without, 11.2
+    // so, 17.4 in gemm_simt.cu; 1,000 tokens: 62.6 with launches of 512, 12.1 so, 27.0)
+    const int rows = bw::num_sms() / cut.ctas < tiles_m ? bw::num_sms() / cut.ctas : tiles_m;
+    bw::launch(gemm_f32_tc_kernel, dim3(cut.ctas, rows < 1 ? 1 : rows), dim3(THREADS), (size_t)ring_bytes(bn) + 1024, s, tm_w, tm_x, o, bn, cut,
                tiles_m);
     BW_LAUNCH_CHECK();
     if (shared) {

@@ -8,7 +8,7 @@ from __future__ import annotations
 import ctypes
 import math
 import os
-from typing import List, Optional
+from typing import List, Optional, Tuple
 
 import torch
 
@@ -484,7 +484,6 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = N
 # ------------------------------------------------------------------ attention
 
 _GEMM_F32_TC_ARGS = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_int, c_void_p, c_void_p, c_ll, c_void_p]
-_GEMM_F32_TOKENS = 512       # tokens of one launch: the pieces of shared tiles stay below 80 MB on 148 SMs, whatever the weight's size
 
 
 def gemm_f32_tc_supports(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -494,9 +493,12 @@ def gemm_f32_tc_supports(x: torch.Tensor, w: torch.Tensor) -> bool:
             and x.dim() == 2 and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
-def gemm_f32_part_floats(N: int, K: int) -> int:
-    """The scratch of a split product per token on the current device, in floats."""
-    return _fn("gemm_f32_tc", "bw_gemm_f32_tc_part_floats", [c_int, c_int])(N, K)
+def gemm_f32_scratch(N: int, K: int) -> Tuple[int, int]:
+    """The scratch of a split product's shared tiles per token on the current device, in floats, and the tokens of one launch: 512, or
+    more of a small weight, as long as that scratch stays below 80 MB and the tokens' parts below 64."""
+    floats = _fn("gemm_f32_tc", "bw_gemm_f32_tc_part_floats", [c_int, c_int])(N, K)
+    most = min(20_000_000 // floats if floats else 65535, 8_000_000 // K, 65535)
+    return floats, max(512, most // 128 * 128)
 
 
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
@@ -520,13 +522,14 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = No
         _dev(bias, "bias")
         if bias.numel() != N:
             raise KernelError("gemm: bias must have N entries")
-    most = min(M, _GEMM_F32_TOKENS)
-    split = torch.empty((2 * most * K,), dtype=torch.float32, device=x.device)
-    floats = most * gemm_f32_part_floats(N, K)
+    floats, most = gemm_f32_scratch(N, K)
+    tokens = min(M, most)
+    floats *= tokens
+    split = torch.empty((2 * tokens * K,), dtype=torch.float32, device=x.device)
     part = torch.empty((floats,), dtype=torch.float32, device=x.device) if floats else None
     fn = _fn("gemm_f32_tc", "bw_gemm_f32_tc", _GEMM_F32_TC_ARGS, tag=f"{M}x{N}x{K}")
-    for at in range(0, M, _GEMM_F32_TOKENS):
-        n = min(_GEMM_F32_TOKENS, M - at)
+    for at in range(0, M, most):
+        n = min(most, M - at)
         _check(fn(_ptr(x[at:]), _ptr(w), _ptr(bias), _code(bias, "bias") if bias is not None else 0, _ptr(out[at:]), n, N, K, x.stride(0),
                   out.stride(0), int(accumulate), _ptr(split), _ptr(part), floats, _stream()), "gemm_f32_tc")
     return out

@@ -52,7 +52,7 @@ def test_split_products(ops, M, N, K):
         assert torch.equal(ops.gemm_f32(x[rows], w), plain[rows])
 
 
-@pytest.mark.parametrize("M,N,K", [(301, 6144, 4096), (301, 4096, 4096), (128, 4096, 2048), (17, 6144, 4096)])
+@pytest.mark.parametrize("M,N,K", [(301, 6144, 4096), (301, 4096, 4096), (128, 4096, 2048), (17, 6144, 4096), (1500, 1024, 512)])
 def test_queued_products_repeat_themselves(ops, M, N, K):
     """Products right behind other kernels, nothing waited for in between: every one the bits of the same product by itself.  (The
     product's blocks start beside those of the kernels before, whose memory traffic holds up their reads of shared memory.)"""
