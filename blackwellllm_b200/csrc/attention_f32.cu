@@ -61,7 +61,7 @@ __device__ __forceinline__ int slices_of(int base, int end, int keys) { return (
 // SLICES: work items (request, slice, slices, first slot), all tokens of the request's segment, whose slices are of one size; else (request, first token).
 // CH: groups of four channels of a lane.
 template <int ROWS, int CH, bool SLICES>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, SLICES ? 3 : 1)
 attention_f32_kernel(Params p, const int4* __restrict__ work) {
     BW_PDL_TRIGGER();
     extern __shared__ float4 smem4[];
@@ -89,10 +89,9 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
     const bool same = !SLICES && slice_keys(p, end - 1) == keys && (p.chunk <= 0 || p.chunk <= SLICE * MOST);
     BW_PDL_WAIT();
 
-    for (int i = warp; i < ROWS; i += WARPS) {      // rows beyond the tile's are zeros
-        const float* src = p.q + ((size_t)(row0 + t0 + i / G) * p.nh + (size_t)kvh * G + i % G) * hd;
-        for (int c = lane * 4; c < hd; c += 128)
-            *reinterpret_cast<float4*>(qs + i * ldk + c) = i < rows ? *reinterpret_cast<const float4*>(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = warp; i < ROWS; i += WARPS) {      // with the first tile of keys; rows beyond the tile's are zeros
+        const float* src = p.q + (i < rows ? ((size_t)(row0 + t0 + i / G) * p.nh + (size_t)kvh * G + i % G) * hd : 0);
+        for (int c = lane * 4; c < hd; c += 128) copy16(qs + i * ldk + c, src + c, i < rows);
     }
     auto fetch = [&](int tile) {                    // a warp brings four keys and their values
         const int st = tile & 1;
@@ -169,18 +168,24 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
             }
         }
         __syncthreads();
+        // (a warp's rows side by side: one after another their shuffles and exponentials are the kernel's latency at few keys)
+        float sc[RW], m_new[RW], e[RW], sum[RW];
         bool zero = false;
 #pragma unroll
+        for (int i = 0; i < RW; ++i) sc[i] = ps[(warp * RW + i) * LDP + lane];
+#pragma unroll
+        for (int i = 0; i < RW; ++i) m_new[i] = fmaxf(m[i], bw::warp_max(sc[i]));
+#pragma unroll
+        for (int i = 0; i < RW; ++i) e[i] = sc[i] == -INFINITY ? 0.f : expf(sc[i] - m_new[i]);
+#pragma unroll
+        for (int i = 0; i < RW; ++i) sum[i] = bw::warp_sum(e[i]);
+#pragma unroll
         for (int i = 0; i < RW; ++i) {
-            float* pr = ps + (warp * RW + i) * LDP;
-            const float sc = pr[lane];
-            const float m_new = fmaxf(m[i], bw::warp_max(sc));
-            const float corr = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
-            const float e = sc == -INFINITY ? 0.f : expf(sc - m_new);
-            l[i] = l[i] * corr + bw::warp_sum(e);
-            m[i] = m_new;
-            pr[lane] = e;
-            zero |= e == 0.f && warp * RW + i < rows;
+            const float corr = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new[i]);
+            l[i] = l[i] * corr + sum[i];
+            m[i] = m_new[i];
+            ps[(warp * RW + i) * LDP + lane] = e[i];
+            zero |= e[i] == 0.f && warp * RW + i < rows;
 #pragma unroll
             for (int c = 0; c < CH * 4; ++c) o[i][c] *= corr;
         }
