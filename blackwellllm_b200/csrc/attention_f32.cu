@@ -5,15 +5,16 @@
 // A block of eight warps takes a tile of ROWS stacked query rows (token-major, then the heads of the group) of one request and
 // kv head and walks 32 keys at a time (two stages, cp.async).  Scores: each thread a few rows times a few keys.  Softmax and
 // values: warp w owns rows w ROWS / 8 on, a lane four channels (twice that for heads above 128), so probabilities pass through
-// shared memory inside the warp only.  ROWS = 64 for prompt portions, 16 for the few rows of a decoding request, whose slices of
-// keys have blocks of their own; a second kernel adds them up.
+// shared memory inside the warp only.  ROWS = 64 for prompt portions, 16 for the few rows of a decoding request.  The keys of a tile
+// are one block's, or dealt out by slices to several, whose results a second kernel adds up.
 // A row's result is the same bits whatever else is in the batch: both forms make a softmax per slice of keys, counted from position 0,
 // in the same order of operations, and fold the slices in their order (fold()).  A slice has SLICE keys, or as many times SLICE that a
 // row sees MOST slices or hardly more: what a row sees decides, and no batch.  (So a decoding request has at most MOST + 2 blocks and
 // partial results per kv head at any context: 64 requests of 8 kv heads and groups of 4 at 131,072 tokens 69 MB.)
-// What bounds it: decode, the bytes of keys and values; prompts, shared-memory reads (six 16-byte reads per 32 FMAs).  Measured at
-// head size 128, groups of 4, 8 kv heads, against attention_simt.cu (a block per token and head, a lane a key): 4 requests at
-// 1,000 keys 45 us with the merge against 347, 301 prompt tokens 84 us against 827.
+// What bounds it: decode, the bytes of keys and values; prompts, shared-memory reads (six 16-byte reads per 32 FMAs); few keys, latency.
+// Measured at head size 128, groups of 4, 8 kv heads, against attention_simt.cu (a block per token and head, a lane a key): 4 requests
+// at 1,000 keys 29 us with the merge against 167, 4 portions of 200 tokens 126 against 1,402, 9 tokens 6.1 against 9.5.  Slower than
+// that kernel is what keeps a tile's rows idle: 64 requests at 300 keys, groups of 1, 8 kv heads of 64: 92 us against 66.
 #include <type_traits>
 #include "common.cuh"
 
@@ -27,8 +28,7 @@ struct Params {
     const int *cu_q, *q_start, *block_table;
     int max_blocks, nh, nkv, hd, page_size, num_pages, window, chunk;
     float scale;
-    float *part_o, *part_ml;      // [slot][kv head][slot_rows][hd] and [..][2] (maximum, sum)
-    int slot_rows;                // stacked rows of the largest segment that is sliced
+    float *part_o, *part_ml;      // [row of a tile and slice][hd] and [..][2] (maximum, sum), see part_row()
 };
 
 __device__ __forceinline__ void copy16(float* dst, const float* src, bool valid) {
@@ -58,10 +58,16 @@ __device__ __forceinline__ int slice_keys(const Params& p, int pos) {
 __device__ __forceinline__ int slices_from(const Params& p, int pos, int keys) { return bw::first_visible(pos, p.window, p.chunk) / keys * keys; }
 __device__ __forceinline__ int slices_of(int base, int end, int keys) { return (end - base + keys - 1) / keys; }
 
-// SLICES: work items (request, slice, slices, first slot), all tokens of the request's segment, whose slices are of one size; else (request, first token).
+// Where a tile of `rows` stacked rows leaves a slice's results: `where` rows per kv head lie before its own.
+__device__ __forceinline__ size_t part_row(const Params& p, int where, int slice, int rows, int kvh) {
+    return (size_t)(where + slice * rows) * p.nkv + (size_t)kvh * rows;
+}
+
+// Work items (request, first token); SLICES: (request, first token, block | blocks << 16, where), a block of the `blocks` that share
+// the tile's slices, whose rows have slices of one size.  Of a single slice the block writes the tile's result (its fold is it).
 // CH: groups of four channels of a lane.
 template <int ROWS, int CH, bool SLICES>
-__global__ void __launch_bounds__(THREADS, SLICES ? 3 : 1)
+__global__ void __launch_bounds__(THREADS, !SLICES ? 1 : ROWS == 64 ? 2 : 3)
 attention_f32_kernel(Params p, const int4* __restrict__ work) {
     BW_PDL_TRIGGER();
     extern __shared__ float4 smem4[];
@@ -76,15 +82,22 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
     const int4 item = work[blockIdx.x];
     const int r = item.x;
     const int row0 = p.cu_q[r], q_len = p.cu_q[r + 1] - row0;
-    const int t0 = SLICES ? 0 : item.y;
+    const int t0 = item.y;
     const int tokens = min(ROWS / G, q_len - t0), rows = tokens * G;
     const int pos0 = p.q_start[r] + t0, end = pos0 + tokens;
     const int* bt = p.block_table + (size_t)r * p.max_blocks;
     const int keys = slice_keys(p, pos0), per = keys / KEYS;      // of the first row's slices: keys, tiles
     const int base = slices_from(p, pos0, SLICES ? keys : SLICE);
-    if (SLICES && item.y >= slices_of(base, end, keys)) return;   // (the list is as long as the longest context may get)
     const int all = (end - base + KEYS - 1) / KEYS;
-    const int first = SLICES ? item.y * per : 0, last = SLICES ? min(first + per, all) : all;
+    int first = 0, last = all;
+    bool whole = !SLICES;                                 // this block makes the tile's result
+    if constexpr (SLICES) {
+        const int block = item.z & 0xffff, blocks = item.z >> 16, slices = slices_of(base, end, keys), share = (slices + blocks - 1) / blocks;
+        whole = slices == 1;
+        first = block * share * per;
+        last = min(first + share * per, all);
+        if (first >= last) return;                        // (the list is as long as the longest context may get)
+    }
     // a portion's rows may differ in the size of their slices (it never shrinks, except where a block of positions begins)
     const bool same = !SLICES && slice_keys(p, end - 1) == keys && (p.chunk <= 0 || p.chunk <= SLICE * MOST);
     BW_PDL_WAIT();
@@ -220,7 +233,25 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
         };
         if (__any_sync(0xffffffffu, zero)) add_values(std::true_type{});
         else add_values(std::false_type{});
-        if constexpr (!SLICES) {
+        if constexpr (SLICES) {
+            if (!whole && ((tile + 1) % per == 0 || tile + 1 == last)) {
+                const size_t at = part_row(p, item.w, tile / per, rows, kvh);
+#pragma unroll
+                for (int i = 0; i < RW; ++i) {
+                    const int row = warp * RW + i;
+                    if (row >= rows) continue;
+                    if (lane == 0) *reinterpret_cast<float2*>(p.part_ml + 2 * (at + row)) = make_float2(m[i], l[i]);
+#pragma unroll
+                    for (int h = 0; h < CH; ++h) {
+                        const int c = lane * 4 + 128 * h;
+                        if (c < hd) *reinterpret_cast<float4*>(p.part_o + (at + row) * hd + c) = make_float4(o[i][4 * h], o[i][4 * h + 1], o[i][4 * h + 2], o[i][4 * h + 3]);
+                    }
+#pragma unroll
+                    for (int c = 0; c < CH * 4; ++c) o[i][c] = 0.f;
+                    m[i] = -INFINITY; l[i] = 0.f;
+                }
+            }
+        } else {
             const int done = base / KEYS + tile + 1;      // tiles from position 0
             if (same ? done % per == 0 || tile + 1 == last : done % (SLICE / KEYS) == 0 || tile + 1 == last) {
 #pragma unroll
@@ -235,21 +266,13 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
         }
         __syncthreads();        // (the next fetch overwrites this stage, the next scores the probabilities)
     }
+    if (!whole) return;
 #pragma unroll
     for (int i = 0; i < RW; ++i) {
         const int row = warp * RW + i;
         if (row >= rows) continue;
-        float f = 1.f;
-        float* dst;
-        if (SLICES && item.z > 1) {
-            const size_t slot = ((size_t)(item.w + item.y) * p.nkv + kvh) * p.slot_rows + row;
-            dst = p.part_o + slot * hd;
-            if (lane == 0) { p.part_ml[2 * slot] = m[i]; p.part_ml[2 * slot + 1] = l[i]; }
-        } else {
-            const float sum = SLICES ? l[i] : L[i];
-            f = sum > 0.f ? 1.f / sum : 0.f;
-            dst = p.out + ((size_t)(row0 + t0 + row / G) * p.nh + (size_t)kvh * G + row % G) * hd;
-        }
+        const float sum = SLICES ? l[i] : L[i], f = sum > 0.f ? 1.f / sum : 0.f;
+        float* dst = p.out + ((size_t)(row0 + t0 + row / G) * p.nh + (size_t)kvh * G + row % G) * hd;
         float res[CH * 4];
 #pragma unroll
         for (int c = 0; c < CH * 4; ++c) {
@@ -264,16 +287,17 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
     }
 }
 
-// Slices of one (request, kv head, row), in slice order; a thread four channels.
+// Slices of one (tile, kv head, row) of several, in slice order; a thread four channels.  Items (request, first token, rows, where).
 __global__ void __launch_bounds__(64)
 attention_f32_merge_kernel(Params p, const int4* __restrict__ work) {
     BW_PDL_TRIGGER();
     const int4 item = work[blockIdx.x];
-    const int r = item.x, kvh = blockIdx.y, row = blockIdx.z, G = p.nh / p.nkv, hd = p.hd, c = threadIdx.x * 4;
-    const int row0 = p.cu_q[r], q_len = p.cu_q[r + 1] - row0, pos0 = p.q_start[r];
-    if (row >= q_len * G || c >= hd) return;
-    const int keys = slice_keys(p, pos0), slices = slices_of(slices_from(p, pos0, keys), pos0 + q_len, keys);
-    BW_PDL_WAIT();
+    const int r = item.x, t0 = item.y, kvh = blockIdx.y, row = blockIdx.z, G = p.nh / p.nkv, hd = p.hd, c = threadIdx.x * 4;
+    const int row0 = p.cu_q[r] + t0, tokens = min(item.z / G, p.cu_q[r + 1] - row0), rows = tokens * G, pos0 = p.q_start[r] + t0;
+    if (row >= rows || c >= hd) return;
+    const int keys = slice_keys(p, pos0), slices = slices_of(slices_from(p, pos0, keys), pos0 + tokens, keys);
+    BW_PDL_WAIT();            // (also where nothing is left to do: who waits for this kernel waits for the slices')
+    if (slices == 1) return;
     float M = -INFINITY, L = 0.f, O[4] = {0.f, 0.f, 0.f, 0.f};
     constexpr int AHEAD = 8;             // slices whose loads are in flight together
     for (int s0 = 0; s0 < slices; s0 += AHEAD) {
@@ -281,9 +305,9 @@ attention_f32_merge_kernel(Params p, const int4* __restrict__ work) {
         float2 ml[AHEAD];
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i) {
-            const size_t slot = ((size_t)(item.w + min(s0 + i, slices - 1)) * p.nkv + kvh) * p.slot_rows + row;
-            ml[i] = *reinterpret_cast<const float2*>(p.part_ml + 2 * slot);
-            v[i] = *reinterpret_cast<const float4*>(p.part_o + slot * hd + c);
+            const size_t at = part_row(p, item.w, min(s0 + i, slices - 1), rows, kvh) + row;
+            ml[i] = *reinterpret_cast<const float2*>(p.part_ml + 2 * at);
+            v[i] = *reinterpret_cast<const float4*>(p.part_o + at * hd + c);
         }
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i) {
@@ -313,24 +337,27 @@ int go(const Params& p, const int* work, int n, cudaStream_t s) {
 BW_EXPORT int bw_attention_f32_slice() { return SLICE; }
 BW_EXPORT int bw_attention_f32_slices() { return MOST; }
 
-// rows_w: int32 [n_rows][4] (request, first token, 0, 0), tiles of 64 / (nh / nkv) tokens; keys_w: [n_keys][4] (request, slice,
-// slices, first slot) for segments of at most slot_rows <= 16 stacked rows whose slices are of one size, at least as many slices as the
-// segment's rows see; merge_w: [n_merge][4] (request, 0, slices, first slot).  part_o,
-// part_ml: float32 [slots][nkv][slot_rows][hd] and [..][2] (null without merge items).  hd % 4 == 0, hd <= 256, nh / nkv <= 64.
+// rows_w: int32 [n_rows][4] (request, first token, 0, 0), tiles of 64 / (nh / nkv) tokens; wide_w: such tiles, and keys_w: segments of at
+// most 16 stacked rows, whose slices are dealt out to blocks: [..][4] (request, first token, block | blocks << 16, where), every row's
+// slices of one size; merge_w: [n_merge][4] (request, first token, rows, where), at most merge_rows rows each.  part_o, part_ml: float32
+// [part_rows * nkv][hd] and [..][2] (null without merge items), part_rows at least the sum of slices times rows of the merged tiles,
+// of which `where` counts those before.  hd % 4 == 0, hd <= 256, nh / nkv <= 64.
 BW_EXPORT int bw_attention_f32(const float* q, const float* k_pages, const float* v_pages, float* out, const int* cu_q,
                                const int* q_start, const int* block_table, int max_blocks, const int* rows_w, int n_rows,
-                               const int* keys_w, int n_keys, const int* merge_w, int n_merge, float* part_o, float* part_ml, int slot_rows, int nh,
-                               int nkv, int hd, int page_size, int num_pages, int window, int chunk, float scale, void* stream) {
+                               const int* wide_w, int n_wide, const int* keys_w, int n_keys, const int* merge_w, int n_merge,
+                               int merge_rows, float* part_o, float* part_ml, int nh, int nkv, int hd, int page_size, int num_pages,
+                               int window, int chunk, float scale, void* stream) {
     if (nkv <= 0 || nh % nkv || nh / nkv > 64 || hd <= 0 || hd % 4 || hd > 256) return BW_ERR_UNSUPPORTED;
-    if (n_merge && (!part_o || !part_ml || slot_rows <= 0 || slot_rows > SLICE_ROWS)) return BW_ERR_BAD_ARG;
+    if (n_merge && (!part_o || !part_ml || merge_rows <= 0 || merge_rows > 64)) return BW_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     const Params p = {q, k_pages, v_pages, out, cu_q, q_start, block_table, max_blocks, nh, nkv, hd, page_size, num_pages, window, chunk,
-                      scale, part_o, part_ml, slot_rows};
+                      scale, part_o, part_ml};
     int rc = 0;
     if (n_rows) rc = hd <= 128 ? go<64, 1, false>(p, rows_w, n_rows, s) : go<64, 2, false>(p, rows_w, n_rows, s);
+    if (rc == 0 && n_wide) rc = hd <= 128 ? go<64, 1, true>(p, wide_w, n_wide, s) : go<64, 2, true>(p, wide_w, n_wide, s);
     if (rc == 0 && n_keys) rc = hd <= 128 ? go<SLICE_ROWS, 1, true>(p, keys_w, n_keys, s) : go<SLICE_ROWS, 2, true>(p, keys_w, n_keys, s);
     if (rc == 0 && n_merge) {
-        bw::launch(attention_f32_merge_kernel, dim3(n_merge, nkv, slot_rows), dim3(64), 0, s, p, (const int4*)merge_w);
+        bw::launch(attention_f32_merge_kernel, dim3(n_merge, nkv, merge_rows), dim3(64), 0, s, p, (const int4*)merge_w);
         BW_LAUNCH_CHECK();
     }
     return rc;

@@ -588,62 +588,97 @@ def attention_f32(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
     if q.shape[1] != nh * hd:
         raise KernelError("attention: q must be [T, nh * head_dim]")
     out = torch.empty_like(q)
-    rows_w, n_rows, keys_w, n_keys, merge_w, n_merge, slices, slot_rows = _attention_f32_work(batch, nh // nkv, window, chunk)
+    work, part_rows, merge_rows = _attention_f32_work(batch, nh // nkv, nkv, window, chunk)
     part_o = part_ml = None
-    if n_merge:
-        part_o = torch.empty((slices * nkv * slot_rows, hd), dtype=torch.float32, device=out.device)
-        part_ml = torch.empty((slices * nkv * slot_rows, 2), dtype=torch.float32, device=out.device)
+    if part_rows:
+        part_o = torch.empty((part_rows * nkv, hd), dtype=torch.float32, device=out.device)
+        part_ml = torch.empty((part_rows * nkv, 2), dtype=torch.float32, device=out.device)
+    lists = [v for items in work for v in (_ptr(items), 0 if items is None else items.shape[0])]
     fn = _fn("attention_f32", "bw_attention_f32", _ATTN_F32_ARGS)
     _check(fn(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(batch.cu_q), _ptr(batch.q_start), _ptr(block_table),
-              block_table.shape[1], _ptr(rows_w), n_rows, _ptr(keys_w), n_keys, _ptr(merge_w), n_merge, _ptr(part_o),
-              _ptr(part_ml), slot_rows, nh, nkv, hd, page_size, num_pages, int(window or 0), int(chunk or 0), float(scale), _stream()),
-           "attention_f32")
+              block_table.shape[1], *lists, merge_rows, _ptr(part_o), _ptr(part_ml), nh, nkv, hd, page_size, num_pages, int(window or 0),
+              int(chunk or 0), float(scale), _stream()), "attention_f32")
     return out
 
 
-def plan_attention_f32(q_len, q_start, kv_len, G: int, window: Optional[int], chunk: Optional[int], slice_keys: int,
-                       most: int, static_bound: Optional[int] = None):
-    """The work lists of the tiled float32 attention as plain lists, of the form of :func:`plan_attention_work`, and the stacked rows
-    of the largest sliced segment.  A segment of at most 16 stacked rows whose rows have slices of one size (``slice_keys`` keys, or as
-    many times that as makes ``most`` slices of what a row sees) has a block for every slice that its rows may see."""
-    def of(pos):
-        lo = max(pos - window + 1 if window else 0, pos - pos % chunk if chunk else 0, 0)
-        return -(-(pos + 1 - lo) // (slice_keys * most))
-    rows, keys, merge, slots, slot_rows = [], [], [], 0, 0
+def plan_attention_f32(q_len, q_start, G: int, nkv: int, window: Optional[int], chunk: Optional[int], slice_keys: int,
+                       most: int, sms: int = 148, static_bound: Optional[int] = None):
+    """The work of the tiled float32 attention as plain lists: (tiles whose keys one block walks, tiles whose slices several share,
+    segments of at most 16 stacked rows whose slices several share, the tiles to be merged), the rows of partial results per kv head,
+    and the most rows of a merged tile.  A row's slices have ``slice_keys`` keys, or as many times that as makes ``most`` slices of
+    what it sees; the rows of a tile that is sliced have slices of one size.  How many blocks share a tile does not change a bit."""
+    def first(pos):
+        return max(pos - window + 1 if window else 0, pos - pos % chunk if chunk else 0, 0)
+
+    def slices(r, t0, n):      # at most, of the tile's keys; 0: of several sizes
+        if n > 1 and len({-(-(p + 1 - first(p)) // (slice_keys * most)) for p in range(q_start[r] + t0, q_start[r] + t0 + n)}) > 1:
+            return 0
+        end = static_bound or q_start[r] + t0 + n
+        if not window and not chunk:
+            return min(-(-end // slice_keys), most)
+        # the keys before its first row that a tile reaches back to, from a slice's start
+        return min([-(-end // slice_keys), most + 2] + [-(-(reach + n + slice_keys - 1) // slice_keys) for reach in (window, chunk) if reach])
+
+    few, tiles = [], []
     for r, n_q in enumerate(q_len):
-        if n_q * G > 16 or (n_q > 1 and len({of(q_start[r] + i) for i in range(n_q)}) > 1):
-            rows += [(r, t0, 0, 0) for t0 in range(0, n_q, 64 // G)]
-            continue
-        n = min(-(-(static_bound or kv_len[r]) // slice_keys), most)
-        if window or chunk:     # the keys before its first row that a segment reaches back to, from a slice's start
-            n = min([-(-(static_bound or kv_len[r]) // slice_keys), most + 2]
-                    + [-(-(reach + n_q + slice_keys - 1) // slice_keys) for reach in (window, chunk) if reach])
-        keys += [(r, s, n, slots) for s in range(n)]
-        if n > 1:
-            merge.append((r, 0, n, slots))
-        slots += n
-        slot_rows = max(slot_rows, n_q * G)
+        if n_q * G <= 16 and (n_q == 0 or slices(r, 0, n_q)):
+            few.append((r, 0, n_q))
+        else:
+            tiles += [(r, t0, min(64 // G, n_q - t0)) for t0 in range(0, n_q, 64 // G)]
+
+    def small(items):       # 64 MB hold the partial results of 256 channels
+        return sum(slices(*t) * t[2] * G for t in items if slices(*t) > 1) * nkv * 258 * 4 <= 64e6
+    # a few tiles of few keys that leave three SMs of four idle: as tiles of 16 rows, whose blocks are done sooner
+    # (33 tokens, groups of 4, 8 kv heads of 128: 19.2 us and 9.8 so; groups of 2, 2 kv heads of 16: 14.0 and 7.3)
+    if tiles and G <= 16 and 4 * len(tiles) * nkv <= sms:
+        pieces = [(r, t0, min(16 // G, q_len[r] - t0)) for r in dict.fromkeys(t[0] for t in tiles) for t0 in range(0, q_len[r], 16 // G)]
+        if all(0 < slices(*t) < 4 for t in pieces):
+            few, tiles = few + pieces, []
+    rows, wide, keys, merge, part_rows, merge_rows = [], [], [], [], 0, 0
+
+    def share(items, to, blocks):
+        nonlocal part_rows, merge_rows
+        for r, t0, n in items:
+            s = slices(r, t0, n)
+            b = max(1, min(s, blocks))
+            to += [(r, t0, i | b << 16, part_rows) for i in range(b)]
+            if s > 1:
+                merge.append((r, t0, n * G, part_rows))
+                part_rows += s * n * G
+                merge_rows = max(merge_rows, n * G)
+    # blocks for eight rounds of two an SM: a block's slices follow one another, and a bound's slices that a short request does not have
+    # cost their blocks' starts (64 requests of 20 tokens at a bound of 8,320, groups of 4, 8 kv heads of 128: 93 us
+    # with a block a slice, 21 so; groups of 1, 32 kv heads: 337 and 55)
+    share(few, keys, -(-8 * sms // max(1, len(few) * nkv)))
+    # tiles that leave half of the SMs idle share their slices, where they have some (40 tokens at 2,000,
+    # groups of 64, one kv head of 8: 403 us unshared, 143 so; groups of 4, 8 kv heads of 128: 585 and 113)
+    sliced = [t for t in tiles if slices(*t) >= 4] if 2 * len(tiles) * nkv <= sms else []
+    if not small(sliced):
+        sliced = []
+    share(sliced, wide, -(-2 * sms // max(1, len(sliced) * nkv)))
+    rows = [(r, t0, 0, 0) for r, t0, n in tiles if (r, t0, n) not in sliced]
     rows.sort(key=lambda it: -(q_start[it[0]] + it[1]))     # the tiles with the most keys first
-    return rows, keys, merge, slots, slot_rows
+    return (rows, wide, keys, merge), part_rows, merge_rows
 
 
-def _attention_f32_work(batch, G: int, window: Optional[int], chunk: Optional[int]):
-    """:func:`plan_attention_f32` for this batch on the device, made once per step and shared by its layers."""
-    key = ("attn_f32_work", G, window, chunk)
+def _attention_f32_work(batch, G: int, nkv: int, window: Optional[int], chunk: Optional[int]):
+    """:func:`plan_attention_f32` for this batch with its lists on the device, made once per step and shared by its layers."""
+    key = ("attn_f32_work", G, nkv, window, chunk)
     work = batch.static_extras.get(key)
     if work is None:
         R, dev = batch.R, batch.token_ids.device
-        rows, keys, merge, slots, slot_rows = plan_attention_f32(
-            batch.h_q_len[:R], batch.h_q_start[:R], batch.h_kv_len[:R], G, window, chunk, _fn("attention_f32", "bw_attention_f32_slice", [])(),
-            _fn("attention_f32", "bw_attention_f32_slices", [])(), batch.static_bound)
+        lists, part_rows, merge_rows = plan_attention_f32(
+            batch.h_q_len[:R], batch.h_q_start[:R], G, nkv, window, chunk,
+            _fn("attention_f32", "bw_attention_f32_slice", [])(), _fn("attention_f32", "bw_attention_f32_slices", [])(), num_sms(dev),
+            batch.static_bound)
 
         def up(items):
             return torch.tensor(items, dtype=torch.int32).pin_memory().to(dev, non_blocking=True) if items else None
-        work = batch.static_extras[key] = (up(rows), len(rows), up(keys), len(keys), up(merge), len(merge), slots, slot_rows)
+        work = batch.static_extras[key] = ([up(items) for items in lists], part_rows, merge_rows)
     return work
 
 
-_ATTN_F32_ARGS = [c_void_p] * 7 + [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p] + [c_int] * 8 + [c_float, c_void_p]
+_ATTN_F32_ARGS = [c_void_p] * 7 + [c_int] + [c_void_p, c_int] * 4 + [c_int, c_void_p, c_void_p] + [c_int] * 7 + [c_float, c_void_p]
 
 
 def _gate_args(gate: Optional[tuple], T: int, nh: int, hd: int):

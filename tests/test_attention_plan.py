@@ -74,47 +74,71 @@ def test_a_graph_replay_depends_on_the_bound_only():
     assert alone[3] > many[3] // 64 >= 1   # fewer slices a request when more requests fill the GPU
 
 
-@pytest.mark.parametrize("G", (1, 3, 4, 16, 20))
+@pytest.mark.parametrize("G,nkv", ((1, 32), (3, 2), (4, 8), (16, 1), (20, 1), (64, 1)))
 @pytest.mark.parametrize("window,chunk", [(None, None), (48, None), (9000, None), (None, 100), (None, 9000), (20000, 30000)])
-def test_float32_slices(G, window, chunk):
-    """The float32 kernel's lists: every token once, and slices for all that a segment's rows may see (counted as the kernel does)."""
+def test_float32_work(G, nkv, window, chunk):
+    """The float32 kernel's lists: every token in one tile, every slice that a tile's rows may see in one block (counted as the kernel
+    counts), and results of slices that neither overlap nor leave the scratch."""
     rng = random.Random(G)
     first = lambda pos: max(0, pos - window + 1 if window else 0, pos - pos % chunk if chunk else 0)
     keys_of = lambda pos: 128 * -(-(pos + 1 - first(pos)) // 8192)
     for trial in range(60):
-        q_len, q_start, kv_len = random_batch(rng, rng.randint(1, 20), G)
+        q_len, q_start, _ = random_batch(rng, rng.randint(1, 20), G)
+        if trial % 4 == 3:
+            q_len = [rng.choice((1, 20, 45)) for _ in q_len[:2]]
         if trial % 2:
             q_start = [s + rng.choice((0, 8185, 16380, 40000, 120000)) for s in q_start]
-            kv_len = [s + n for s, n in zip(q_start, q_len)]
         bound = None
         if trial % 3 == 0:
-            q_len, kv_len, bound = [1] * len(q_len), [s + 1 for s in q_start], max(q_start) + 1 + rng.randint(0, 100000)
-        rows, keys, merge, slots, slot_rows = plan_attention_f32(q_len, q_start, kv_len, G, window, chunk, 128, 64, bound)
-        tiled, sliced = {}, {}
+            q_len, bound = [1] * len(q_len), max(q_start) + 1 + rng.randint(0, 100000)
+        q_start = q_start[:len(q_len)]
+        (rows, wide, keys, merge), part_rows, merge_rows = plan_attention_f32(q_len, q_start, G, nkv, window, chunk, 128, 64, 148, bound)
+        merged, covered, parts = {(r, t0): (n, w) for r, t0, n, w in merge}, [], []
+        assert len(merged) == len(merge)
         for r, t0, _, _ in rows:
-            tiled.setdefault(r, []).append(t0)
-        for r, s, n, slot in keys:
-            sliced.setdefault(r, []).append((s, n, slot))
-        at = 0
+            covered.append((r, t0, min(64 // G, q_len[r] - t0)))
+        for items, tile in ((wide, 64), (keys, 16)):
+            tiles = {}
+            for r, t0, z, where in items:
+                tiles.setdefault((r, t0), []).append((z & 0xffff, z >> 16, where))
+            for (r, t0), blocks in tiles.items():
+                n = min(tile // G, q_len[r] - t0)
+                covered.append((r, t0, n))
+                B, where = blocks[0][1:]
+                assert 1 <= B <= 66 and blocks == [(i, B, where) for i in range(B)] and n * G <= tile
+                sizes = {keys_of(q_start[r] + t0 + i) for i in range(n)}
+                assert len(sizes) == 1
+                size = sizes.pop()
+                base = first(q_start[r] + t0) // size * size
+                real = -(-(q_start[r] + t0 + n - base) // size)
+                share = -(-real // B)
+                assert share * B >= real
+                if (r, t0) not in merged:
+                    assert real <= 1 and B == 1
+                else:
+                    assert merged[(r, t0)] == (n * G, where) and n * G <= merge_rows <= 64
+                    parts.append((where, where + real * n * G))
+        covered.sort()
         for r, n_q in enumerate(q_len):
-            sizes = {keys_of(q_start[r] + i) for i in range(n_q)}
-            if r in tiled:
-                assert r not in sliced and sorted(tiled[r]) == list(range(0, n_q, 64 // G)) and (n_q * G > 16 or len(sizes) > 1)
-                continue
-            n = len(sliced[r])
-            assert sliced[r] == [(s, n, at) for s in range(n)] and len(sizes) == 1 and n_q * G <= slot_rows <= 16
-            size = sizes.pop()
-            base = first(q_start[r]) // size * size
-            assert -(-(kv_len[r] - base) // size) <= n <= 66
-            assert ((r, 0, n, at) in merge) == (n > 1)
-            at += n
-        assert at == slots
+            at = 0
+            for _, t0, n in (c for c in covered if c[0] == r):
+                assert t0 == at
+                at += n
+            assert at == n_q
+        parts.sort()
+        assert all(a[1] <= b[0] for a, b in zip(parts, parts[1:])) and (not parts or parts[-1][1] <= part_rows)
 
 
 @pytest.mark.parametrize("bound", (131072, 340000))
-def test_float32_decode_graphs_stay_small(bound):
-    """A decode graph's lists are made for the longest context: blocks and partial results per request are bounded all the same."""
-    R, G, nkv, hd = 64, 4, 8, 128
-    rows, keys, merge, slots, slot_rows = plan_attention_f32([1] * R, [700] * R, [701] * R, G, None, None, 128, 64, bound)
-    assert not rows and len(keys) == slots == 64 * R and slot_rows == G
-    assert 4 * slots * nkv * slot_rows * (hd + 2) <= 70e6
+@pytest.mark.parametrize("R,G,nkv", [(64, 4, 8), (64, 1, 32), (8, 4, 8), (2, 64, 1)])
+def test_float32_decode_graphs_stay_small(bound, R, G, nkv):
+    """A decode graph's lists are made for the longest context: its blocks and partial results are bounded all the same."""
+    (rows, wide, keys, merge), part_rows, _ = plan_attention_f32([1] * R, [700] * R, G, nkv, None, None, 128, 64, 148, bound)
+    assert len(rows + wide + keys) * nkv <= 8 * 148 + R * nkv
+    assert part_rows <= 64 * R * G and 4 * part_rows * nkv * (128 + 2) <= 70e6
+
+
+def test_float32_prompts_scratch_is_bounded():
+    for nkv, n in ((1, 500), (2, 250), (8, 64), (37, 16)):
+        (rows, wide, keys, merge), part_rows, _ = plan_attention_f32([n], [100000], 4, nkv, None, None, 128, 64)
+        assert 4 * part_rows * nkv * 258 <= 64e6
