@@ -47,15 +47,19 @@ def uniform_many(seeds: Sequence[int], indices: Sequence[int]) -> np.ndarray:
     from ..cache.manager import native
     if len(seeds) != len(indices):
         raise ValueError(f"one index per seed: {len(seeds)} seeds, {len(indices)} indices")
-    out = np.empty(len(seeds), dtype=np.float32)
-    s, i = (np.array([operator.index(v) & 0xFFFFFFFFFFFFFFFF for v in vals], dtype=np.uint64) for vals in (seeds, indices))
-    native().bwh_uniform(len(out), s.ctypes.data, i.ctypes.data, out.ctypes.data)
+    n = len(seeds)
+    out = np.empty(n, dtype=np.float32)
+    both = np.array([operator.index(v) & 0xFFFFFFFFFFFFFFFF for vals in (seeds, indices) for v in vals], dtype=np.uint64)
+    at = both.ctypes.data
+    native().bwh_uniform(n, at, at + 8 * n, out.ctypes.data)
     return out
 
 
 def row_draws(params: Sequence["SamplingParams"], seeds: Sequence[int], draw_index: Sequence[int]) -> np.ndarray:
     """The random number of every row, float32.  Greedy rows draw nothing (0) and theirs are not looked at."""
     rows = [r for r, p in enumerate(params) if not p.greedy]
+    if len(rows) == len(params) == len(seeds) == len(draw_index):
+        return uniform_many(seeds, draw_index)
     out = np.zeros(len(params), dtype=np.float32)
     out[rows] = uniform_many([seeds[r] for r in rows], [draw_index[r] for r in rows])
     return out

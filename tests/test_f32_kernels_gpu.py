@@ -98,7 +98,8 @@ def test_queued_steps_repeat_themselves():
 
 
 def test_split_products_over_the_range_of_float32(ops):
-    """Magnitudes from the smallest normal products to large ones, in one product each: the split is relative to each value."""
+    """Products of magnitudes from 1e-30 to 1e30: the split is relative to each value.  (Smaller ones:
+    test_single_products_and_small_magnitudes.)"""
     for scale_x, scale_w in ((1e-15, 1e-15), (1e15, 1e15), (1e-18, 1e18)):
         x, w = rand(40, 512, seed=1) * scale_x, rand(256, 512, seed=2) * scale_w
         want = x.double() @ w.double().T
