@@ -1,8 +1,8 @@
-// out[M, N] (=|+=) x[M, K] . w[N, K]^T (+ bias), float32 in and out, on the tensor cores without losing float32's precision.
+// out[M, N] (=|+=) x[M, K] . w[N, K]^T (+ bias), float32 in and out, on the tensor cores.
 //
 // Every operand is split into two TF32 numbers, hi = x rounded to 11 bits and lo = x - hi, which is exact and has at most 12 bits, of
-// which the tensor cores read 11 (what they drop is below 2^-23 |x|), and three products are summed, hi hi apart from hi lo + lo hi (lo lo is below 2^-22 of the product).  The
-// tensor cores' own sums are kept short: an accumulator takes 64 channels and is then added into float32 registers, rounded to
+// which the tensor cores read 11 (what they drop is at most 2^-23 |x|), and three products are summed, hi hi apart from hi lo + lo hi (lo
+// lo is below 2^-22 of the product).  The tensor cores' own sums are kept short: an accumulator takes 64 channels and is then added into float32 registers, rounded to
 // nearest, so no long chain runs through the tensor cores' accumulation.  Measured against 64 bits over the products of an 8B
 // decoder (K 4096 and 14336): relative error 2.2e-7 to 2.6e-7, where one chain of float32 FMAs (gemm_simt.cu) has 1.2e-6 to 2.2e-6.
 // What the split drops of an operand is at most 2^-23 of it, one unit of float32's last place: a product by itself (a row of x with one
@@ -23,10 +23,10 @@
 // Roles (896 threads): warp 0 loads weights; warp 1 TMEM owner and MMAs; warp 2 loads tokens; warps 4..11 split the weights, two
 // groups that take stages in turn; warps 12..27 add the accumulators up, 32 tokens each group of four, and write the result.  Every
 // wait is bounded; a timeout sets the status word and all roles fall through to the exit.
-// What bounds it: the MMA warp, in its waits (about 300 cycles a stage of 32 channels, of 1,369 at 128 tokens; 768 are MMAs) and its
-// issue.  Measured, x 28672 x 4096: 1 to 16 tokens 84 to 88 us (5.6 TB/s), 64 tokens 122 us, 128 tokens 167 us (180 TFLOP/s), 301 tokens
-// 454 us; with loop bounds that the compiler could not know to be the same in all lanes 91, 127, 173 and 476 us.  gemm_simt.cu's tiles:
-// eight layers of the 8B shape with logits at each of 301 tokens 72.2 ms, of which 65.0 were products.
+// What bounds it: up to 16 tokens the weights' bytes; beyond, what a stage of 32 channels takes from its split to its sums: at 128 tokens
+// about 1,700 cycles, the two small kernels' share included, of which its twelve MMAs are 768 (64 each, measured by themselves).
+// Measured, x 28672 x 4096, with the small kernels, on several B200s: 1 to 16 tokens 86 to 93 us (5.0 to 5.5 TB/s), 64 tokens 122 to
+// 129, 128 tokens 168 to 176 (about 175 TFLOP/s), 301 tokens 490 to 527.  gemm_simt.cu: 301 tokens 3.1 ms.
 #include "tcgen05.cuh"
 
 using bf16 = __nv_bfloat16;
@@ -239,14 +239,14 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        // the whole warp walks the stages, one elected lane issues: operands the compiler knows to be the same in all lanes (in a branch
-        // of one lane an MMA took 100 to 150 cycles to issue, whatever its size; so 9, or what the tensor pipe needs)
+        // the whole warp walks the stages and one elected lane issues (see tcgen05.cuh, elect_one; in a branch of one lane an MMA took
+        // 100 to 150 cycles to issue, whatever its size; so 9, or what the tensor pipe needs)
         const uint32_t small = __shfl_sync(0xffffffffu, tmem, 0), cols_a = small + 3 * acc_cols(bn);
         const uint32_t idesc = idesc_tf32(bn), smem0 = bw::smem_u32(smem_x), lo_units = (uint32_t)bn * BK * 4 / 16;
         int xst = 0, xph = 0, tst = 0, tph = 0, p = 0, items = 0;
         bool ok = true;
         while (ok && __shfl_sync(0xffffffffu, (int)it.next(), 0)) {
-            const int n = __shfl_sync(0xffffffffu, it.n, 0);      // (known to be the same in all lanes, like all that the loop changes)
+            const int n = __shfl_sync(0xffffffffu, it.n, 0);      // (each lane's own: 301 tokens 476 us, so 454 on the same GPU)
             ok = __all_sync(0xffffffffu, bw::mbar_wait(small_free, (items++ & 1) ^ 1, &g_status, 3));
             for (int i = 0; ok && i < n; ++i) {
                 const int buf = p & 1;

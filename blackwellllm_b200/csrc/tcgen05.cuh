@@ -21,8 +21,8 @@ namespace bw {
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
-// True in one lane of a converged warp.  A warp that issues MMAs walks its loop as a whole and issues under this: the operands are
-// then known to be the same in all lanes.  Measured, cycles between MMAs of M 128 under it / in a branch of lane 0: A from tensor
+// True in one lane of a converged warp.  A warp that issues MMAs walks its loop as a whole, with the same operands in all lanes, and
+// issues under this.  Measured, cycles between MMAs of M 128 under it / in a branch of lane 0: A from tensor
 // memory, N 16: 9 / 46, N 64: 32 / 46; A from shared memory, N 16: 39 / 48, N 64: 48 / 48 (100 to 150 in the branch where sizes are
 // not known at compile time); from N 128 on the tensor pipe's own 64 or more.
 __device__ __forceinline__ bool elect_one() {

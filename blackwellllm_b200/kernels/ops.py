@@ -487,8 +487,9 @@ _GEMM_F32_TC_ARGS = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int
 
 
 def gemm_f32_tc_supports(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether the tensor-core product of split float32 operands takes these: channels in fours, rows that begin on 16 bytes, and a
-    weight of at least one tile's rows and eight stages' channels (a smaller one is all latency there, and its chains too short to err more)."""
+    """Whether the tensor-core product of split float32 operands takes these, whatever the number of tokens: channels in fours, rows
+    that begin on 16 bytes, and a weight of at least one tile's rows (of fewer the tile is mostly padding) and eight stages' channels
+    (fewer are all filling and draining, and a chain of FMAs over them errs no more)."""
     return (x.dtype == torch.float32 and w.dtype == torch.float32 and w.shape[0] >= 128 and w.shape[1] >= 256 and w.shape[1] % 4 == 0
             and x.dim() == 2 and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
@@ -504,7 +505,8 @@ def gemm_f32_scratch(N: int, K: int) -> Tuple[int, int]:
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
              accumulate: bool = False) -> torch.Tensor:
     """out (=|+=) x @ w.T (+ bias) in float32, a row's result independent of the other rows: on the tensor cores from operands split
-    into two TF32 parts, whose error is no larger than that of float32 FMAs; forms that kernel does not take on the CUDA cores."""
+    into two TF32 parts, or, in forms that kernel does not take, on the CUDA cores.  Against 64 bits sums of many products err less than
+    a chain of float32 FMAs; a product by itself is off by up to 2^-21 of it, and operands below 1e-34 keep multiples of 2^-136 only."""
     if not gemm_f32_tc_supports(x, w):
         return gemm_simt(x, w, bias, out=out, accumulate=accumulate)
     _dev(x, "x", torch.float32, contiguous=False); _dev(w, "w", torch.float32)

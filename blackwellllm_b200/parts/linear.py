@@ -1,9 +1,10 @@
 """A weight matrix [out, in] with an optional bias, and the one place that picks
 the matrix-product kernel for it.
 
-float32 weights are multiplied in float32 (the true 32-bit path): on the CUDA cores for a few
-tokens and for small weights, else on the tensor cores from operands split in two, with an
-error no larger than that of a chain of float32 FMAs.
+float32 weights are multiplied in float32 (the true 32-bit path): on the tensor cores from
+operands split in two, or on the CUDA cores where the weight is small or rows do not begin on
+16 bytes, never by the number of tokens.  Sums of many products err less than a chain of
+float32 FMAs; a product by itself may be off by 2^-21 of it.
 bfloat16 weights run on the tcgen05 tensor-core kernel; a shape that kernel
 refuses (an inner size that is no multiple of 8, which a TMA row stride cannot
 express) runs on the CUDA-core kernel with bfloat16 operands and float32 sums.
