@@ -250,6 +250,35 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     }
 }
 
+// The greedy choice of one row per block: the row is read once and nothing else is done.
+__global__ void __launch_bounds__(THREADS)
+argmax_kernel(const float* __restrict__ logits, int* __restrict__ out, int V, size_t ld) {
+    BW_PDL_TRIGGER();
+    BW_PDL_WAIT();
+    __shared__ float sv[WARPS];
+    __shared__ int si[WARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float* row = logits + (size_t)blockIdx.x * ld;
+    float mx = -INFINITY;
+    int arg = 0x7fffffff;
+    for (int c = threadIdx.x; c < V; c += THREADS) argmax_pair(mx, arg, row[c], c);
+    auto over_warp = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, mx, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, arg, o);
+            argmax_pair(mx, arg, ov, oi);
+        }
+    };
+    over_warp();
+    if (lane == 0) { sv[warp] = mx; si[warp] = arg; }
+    __syncthreads();
+    if (warp) return;
+    mx = sv[lane]; arg = si[lane];
+    over_warp();
+    if (lane == 0) out[blockIdx.x] = arg == 0x7fffffff ? 0 : arg;
+}
+
 // Repetition penalty in place, one block per row: every DISTINCT id of the row's history
 // ids[begin[r] .. begin[r+1]) has its logit divided by penalty[r] when positive and multiplied
 // by it when not, once however often the id occurs (only an id's first occurrence acts).
@@ -326,14 +355,20 @@ BW_EXPORT int bw_sample(const float* logits, const float* temperature, const flo
     while ((1ll << bits) < V) ++bits;
     const float scale = (float)(1ull << (62 - bits < 45 ? 62 - bits : 45));
     const dim3 block(THREADS);
-    // One block a row where that is faster: a row that fits a block's registers (64 rows of 5,000: nucleus 14 us, 69 on clusters; alone
-    // 13 and 20), or so many rows that their clusters take turns for longer than a block walks its row (greedy / temperature / nucleus,
-    // on clusters and in blocks: 64 rows of 32,000 13 / 19 / 75 and 9 / 27 / 63, 128 of 64,000 24 / 47 / 158 and 16 / 55 / 137, 256 of
-    // 128,256 72 / 168 / 404 and 70 / 157 / 366; of 256,000, which a cluster's registers do not hold, 356 / 479 / 1,180 and
-    // 128 / 323 / 717).
-    const int many = V > 160 * 1024 ? 100 : V / (!temperature && V <= 64 * 1024 ? 870 : 500);
-    if (V <= 8 * THREADS || R > many) {
-        const auto kernel = V <= 8 * THREADS && (temperature || R <= bw::num_sms()) ? sample_kernel<8, false, 1> : sample_kernel<0, false, 1>;
+    // The greedy choice alone needs one pass, and clusters take turns of 17 rows or so: a block a row, but for a few long rows (us on
+    // clusters and in blocks: 8 rows of 24,000 3.1 and 3.2, of 32,000 3.2 and 3.8, of 128,256 4.1 and 8.1; 18 of 32,000 5.4 and 3.8; 36
+    // of 128,256 10.4 and 8.3; 256 of them 71 and 25; 18 of 200,000 14.6 and 11.2).
+    if (!temperature && (V <= 24 * 1024 || R > (V > 100 * 1024 && V <= 160 * 1024 ? 32 : 16))) {
+        bw::launch(argmax_kernel, dim3((unsigned)R), block, 0, (cudaStream_t)stream, logits, out, V, (size_t)ld);
+        BW_LAUNCH_CHECK();
+        return 0;
+    }
+    // Else one block a row where that is faster: a row that fits a block's registers (64 rows of 5,000: nucleus 14 us, 69 on clusters;
+    // alone 13 and 20), or so many rows that their clusters take turns for longer than a block walks its row (temperature / nucleus, on
+    // clusters and in blocks: 64 rows of 32,000 19 / 75 and 27 / 63, 128 of 64,000 47 / 158 and 55 / 137, 256 of 128,256 168 / 404 and
+    // 156 / 365; of 256,000, which a cluster's registers do not hold, 479 / 1,180 and 323 / 717).
+    if (V <= 8 * THREADS || R > (V > 160 * 1024 ? 100 : V / 512)) {
+        const auto kernel = V <= 8 * THREADS ? sample_kernel<8, false, 1> : sample_kernel<0, false, 1>;
         bw::launch(kernel, dim3((unsigned)R), block, 0, (cudaStream_t)stream, logits, temperature, top_p, u, out, V, (size_t)ld, scale);
         BW_LAUNCH_CHECK();
         return 0;

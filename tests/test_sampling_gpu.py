@@ -90,3 +90,8 @@ def test_rows_choose_the_same_token_in_every_form(R, V):
         whole = ops.sample(x, *args)
         for at in range(0, R, 9):
             assert torch.equal(ops.sample(x[at:at + 9], *(a[at:at + 9] if a is not None else None for a in args)), whole[at:at + 9])
+    # greedy rows of masks and of no numbers alone, and the lowest index of a tie
+    x[0], x[1], x[2] = float("-inf"), float("nan"), 3.0
+    x[0, V - 1], x[2, V // 3], x[2, V // 2] = -1e30, 4.0, 4.0
+    for part in (x, x[:3]):
+        assert ops.sample(part, None, None, None)[:3].tolist() == [V - 1, 0, V // 3]
