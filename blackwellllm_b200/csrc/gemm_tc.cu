@@ -17,7 +17,7 @@
 // (the residual stream), or SwiGLU over interleaved gate/up features -> bfloat16, or rotary
 // position encoding of a fused q/k/v projection with the keys and values written to their pages.
 //
-// With 512 tokens or more and no K split the product runs on CTA PAIRS instead
+// With more than 128 tokens most products run on CTA PAIRS instead
 // (gemm_pair_kernel, cta_group::2): two CTAs of a cluster share a tile of 256 tokens, each loads
 // half of the weight tile, and the leader's MMAs read both CTAs' shared memory.
 //
@@ -37,8 +37,8 @@ constexpr int UMMA_K = 16;
 constexpr int A_BYTES = BM * BK * 2;
 constexpr int THREADS = 192;
 // Epilogue staging, per epilogue warp a 32 x 33 float block or two 32 x 32 boxes for TMA.  Only the normal
-// orientation uses it, and that has tiles of 128 columns or more: the narrow kernels do without.
-template <int BN> __host__ __device__ constexpr int staging_bytes() { return BN >= 128 ? 4 * 2 * 4096 : 0; }
+// orientation and the pairs use it, and those have tiles of 96 columns or more: the narrow kernels do without.
+template <int BN> __host__ __device__ constexpr int staging_bytes() { return BN >= 96 ? 4 * 2 * 4096 : 0; }
 constexpr int SMEM_BUDGET = 226 * 1024 - staging_bytes<256>() - 2048;
 constexpr int FUSED_REDUCE_MAX_TOKENS = 16;   // split-K sums inside the kernel up to this many tokens
 constexpr int SWIGLU_BLOCK = 16;   // gate/up features are interleaved in blocks of 16 rows of the weight
@@ -260,6 +260,29 @@ __device__ __forceinline__ void emit(const Epilogue& ep, float* part, const floa
     }
 }
 
+// The biases of the 32 features f0 .. f0 + 31 (f0 a multiple of 32; the same for every lane), zeros from feature
+// `limit` on: 16-byte loads where the address and the limit allow them.
+__device__ __forceinline__ void load_bias32(const Epilogue& ep, int f0, int limit, float (&b)[32]) {
+    const bool whole = f0 + 32 <= limit && (((uintptr_t)ep.bias) & 15) == 0;
+    if (whole && ep.bias_type == BW_F32) {
+        const float4* src = reinterpret_cast<const float4*>((const float*)ep.bias + f0);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { const float4 t = __ldg(src + i); b[4 * i] = t.x; b[4 * i + 1] = t.y; b[4 * i + 2] = t.z; b[4 * i + 3] = t.w; }
+    } else if (whole) {
+        const uint4* src = reinterpret_cast<const uint4*>((const bf16*)ep.bias + f0);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint4 t = __ldg(src + i);
+            const uint32_t w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { b[8 * i + 2 * k] = __uint_as_float(w[k] << 16); b[8 * i + 2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u); }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) b[i] = f0 + i < limit ? bias_at(ep, f0 + i) : 0.f;
+    }
+}
+
 // Rotary epilogue in the normal orientation: the thread holds 32 consecutive features f0 .. f0 + 31
 // (the first n_features of them belong to this tile; a multiple of 16) of ONE token (v, float32 bits straight from TMEM).  Partners are neighbours in its registers, the
 // cache slot of the token is read once per tile (kv_slot < 0: no keys and values are written), and
@@ -268,6 +291,8 @@ __device__ __forceinline__ void rope_direct(const Epilogue& ep, const uint32_t (
                                          int n_features, int kv_slot) {
     const RopeOut& ro = ep.rope;
     const int half = ro.rd >> 1;
+    float b[32];
+    if (ep.bias) load_bias32(ep, f0, ep.features, b);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const int fh = f0 + 16 * h;
@@ -283,7 +308,7 @@ __device__ __forceinline__ void rope_direct(const Epilogue& ep, const uint32_t (
         }
         float x[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(v[16 * h + i]) + bias_at(ep, fh + i);
+        for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(v[16 * h + i]) + (ep.bias ? b[16 * h + i] : 0.f);
         const bool rotated_head = head < ro.nh + ro.nkv;
         if ((ro.rd & 15) == 0) {
             if (rotated_head && li0 < ro.rd) {
@@ -325,29 +350,6 @@ __device__ __forceinline__ void rope_direct(const Epilogue& ep, const uint32_t (
                 }
             }
         }
-    }
-}
-
-// The biases of the 32 features f0 .. f0 + 31 (f0 a multiple of 32; the same for every lane), zeros from feature
-// `limit` on: 16-byte loads where the address and the limit allow them.
-__device__ __forceinline__ void load_bias32(const Epilogue& ep, int f0, int limit, float (&b)[32]) {
-    const bool whole = f0 + 32 <= limit && (((uintptr_t)ep.bias) & 15) == 0;
-    if (whole && ep.bias_type == BW_F32) {
-        const float4* src = reinterpret_cast<const float4*>((const float*)ep.bias + f0);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { const float4 t = __ldg(src + i); b[4 * i] = t.x; b[4 * i + 1] = t.y; b[4 * i + 2] = t.z; b[4 * i + 3] = t.w; }
-    } else if (whole) {
-        const uint4* src = reinterpret_cast<const uint4*>((const bf16*)ep.bias + f0);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint4 t = __ldg(src + i);
-            const uint32_t w[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) { b[8 * i + 2 * k] = __uint_as_float(w[k] << 16); b[8 * i + 2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u); }
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) b[i] = f0 + i < limit ? bias_at(ep, f0 + i) : 0.f;
     }
 }
 
@@ -780,7 +782,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // k-block costs it 16 + BN / 8 KB instead of 16 + BN / 4: less traffic from L2 per flop, and room
 // for more stages), the leader CTA's MMA thread issues one M = 256 instruction that reads both
 // CTAs' shared memory and writes each CTA's 128 accumulator rows into its own TMEM, and each CTA
-// runs the epilogue of its own rows.  Normal orientation only, no K split.
+// runs the epilogue of its own rows.  SwiGLU also in the other orientation (256 features x BN tokens, no K split): a tile of tokens is then
+// as wide as the tokens need.  Tiles that share weight rows follow one another in either, so weights come from memory once.
 //   full[s]   on the leader: both CTAs' loads of stage s count their bytes there;
 //   empty[s]  on each CTA: the leader's commit reaches both;
 //   tfull[a]  on each CTA (the leader's commit reaches both); tempty[a] on the leader: the four
@@ -837,7 +840,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             Item im;
             BW_PDL_WAIT();
             while (ok && items.next(im)) {
-                const int tile_a = im.tile % tiles_a, tile_b = im.tile / tiles_a;
+                const int tile_a = ep.transposed ? im.tile / tiles_b : im.tile % tiles_a, tile_b = ep.transposed ? im.tile % tiles_b : im.tile / tiles_a;
                 for (int i = 0; i < im.nkb; ++i, ++it) {
                     const int s = it % STAGES;
                     const uint32_t ph = (it / STAGES) & 1;
@@ -885,12 +888,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         BW_PDL_WAIT();
         const int quarter = warp & 3;
         float* stage = staging + (warp - 2) * (32 * 33);
-        const int a_rows = ep.tokens, b_rows = ep.features;
+        const int a_rows = ep.transposed ? ep.features : ep.tokens, b_rows = ep.transposed ? ep.tokens : ep.features;
         uint32_t n = 0;
         Items items(ep, kb_total, kb_per_split, tiles, num_work, pair, n_pairs);
         Item im;
         for (; items.next(im); ++n) {
-            const int tile_a = im.tile % tiles_a, tile_b = im.tile / tiles_a;
+            const int tile_a = ep.transposed ? im.tile / tiles_b : im.tile % tiles_a, tile_b = ep.transposed ? im.tile % tiles_b : im.tile / tiles_a;
             const uint32_t acc = n & 1, accph = (n >> 1) & 1;
             if (!bw::mbar_wait_cluster(tfull0 + 8 * acc, accph, &g_status, 33)) break;
             bw::tc_fence_after();
@@ -903,7 +906,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 uint32_t v[32];
                 bw::tmem_ld_32x32(lane_addr + c0, v);
                 bw::tmem_ld_wait();
-                if (part) {
+                if (ep.transposed) {
+                    // SwiGLU: lanes hold the 16 gate and 16 up sums of 32 tokens; turned through shared memory, a lane holds a token's
+                    if constexpr (!ROPE) {
+#pragma unroll
+                        for (int c = 0; c < 32; ++c) stage[c * 33 + lane] = __uint_as_float(v[c]);
+                        __syncwarp();
+#pragma unroll
+                        for (int f = 0; f < 32; ++f) v[f] = __float_as_uint(stage[lane * 33 + f]);
+                        __syncwarp();
+                        const int token = tile_b * BN + c0 + lane;
+                        if (token < b_rows && row0 < a_rows) swiglu_direct(ep, v, token, row0);
+                    }
+                } else if (part) {
                     // a K split: this item's sums go to its plane of the scratch as they are (the lane's token,
                     // 32 consecutive features); a second kernel adds the planes in split order
                     const int token = row0 + lane, f0 = tile_b * BN + c0;
@@ -985,6 +1000,62 @@ __global__ void splitk_reduce_kernel(Epilogue ep) {
             float4* o = reinterpret_cast<float4*>((float*)ep.out + (size_t)token * ep.ldo + j);
             if (ep.accumulate) { const float4 old = *o; v.x = old.x + v.x; v.y = old.y + v.y; v.z = old.z + v.z; v.w = old.w + v.w; }
             *o = v;
+        }
+        return;
+    }
+    if (ep.rope_on && (ep.features & 3) == 0 && (ep.rope.hd & 3) == 0 && ((uintptr_t)ep.partial & 15) == 0 &&
+        (((uintptr_t)ep.rope.q_out | (uintptr_t)ep.rope.k_pages | (uintptr_t)ep.rope.v_pages) & 3) == 0) {
+        // rotary: two pairs a thread, 16-byte loads of every plane (a thread a feature, each pair's planes read twice: 93 tokens of
+        // 6144 x 4096 with their product 21.9 us)
+        const RopeOut& ro = ep.rope;
+        const int half = ro.rd >> 1, per_row = ep.features / 4;
+        const size_t quads = total / 4;
+        for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < quads; q += (size_t)gridDim.x * blockDim.x) {
+            const int token = (int)(q / per_row), j = (int)(q - (size_t)token * per_row) * 4;
+            const int head = j / ro.hd, li = j - head * ro.hd;
+            const bool is_q = head < ro.nh, rotates = head < ro.nh + ro.nkv;
+            float cs[2], sn[2];
+            bool rot[2];
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                rot[p] = rotates && li + 2 * p < ro.rd;
+                const float* tab = ro.table + (size_t)token * ro.rd + (li >> 1) + p;
+                cs[p] = rot[p] ? __ldg(tab) : 1.f;
+                sn[p] = rot[p] ? __ldg(tab + half) : 0.f;
+            }
+            const int kv = !is_q && ro.kv_slot ? __ldg(ro.kv_slot + token) : -1;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+            for (int s = 0; s < ep.splits; ++s) {
+                const float4 t = *reinterpret_cast<const float4*>(ep.partial + (size_t)s * plane + 4 * q);
+                v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+            }
+            bf16* dst = ro.q_out + ((size_t)token * ro.nh + head) * ro.hd;
+            if (!is_q) {
+                const long long row = rope_page_row(ro, kv, head - ro.nh - (rotates ? 0 : ro.nkv));
+                if (row < 0) continue;
+                dst = (rotates ? ro.k_pages : ro.v_pages) + (size_t)row * ro.hd;
+            }
+            const float x[4] = {v.x + bias_at(ep, j), v.y + bias_at(ep, j + 1), v.z + bias_at(ep, j + 2), v.w + bias_at(ep, j + 3)};
+            float a[2], b[2];       // of each pair: the first half's channel and the second's
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                a[p] = rot[p] ? x[2 * p] * cs[p] + x[2 * p + 1] * -sn[p] : x[2 * p];
+                b[p] = rot[p] ? x[2 * p + 1] * cs[p] + x[2 * p] * sn[p] : x[2 * p + 1];
+            }
+            if (rot[1]) {           // (both: the rotated channels come first)
+                const int c = li >> 1;
+                *reinterpret_cast<uint32_t*>(dst + c) = bw::pack_bf16x2(a[0], a[1]);
+                if ((half & 1) == 0) *reinterpret_cast<uint32_t*>(dst + c + half) = bw::pack_bf16x2(b[0], b[1]);
+                else { dst[c + half] = __float2bfloat16_rn(b[0]); dst[c + half + 1] = __float2bfloat16_rn(b[1]); }
+            } else {
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    const int c = rot[p] ? (li >> 1) + p : li + 2 * p;
+                    dst[c] = __float2bfloat16_rn(a[p]);
+                    dst[c + (rot[p] ? half : 1)] = __float2bfloat16_rn(b[p]);
+                }
+            }
         }
         return;
     }
@@ -1173,15 +1244,22 @@ double gemm_single_cost(int M, int N, int K, int bn, long long tiles, int splits
 }
 }  // namespace
 
-// CTA pairs for out[M, N] = x[M, K] . w[N, K]^T with M > 256: the tile width (256 or 224) and the number of K
-// splits (1 to 4, each of 8 k-blocks or more, their planes within the scratch) with the lowest estimate, which
-// is returned (negative: pairs cannot take it).  force_splits > 0 fixes the splits.
-BW_EXPORT double bw_gemm_tc_pair_plan(int M, int N, int K, int force_splits, long long workspace_elems, int* width, int* splits) {
+// CTA pairs for out[M, N] = x[M, K] . w[N, K]^T with M > 128: the tile width (256 or 224, with `narrow` also 192 or 128) and the number
+// of K splits (1 to 4, each of 8 k-blocks or more, their planes within the scratch) with the lowest estimate, which is returned
+// (negative: pairs cannot take it).  force_splits > 0 fixes the splits.
+// A tile's cost in columns of a 256-wide one: a narrow tile draws nearly as many bytes per k-block (the tokens' half), and from 192
+// columns down those bound it.  Measured, us in one round of the pairs: K 4096, 512 tokens: 26.4 (256), 24.5 (224), 22.5 (192), 21.3
+// (160), 20.4 (128); K 14336, 648 tokens 78.6, 69.8, 67.0; per k-block over many rounds 0.38, 0.35, 0.30, 0.30, 0.29.  (240 columns
+// were no faster than 256, 160 hardly faster than 192 where both fit a round.)  What the two narrow ones give: o of 3584 at 648 and 1,536
+// tokens 22.5 -> 20.3 and 37.4 -> 34.0, its down projection 87.4 -> 81.8 and 171 -> 161, q/k/v of 6144 x 4096 at 512 and 1,024 tokens
+// 31.9 -> 28.8 and 48.0 -> 44.5, o of 5120 at 2,048 82 -> 77, its down projection 217 -> 197.
+static double pair_plan(int M, int N, int K, int force_splits, long long workspace_elems, bool narrow, int* width, int* splits) {
     const int NUM_SMS = bw::num_sms();
     const int kb_total = ceil_div(K, BK), pa = ceil_div(M, 2 * BM);
-    const int widths[2] = {256, 224};   // (240 works but was measured no faster than 256)
+    const int widths[4] = {256, 224, 192, 128};
+    const double columns[4] = {256.0, narrow ? 236.0 : 224.0, 205.0, 184.0};
     double best = -1.0;
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < (narrow ? 4 : 2); ++i) {
         const long long t = (long long)pa * ceil_div(N, widths[i]);
         for (int ps = 1; ps <= 4; ++ps) {
             if (force_splits > 0 && ps != (force_splits > kb_total ? kb_total : force_splits)) continue;
@@ -1191,11 +1269,82 @@ BW_EXPORT double bw_gemm_tc_pair_plan(int M, int N, int K, int force_splits, lon
             // way through memory costs more than the idle pairs (o at 512 tokens: 38 against 26 us).
             if (ps > 1 && force_splits <= 0 && (ps != 2 || kb_total < 128 || t * ps > NUM_SMS / 2)) continue;
             if (ps > kb_total || (ps > 1 && (long long)ps * M * N > workspace_elems)) continue;
-            const double cost = (double)ceil_div(t * ps, NUM_SMS / 2) * ceil_div(kb_total, ps) * widths[i] + split_sum_cost(M, N, ps);
+            const double cost = (double)ceil_div(t * ps, NUM_SMS / 2) * ceil_div(kb_total, ps) * columns[i] + split_sum_cost(M, N, ps);
             if (best < 0.0 || cost < best * 0.995) { best = cost; *width = widths[i]; *splits = ps; }
         }
     }
     return best;
+}
+// The same among the wide tiles.
+BW_EXPORT double bw_gemm_tc_pair_plan(int M, int N, int K, int force_splits, long long workspace_elems, int* width, int* splits) {
+    return pair_plan(M, N, K, force_splits, workspace_elems, false, width, splits);
+}
+
+// SwiGLU on CTA pairs in the other orientation, tiles of 256 features x 96 to 256 tokens: the tokens need no whole tiles of 256.  The
+// estimate as pair_plan makes it (columns of a tile as long as 256 of them would take; measured per k-block over many rounds 0.38 us at 256
+// tokens a tile, 0.33, 0.29, 0.27, 0.25, 0.22), *width set.  Against tiles of 256 tokens (us, 28672 x 4096: 300 tokens 86 -> 74, 550 120 -> 103,
+// 648 123 -> 115, 1,100 197 -> 176, 1,300 229 -> 213; 37888 x 3584: 648 136 -> 126, 1,300 302 -> 234); where the estimates differ by less than
+// 7 % either may be the faster one by 4 %.
+static double swiglu_pair_plan(int M, int N, int K, int* width) {
+    const int widths[6] = {256, 224, 192, 160, 128, 96};
+    const double columns[6] = {256.0, 222.0, 197.0, 182.0, 167.0, 148.0};
+    double best = -1.0;
+    for (int i = 0; i < 6; ++i) {
+        const long long t = (long long)ceil_div(N, 2 * BM) * ceil_div(M, widths[i]);
+        const double cost = (double)ceil_div(t, bw::num_sms() / 2) * ceil_div(K, BK) * columns[i];
+        if (best < 0.0 || cost < best) { best = cost; *width = widths[i]; }
+    }
+    return best;
+}
+
+// How a product runs, from bw_gemm_tc_plan's decision (transposed, bn, splits) and the pairs' estimate.  kind: 0 plain, 1 SwiGLU, 2 rotary,
+// 3 sums left open.  pair_mode: bw_gemm_tc_pair_mode's.  Returns 1 for CTA pairs (bn: a pair's features; transposed: its tokens), 0 for single CTAs.
+BW_EXPORT int bw_gemm_tc_route(int M, int N, int K, int kind, int pair_mode, int force_splits, long long workspace_elems, int* transposed,
+                               int* bn, int* splits) {
+    const int NUM_SMS = bw::num_sms();
+    const int kb_total = ceil_div(K, BK);
+    int width = 0, ps = 1;
+    if (*transposed) {
+        if (force_splits > 0 || kind == 3) return 0;
+        if (kind == 1 && M > 64 && M <= BM && ceil_div(N, BM) > NUM_SMS) {
+            // Gate/up of 65 to 128 tokens in more tiles of 128 features than SMs: whole tiles of 128 tokens and 224 or 256 features where
+            // those take no more columns a CTA.  The other orientation's SwiGLU, two lanes a value and stores of two bytes, takes longer
+            // than a tile's products (28672 x 4096, 93 / 128 tokens: 59 / 62 us, so 50 / 50; 37888 x 3584: 56 / 59 and 53 / 53; 64 tokens
+            // 51.6 and 49.7, 48 tokens 50.0 and 49.7).
+            long long least = (long long)ceil_div(ceil_div(N, BM), NUM_SMS) * BM;
+            for (const int wd : {224, 256}) {
+                const long long cost = (long long)ceil_div(ceil_div(N, wd), NUM_SMS) * wd;
+                if (cost < least || (cost == least && *transposed)) { least = cost; *transposed = 0; *bn = wd; *splits = 1; }
+            }
+        }
+        // 129 to 256 tokens on one pair tile of tokens, but for a long K, whose splits the 128-row tiles of features deal out better (us, as
+        // they were / on pairs: gate/up of 28672 x 4096 at 160 and 256 tokens 77 / 54 and 92 / 56, q/k/v of 6144 x 4096 31 / 24 and 39 / 25,
+        // o of 4096 at 160, 200 and 256 17.5 / 19.2, 20.7 / 19.4 and 21.4 / 19.4, its down projection 36 to 40 / 54)
+        if (pair_mode > 0 && M > BM && (kind != 0 || (kb_total < 128 && (M > 160 || *splits == 1)))) {
+            const double pair = pair_plan(M, N, K, 0, workspace_elems, true, &width, &ps);
+            if (pair < 0.0) return 0;
+            *transposed = 0; *bn = width; *splits = ps;
+            if (kind == 1 && swiglu_pair_plan(M, N, K, &width) < 0.93 * pair) { *transposed = 1; *bn = width; *splits = 1; }
+            return 1;
+        }
+        return 0;
+    }
+    // More than 256 tokens: CTA pairs on tiles of 256 tokens, or single CTAs: whichever the estimate says
+    // is faster (mode 0: never pairs; 1: the estimate; 2: pairs whenever they can; BW_GEMM_PAIR or
+    // bw_gemm_tc_pair_mode).  With few tiles for the 74 pairs (steps of 300 to 1,000 tokens on the
+    // products with few output features) the pairs split K as well; the partial sums are added in split
+    // order by the second kernel.
+    if (pair_mode <= 0 || M <= 2 * BM) return 0;
+    const double pair = pair_plan(M, N, K, force_splits, workspace_elems, true, &width, &ps);
+    const double single = gemm_single_cost(M, N, K, *bn, (long long)ceil_div(M, BM) * ceil_div(N, *bn), *splits);
+    int other = 0;
+    if (kind == 1 && force_splits <= 0 && swiglu_pair_plan(M, N, K, &other) < 0.93 * (pair >= 0.0 && (pair_mode == 2 || pair <= single) ? pair : single)) {
+        *transposed = 1; *bn = other; *splits = 1;
+        return 1;
+    }
+    if (pair < 0.0 || (pair_mode != 2 && pair > single)) return 0;
+    *bn = width; *splits = ps;
+    return 1;
 }
 
 constexpr int PLANES_MAX_TOKENS = 256;   // bw_gemm_tc_planes: the orientation with the features in the 128-row dimension
@@ -1235,35 +1384,24 @@ static int run_gemm_tc(const void* x, const void* w, const void* bias, int bias_
     int splits = bw_gemm_tc_plan(M, N, K, swiglu, can_split ? workspace_elems : 0, can_split ? n_counters : 0, &tr, &bn);
     if (!tr && bn < 128) return BW_ERR_BAD_ARG;   // only tiles of 128 columns or more have the normal orientation's staging
     const int kb_total = ceil_div(K, BK);
-    const long long a_rows = tr ? N : M, b_rows = tr ? M : N;
-    const int tiles_a = ceil_div(a_rows, BM), tiles_b = ceil_div(b_rows, bn);
+    const long long plan_tiles = (long long)ceil_div(tr ? N : M, BM) * ceil_div(tr ? M : N, bn);
     if (force_splits > 0) {
         splits = force_splits > kb_total ? kb_total : force_splits;
-        if (splits > 1 && (!can_split || (long long)splits * M * N > workspace_elems ||
-                           (long long)tiles_a * tiles_b * 4 > n_counters))
+        if (splits > 1 && (!can_split || (long long)splits * M * N > workspace_elems || plan_tiles * 4 > n_counters))
             return BW_ERR_BAD_ARG;
     }
-    // More than 256 tokens: CTA pairs on tiles of 256 tokens, or single CTAs: whichever the estimate says
-    // is faster (mode 0: never pairs; 1: the estimate; 2: pairs whenever they can; BW_GEMM_PAIR or
-    // bw_gemm_tc_pair_mode).  With few tiles for the 74 pairs (steps of 300 to 1,000 tokens on the
-    // products with few output features) the pairs split K as well; the partial sums are added in split
-    // order by the second kernel.
     if (g_pair_mode < 0) { const char* e = getenv("BW_GEMM_PAIR"); g_pair_mode = (e && e[0] >= '0' && e[0] <= '2') ? e[0] - '0' : 1; }
-    int pbn = 256, psplits = 1;
-    bool use_pairs = false;
-    if (g_pair_mode > 0 && !tr && M > 256) {
-        const double pair = bw_gemm_tc_pair_plan(M, N, K, force_splits, can_split ? workspace_elems : 0, &pbn, &psplits);
-        const double single = gemm_single_cost(M, N, K, bn, (long long)tiles_a * tiles_b, splits);
-        use_pairs = pair >= 0.0 && (g_pair_mode == 2 || pair <= single);
-        if (use_pairs) splits = psplits;
-    }
+    const bool use_pairs = bw_gemm_tc_route(M, N, K, planes ? 3 : rope ? 2 : swiglu ? 1 : 0, g_pair_mode, force_splits,
+                                            can_split ? workspace_elems : 0, &tr, &bn, &splits) != 0;
     const int kb_per_split = ceil_div(kb_total, splits);
     splits = ceil_div(kb_total, kb_per_split);   // no empty split
+    const long long a_rows = tr ? N : M, b_rows = tr ? M : N;
+    const int tiles_a = ceil_div(a_rows, BM), tiles_b = ceil_div(b_rows, bn);
 
     CUtensorMap ta, tb;
     const void* a_ptr = tr ? w : x; const void* b_ptr = tr ? x : w;
     const long long a_ld = tr ? K : ldx, b_ld = tr ? ldx : K;
-    if (!make_map(&ta, a_ptr, a_rows, K, a_ld, BM) || !make_map(&tb, b_ptr, b_rows, K, b_ld, bn)) return BW_ERR_DRIVER;
+    if (!make_map(&ta, a_ptr, a_rows, K, a_ld, BM) || !make_map(&tb, b_ptr, b_rows, K, b_ld, use_pairs ? bn / 2 : bn)) return BW_ERR_DRIVER;
 
     Epilogue ep;
     // few tokens: the last warp of each tile sums the splits inside the kernel; more: a second kernel
@@ -1294,7 +1432,7 @@ static int run_gemm_tc(const void* x, const void* w, const void* bias, int bias_
     if (!tr && splits == 1 && !rope && !swiglu && !planes && ((uintptr_t)out & 15) == 0 && ldo % (out_type == BW_F32 ? 4 : 8) == 0) {
         // (boxes that are written need tiles of whole boxes: 240 columns are seven and a half)
         if (accumulate) ep.tma_add = BOX_ADD;
-        else if (use_pairs ? pbn % 32 == 0 : bn % 32 == 0) ep.tma_add = out_type == BW_F32 ? BOX_F32 : BOX_BF16;
+        else if (bn % 32 == 0) ep.tma_add = out_type == BW_F32 ? BOX_F32 : BOX_BF16;
         if (ep.tma_add && !make_out_map(&tc, out, M, N, ldo, out_type == BW_F32)) return BW_ERR_DRIVER;
     }
     const int num_work = stream_k ? NUM_SMS : tiles_a * tiles_b * splits;
@@ -1309,12 +1447,12 @@ static int run_gemm_tc(const void* x, const void* w, const void* bias, int bias_
         case 256: rc = launch<256, R>(ta, tb, tc, ep, kb_total, kb_per_split, tiles_a, tiles_b, num_work, s); break; \
         default: return BW_ERR_BAD_ARG; }
     if (use_pairs) {
-        CUtensorMap tb2;
-        if (!make_map(&tb2, b_ptr, b_rows, K, b_ld, pbn / 2)) return BW_ERR_DRIVER;
-        const int pa = ceil_div(M, 2 * BM), pb = ceil_div(N, pbn);
-#define BW_PAIR_LAUNCH(W) (rope ? launch_pair<W, true>(ta, tb2, tc, ep, kb_total, kb_per_split, pa, pb, s) \
-                                : launch_pair<W, false>(ta, tb2, tc, ep, kb_total, kb_per_split, pa, pb, s))
-        rc = pbn == 256 ? BW_PAIR_LAUNCH(256) : BW_PAIR_LAUNCH(224);
+        const int pa = ceil_div(a_rows, 2 * BM), pb = ceil_div(b_rows, bn);
+#define BW_PAIR_LAUNCH(W) (rope ? launch_pair<W, true>(ta, tb, tc, ep, kb_total, kb_per_split, pa, pb, s) \
+                                : launch_pair<W, false>(ta, tb, tc, ep, kb_total, kb_per_split, pa, pb, s))
+        rc = bn == 256 ? BW_PAIR_LAUNCH(256) : bn == 224 ? BW_PAIR_LAUNCH(224) : bn == 192 ? BW_PAIR_LAUNCH(192) : bn == 128 ? BW_PAIR_LAUNCH(128)
+           : bn == 160 ? launch_pair<160, false>(ta, tb, tc, ep, kb_total, kb_per_split, pa, pb, s)      // (SwiGLU only)
+                       : launch_pair<96, false>(ta, tb, tc, ep, kb_total, kb_per_split, pa, pb, s);
 #undef BW_PAIR_LAUNCH
     } else
     if (rope) BW_GEMM_LAUNCH(true) else BW_GEMM_LAUNCH(false)

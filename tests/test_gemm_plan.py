@@ -116,3 +116,29 @@ def test_pair_plan_splits_k_only_where_the_pairs_would_idle():
     assert plan(512, 4096, 4096)[2] == 1 and plan(768, 4096, 14336)[2] == 1
     assert plan(2048, 28672, 4096)[2] == 1                       # gate/up at 2,048 tokens: rounds of whole tiles
     assert plan(700, 520, 2240, force=3)[2] == 3                 # a forced split is taken as it is
+
+
+@pytest.mark.parametrize("kind", (0, 1, 2, 3))
+def test_every_route_is_one_the_kernels_are_built_for(plan, kind):
+    """``bw_gemm_tc_route``: single CTAs in either orientation or CTA pairs (kind 0 plain, 1 SwiGLU, 2 rotary, 3 sums left open)."""
+    from blackwellllm_b200.kernels.build import load_library
+    fn = load_library("gemm_tc").bw_gemm_tc_route
+    fn.argtypes = [ctypes.c_int] * 6 + [ctypes.c_longlong] + [ctypes.POINTER(ctypes.c_int)] * 3
+    for M, (N, K), mode, force in itertools.product(TOKENS + (129, 160, 161, 200, 640), PRODUCTS, (0, 1, 2), (0, 3)):
+        if kind == 1 and N % 32 or kind == 3 and M > 256:
+            continue
+        for workspace in (0, 3 * M * N, 1 << 24):
+            planned, tr0, bn0 = plan(M, N, K, int(kind == 1), workspace)
+            tr, bn, splits = ctypes.c_int(tr0), ctypes.c_int(bn0), ctypes.c_int(planned)
+            pairs = fn(M, N, K, kind, mode, force, workspace, ctypes.byref(tr), ctypes.byref(bn), ctypes.byref(splits))
+            what = f"M={M} N={N} K={K} kind={kind} mode={mode} force={force}: pairs={pairs} {tr.value} {bn.value} {splits.value}"
+            assert splits.value == 1 or splits.value * M * N <= workspace, what
+            if pairs:
+                assert mode and M > 128 and kind != 3, what
+                if tr.value:        # the SwiGLU of 256 features x bn tokens
+                    assert kind == 1 and bn.value in (96, 128, 160, 192, 224, 256) and splits.value == 1 and not force, what
+                else:
+                    assert bn.value in (128, 192, 224, 256), what
+                assert not force or M > 256, what
+            elif (tr.value, bn.value, splits.value) != (tr0, bn0, planned):
+                assert kind == 1 and 64 < M <= 128 and tr.value == 0 and bn.value in (224, 256) and splits.value == 1, what

@@ -321,6 +321,50 @@ def test_gemm_tc_rotary_epilogue(ops, M, splits, nh, nkv, hd, rd, page):
     assert ops.gemm_tc_status() == 0
 
 
+# the edges of the routes (64 | 65, 128 | 129, 256 | 257 tokens), tokens that leave a tile ragged, and products of fewer or more
+# tiles than SMs
+@pytest.mark.parametrize("M", [65, 93, 128, 129, 161, 200, 256, 257, 300, 550, 648])
+@pytest.mark.parametrize("I,K", [(176, 264), (528, 1000), (9616, 72)])
+def test_gemm_tc_swiglu_of_65_to_648_tokens(ops, M, I, K):
+    """Single CTAs on 128 tokens, CTA pairs in either orientation; biases; an output whose rows are further apart than they are long."""
+    x = rand(M, K, dtype=torch.bfloat16, seed=1).to(DEV)
+    wg, wu = (rand(I, K, dtype=torch.bfloat16, seed=2 + i, scale=0.05).to(DEV) for i in range(2))
+    bg, bu = (rand(I, seed=4 + i, scale=0.2).to(DEV) for i in range(2))
+    bias = ops.interleave_gate_up(bg.view(-1, 1), bu.view(-1, 1)).view(-1)
+    wide = torch.full((M, I + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.gemm_tc(x, ops.interleave_gate_up(wg, wu), bias, out=wide[:, :I], swiglu=True)
+    ref = plain_swiglu(x.double() @ wg.double().T + bg.double(), x.double() @ wu.double().T + bu.double())
+    assert ops.gemm_tc_status() == 0
+    # the product's 2^-9 (bfloat16) of each value, silu's derivative below 1.1 and the factor u: 2^-7 of the largest leaves room for both
+    assert float((wide[:, :I].double() - ref).abs().max()) <= 2 ** -7 * float(ref.abs().max())
+    assert bool((wide[:, I:] == 7.0).all())
+
+
+@pytest.mark.parametrize("M", [17, 65, 128, 129, 200, 256, 257, 650])
+@pytest.mark.parametrize("nh,nkv,hd,rd,bias_dtype", [(28, 4, 128, 128, torch.bfloat16), (5, 1, 48, 32, torch.float32), (3, 1, 16, 6, None)])
+def test_gemm_tc_rotary_routes(ops, M, nh, nkv, hd, rd, bias_dtype):
+    """The rotation in each route's epilogue and in the second kernel, against the plain product and :func:`rope_append`."""
+    K, page = 520, 16
+    N = (nh + 2 * nkv) * hd
+    x, w = rand(M, K, dtype=torch.bfloat16, seed=1).to(DEV), rand(N, K, dtype=torch.bfloat16, seed=2, scale=0.1).to(DEV)
+    b = None if bias_dtype is None else rand(N, seed=3, scale=0.5).to(DEV, bias_dtype)
+    positions = (torch.randperm(M, generator=torch.Generator().manual_seed(5)).to(torch.int32) + 900).to(DEV)
+    blocks = (M + 900) // page + 1
+    table = torch.arange(blocks, dtype=torch.int32, device=DEV).flip(0).contiguous().view(1, blocks)
+    req = torch.zeros(M, dtype=torch.int32, device=DEV)
+    inv = plain_inv_freq(hd, 10000.0, None, rotary_dim=rd).float().to(DEV)
+    tab = ops.rope_table(positions, inv, rd)
+    slots = ops.kv_slots(positions, req, table, page, blocks)
+    pages = torch.zeros(2, 2, blocks, nkv, page, hd, dtype=torch.bfloat16, device=DEV)
+    got = ops.gemm_tc_rope(x, w, b, tab, slots, pages[0, 0], pages[0, 1], nh, nkv, hd, rd)
+    qkv = (x.double() @ w.double().T + (0.0 if b is None else b.double())).float()
+    want = ops.rope_append(qkv, positions, req, table, inv, rd, pages[1, 0], pages[1, 1], nh, nkv, hd, table=tab, paired=True)
+    assert ops.gemm_tc_status() == 0
+    # both round the same sums to bfloat16 once: where float32 sums differ in their last bits, by 2^-8 of the value at most
+    for a, r in ((got, want), (pages[0, 0], pages[1, 0]), (pages[0, 1], pages[1, 1])):
+        assert float((a.float() - r.float()).abs().max()) <= 2 ** -8 * float(r.float().abs().max())
+
+
 def test_gemm_tc_row_independent_of_batch(ops):
     """A token's row does not depend on which other tokens share the launch."""
     K, N = 1024, 768
