@@ -1108,30 +1108,50 @@ def plan_attention_work(q_len, q_start, kv_len, G: int, nkv: int, window: Option
     slot) for requests with more than one slice; and the number of partial-result slots."""
     tpt = rows_tile // G   # tokens of one tile of stacked rows
     rows_items, keys_items, merge_items = [], [], []
-    n_small = sum(1 for n in q_len if n * G <= 16)
     # CTAs of the key-slice kernel that fit on the GPU at once (shared memory bound)
     if hd % 64 == 0 and page_size in (8, 16, 32, 64):   # the TMA-fed kernel: 2 stages of unpadded tiles
         smem = 2 * 2 * 64 * hd * 2 + 16 * (hd * 2 + 16) + 2048
     else:
         smem = (16 + 4 * 64) * (hd * 2 + 16)
     slots = sms * max(1, min(8, (227 * 1024) // (smem + 1024)))
-    heads = max(1, n_small * nkv)
-    if heads <= slots:
-        want = slots // heads            # one full wave: all slices run side by side, no tail
-    else:
-        want = -(-4 * slots // heads)    # many short CTAs: at least four waves smooth the tail
-    total_slices = 0
+    spans = {}      # key tiles of every request that is cut into slices
     for r, n_q in enumerate(q_len):
         if n_q * G > 16:
-            rows_items += [(r, t0, 0, 0) for t0 in range(0, n_q, tpt)]
             continue
         span = static_bound or kv_len[r]
         if window:   # (kept first keys lie in tiles of their own before the window's)
             span = min(span, window + n_q + (-(-keep_first // 64) * 64 if keep_first else 0))
         if chunk:   # a query sees no key before the start of its block of positions
             span = min(span, chunk + n_q)
-        tiles = -(-span // 64)
-        n = max(1, min(want, tiles // 2, 64))
+        spans[r] = -(-span // 64)
+    heads = max(1, len(spans) * nkv)
+    if heads <= slots:
+        want = slots // heads            # one full wave: all slices run side by side, no tail
+    else:
+        want = -(-4 * slots // heads)    # many short CTAs: at least four waves smooth the tail
+    cut = {r: max(1, min(want, tiles // 2, 64)) for r, tiles in spans.items()}
+    if len(set(spans.values())) > 1:
+        # Requests of different lengths get slices of one length, the shortest with which their number stays what it was: with one
+        # number of slices for all, the longest request's are alone at the end (31 requests at 512 to 4,096 keys, 4 kv heads of 128,
+        # 28 query heads: 53 us, 35 so)
+        most = want * len(spans)
+
+        def slices(per):
+            return {r: max(1, min(-(-tiles // per), tiles // 2, 64)) for r, tiles in spans.items()}
+        lo, hi = 2, max(spans.values())
+        while lo < hi:
+            mid = (lo + hi) // 2
+            if sum(slices(mid).values()) <= most:
+                hi = mid
+            else:
+                lo = mid + 1
+        cut = slices(lo)
+    total_slices = 0
+    for r, n_q in enumerate(q_len):
+        if n_q * G > 16:
+            rows_items += [(r, t0, 0, 0) for t0 in range(0, n_q, tpt)]
+            continue
+        n = cut[r]
         keys_items += [(r, s, n, total_slices) for s in range(n)]
         if n > 1:
             merge_items.append((r, 0, n, total_slices))
