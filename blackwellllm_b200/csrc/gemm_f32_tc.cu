@@ -23,10 +23,10 @@
 // Roles (896 threads): warp 0 loads weights; warp 1 TMEM owner and MMAs; warp 2 loads tokens; warps 4..11 split the weights, two
 // groups that take stages in turn; warps 12..27 add the accumulators up, 32 tokens each group of four, and write the result.  Every
 // wait is bounded; a timeout sets the status word and all roles fall through to the exit.
-// What bounds it: up to 16 tokens the weights' bytes; beyond, what a stage of 32 channels takes from its split to its sums: at 128 tokens
-// about 1,700 cycles, the two small kernels' share included, of which its twelve MMAs are 768 (64 each, measured by themselves).
-// Measured, x 28672 x 4096, with the small kernels, on several B200s: 1 to 16 tokens 86 to 93 us (5.0 to 5.5 TB/s), 64 tokens 122 to
-// 129, 128 tokens 168 to 176 (about 175 TFLOP/s), 301 tokens 490 to 527.  gemm_simt.cu: 301 tokens 3.1 ms.
+// What bounds it: up to 16 tokens the weights' bytes; beyond, shared memory: a stage of 32 channels at 112 tokens moves 103 KB of it (the
+// weights' tile in and out 32, the tokens' in 28, what its twelve MMAs read 43), 800 cycles at 128 bytes, of which the MMAs alone need 670.
+// Measured, x 28672 x 4096, with the small kernels, on several B200s: 1 to 16 tokens 79 to 84 us (5.6 to 6.0 TB/s), 64 tokens 114, 128
+// tokens 149 (202 TFLOP/s), 301 tokens 404 to 415.  gemm_simt.cu: 301 tokens 3.1 ms.
 #include "tcgen05.cuh"
 
 using bf16 = __nv_bfloat16;
@@ -56,13 +56,22 @@ __host__ __device__ constexpr int w_stages(int bn) {
 }
 // A warp that waits for a phase by its parity must not be two phases ahead of it.  The split groups take stages in turn, and what holds
 // a group back is its own slot among the split weights: behind it at most t_stages stages are unfinished.  So no slot may have two
-// groups waiting for it, and a stage of the weights' ring may come round again only after the group that had it before is done.
+// groups waiting for it, and a stage of the weights' ring may come round again only after the group that had it before is done.  A
+// slot of the tokens' ring is always the same group's.
 constexpr bool rings_hold() {
     for (int bn = 16; bn <= MAX_BN; bn += 16)
-        if (t_stages(bn) < SPLIT_GROUPS || w_stages(bn) < t_stages(bn) + SPLIT_GROUPS) return false;
+        if (t_stages(bn) < SPLIT_GROUPS || w_stages(bn) < t_stages(bn) + SPLIT_GROUPS || x_stages(bn) % SPLIT_GROUPS) return false;
     return true;
 }
 static_assert(rings_hold(), "a split group could pass a wait two phases early");
+// More than 64 tokens: the warps that split the weights, which wait most of the time, also wait, in the MMA warp's place, for the stage's
+// tokens and for the accumulator that a pair of stages begins: each wait between two stages' products leaves the tensor pipe without
+// work (it has about two instructions queued): x 28672 x 4096, 93 tokens 140 us, 129 so; 128 tokens 163 and 152, K 14336, 301 tokens 234
+// and 217.  Up to 64 tokens the weights' bytes bound, and the split is on their way (16 tokens 86 us, 89 so).  A wait for an accumulator of
+// stage i, the first of a pair p, must find the wait of pair p - 2 over: that pair begins with stage i - 2, the group's own, or with an
+// earlier one, done as the group knows from its wait for the slot of stage i, if there are three slots at most.
+__host__ __device__ constexpr bool split_waits(int bn) { return bn > 64; }
+static_assert(t_stages(80) <= 3 && t_stages(128) <= 3, "with four slots stage i - 3 may be another group's, unfinished");
 __host__ __device__ constexpr int ring_bytes(int bn) { return w_stages(bn) * A_BYTES + x_stages(bn) * x_bytes(bn); }
 
 // x rounded to TF32, halves away from zero (three integer instructions fewer than the conversion instruction takes; a NaN whose
@@ -173,6 +182,7 @@ split_kernel(const float* __restrict__ x, float* __restrict__ xs, int M, int K, 
     }
 }
 
+template <bool SPLIT_WAITS>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, Out o, int bn, Cut cut,
                    int tiles_m) {
@@ -251,8 +261,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             for (int i = 0; ok && i < n; ++i) {
                 const int buf = p & 1;
                 const bool fresh = i % SUM_STAGES == 0, last = i % SUM_STAGES == SUM_STAGES - 1 || i == n - 1;
-                ok = bw::mbar_wait(xfull0 + 8 * xst, xph, &g_status, 4) && bw::mbar_wait(ready0 + 8 * tst, tph, &g_status, 5);
-                if (fresh) ok = ok && bw::mbar_wait(sum_free0 + 8 * buf, ((p >> 1) & 1) ^ 1, &g_status, 6);
+                if constexpr (SPLIT_WAITS) {     // (the warps that say `ready` have waited for the tokens' tile and the accumulator)
+                    ok = bw::mbar_wait(ready0 + 8 * tst, tph, &g_status, 5);
+                } else {
+                    ok = bw::mbar_wait(xfull0 + 8 * xst, xph, &g_status, 4) && bw::mbar_wait(ready0 + 8 * tst, tph, &g_status, 5);
+                    if (fresh) ok = ok && bw::mbar_wait(sum_free0 + 8 * buf, ((p >> 1) & 1) ^ 1, &g_status, 6);
+                }
                 if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
                 bw::tc_fence_after();
                 const uint32_t d = small + (1 + buf) * acc_cols(bn), hi = cols_a + tst * 64;
@@ -277,11 +291,13 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         }
     } else if (warp >= 4 && warp < 4 + 4 * SPLIT_GROUPS) {
         const int quarter = warp & 3, row = quarter * 32 + lane;
-        const int mine = (tiles_m - (int)blockIdx.y + (int)gridDim.y - 1) / (int)gridDim.y;            // tiles of tokens
-        const long long all = (cut.begin(blockIdx.x + 1) - cut.begin(blockIdx.x)) * mine;         // stages of all items
         const uint32_t tmem_a = tmem + 3 * acc_cols(bn) + ((uint32_t)(quarter * 32) << 16);
         const int group = (warp - 4) / 4;
-        int s = group, ph = 0, slot = group, tph = 1;
+        const int mine = (tiles_m - (int)blockIdx.y + (int)gridDim.y - 1) / (int)gridDim.y;            // tiles of tokens
+        const long long all = (cut.begin(blockIdx.x + 1) - cut.begin(blockIdx.x)) * mine;         // stages of all items
+        int s = group, ph = 0, slot = group, tph = 1, xst = group, xph = 0;
+        int at = group, before = 0;              // the stage within its item; the pairs of stages in the items before
+        if constexpr (SPLIT_WAITS) it.next();
         for (long long i = group; i < all; i += SPLIT_GROUPS) {
             if (!__all_sync(0xffffffffu, bw::mbar_wait(wfull0 + 8 * s, ph, &g_status, 7))) break;
             const uint8_t* src = smem + s * A_BYTES + row * 128;
@@ -314,6 +330,17 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 bw::tmem_st_32x16(dst + 32 + 16 * h, lo);
             }
             bw::tmem_st_wait();
+            if constexpr (SPLIT_WAITS) {
+                while (at >= it.n) { at -= it.n; before += (it.n + SUM_STAGES - 1) / SUM_STAGES; if (!it.next()) break; }
+                const int p = before + at / SUM_STAGES;
+                bool ok = bw::mbar_wait(xfull0 + 8 * xst, xph, &g_status, 4);
+                if (at % SUM_STAGES == 0) ok = ok && bw::mbar_wait(sum_free0 + 8 * (p & 1), ((p >> 1) & 1) ^ 1, &g_status, 6);
+                if (!__all_sync(0xffffffffu, ok)) break;
+                bw::tc_fence_after();
+                at += SPLIT_GROUPS;
+                xst += SPLIT_GROUPS;
+                if (xst >= xs) { xst -= xs; xph ^= 1; }
+            }
             bw::tc_fence_before();
             __syncwarp();
             if (lane == 0) bw::mbar_arrive(ready0 + 8 * slot);
@@ -395,34 +422,75 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     if (warp == 1) bw::tmem_dealloc(tmem, 512);
 }
 
-// The parts of the tiles that several ranges share, in their order; four features a thread where V is 4.
+// The parts of the tiles that several ranges share, in their order; V features of SUM_TOKENS tokens a thread.  Where the parts lie takes
+// some 64-bit divisions, made before the wait for the products and once for the tokens (the whole product, x 6144 x 4096, with a token a
+// thread and so: 301 tokens 106 and 101 us, 1 token 29.6 and 27.9).  V 4: rows of the result begin on 16 bytes.
+constexpr int SUM_TOKENS = 4;
 template <int V>
 __global__ void __launch_bounds__(256)
 sum_kernel(Out o, Cut cut) {
     BW_PDL_TRIGGER();
-    BW_PDL_WAIT();
-    const int n = (blockIdx.x * blockDim.x + threadIdx.x) * V, m = blockIdx.y;
+    const int n = (blockIdx.x * blockDim.x + threadIdx.x) * V, m0 = blockIdx.y * SUM_TOKENS, tokens = min(SUM_TOKENS, o.M - m0);
     const bool in = n < o.N;
     const int tile = min(n, o.N - 1) / BM, parts = cut.parts(tile), first = cut.first_part(tile);
+    constexpr int KNOWN = 4;
+    size_t at[KNOWN];                // of the first parts; a weight of few features and many channels has more
+#pragma unroll
+    for (int i = 0; i < KNOWN; ++i) at[i] = i < parts ? (size_t)cut.piece(first + i, tile) * o.M * BM : 0;
+    float bias[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) bias[e] = in ? bias_at(o, n + e) : 0.f;
+    BW_PDL_WAIT();
     if (parts == 1) return;          // (a warp's features lie in one tile)
-    float s[V];
+    const float* p = o.part + (size_t)m0 * BM + (n - tile * BM);
+    float* dst = o.out + m0 * o.ldo + n;
+    auto load = [&](const float* from, bool there, float (&v)[V]) {
+        if constexpr (V == 4) {
+            const float4 t = there ? *reinterpret_cast<const float4*>(from) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+        } else v[0] = there ? *from : 0.f;
+    };
+    float s[SUM_TOKENS][V], old[SUM_TOKENS][V];
 #pragma unroll
-    for (int e = 0; e < V; ++e) s[e] = 0.f;
-    for (int i = 0; in && i < parts; ++i) {
-        const float* p = o.part + ((size_t)cut.piece(first + i, tile) * o.M + m) * BM + (n - tile * BM);
-        float v[V];
-        if constexpr (V == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
-        else v[0] = *p;
-#pragma unroll
-        for (int e = 0; e < V; ++e) s[e] = i ? s[e] + v[e] : v[e];
+    for (int t = 0; t < SUM_TOKENS; ++t) {
+        load(dst + t * o.ldo, o.accumulate && in && t < tokens, old[t]);
+        load(p + at[0] + t * BM, in && t < tokens, s[t]);
     }
-    float* dst = o.out + m * o.ldo + n;
+    auto add = [&](size_t from) {
+        float v[SUM_TOKENS][V];
 #pragma unroll
-    for (int e = 0; e < V; ++e) {
-        s[e] = chains(o, s[e] != s[e], s[e], m, n + e);
-        if (!in) continue;
-        s[e] += bias_at(o, n + e);
-        dst[e] = o.accumulate ? s[e] + dst[e] : s[e];
+        for (int t = 0; t < SUM_TOKENS; ++t) load(p + from + t * BM, in && t < tokens, v[t]);
+#pragma unroll
+        for (int t = 0; t < SUM_TOKENS; ++t)
+#pragma unroll
+            for (int e = 0; e < V; ++e) s[t][e] += v[t][e];
+    };
+#pragma unroll
+    for (int i = 1; i < KNOWN; ++i) if (i < parts) add(at[i]);
+    for (int i = KNOWN; i < parts; ++i) add((size_t)cut.piece(first + i, tile) * o.M * BM);
+    unsigned again = 0;              // the results that chain() makes
+#pragma unroll
+    for (int t = 0; t < SUM_TOKENS; ++t) {
+        if (!in || t >= tokens) continue;
+        unsigned nan = 0;
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            nan |= s[t][e] != s[t][e] ? 1u << e : 0u;
+            s[t][e] += bias[e];
+            if (o.accumulate) s[t][e] += old[t][e];
+        }
+        again |= nan << (t * V);
+        if (V == 4 && !nan) *reinterpret_cast<float4*>(dst + t * o.ldo) = make_float4(s[t][0], s[t][1 % V], s[t][2 % V], s[t][3 % V]);
+        else {
+#pragma unroll
+            for (int e = 0; e < V; ++e) if (!(nan >> e & 1)) dst[t * o.ldo + e] = s[t][e];
+        }
+    }
+    for (unsigned any = __reduce_or_sync(0xffffffffu, again); any; any &= any - 1) {
+        const int k = __ffs(any) - 1, t = k / V, e = k % V;
+        const bool wanted = again >> k & 1;
+        const float v = chains(o, wanted, 0.f, m0 + t, n + e) + (wanted ? bias_at(o, n + e) : 0.f);
+        if (wanted) dst[t * o.ldo + e] = o.accumulate ? v + dst[t * o.ldo + e] : v;
     }
 }
 
@@ -476,19 +544,21 @@ BW_EXPORT int bw_gemm_f32_tc(const float* x, const float* w, const void* bias, i
     const long long pieces = ((long long)M * (K / 4) + 255) / 256;
     bw::launch(split_kernel, dim3((unsigned)(pieces < 4 * bw::num_sms() ? pieces : 4 * bw::num_sms())), dim3(256), 0, s, x, xs, M, K, ldx);
     BW_LAUNCH_CHECK();
-    static bool done[bw::MAX_DEVICES] = {};
-    const cudaError_t e = bw::allow_dynamic_smem(gemm_f32_tc_kernel, SMEM_BUDGET + 1024, done);
+    static bool done[2][bw::MAX_DEVICES] = {};
+    const auto kernel = split_waits(bn) ? gemm_f32_tc_kernel<true> : gemm_f32_tc_kernel<false>;
+    const cudaError_t e = bw::allow_dynamic_smem(kernel, SMEM_BUDGET + 1024, done[split_waits(bn)]);
     if (e != cudaSuccess) return (int)e;
     const Out o = {out, bias, part, x, w, ldo, ldx, bias_type, accumulate, M, N, K};
     // a small weight's ranges leave SMs idle: they take tiles of tokens (300 tokens x 1024 x 256: 23.6 us without, 11.2
     // so, 17.4 in gemm_simt.cu; 1,000 tokens: 62.6 with launches of 512, 12.1 so, 27.0)
     const int rows = bw::num_sms() / cut.ctas < tiles_m ? bw::num_sms() / cut.ctas : tiles_m;
-    bw::launch(gemm_f32_tc_kernel, dim3(cut.ctas, rows < 1 ? 1 : rows), dim3(THREADS), (size_t)ring_bytes(bn) + 1024, s, tm_w, tm_x, o, bn, cut,
+    bw::launch(kernel, dim3(cut.ctas, rows < 1 ? 1 : rows), dim3(THREADS), (size_t)ring_bytes(bn) + 1024, s, tm_w, tm_x, o, bn, cut,
                tiles_m);
     BW_LAUNCH_CHECK();
     if (shared) {
-        if (N % 4 == 0) bw::launch(sum_kernel<4>, dim3((N / 4 + 255) / 256, M), dim3(256), 0, s, o, cut);
-        else bw::launch(sum_kernel<1>, dim3((N + 255) / 256, M), dim3(256), 0, s, o, cut);
+        const int groups = (M + SUM_TOKENS - 1) / SUM_TOKENS;
+        if (N % 4 == 0 && ldo % 4 == 0 && ((uintptr_t)out & 15) == 0) bw::launch(sum_kernel<4>, dim3((N / 4 + 255) / 256, groups), dim3(256), 0, s, o, cut);
+        else bw::launch(sum_kernel<1>, dim3((N + 255) / 256, groups), dim3(256), 0, s, o, cut);
         BW_LAUNCH_CHECK();
     }
     return 0;
