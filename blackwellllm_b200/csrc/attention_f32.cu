@@ -36,8 +36,13 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool valid)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
-__host__ __device__ constexpr int smem_floats(int rows, int hd) {
-    return rows * (hd + 4) + 2 * KEYS * (hd + 4) + 2 * KEYS * hd + rows * (KEYS + 4) + 2 * KEYS;
+// Tiles of keys in flight or at work: prompts work on a tile for longer than the next one takes to come; a decoding request's few rows do not.
+__host__ __device__ constexpr int stages(int rows) { return rows == 64 ? 2 : 3; }
+// Keys that a block fetches and scores at once (the softmax takes KEYS of them at a time).  Of a prompt's 64 rows a thread scores 4 x 4 with
+// 64 keys, eight 16-byte reads of shared memory per 64 FMAs; with 32 keys 2 x 4, six reads per 32, which the reads bound.
+__host__ __device__ constexpr int fetched(int rows, int ch, bool slices) { return rows == 64 && ch == 1 && !slices ? 64 : KEYS; }
+__host__ __device__ constexpr int smem_floats(int rows, int hd, int kt) {
+    return rows * (hd + 4) + stages(rows) * (kt * (hd + 4) + kt * hd + kt) + rows * (kt + 4);
 }
 
 // One more slice (maximum m, sum l) of a row: the factors of what was there (M, L) and of the slice; M and L are updated.  A slice in
@@ -67,17 +72,17 @@ __device__ __forceinline__ size_t part_row(const Params& p, int where, int slice
 // the tile's slices, whose rows have slices of one size.  Of a single slice the block writes the tile's result (its fold is it).
 // CH: groups of four channels of a lane.
 template <int ROWS, int CH, bool SLICES>
-__global__ void __launch_bounds__(THREADS, !SLICES ? 1 : ROWS == 64 ? 2 : 3)
+__global__ void __launch_bounds__(THREADS, !SLICES ? 1 : 2)
 attention_f32_kernel(Params p, const int4* __restrict__ work) {
     BW_PDL_TRIGGER();
     extern __shared__ float4 smem4[];
     const int hd = p.hd, ldk = hd + 4, G = p.nh / p.nkv;
     float* qs = reinterpret_cast<float*>(smem4);          // [ROWS][ldk]
-    float* ks = qs + ROWS * ldk;                          // [2][KEYS][ldk]
-    float* vs = ks + 2 * KEYS * ldk;                      // [2][KEYS][hd]
-    float* ps = vs + 2 * KEYS * hd;                       // [ROWS][KEYS + 4]
-    int* known = reinterpret_cast<int*>(ps + ROWS * (KEYS + 4));   // [2][KEYS]: the key has a page
-    constexpr int LDP = KEYS + 4;
+    constexpr int STAGES = stages(ROWS), KT = fetched(ROWS, CH, SLICES), PARTS = KT / KEYS, LDP = KT + 4;
+    float* ks = qs + ROWS * ldk;                          // [STAGES][KT][ldk]
+    float* vs = ks + STAGES * KT * ldk;                   // [STAGES][KT][hd]
+    float* ps = vs + STAGES * KT * hd;                    // [ROWS][LDP]
+    int* known = reinterpret_cast<int*>(ps + ROWS * LDP); // [STAGES][KT]: the key has a page
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kvh = blockIdx.y;
     const int4 item = work[blockIdx.x];
     const int r = item.x;
@@ -100,28 +105,41 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
     }
     // a portion's rows may differ in the size of their slices (it never shrinks, except where a block of positions begins)
     const bool same = !SLICES && slice_keys(p, end - 1) == keys && (p.chunk <= 0 || p.chunk <= SLICE * MOST);
+    int pages[KT / WARPS];                          // of the keys that are fetched next, looked up before
+    auto look_up = [&](int tile) {
+#pragma unroll
+        for (int j = 0; j < KT / WARPS; ++j) {
+            const int kp = base + tile * KEYS + warp * (KT / WARPS) + j;
+            pages[j] = tile < last && kp < end ? bt[kp / p.page_size] : -1;
+        }
+    };
+    look_up(first);      // (block tables are on the device before the step's first kernel, as the work lists are)
     BW_PDL_WAIT();
 
     for (int i = warp; i < ROWS; i += WARPS) {      // with the first tile of keys; rows beyond the tile's are zeros
         const float* src = p.q + (i < rows ? ((size_t)(row0 + t0 + i / G) * p.nh + (size_t)kvh * G + i % G) * hd : 0);
         for (int c = lane * 4; c < hd; c += 128) copy16(qs + i * ldk + c, src + c, i < rows);
     }
-    auto fetch = [&](int tile) {                    // a warp brings four keys and their values
-        const int st = tile & 1;
+    auto fetch = [&](int tile, int st) {            // the KT keys from this tile on: a warp brings some and their values
 #pragma unroll
-        for (int j = 0; j < KEYS / WARPS; ++j) {
-            const int key = warp * (KEYS / WARPS) + j, kp = base + tile * KEYS + key;
-            const int page = kp < end ? bt[kp / p.page_size] : -1;
+        for (int j = 0; j < KT / WARPS; ++j) {
+            const int key = warp * (KT / WARPS) + j, kp = base + tile * KEYS + key, page = pages[j];
             const bool ok = page >= 0 && page < p.num_pages;
             const size_t at = ok ? (((size_t)page * p.nkv + kvh) * p.page_size + (kp % p.page_size)) * hd : 0;
             for (int c = lane * 4; c < hd; c += 128) {
-                copy16(ks + (st * KEYS + key) * ldk + c, p.k_pages + at + c, ok);
-                copy16(vs + (st * KEYS + key) * hd + c, p.v_pages + at + c, ok);
+                copy16(ks + (st * KT + key) * ldk + c, p.k_pages + at + c, ok);
+                copy16(vs + (st * KT + key) * hd + c, p.v_pages + at + c, ok);
             }
-            if (lane == 0) known[st * KEYS + key] = ok;
+            if (lane == 0) known[st * KT + key] = ok;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
+        look_up(tile + PARTS);
     };
+    // Rows that a warp takes through the softmax and the values: side by side in a tile of 64; of few rows one each for as many warps
+    // as there are (with their neighbours, and all warps through the products of empty rows, two stages and a page looked up where it was
+    // needed: 4 requests at 1,000 keys, groups of 4, 8 kv heads of 128, 30.4 us with the merge, 20.3 so; 16 at 1,500 155 and 105; 64 at
+    // 20 17.3 and 11.6)
+    auto row_of = [&](int i) { return ROWS == 64 ? warp * (ROWS / WARPS) + i : warp + i * WARPS; };
 
     constexpr int RW = ROWS / WARPS;                // rows of a warp
     float o[RW][CH * 4], m[RW], l[RW];
@@ -139,128 +157,155 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
 #pragma unroll
         for (int c = 0; c < CH * 4; ++c) O[i][c] = 0.f;
     }
-    constexpr int TX = ROWS == 64 ? 8 : 16, RPT = ROWS == 64 ? 2 : 1, KPT = KEYS / TX, TY = THREADS / TX;
+    constexpr int TX = KT / 4, RPT = KT / 16, KPT = 4, TY = THREADS / TX;      // (64 rows)
     const int tx = tid % TX, ty = tid / TX;
-    if (first < last) fetch(first);
-    for (int tile = first; tile < last; ++tile) {
-        const int st = tile & 1;
-        if (tile + 1 < last) {
-            fetch(tile + 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; ++i)
+        if (first + i * PARTS < last) fetch(first + i * PARTS, i);
+    for (int from = first, st = 0; from < last; from += PARTS, st = st + 1 == STAGES ? 0 : st + 1) {
+        const int next = from + (STAGES - 1) * PARTS;
+        if (next < last) fetch(next, st == 0 ? STAGES - 1 : st - 1);
+        // these keys have come, however many of those behind them have not
+        if (next < last) asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+        else if (STAGES > 2 && from + PARTS < last) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        float s[RPT][KPT];
+        const float* kt = ks + st * KT * ldk;
+        if constexpr (ROWS == 16) {
+            // a warp a row, a lane a key
 #pragma unroll
-        for (int i = 0; i < RPT; ++i)
-#pragma unroll
-            for (int j = 0; j < KPT; ++j) s[i][j] = 0.f;
-        const float* kt = ks + st * KEYS * ldk;
-        for (int c = 0; c < hd; c += 4) {
-            float4 a[RPT], b[KPT];
-#pragma unroll
-            for (int i = 0; i < RPT; ++i) a[i] = *reinterpret_cast<const float4*>(qs + (ty + i * TY) * ldk + c);
-#pragma unroll
-            for (int j = 0; j < KPT; ++j) b[j] = *reinterpret_cast<const float4*>(kt + (tx + j * TX) * ldk + c);
+            for (int i = 0; i < ROWS / WARPS; ++i) {
+                const int row = row_of(i), q_pos = pos0 + row / G, kp = base + from * KEYS + lane;
+                if (row >= rows) continue;
+                float s = 0.f;
+#pragma unroll 8
+                for (int c = 0; c < hd; c += 4) {
+                    const float4 a = *reinterpret_cast<const float4*>(qs + row * ldk + c), b = *reinterpret_cast<const float4*>(kt + lane * ldk + c);
+                    s = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
+                }
+                const bool seen = kp <= q_pos && kp >= bw::first_visible(q_pos, p.window, p.chunk) && known[st * KT + lane];
+                ps[row * LDP + lane] = seen ? s * p.scale : -INFINITY;
+            }
+            __syncwarp();
+        } else {
+            float s[RPT][KPT];
 #pragma unroll
             for (int i = 0; i < RPT; ++i)
 #pragma unroll
-                for (int j = 0; j < KPT; ++j)
-                    s[i][j] = fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, s[i][j]))));
-        }
+                for (int j = 0; j < KPT; ++j) s[i][j] = 0.f;
+            for (int c = 0; c < hd; c += 4) {
+                float4 a[RPT], b[KPT];
 #pragma unroll
-        for (int i = 0; i < RPT; ++i) {
-            const int row = ty + i * TY, q_pos = pos0 + row / G;
-            const int lo = bw::first_visible(q_pos, p.window, p.chunk);
+                for (int i = 0; i < RPT; ++i) a[i] = *reinterpret_cast<const float4*>(qs + (ty + i * TY) * ldk + c);
 #pragma unroll
-            for (int j = 0; j < KPT; ++j) {
-                const int key = tx + j * TX, kp = base + tile * KEYS + key;
-                const bool seen = row < rows && kp <= q_pos && kp >= lo && known[st * KEYS + key];
-                ps[row * LDP + key] = seen ? s[i][j] * p.scale : -INFINITY;
+                for (int j = 0; j < KPT; ++j) b[j] = *reinterpret_cast<const float4*>(kt + (tx + j * TX) * ldk + c);
+#pragma unroll
+                for (int i = 0; i < RPT; ++i)
+#pragma unroll
+                    for (int j = 0; j < KPT; ++j)
+                        s[i][j] = fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, s[i][j]))));
             }
-        }
-        __syncthreads();
-        // (a warp's rows side by side: one after another their shuffles and exponentials are the kernel's latency at few keys)
-        float sc[RW], m_new[RW], e[RW], sum[RW];
-        bool zero = false;
 #pragma unroll
-        for (int i = 0; i < RW; ++i) sc[i] = ps[(warp * RW + i) * LDP + lane];
+            for (int i = 0; i < RPT; ++i) {
+                const int row = ty + i * TY, q_pos = pos0 + row / G;
+                const int lo = bw::first_visible(q_pos, p.window, p.chunk);
 #pragma unroll
-        for (int i = 0; i < RW; ++i) m_new[i] = fmaxf(m[i], bw::warp_max(sc[i]));
-#pragma unroll
-        for (int i = 0; i < RW; ++i) e[i] = sc[i] == -INFINITY ? 0.f : expf(sc[i] - m_new[i]);
-#pragma unroll
-        for (int i = 0; i < RW; ++i) sum[i] = bw::warp_sum(e[i]);
-#pragma unroll
-        for (int i = 0; i < RW; ++i) {
-            const float corr = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new[i]);
-            l[i] = l[i] * corr + sum[i];
-            m[i] = m_new[i];
-            ps[(warp * RW + i) * LDP + lane] = e[i];
-            zero |= e[i] == 0.f && warp * RW + i < rows;
-#pragma unroll
-            for (int c = 0; c < CH * 4; ++c) o[i][c] *= corr;
-        }
-        __syncwarp();
-        // A key without weight (masked, or too far below the largest score) must not add its value, which may be no number: 0 times an
-        // infinity is none.  Rare beside the diagonal and a window's edges, so a warp asks once per tile.
-        const float* vt = vs + st * KEYS * hd;
-        auto add_values = [&](auto skip) {
-#pragma unroll 2
-            for (int k4 = 0; k4 < KEYS; k4 += 4) {
-                float4 w[RW];
-#pragma unroll
-                for (int i = 0; i < RW; ++i) w[i] = *reinterpret_cast<const float4*>(ps + (warp * RW + i) * LDP + k4);
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-                    for (int h = 0; h < CH; ++h) {
-                        const int c = lane * 4 + 128 * h;
-                        if (c >= hd) continue;
-                        const float4 v = *reinterpret_cast<const float4*>(vt + (k4 + kk) * hd + c);
-#pragma unroll
-                        for (int i = 0; i < RW; ++i) {
-                            const float e = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
-                            if (decltype(skip)::value && e == 0.f) continue;
-                            o[i][4 * h] = fmaf(e, v.x, o[i][4 * h]);
-                            o[i][4 * h + 1] = fmaf(e, v.y, o[i][4 * h + 1]);
-                            o[i][4 * h + 2] = fmaf(e, v.z, o[i][4 * h + 2]);
-                            o[i][4 * h + 3] = fmaf(e, v.w, o[i][4 * h + 3]);
-                        }
-                    }
-            }
-        };
-        if (__any_sync(0xffffffffu, zero)) add_values(std::true_type{});
-        else add_values(std::false_type{});
-        if constexpr (SLICES) {
-            if (!whole && ((tile + 1) % per == 0 || tile + 1 == last)) {
-                const size_t at = part_row(p, item.w, tile / per, rows, kvh);
-#pragma unroll
-                for (int i = 0; i < RW; ++i) {
-                    const int row = warp * RW + i;
-                    if (row >= rows) continue;
-                    if (lane == 0) *reinterpret_cast<float2*>(p.part_ml + 2 * (at + row)) = make_float2(m[i], l[i]);
-#pragma unroll
-                    for (int h = 0; h < CH; ++h) {
-                        const int c = lane * 4 + 128 * h;
-                        if (c < hd) *reinterpret_cast<float4*>(p.part_o + (at + row) * hd + c) = make_float4(o[i][4 * h], o[i][4 * h + 1], o[i][4 * h + 2], o[i][4 * h + 3]);
-                    }
-#pragma unroll
-                    for (int c = 0; c < CH * 4; ++c) o[i][c] = 0.f;
-                    m[i] = -INFINITY; l[i] = 0.f;
+                for (int j = 0; j < KPT; ++j) {
+                    const int key = tx + j * TX, kp = base + from * KEYS + key;
+                    const bool seen = row < rows && kp <= q_pos && kp >= lo && known[st * KT + key];
+                    ps[row * LDP + key] = seen ? s[i][j] * p.scale : -INFINITY;
                 }
             }
-        } else {
-            const int done = base / KEYS + tile + 1;      // tiles from position 0
-            if (same ? done % per == 0 || tile + 1 == last : done % (SLICE / KEYS) == 0 || tile + 1 == last) {
+            __syncthreads();
+        }
+#pragma unroll 1
+        for (int part = 0; part < PARTS; ++part) {
+            const int tile = from + part;
+            if (tile >= last) break;
+            float* pt = ps + part * KEYS;
+            if (ROWS == 64 || warp < rows) {
+                // (a warp's rows side by side: one after another their shuffles and exponentials are the kernel's latency at few keys)
+                float sc[RW], m_new[RW], e[RW], sum[RW];
+                bool zero = false;
+#pragma unroll
+                for (int i = 0; i < RW; ++i) sc[i] = ROWS == 64 || row_of(i) < rows ? pt[row_of(i) * LDP + lane] : -INFINITY;
+#pragma unroll
+                for (int i = 0; i < RW; ++i) m_new[i] = fmaxf(m[i], bw::warp_max(sc[i]));
+#pragma unroll
+                for (int i = 0; i < RW; ++i) e[i] = sc[i] == -INFINITY ? 0.f : expf(sc[i] - m_new[i]);
+#pragma unroll
+                for (int i = 0; i < RW; ++i) sum[i] = bw::warp_sum(e[i]);
 #pragma unroll
                 for (int i = 0; i < RW; ++i) {
-                    if (!same && tile + 1 < last && done % (slice_keys(p, pos0 + (warp * RW + i) / G) / KEYS)) continue;
-                    const float2 f = fold(M[i], L[i], m[i], l[i]);
+                    const float corr = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new[i]);
+                    l[i] = l[i] * corr + sum[i];
+                    m[i] = m_new[i];
+                    pt[row_of(i) * LDP + lane] = e[i];
+                    zero |= e[i] == 0.f && row_of(i) < rows;
 #pragma unroll
-                    for (int c = 0; c < CH * 4; ++c) { O[i][c] = folded(O[i][c], o[i][c], f); o[i][c] = 0.f; }
-                    m[i] = -INFINITY; l[i] = 0.f;
+                    for (int c = 0; c < CH * 4; ++c) o[i][c] *= corr;
+                }
+                __syncwarp();
+                // A key without weight (masked, or too far below the largest score) must not add its value, which may be no number: 0 times an
+                // infinity is none.  Rare beside the diagonal and a window's edges, so a warp asks once per tile.
+                const float* vt = vs + (st * KT + part * KEYS) * hd;
+                auto add_values = [&](auto skip) {
+#pragma unroll 2
+                    for (int k4 = 0; k4 < KEYS; k4 += 4) {
+                        float4 w[RW];
+#pragma unroll
+                        for (int i = 0; i < RW; ++i) w[i] = *reinterpret_cast<const float4*>(pt + row_of(i) * LDP + k4);
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                            for (int h = 0; h < CH; ++h) {
+                                const int c = lane * 4 + 128 * h;
+                                if (c >= hd) continue;
+                                const float4 v = *reinterpret_cast<const float4*>(vt + (k4 + kk) * hd + c);
+#pragma unroll
+                                for (int i = 0; i < RW; ++i) {
+                                    const float e = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
+                                    if (decltype(skip)::value && e == 0.f) continue;
+                                    o[i][4 * h] = fmaf(e, v.x, o[i][4 * h]);
+                                    o[i][4 * h + 1] = fmaf(e, v.y, o[i][4 * h + 1]);
+                                    o[i][4 * h + 2] = fmaf(e, v.z, o[i][4 * h + 2]);
+                                    o[i][4 * h + 3] = fmaf(e, v.w, o[i][4 * h + 3]);
+                                }
+                            }
+                    }
+                };
+                if (__any_sync(0xffffffffu, zero)) add_values(std::true_type{});
+                else add_values(std::false_type{});
+            }
+            if constexpr (SLICES) {
+                if (!whole && ((tile + 1) % per == 0 || tile + 1 == last)) {
+                    const size_t at = part_row(p, item.w, tile / per, rows, kvh);
+#pragma unroll
+                    for (int i = 0; i < RW; ++i) {
+                        const int row = row_of(i);
+                        if (row >= rows) continue;
+                        if (lane == 0) *reinterpret_cast<float2*>(p.part_ml + 2 * (at + row)) = make_float2(m[i], l[i]);
+#pragma unroll
+                        for (int h = 0; h < CH; ++h) {
+                            const int c = lane * 4 + 128 * h;
+                            if (c < hd) *reinterpret_cast<float4*>(p.part_o + (at + row) * hd + c) = make_float4(o[i][4 * h], o[i][4 * h + 1], o[i][4 * h + 2], o[i][4 * h + 3]);
+                        }
+#pragma unroll
+                        for (int c = 0; c < CH * 4; ++c) o[i][c] = 0.f;
+                        m[i] = -INFINITY; l[i] = 0.f;
+                    }
+                }
+            } else {
+                const int done = base / KEYS + tile + 1;      // tiles from position 0
+                if (same ? done % per == 0 || tile + 1 == last : done % (SLICE / KEYS) == 0 || tile + 1 == last) {
+#pragma unroll
+                    for (int i = 0; i < RW; ++i) {
+                        if (!same && tile + 1 < last && done % (slice_keys(p, pos0 + row_of(i) / G) / KEYS)) continue;
+                        const float2 f = fold(M[i], L[i], m[i], l[i]);
+#pragma unroll
+                        for (int c = 0; c < CH * 4; ++c) { O[i][c] = folded(O[i][c], o[i][c], f); o[i][c] = 0.f; }
+                        m[i] = -INFINITY; l[i] = 0.f;
+                    }
                 }
             }
         }
@@ -269,7 +314,7 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
     if (!whole) return;
 #pragma unroll
     for (int i = 0; i < RW; ++i) {
-        const int row = warp * RW + i;
+        const int row = row_of(i);
         if (row >= rows) continue;
         const float sum = SLICES ? l[i] : L[i], f = sum > 0.f ? 1.f / sum : 0.f;
         float* dst = p.out + ((size_t)(row0 + t0 + row / G) * p.nh + (size_t)kvh * G + row % G) * hd;
@@ -324,9 +369,10 @@ attention_f32_merge_kernel(Params p, const int4* __restrict__ work) {
 template <int ROWS, int CH, bool SLICES>
 int go(const Params& p, const int* work, int n, cudaStream_t s) {
     static bool done[bw::MAX_DEVICES] = {};
-    const cudaError_t e = bw::allow_dynamic_smem(attention_f32_kernel<ROWS, CH, SLICES>, 4 * smem_floats(ROWS, CH * 128), done);
+    constexpr int KT = fetched(ROWS, CH, SLICES);
+    const cudaError_t e = bw::allow_dynamic_smem(attention_f32_kernel<ROWS, CH, SLICES>, 4 * smem_floats(ROWS, CH * 128, KT), done);
     if (e != cudaSuccess) return (int)e;
-    bw::launch(attention_f32_kernel<ROWS, CH, SLICES>, dim3(n, p.nkv), dim3(THREADS), 4 * (size_t)smem_floats(ROWS, p.hd), s, p, (const int4*)work);
+    bw::launch(attention_f32_kernel<ROWS, CH, SLICES>, dim3(n, p.nkv), dim3(THREADS), 4 * (size_t)smem_floats(ROWS, p.hd, KT), s, p, (const int4*)work);
     BW_LAUNCH_CHECK();
     return 0;
 }
