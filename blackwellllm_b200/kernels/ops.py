@@ -44,13 +44,14 @@ def _check(code: int, what: str) -> None:
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return c_void_p(0 if t is None else t.data_ptr())
+    # (a plain number: ctypes makes the pointer; an object of it for every argument cost a tenth of a launcher call)
+    return None if t is None else t.data_ptr()
 
 
 def _stream():
     # the raw handle of the current stream of the current device (torch.cuda.current_stream() builds a
     # Stream object around the same number, several microseconds a call)
-    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _dev(t: torch.Tensor, name: str, dtype=None, contiguous=True):
