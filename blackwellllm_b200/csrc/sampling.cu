@@ -21,6 +21,14 @@ constexpr int THREADS = 1024;
 constexpr int WARPS = THREADS / 32;
 constexpr int ROW_BLOCKS = 8;       // blocks of a row, a cluster
 constexpr int BINS = 1024;          // one per thread: ten bits of a weight's float pattern at a time
+constexpr int VALUE_ROWS = 64;      // rows whose parameters travel with the launch
+
+// The rows' parameters: arrays on the device (any null: greedy, or no nucleus), or values in the launch itself.
+struct Rows {
+    const float *temperature, *top_p, *u;
+    int by_value;
+    float v[3][VALUE_ROWS];
+};
 
 __device__ __forceinline__ void argmax_pair(float& v, int& i, float ov, int oi) {
     if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
@@ -40,6 +48,14 @@ __device__ __forceinline__ u64 warp_scan_u64(u64 v) {   // inclusive
     return v;
 }
 
+// What the warps before this one left in sums[], and all warps: the same in all lanes.
+__device__ __forceinline__ void over_warps(const u64* sums, u64& before, u64& total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const u64 mine = sums[lane], upto = warp_scan_u64(mine);
+    total = __shfl_sync(0xffffffffu, upto, 31);
+    before = __shfl_sync(0xffffffffu, upto - mine, warp);
+}
+
 // A histogram of masses as two words per bin (shared memory adds 32-bit integers natively).
 struct Hist { unsigned lo[BINS], hi[BINS]; };
 __device__ __forceinline__ void hist_add(Hist& h, unsigned bin, u64 q) {
@@ -49,6 +65,10 @@ __device__ __forceinline__ void hist_add(Hist& h, unsigned bin, u64 q) {
     if (up) atomicAdd(&h.hi[bin], up);
 }
 
+// The cuts of the lists of largest weights, from the highest: 2^-6, 2^-8 .. 2^-16 of the largest; a row's lists have LISTED tokens at most.
+constexpr int LEVELS = 6, LISTED = 4 * THREADS;
+__device__ __forceinline__ float level_cut(int l) { return __uint_as_float((unsigned)(127 - 6 - 2 * l) << 23); }
+
 // One row per cluster (of CLUSTER blocks).  The weights e = exp((x - max) / T) are made once and stay in registers (NV a thread; NV = 0: a row too
 // long for that is read again for every pass) or, with more rows than clusters that fit at one block an SM, in shared memory (IN_SMEM:
 // two blocks an SM at 32 registers a thread).  Masses are integers, e * 2^shift rounded (`scale` = 2^shift, shift at most 45 and
@@ -56,13 +76,16 @@ __device__ __forceinline__ void hist_add(Hist& h, unsigned bin, u64 q) {
 // The nucleus threshold, the largest weight whose mass together with all larger ones reaches the target, is found ten bits of the
 // float pattern at a time (30 bits: e <= 1) from histograms that the blocks read from one another's shared memory: three passes
 // over registers, in place of the 30 passes over the row that a bisection takes.
-// What bounds it: latency (five cluster barriers, three histogram passes); a row of 128,256 is 0.5 MB.  Measured, temperature 0.6,
-// top_p 0.9: a row of 128,256 in 26 us, 32 rows of 152,064 in 63 us (79 in registers; one block per row and the bisection: 728 and
-// 1,162 us).
+// Before that, the nucleus is looked for among the row's largest weights alone: every block lists its tokens down to the lowest of LEVELS
+// cuts of which it has few enough, in index order, and the row's first block, with all lists and the row's mass, selects and draws
+// among them by itself: up to 32 tokens in one warp, more (up to four a thread) from histograms of its own.  Where they do not reach the
+// target mass (a flat row), or a weight is no number, the histograms over all blocks decide; both find the same token.
+// What bounds it: latency (three cluster barriers, with the histograms over all blocks five; 20 exponentials, masses and votes a thread); a
+// row of 128,256 is 0.5 MB.  Measured, temperature 0.6, top_p 0.9, logits as a language model gives them: a row of 128,256 in 14 us, 32 rows
+// of 152,064 in 32 us (25 and 61 with the histograms over all blocks alone; one block per row and a bisection: 728 and 1,162).
 template <int NV, bool IN_SMEM = false, int CLUSTER = ROW_BLOCKS>
 __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(THREADS, IN_SMEM || (NV == 0 && CLUSTER == 1) ? 2 : 1)
-sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
-              const float* __restrict__ top_p, const float* __restrict__ u, int* __restrict__ out,
+sample_kernel(const float* __restrict__ logits, const __grid_constant__ Rows rows, int* __restrict__ out,
               int V, size_t ld, float scale) {
     BW_PDL_TRIGGER();
     BW_PDL_WAIT();
@@ -71,15 +94,16 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     __shared__ float sv[WARPS], all_max[CLUSTER];
     __shared__ int si[WARPS], all_arg[CLUSTER];
     __shared__ u64 sums[WARPS], all_mass[CLUSTER], above;
-    __shared__ unsigned bin_found;
+    __shared__ unsigned bin_found, all_cut[CLUSTER];
+    __shared__ int all_listed[CLUSTER], counts[LEVELS][WARPS], own_level, again;
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), r = blockIdx.x / CLUSTER;
     cluster.barrier_arrive();       // (waited for before the first access to another block's memory: that block has then begun)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float* row = logits + (size_t)r * ld;
-    const float T = temperature ? temperature[r] : 0.f;
+    const float T = rows.by_value ? rows.v[0][r] : rows.temperature ? rows.temperature[r] : 0.f;
     const bool greedy = !(T > 0.f);
-    const float tp = (!greedy && top_p) ? top_p[r] : 1.f;
+    const float tp = greedy ? 1.f : rows.by_value ? rows.v[1][r] : rows.top_p ? rows.top_p[r] : 1.f;
 
     // this warp's tokens: a contiguous stretch of the block's contiguous stretch of the row
     const int per_block = (V + CLUSTER - 1) / CLUSTER;
@@ -100,11 +124,18 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
 #pragma unroll
         for (int i = 0; i < NV; ++i)
             if (32 * i < left) argmax_pair(mx, arg, e[i], first + 32 * i);
+    } else if constexpr (IN_SMEM) {
+        // (each lane its own tokens, all asked for at once: through registers, four at a time, the 19 of 152,064 took 12 us)
+        float* to = kept_smem + warp * per_warp + lane;
+        for (int i = 0; i < iters; ++i)
+            if (32 * i < left)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(to + 32 * i)), "l"(row + first + 32 * i) : "memory");
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        for (int i = 0; 32 * i < left; ++i) argmax_pair(mx, arg, to[32 * i], first + 32 * i);
     } else {
 #pragma unroll 4
         for (int i = 0; i < iters; ++i) {
             const float x = 32 * i < left ? row[first + 32 * i] : -INFINITY;
-            if constexpr (IN_SMEM) kept_smem[warp * per_warp + 32 * i + lane] = x;
             if (32 * i < left) argmax_pair(mx, arg, x, first + 32 * i);
         }
     }
@@ -147,17 +178,210 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
         else if constexpr (IN_SMEM) return kept_smem[warp * per_warp + 32 * i + lane];
         else return 32 * i < left ? expf((row[first + 32 * i] - mx) * invT) : -1.f;
     };
-    auto mass = [&](float w) { return __float2ull_rn(w * scale); };
-    const int passes = NV > 0 ? NV : iters;
-    if constexpr (NV > 0) {
-#pragma unroll
-        for (int i = 0; i < NV; ++i) e[i] = 32 * i < left ? expf((e[i] - mx) * invT) : -1.f;
-    }
-    if constexpr (IN_SMEM) {       // (each thread its own)
-        for (int i = 0; i < iters; ++i) {
+    auto make_weight = [&](int i) {     // from the logit that is kept
+        if constexpr (NV > 0) e[i] = 32 * i < left ? expf((e[i] - mx) * invT) : -1.f;
+        else if constexpr (IN_SMEM) {
             float& k = kept_smem[warp * per_warp + 32 * i + lane];
             k = 32 * i < left ? expf((k - mx) * invT) : -1.f;
         }
+        return weight(i);
+    };
+    auto mass = [&](float w) { return __float2ull_rn(w * scale); };
+    const int passes = NV > 0 ? NV : iters;
+    const float uniform = rows.by_value ? rows.v[2][r] : rows.u[r];
+    // this thread's bin of a histogram, counted from the largest weights, m its mass: where the target lies
+    auto select = [&](unsigned bin, u64 m, auto&& set_target, u64& target, unsigned& prefix) {
+        u64 sum = warp_scan_u64(m);
+        if (lane == 31) sums[warp] = sum;
+        __syncthreads();
+        u64 before, total;
+        over_warps(sums, before, total);
+        sum += before;
+        set_target(total);
+        if (sum - m < target && target <= sum) { bin_found = bin; above = sum - m; }
+        if (tid == 0 && total == 0) { bin_found = 0; above = 0; }
+        __syncthreads();
+        prefix = (prefix << 10) | bin_found;
+        target -= above;
+    };
+    auto nucleus_target = [&](u64 total) {
+        u64 t = __double2ull_ru((double)tp * (double)total);
+        if (t < 1) t = 1;        // (top_p <= 0 keeps the most probable token)
+        return t > total ? total : t;
+    };
+    auto drawn = [&](u64 total) {
+        const double at = (double)uniform * (double)total;
+        const u64 goal = at > 0.0 ? __double2ull_rd(at) : 0;
+        return goal >= total ? total - 1 : goal;
+    };
+
+    if (!(tp < 1.f)) {
+        if constexpr (NV > 0 || IN_SMEM) {
+#pragma unroll
+            for (int i = 0; i < passes; ++i) make_weight(i);
+        }
+    } else {
+        // the weights, their mass, and how many tokens lie above each cut
+        u64 q = 0;
+        int many[LEVELS] = {};
+        bool number = true;
+#pragma unroll
+        for (int i = 0; i < passes; ++i) {
+            const float w = make_weight(i), x = w * scale;
+            number &= w == w;
+            // (most masses fit 32 bits, whose conversion is a fraction of the other's)
+            if (x < 0x1p31f) q += __float2uint_rn(x);              // (none: -1, no mass)
+            if (__any_sync(0xffffffffu, !(x < 0x1p31f))) { if (x >= 0x1p31f) q += mass(w); }
+            if (__any_sync(0xffffffffu, w >= level_cut(LEVELS - 1))) {
+#pragma unroll
+                for (int l = 0; l < LEVELS; ++l) many[l] += __popc(__ballot_sync(0xffffffffu, w >= level_cut(l)));
+            }
+        }
+        q = warp_sum_u64(q);
+        number = __all_sync(0xffffffffu, number);
+        if (lane == 0) {
+            sums[warp] = q;
+#pragma unroll
+            for (int l = 0; l < LEVELS; ++l) counts[l][warp] = number ? many[l] : LISTED + 1;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const u64 block = warp_sum_u64(sums[lane]);
+            int l = LEVELS - 1, listed = 0, mine = 0;
+            for (; l >= 0; --l) {
+                mine = counts[l][lane];
+                listed = __reduce_add_sync(0xffffffffu, mine);
+                if (listed <= (CLUSTER > 1 ? LISTED / CLUSTER : BINS)) break;
+            }
+            int upto = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += t; }
+            si[lane] = upto - mine;             // where this warp's tokens begin in the block's list
+            const unsigned cut = l < 0 ? 0xffffffffu : __float_as_uint(level_cut(l));
+            if (lane < CLUSTER) {
+                *cluster.map_shared_rank(&all_mass[rank], lane) = block;
+                *cluster.map_shared_rank(&all_listed[rank], lane) = l < 0 ? 0 : listed;
+                *cluster.map_shared_rank(&all_cut[rank], lane) = cut;
+            }
+            if (lane == 0) { bin_found = cut; own_level = l; }
+        }
+        __syncthreads();
+        Hist& list = hist[2];                   // the block's list: weights, tokens
+        if (own_level >= 0 && counts[own_level][warp] > 0) {
+            const float own_cut = __uint_as_float(bin_found);
+            int at = si[warp];
+#pragma unroll
+            for (int i = 0; i < passes; ++i) {
+                const float w = weight(i);
+                const bool in = w >= own_cut;
+                const unsigned who = __ballot_sync(0xffffffffu, in);
+                if (in) {
+                    const int to = at + __popc(who & ((1u << lane) - 1));
+                    list.lo[to] = __float_as_uint(w);
+                    list.hi[to] = (unsigned)(first + 32 * i);
+                }
+                at += __popc(who);
+            }
+        }
+        cluster.sync();
+        if (rank == 0) {
+            u64 total = 0;
+            unsigned cut = 0;
+            int n = 0;
+#pragma unroll
+            for (int c = 0; c < CLUSTER; ++c) { total += all_mass[c]; cut = max(cut, all_cut[c]); n += all_listed[c]; }
+            // entry j of the blocks' lists end to end (tokens in index order); one below the row's cut counts as none
+            auto entry = [&](int j, unsigned& bits, unsigned& token) {
+                int c = 0;
+                bits = token = 0;
+                if (j >= n) return;
+                while (j >= all_listed[c]) j -= all_listed[c++];
+                const Hist* h = cluster.map_shared_rank(&hist[2], c);
+                bits = h->lo[j]; token = h->hi[j];
+                if (bits < cut) bits = 0;
+            };
+            u64 target = nucleus_target(total);
+            bool found = false;
+            if (cut == 0xffffffffu || total == 0 || n == 0) {
+                // the histograms decide
+            } else if (n <= 32) {
+                if (warp == 0) {                // a lane an entry, all in one warp
+                    unsigned bits, token;
+                    entry(lane, bits, token);
+                    const u64 m = bits ? mass(__uint_as_float(bits)) : 0;
+                    u64 larger = 0, upto = 0;   // the mass of larger weights; of those and this weight's ties
+                    for (int k = 0; k < n; ++k) {
+                        const unsigned b = __shfl_sync(0xffffffffu, bits, k);
+                        const u64 mk = __shfl_sync(0xffffffffu, m, k);
+                        if (b > bits) larger += mk;
+                        if (b >= bits) upto += mk;
+                    }
+                    const unsigned hit = __ballot_sync(0xffffffffu, m && larger < target && target <= upto);
+                    found = hit != 0;
+                    if (found) {
+                        const unsigned least = __shfl_sync(0xffffffffu, bits, __ffs(hit) - 1);
+                        const u64 kept = bits >= least ? m : 0, sum = warp_scan_u64(kept);
+                        const u64 goal = drawn(__shfl_sync(0xffffffffu, sum, 31));
+                        if (kept && goal < sum && goal >= sum - kept) out[r] = (int)token;
+                    }
+                }
+            } else {
+                constexpr int PER = LISTED / THREADS;
+                const int per = (n + THREADS - 1) / THREADS;
+                unsigned bits[PER], token[PER];
+                u64 reached = 0;
+#pragma unroll
+                for (int k = 0; k < PER; ++k) {
+                    bits[k] = token[k] = 0;
+                    if (k < per) entry(tid * per + k, bits[k], token[k]);
+                    if (bits[k]) reached += mass(__uint_as_float(bits[k]));
+                }
+                reached = warp_sum_u64(reached);
+                __syncthreads();                // (the list has been read, sums too)
+                if (lane == 0) sums[warp] = reached;
+                hist[2].lo[tid] = hist[2].hi[tid] = 0;
+                __syncthreads();
+                u64 before;
+                over_warps(sums, before, reached);
+                found = reached >= target;
+                if (found) {
+                    unsigned prefix = 0;
+#pragma unroll
+                    for (int round = 0; round < 3; ++round) {
+                        const int shift = 20 - 10 * round;
+#pragma unroll
+                        for (int k = 0; k < PER; ++k)
+                            if (bits[k] && (round == 0 || (bits[k] >> (shift + 10)) == prefix))
+                                hist_add(hist[round], (bits[k] >> shift) & (BINS - 1), mass(__uint_as_float(bits[k])));
+                        __syncthreads();
+                        const unsigned bin = BINS - 1 - tid;
+                        select(bin, ((u64)hist[round].hi[bin] << 32) + hist[round].lo[bin], [](u64) {}, target, prefix);
+                    }
+                    u64 kept = 0;
+#pragma unroll
+                    for (int k = 0; k < PER; ++k) kept += bits[k] >= prefix && bits[k] ? mass(__uint_as_float(bits[k])) : 0;
+                    u64 upto = warp_scan_u64(kept), all;
+                    if (lane == 31) sums[warp] = upto;
+                    __syncthreads();
+                    over_warps(sums, before, all);
+                    upto += before - kept;
+                    const u64 goal = drawn(all);
+#pragma unroll
+                    for (int k = 0; k < PER; ++k) {
+                        const u64 m = bits[k] >= prefix && bits[k] ? mass(__uint_as_float(bits[k])) : 0;
+                        if (m && goal >= upto && goal < upto + m) out[r] = (int)token[k];
+                        upto += m;
+                    }
+                }
+            }
+            if (warp == 0 && lane < CLUSTER) *cluster.map_shared_rank(&again, lane) = !found;
+        }
+        cluster.sync();
+        if (!again) return;
+        if (rank == 0)       // (the other blocks' first two are as they were)
+            for (int i = tid; i < 2 * BINS; i += THREADS) hist[i / BINS].lo[i % BINS] = hist[i / BINS].hi[i % BINS] = 0;
+        hist[2].lo[tid] = hist[2].hi[tid] = 0;
+        __syncthreads();
     }
     float tau = 0.f;
     if (tp < 1.f) {
@@ -186,23 +410,7 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
                 m += ((u64)h->hi[bin] << 32) + h->lo[bin];
             }
             if (round == 0 && __syncthreads_or(tid == 0 && m != 0)) { nucleus = false; break; }
-            u64 sum = warp_scan_u64(m);
-            if (lane == 31) sums[warp] = sum;
-            __syncthreads();
-            u64 before = 0, total = 0;
-#pragma unroll 8
-            for (int w = 0; w < WARPS; ++w) { const u64 s = sums[w]; total += s; if (w < warp) before += s; }
-            sum += before;
-            if (round == 0) {
-                target = __double2ull_ru((double)tp * (double)total);
-                if (target < 1) target = 1;        // (top_p <= 0 keeps the most probable token)
-                if (target > total) target = total;
-            }
-            if (sum - m < target && target <= sum) { bin_found = bin; above = sum - m; }
-            if (tid == 0 && total == 0) { bin_found = 0; above = 0; }
-            __syncthreads();
-            prefix = (prefix << 10) | bin_found;
-            target -= above;
+            select(bin, m, [&](u64 total) { if (round == 0) target = nucleus_target(total); }, target, prefix);
         }
         if (nucleus) tau = __uint_as_float(prefix);
     }
@@ -232,10 +440,10 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
         }
         return;
     }
-    const double at = (double)u[r] * (double)total;
-    u64 goal = at > 0.0 ? __double2ull_rd(at) : 0;
-    if (goal >= total) goal = total - 1;
-    for (int w = 0; w < warp; ++w) before += sums[w];
+    const u64 goal = drawn(total);
+    u64 mine, block;
+    over_warps(sums, mine, block);
+    before += mine;
     if (goal < before || goal >= before + kept) return;
 #pragma unroll
     for (int i = 0; i < passes; ++i) {
@@ -345,12 +553,7 @@ BW_EXPORT int bw_log_prob(const float* logits, const int* target, float* out, in
     return 0;
 }
 
-// temperature, top_p: per row (may be null: greedy / no nucleus); u: per row uniform in [0,1).
-BW_EXPORT int bw_sample(const float* logits, const float* temperature, const float* top_p, const float* u,
-                        int* out, int R, int V, long long ld, void* stream) {
-    if (R <= 0) return 0;
-    if (V <= 0 || ld < V) return BW_ERR_BAD_ARG;
-    if (temperature && !u) return BW_ERR_BAD_ARG;
+static int sample(const float* logits, const Rows& rows, bool greedy, int* out, int R, int V, long long ld, void* stream) {
     int bits = 0;
     while ((1ll << bits) < V) ++bits;
     const float scale = (float)(1ull << (62 - bits < 45 ? 62 - bits : 45));
@@ -358,18 +561,19 @@ BW_EXPORT int bw_sample(const float* logits, const float* temperature, const flo
     // The greedy choice alone needs one pass, and clusters take turns of 17 rows or so: a block a row, but for a few long rows (us on
     // clusters and in blocks: 8 rows of 24,000 3.1 and 3.2, of 32,000 3.2 and 3.8, of 128,256 4.1 and 8.1; 18 of 32,000 5.4 and 3.8; 36
     // of 128,256 10.4 and 8.3; 256 of them 71 and 25; 18 of 200,000 14.6 and 11.2).
-    if (!temperature && (V <= 24 * 1024 || R > (V > 100 * 1024 && V <= 160 * 1024 ? 32 : 16))) {
+    if (greedy && (V <= 24 * 1024 || R > (V > 100 * 1024 && V <= 160 * 1024 ? 32 : 16))) {
         bw::launch(argmax_kernel, dim3((unsigned)R), block, 0, (cudaStream_t)stream, logits, out, V, (size_t)ld);
         BW_LAUNCH_CHECK();
         return 0;
     }
-    // Else one block a row where that is faster: a row that fits a block's registers (64 rows of 5,000: nucleus 14 us, 69 on clusters;
-    // alone 13 and 20), or so many rows that their clusters take turns for longer than a block walks its row (temperature / nucleus, on
-    // clusters and in blocks: 64 rows of 32,000 19 / 75 and 27 / 63, 128 of 64,000 47 / 158 and 55 / 137, 256 of 128,256 168 / 404 and
-    // 156 / 365; of 256,000, which a cluster's registers do not hold, 479 / 1,180 and 323 / 717).
-    if (V <= 8 * THREADS || R > (V > 160 * 1024 ? 100 : V / 512)) {
+    // Else one block a row where that is faster: a row that fits a block's registers, or so many rows that their clusters take turns for
+    // longer than a block walks its row (temperature / nucleus, us, on clusters and in blocks: 64 rows of 9,000 19 / 25 and 12 / 17, 32 of
+    // them 11 / 15 and 11 / 16; 128 of 32,000 38 / 52 and 31 / 54, 256 of them 76 / 96 and 42 / 73; 256 of 64,000 90 / 120 and 79 / 181,
+    // 1,024 of them 342 / 448 and 264 / 367; 256 of 128,256 120 / 162 and 167 / 361; of 200,000, which a cluster's registers do not hold, 128
+    // 201 / 286 and 229 / 517, 256 390 / 559 and 261 / 594).
+    if (V <= 8 * THREADS || R > (V > 160 * 1024 ? 200 : V / 200)) {
         const auto kernel = V <= 8 * THREADS ? sample_kernel<8, false, 1> : sample_kernel<0, false, 1>;
-        bw::launch(kernel, dim3((unsigned)R), block, 0, (cudaStream_t)stream, logits, temperature, top_p, u, out, V, (size_t)ld, scale);
+        bw::launch(kernel, dim3((unsigned)R), block, 0, (cudaStream_t)stream, logits, rows, out, V, (size_t)ld, scale);
         BW_LAUNCH_CHECK();
         return 0;
     }
@@ -377,23 +581,47 @@ BW_EXPORT int bw_sample(const float* logits, const float* temperature, const flo
     const int per_block = (V + ROW_BLOCKS - 1) / ROW_BLOCKS;
     const int iters = ((per_block + WARPS - 1) / WARPS + 31) / 32;
     const dim3 grid((unsigned)R * ROW_BLOCKS);
-    // more rows than clusters at one block an SM: two blocks an SM, weights in shared memory (19 rows of 152,064 61 us, 32 63 us; in registers 79)
+    // more rows than clusters at one block an SM: two blocks an SM, weights in shared memory (nucleus, us, so and in registers: 32 rows of
+    // 32,000 17 and 24, of 128,256 29 and 33, 64 of 152,064 62 and 66)
     const int at_once = bw::num_sms() / ROW_BLOCKS;
     const size_t kept = (size_t)iters * 32 * WARPS * sizeof(float);
-    if (temperature && R > at_once && kept <= 80 * 1024) {      // (two blocks and their histograms in an SM's shared memory)
+    if (!greedy && R > at_once && kept <= 80 * 1024) {      // (two blocks and their histograms in an SM's shared memory)
         static bool done[bw::MAX_DEVICES] = {};
         if (const cudaError_t e = bw::allow_dynamic_smem(sample_kernel<0, true>, 80 * 1024, done); e != cudaSuccess) return (int)e;
-        bw::launch(sample_kernel<0, true>, grid, block, kept, (cudaStream_t)stream, logits, temperature, top_p, u, out, V, (size_t)ld, scale);
+        bw::launch(sample_kernel<0, true>, grid, block, kept, (cudaStream_t)stream, logits, rows, out, V, (size_t)ld, scale);
         BW_LAUNCH_CHECK();
         return 0;
     }
-#define BW_SAMPLE(NV) bw::launch(sample_kernel<NV>, grid, block, 0, (cudaStream_t)stream, logits, temperature, top_p, u, out, V, (size_t)ld, scale)
+#define BW_SAMPLE(NV) bw::launch(sample_kernel<NV>, grid, block, 0, (cudaStream_t)stream, logits, rows, out, V, (size_t)ld, scale)
     // registers for 8 tokens a thread (rows up to 65,536) or 20 (up to 163,840: 64 registers a thread allow no more); longer rows are
-    // read again for every pass (a row of 200,000 in 54 us, 32 rows in 146)
+    // read again for every pass (nucleus, a row of 200,000 in 24 us, 32 rows in 71)
     if (iters <= 8) BW_SAMPLE(8);
     else if (iters <= 20) BW_SAMPLE(20);
     else BW_SAMPLE(0);
 #undef BW_SAMPLE
     BW_LAUNCH_CHECK();
     return 0;
+}
+
+// temperature, top_p: per row (may be null: greedy / no nucleus); u: per row uniform in [0,1).
+BW_EXPORT int bw_sample(const float* logits, const float* temperature, const float* top_p, const float* u,
+                        int* out, int R, int V, long long ld, void* stream) {
+    if (R <= 0) return 0;
+    if (V <= 0 || ld < V) return BW_ERR_BAD_ARG;
+    if (temperature && !u) return BW_ERR_BAD_ARG;
+    Rows rows{};
+    rows.temperature = temperature; rows.top_p = top_p; rows.u = u;
+    return sample(logits, rows, !temperature, out, R, V, ld, stream);
+}
+
+// The same with the rows' parameters in the caller's memory: they travel with the launch, no copy and no buffer on the device.  All three
+// arrays, at most VALUE_ROWS rows.
+BW_EXPORT int bw_sample_values(const float* logits, const float* temperature, const float* top_p, const float* u, int* out, int R, int V,
+                               long long ld, void* stream) {
+    if (R <= 0) return 0;
+    if (V <= 0 || ld < V || !temperature || !top_p || !u || R > VALUE_ROWS) return BW_ERR_BAD_ARG;
+    Rows rows{};
+    rows.by_value = 1;
+    for (int r = 0; r < R; ++r) { rows.v[0][r] = temperature[r]; rows.v[1][r] = top_p[r]; rows.v[2][r] = u[r]; }
+    return sample(logits, rows, false, out, R, V, ld, stream);
 }

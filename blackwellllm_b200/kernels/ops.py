@@ -10,6 +10,7 @@ import math
 import os
 from typing import List, Optional, Tuple
 
+import numpy as np
 import torch
 
 from .build import load_library
@@ -749,24 +750,39 @@ def distance_bucket_table(rows: int, far: float) -> torch.Tensor:
 
 # ------------------------------------------------------------------ sampling
 
-def sample(logits: torch.Tensor, temperature: Optional[torch.Tensor], top_p: Optional[torch.Tensor],
-           u: Optional[torch.Tensor]) -> torch.Tensor:
-    """One token per row of ``logits`` [R, V]; greedy where temperature is None or <= 0."""
+SAMPLE_VALUE_ROWS = 64   # rows whose parameters travel with the launch (sampling.cu: VALUE_ROWS)
+
+
+def sample(logits: torch.Tensor, temperature, top_p, u) -> torch.Tensor:
+    """One token per row of ``logits`` [R, V]; greedy where temperature is None or <= 0.  The parameters are float32 tensors on the device,
+    or, for at most SAMPLE_VALUE_ROWS rows, all three float32 numpy arrays: those are read before this returns and travel with the
+    launch (no copy to the device)."""
     _dev(logits, "logits", torch.float32, contiguous=False)
     if logits.dim() != 2 or logits.stride(1) != 1:
         raise KernelError("sample: logits must be [R, V] with contiguous rows")
     R, V = logits.shape
-    for name, t in (("temperature", temperature), ("top_p", top_p), ("u", u)):
-        if t is not None:
-            _dev(t, name, torch.float32)
-            if t.numel() != R:
-                raise KernelError(f"sample: {name} must have one entry per row")
+    host = isinstance(temperature, np.ndarray)
+    if host:
+        at = []
+        for t in (temperature, top_p, u):
+            i = t.__array_interface__ if isinstance(t, np.ndarray) else None
+            if i is None or i["typestr"] != "<f4" or i["shape"] != (R,) or i["strides"] is not None or R > SAMPLE_VALUE_ROWS:
+                raise KernelError(f"sample: host values are three contiguous float32 arrays [R], R at most {SAMPLE_VALUE_ROWS}")
+            at.append(i["data"][0])
+    else:
+        for name, t in (("temperature", temperature), ("top_p", top_p), ("u", u)):
+            if t is not None:
+                _dev(t, name, torch.float32)
+                if t.numel() != R:
+                    raise KernelError(f"sample: {name} must have one entry per row")
+        at = [_ptr(temperature), _ptr(top_p), _ptr(u)]
     out = torch.empty((R,), dtype=torch.int32, device=logits.device)
-    fn = _fn("sampling", "bw_sample",
-             [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_ll, c_void_p])
-    _check(fn(_ptr(logits), _ptr(temperature), _ptr(top_p), _ptr(u), _ptr(out), R, V, logits.stride(0),
-              _stream()), "sample")
+    fn = _fn("sampling", "bw_sample_values" if host else "bw_sample", _SAMPLE_ARGS)
+    _check(fn(_ptr(logits), *at, _ptr(out), R, V, logits.stride(0), _stream()), "sample")
     return out
+
+
+_SAMPLE_ARGS = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_ll, c_void_p]
 
 
 def repetition_penalty(logits: torch.Tensor, ids: torch.Tensor, begin: torch.Tensor, penalty: torch.Tensor) -> torch.Tensor:

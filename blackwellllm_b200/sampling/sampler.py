@@ -3,14 +3,16 @@
 Per row: an optional repetition penalty on the tokens the request has emitted, then
 greedy, or temperature softmax with an optional nucleus and an inverse CDF draw at a
 uniform number that the host takes from the request's own Philox stream
-(``sampling.params.uniform(seed, draw_index)``).  One small upload of (temperature,
-top_p, u) per step (and one of the penalized ids where a request asks for the
-penalty), one or two kernels, one read-back of the tokens.
+(``sampling.params.uniform(seed, draw_index)``).  (temperature, top_p, u) of a step's rows travel
+with the kernel's launch (a copy to the device took longer than the choice: a row 55 us a call), of more
+rows than fit there in one small upload; one more of the penalized ids where a request asks for the
+penalty, one or two kernels, one read-back of the tokens.
 """
 from __future__ import annotations
 
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from ..kernels import ops
@@ -59,10 +61,17 @@ class Sampler:
             self.penalize(logits, params, generated)
         if all(p.greedy for p in params):
             return ops.sample(logits, None, None, None)
-        host = torch.empty((3, R), dtype=torch.float32, pin_memory=True)
-        rows = host.numpy()   # filled row by row: one assignment each instead of one per request
+        few = R <= ops.SAMPLE_VALUE_ROWS
+        if few:
+            rows = np.empty((3, R), dtype=np.float32)
+        else:
+            host = torch.empty((3, R), dtype=torch.float32, pin_memory=True)
+            rows = host.numpy()
+        # filled row by row: one assignment each instead of one per request
         rows[0] = [0.0 if p.greedy else p.temperature for p in params]
         rows[1] = [p.top_p for p in params]
         rows[2] = row_draws(params, seeds, draw_index)
+        if few:
+            return ops.sample(logits, *rows)
         dev = host.to(self.device, non_blocking=True)
         return ops.sample(logits, dev[0], dev[1], dev[2])

@@ -95,3 +95,18 @@ def test_rows_choose_the_same_token_in_every_form(R, V):
     x[0, V - 1], x[2, V // 3], x[2, V // 2] = -1e30, 4.0, 4.0
     for part in (x, x[:3]):
         assert ops.sample(part, None, None, None)[:3].tolist() == [V - 1, 0, V // 3]
+
+
+@pytest.mark.parametrize("R,V", [(3, 300), (3, 40000), (3, 152064), (20, 152064), (3, 170000)])
+@pytest.mark.parametrize("spread", [0.05, 1.0, 3.0, 12.0])
+def test_nuclei_of_one_token_to_most_of_the_row(R, V, spread):
+    """Found among a few listed tokens, in one warp or in a block, or from the histograms of the whole row; parameters on the device
+    and with the launch alike."""
+    from blackwellllm_b200.kernels import ops
+    g = torch.Generator().manual_seed(V + R)
+    rows = (torch.randn(R, V, generator=g) * spread).to(DEV)
+    values = torch.stack([torch.full((R,), 0.8), torch.full((R,), 0.95), torch.rand(R, generator=g)])
+    got = ops.sample(rows, *values.numpy())
+    assert torch.equal(got, ops.sample(rows, *values.to(DEV)))
+    for r in range(min(R, 3)):
+        assert outside(rows[r].cpu(), 0.8, 0.95, float(values[2, r]), int(got[r])) <= 2e-5      # (as above)
