@@ -172,20 +172,30 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
         __syncthreads();
         const float* kt = ks + st * KT * ldk;
         if constexpr (ROWS == 16) {
-            // a warp a row, a lane a key
-#pragma unroll
-            for (int i = 0; i < ROWS / WARPS; ++i) {
-                const int row = row_of(i), q_pos = pos0 + row / G, kp = base + from * KEYS + lane;
-                if (row >= rows) continue;
-                float s = 0.f;
+            // a warp a row or two, a lane a key
+            static_assert(ROWS == 2 * WARPS || ROWS == 64, "two rows a warp at most");
+            auto score = [&](auto both) {
+                const float *q0 = qs + warp * ldk, *q1 = qs + (warp + WARPS) * ldk, *key = kt + lane * ldk;
+                float s0 = 0.f, s1 = 0.f;
 #pragma unroll 8
                 for (int c = 0; c < hd; c += 4) {
-                    const float4 a = *reinterpret_cast<const float4*>(qs + row * ldk + c), b = *reinterpret_cast<const float4*>(kt + lane * ldk + c);
-                    s = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
+                    const float4 a = *reinterpret_cast<const float4*>(q0 + c), b = *reinterpret_cast<const float4*>(key + c);
+                    s0 = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s0))));
+                    if constexpr (decltype(both)::value) {
+                        const float4 d = *reinterpret_cast<const float4*>(q1 + c);
+                        s1 = fmaf(d.w, b.w, fmaf(d.z, b.z, fmaf(d.y, b.y, fmaf(d.x, b.x, s1))));
+                    }
                 }
-                const bool seen = kp <= q_pos && kp >= bw::first_visible(q_pos, p.window, p.chunk) && known[st * KT + lane];
-                ps[row * LDP + lane] = seen ? s * p.scale : -INFINITY;
-            }
+                auto put = [&](int row, float s) {
+                    const int q_pos = pos0 + row / G, kp = base + from * KEYS + lane;
+                    const bool seen = kp <= q_pos && kp >= bw::first_visible(q_pos, p.window, p.chunk) && known[st * KT + lane];
+                    ps[row * LDP + lane] = seen ? s * p.scale : -INFINITY;
+                };
+                put(warp, s0);
+                if constexpr (decltype(both)::value) put(warp + WARPS, s1);
+            };
+            if (warp + WARPS < rows) score(std::true_type{});
+            else if (warp < rows) score(std::false_type{});
             __syncwarp();
         } else {
             float s[RPT][KPT];
