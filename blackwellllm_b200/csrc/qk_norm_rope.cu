@@ -292,6 +292,76 @@ head_norm_rope_kernel(const float* __restrict__ qkv, long long ld, const int* __
     }
 }
 
+// The same for many tokens whose heads rotate as a whole, in halves (rotary_dim == dq == dpad <= 128), and whose values pass as they are.
+// What bounds it is how many rows' loads are in flight: a warp asks for HEADS heads of a token at once, and for the token's angles and
+// the two gains, which all its heads share, once (1,777 tokens of 32 + 8 heads of 128: 45 us in head_norm_rope_kernel, 24 so).  Sums and
+// products are in that kernel's order.
+constexpr int HEADS = 5;
+template <typename OT>
+__global__ void __launch_bounds__(256)
+head_norm_rope_whole_kernel(const float* __restrict__ qkv, long long ld, const int* __restrict__ positions,
+                            const int* __restrict__ req_of_token, const int* __restrict__ block_table, int max_blocks,
+                            const float* __restrict__ table, const float* __restrict__ q_gain, const float* __restrict__ k_gain, float eps,
+                            float q_coef, float q_every, OT* __restrict__ q_out, OT* __restrict__ k_pages, OT* __restrict__ v_pages,
+                            int nh, int nkv, int dq, int dv, int page_size, int num_pages, int has_kv,
+                            const float* __restrict__ q_head_mult, int v_col, float v_scale) {
+    BW_PDL_TRIGGER();
+    const int t = blockIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    const int pos = positions[t], slot = pos % page_size, half = dq >> 1, c = lane * 2, n_heads = nh + (has_kv ? nkv : 0);
+    int page = -1;
+    if (has_kv && num_pages > 0) {
+        page = block_table[(size_t)req_of_token[t] * max_blocks + pos / page_size];
+        if (page >= num_pages) page = -1;
+    }
+    const bool in = c < half;
+    const float2 zero = make_float2(0.f, 0.f), one = make_float2(1.f, 1.f);
+    auto at = [&](const float* p, float2 otherwise) { return in && p ? *reinterpret_cast<const float2*>(p + c) : otherwise; };
+    const float2 gqa = at(q_gain, one), gqb = at(q_gain ? q_gain + half : nullptr, one);
+    const float2 gka = at(k_gain, one), gkb = at(k_gain ? k_gain + half : nullptr, one);
+    float q_mult = 1.f;
+    if (q_coef != 0.f) q_mult = 1.f + q_coef * logf((float)floor((double)(pos + 1) / (double)q_every) + 1.f);
+    BW_PDL_WAIT();
+    const float* row = qkv + (size_t)t * ld;       // queries, then keys
+    const float2 cs = at(table + (size_t)t * dq, zero), sn = at(table + (size_t)t * dq + half, zero);
+    for (int h0 = warp; h0 < n_heads; h0 += HEADS * nwarps) {
+        float2 a[HEADS], b[HEADS];
+        float ss[HEADS];
+#pragma unroll
+        for (int u = 0; u < HEADS; ++u) {
+            const int h = h0 + u * nwarps;
+            const float* src = h < n_heads ? row + (size_t)h * dq : nullptr;
+            a[u] = at(src, zero); b[u] = at(src ? src + half : nullptr, zero);
+        }
+#pragma unroll
+        for (int u = 0; u < HEADS; ++u) {
+            float s = fmaf(a[u].x, a[u].x, 0.f);
+            s = fmaf(a[u].y, a[u].y, s); s = fmaf(b[u].x, b[u].x, s); s = fmaf(b[u].y, b[u].y, s);
+            ss[u] = bw::warp_sum(s);
+        }
+#pragma unroll
+        for (int u = 0; u < HEADS; ++u) {
+            const int h = h0 + u * nwarps;
+            const bool is_q = h < nh;
+            if (h >= n_heads || !in || (!is_q && page < 0)) continue;
+            const float mult = is_q ? (q_head_mult ? q_mult * q_head_mult[h] : q_mult) : 1.f;
+            const float r2 = ((is_q ? q_gain : k_gain) ? rsqrtf(ss[u] / (float)dq + eps) : 1.f) * mult;
+            const float2 ga = is_q ? gqa : gka, gb = is_q ? gqb : gkb;
+            OT* dst = is_q ? q_out + ((size_t)t * nh + h) * dq : k_pages + (((size_t)page * nkv + (h - nh)) * page_size + slot) * dq;
+            const float x0 = a[u].x * r2 * ga.x, x1 = a[u].y * r2 * ga.y, y0 = b[u].x * r2 * gb.x, y1 = b[u].y * r2 * gb.y;
+            put2(dst + c, x0 * cs.x - y0 * sn.x, x1 * cs.y - y1 * sn.y);
+            put2(dst + half + c, y0 * cs.x + x0 * sn.x, y1 * cs.y + x1 * sn.y);
+        }
+    }
+    if (page < 0) return;
+    for (int idx = threadIdx.x * 4; idx < nkv * dq; idx += blockDim.x * 4) {
+        const int h = idx / dq, i = idx - h * dq;
+        float4 o = i < dv ? *reinterpret_cast<const float4*>(row + v_col + (size_t)h * dv + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        o.x *= v_scale; o.y *= v_scale; o.z *= v_scale; o.w *= v_scale;
+        put4(v_pages + (((size_t)page * nkv + h) * page_size + slot) * dq + i, o);
+    }
+}
+
 }  // namespace
 
 // The per-head form (head_norm_rope_kernel).  ld: floats between rows of qkv; q_gain / k_gain: float32 [dq] or
@@ -329,6 +399,17 @@ BW_EXPORT int bw_head_norm_rope_append(const float* qkv, long long ld, const int
     // few tokens: a warp per head where the SMs allow it (8 tokens of 24 heads: 7 us with one block a token, three rounds of heads)
     const int heads = nh + (has_kv ? nkv : 0), spare = 2 * bw::num_sms() / T, rounds = (heads + 7) / 8;
     const int per_token = spare < 1 ? 1 : spare < rounds ? spare : rounds;
+    if (!spare && vec2 && vec_v && rotary_dim == dq && dq == dpad && dq <= 128 && v_eps <= 0.f && !v_first) {
+#define BW_HW(OT) bw::launch((head_norm_rope_whole_kernel<OT>), dim3(T), dim3(256), 0, s, qkv, ld, positions, req_of_token, block_table, \
+        max_blocks, table, q_gain, k_gain, eps, q_coef, q_every, (OT*)q_out, (OT*)k_pages, (OT*)v_pages, nh, nkv, dq, dv, page_size, \
+        num_pages, has_kv, q_head_mult, v_col, v_scale)
+        if (out_type == BW_F32) BW_HW(float);
+        else if (out_type == BW_BF16) BW_HW(bf16);
+        else return BW_ERR_BAD_ARG;
+#undef BW_HW
+        BW_LAUNCH_CHECK();
+        return 0;
+    }
 #define BW_HN(OT) bw::launch((spare ? head_norm_rope_kernel<OT, true> : head_norm_rope_kernel<OT, false>), dim3(T, per_token), dim3(256), 0, s, qkv, ld, positions, req_of_token, block_table, \
         max_blocks, table, rotary_dim, interleaved, q_gain, k_gain, eps, q_coef, q_every, (OT*)q_out, (OT*)k_pages, (OT*)v_pages, \
         nh, nkv, dq, dv, dpad, page_size, num_pages, has_kv, vec, vec2, pairs, vec_v, v_eps, v_first, v_first_ld, v_lam, \

@@ -365,6 +365,37 @@ def test_gemm_tc_rotary_routes(ops, M, nh, nkv, hd, rd, bias_dtype):
         assert float((a.float() - r.float()).abs().max()) <= 2 ** -8 * float(r.float().abs().max())
 
 
+@pytest.mark.parametrize("dq,dv,dtype", [(128, 128, torch.bfloat16), (64, 40, torch.float32), (36, 36, torch.bfloat16), (128, 64, torch.float32)])
+@pytest.mark.parametrize("shared,gains", [(False, True), (False, False), (True, True)])
+def test_heads_of_many_tokens_as_of_few(ops, dq, dv, dtype, shared, gains):
+    """More than two tokens an SM take a kernel of their own where whole heads rotate: what the one for few tokens makes."""
+    import types
+    if shared and dv != dq:
+        pytest.skip("values that are the keys have their size")
+    T, nh, nkv, page = 2 * ops.num_sms(DEV) + 35, 13, 3, 16
+    qkv = rand(T, nh * dq + nkv * (dq if shared else dq + dv) + 4, seed=1).to(DEV)
+    positions = (torch.arange(T, dtype=torch.int32) + 7).to(DEV)
+    req = torch.zeros(T, dtype=torch.int32, device=DEV)
+    blocks = (T + 7) // page + 1
+    table = torch.arange(blocks, dtype=torch.int32, device=DEV).flip(0).contiguous().view(1, blocks)
+    table[0, 3] = -1                                 # a page that is not there
+    cs = ops.rope_table(positions, plain_inv_freq(dq, 10000.0, None).float().to(DEV), dq)
+    gq, gk = (1.0 + rand(dq, seed=2).to(DEV), 1.0 + rand(dq, seed=3).to(DEV)) if gains else (None, None)
+    kw = dict(q_temp=(0.1, 50.0), q_head_mult=rand(nh, seed=4).to(DEV), kv_shared=shared, v_scale=0.7)
+
+    def run(pieces):
+        k, v = (torch.zeros(blocks, nkv, page, dq, dtype=dtype, device=DEV) for _ in range(2))
+        q = [ops.head_norm_rope_append(qkv[a:b], types.SimpleNamespace(positions=positions[a:b], req_of_token=req[a:b]), table, cs[a:b].contiguous(),
+                                       dq, False, gq, gk, 1e-5, k, v, nh, nkv, dq, dv, **kw) for a, b in pieces]
+        return torch.cat(q), k, v
+    # the same products and sums, of which the compiler may contract others: two roundings of a sum of two terms, then one to the type
+    tol = 2 ** -22 if dtype == torch.float32 else 2 ** -8
+    for a, b in zip(run([(0, T)]), run([(0, T // 2), (T // 2, T)])):
+        largest = float(b.float().abs().max())
+        assert largest > 0 and float((a.float() - b.float()).abs().max()) <= tol * largest
+        assert torch.equal(a == 0, b == 0)
+
+
 def test_gemm_tc_row_independent_of_batch(ops):
     """A token's row does not depend on which other tokens share the launch."""
     K, N = 1024, 768
