@@ -30,7 +30,7 @@ hidden_size, ctx)`` builds it.  The spec is any object with a ``kind`` attribute
 """
 from __future__ import annotations
 
-from dataclasses import dataclass
+from dataclasses import dataclass, field
 from typing import Any, Callable, Dict, List, Optional, Tuple
 
 import torch
@@ -58,6 +58,13 @@ class ParamSpec:
 class BuildContext:
     device: torch.device
     dtype: torch.dtype  # torch.float32 (true 32-bit path) or torch.bfloat16
+    _side: Optional[torch.cuda.Stream] = field(default=None, repr=False, compare=False)
+
+    def side_stream(self) -> "torch.cuda.Stream":
+        """The model's own second stream (of high priority, so none that an engine captures graphs on is the same one)."""
+        if self._side is None:
+            object.__setattr__(self, "_side", torch.cuda.Stream(self.device, priority=-1))     # (the rest is frozen)
+        return self._side
 
 
 @dataclass(frozen=True)

@@ -41,3 +41,24 @@ def test_queued_mixed_steps_repeat_themselves():
     for _ in range(8):
         queued = [step(engines[i % 2]) for i in range(50)]
         assert all(torch.equal(out, alone[i % 2]) for i, out in enumerate(queued))
+
+
+def test_two_mixers_as_branches_of_a_graph():
+    """A recorded step runs the two mixers beside each other; its bits are those of uncaptured steps, also of many steps queued."""
+    import tiny_zanivik
+    from blackwellllm_b200 import Engine, StepEntry
+    raw, page = tiny_zanivik.CONFIGS["broad"]
+    weights = {n: t.cuda() for n, t in tiny_zanivik.make_tensors(raw, 5).items()}
+    got = []
+    for graphs in (False, True):
+        e = Engine.from_tensors(raw, weights, dtype="bfloat16", page_size=page, num_pages=40, max_requests=6, max_batch_tokens=512,
+                                max_context=512, cuda_graphs=graphs)
+        for r in range(6):
+            e.step([StepEntry(r, tiny_zanivik.prompt(20 + 37 * r, raw["vocab"], r), [])])
+        logits = []
+        for s in range(60):
+            # (a replay's logits are overwritten by the next one)
+            logits.append(e.step([StepEntry(r, [(31 * s + 7 * r) % raw["vocab"]], [0]) for r in range(6)]).clone())
+        got.append(torch.stack(logits))
+        assert bool(e.graph_kernel_count(6)) == graphs
+    assert torch.equal(*got)
