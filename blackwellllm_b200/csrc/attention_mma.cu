@@ -34,7 +34,8 @@ constexpr int ROW_BYTES = HD * 2 + 16; // padded row: ldmatrix rows land in dist
 constexpr int KSTEPS = HD / 16;
 constexpr int CPR = HD / 8;            // 16-byte chunks per row
 constexpr int TILE_BYTES = BN * ROW_BYTES;
-constexpr int SMEM_KEYS_MERGE_BYTES = (2 * NWARPS * 16 + NWARPS * 16 * HD) * 4;   // finish_keys
+constexpr int FINISH_LD = HD + 8;    // floats between rows in finish_keys: a warp's eight rows of pairs lie in different banks
+constexpr int SMEM_KEYS_MERGE_BYTES = (2 * NWARPS * 16 + NWARPS * 16 * FINISH_LD) * 4;   // finish_keys
 
 struct Params {
     const bf16* q; const bf16* k_pages; const bf16* v_pages; bf16* out;
@@ -439,6 +440,30 @@ attn_rows_kernel(Params p, int toks_per_tile) {
     }
 }
 
+// How a request's walk over key tiles is cut: the lists are made for the longest context that a graph may get, so of `n_slices` only the
+// first `live` have tiles, `per` each.  The others leave at once, and the merge does not look at them (a token at 702 keys under a
+// bound of 8,320: 11 of 55).  A decode step is a chain of such short kernels, bound by what each does before and after its loads.  With that,
+// rows of shared memory that are no power of two long and page look-ups only where pages can be gone: a step of one token, 32 layers,
+// 3,333 -> 3,227 us; of 8 requests at 8,192 keys 4,594 -> 4,555; a narrow hybrid's 17 steps 6,356 -> 6,291.
+struct Walk { int t_first, kept, n, per, live; };
+__device__ __forceinline__ Walk walk_of(const Params& p, int q_pos0, int last_pos, int n_slices) {
+    Walk w;
+    w.t_first = bw::first_visible(q_pos0, p.window, p.chunk) / BN;
+    w.kept = kept_tiles(p.keep_first, w.t_first);      // tiles of kept first keys that lie before the window's
+    w.n = w.kept + last_pos / BN + 1 - w.t_first;
+    w.per = (w.n + n_slices - 1) / n_slices;
+    w.live = w.n > 0 ? (w.n + w.per - 1) / w.per : 0;      // (a request without tokens may see nothing)
+    return w;
+}
+// A block without work leaves before its wait for the earlier kernels, but for the grid's first: whoever waits for this grid then waits for
+// them too, however few blocks have work.
+__device__ __forceinline__ void leave() { if (blockIdx.x + blockIdx.y + blockIdx.z == 0) BW_PDL_WAIT(); }
+// of a merge item's request
+__device__ __forceinline__ int live_slices(const Params& p, int r, int n_slices) {
+    const int q_pos0 = p.q_start[r];
+    return walk_of(p, q_pos0, q_pos0 + p.cu_q[r + 1] - p.cu_q[r] - 1, n_slices).live;
+}
+
 // The end of a key-slice CTA that has a request's only slice, where pairs of query heads become one (bw::DiffHeads): a warp per head.
 __device__ __forceinline__ void finish_pairs(const Params& p, const float* ms, const float* ls, const float* os, int r, int g, int n_rows) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -465,7 +490,7 @@ __device__ __forceinline__ void finish_pairs(const Params& p, const float* ms, c
                 if (c >= HD) break;
                 float acc = 0.f;
 #pragma unroll
-                for (int wv = 0; wv < NWARPS; ++wv) acc += os[((size_t)(wv * 16 + row)) * HD + c] * f[wv];
+                for (int wv = 0; wv < NWARPS; ++wv) acc += os[(wv * 16 + row) * FINISH_LD + c] * f[wv];
                 o[i] = fmaf(acc, mine, o[i]);
             }
         }
@@ -491,7 +516,7 @@ __device__ __forceinline__ void finish_keys(const Params& p, const RowState& st,
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* ms = reinterpret_cast<float*>(smem);            // [4][16]
     float* ls = ms + NWARPS * 16;                          // [4][16]
-    float* os = ls + NWARPS * 16;                          // [4][16][HD]
+    float* os = ls + NWARPS * 16;                          // [4][16][FINISH_LD]
     sync_compute_warps();
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -499,42 +524,44 @@ __device__ __forceinline__ void finish_keys(const Params& p, const RowState& st,
         l += __shfl_xor_sync(0xffffffffu, l, 1);
         l += __shfl_xor_sync(0xffffffffu, l, 2);
         const int row = (lane >> 2) + 8 * h;
+        if (row >= n_rows) continue;
         if ((lane & 3) == 0) { ms[warp * 16 + row] = st.m[h]; ls[warp * 16 + row] = l; }
 #pragma unroll
-        for (int j = 0; j < HD / 8; ++j) {
-            float* d = os + ((size_t)(warp * 16 + row)) * HD + j * 8 + 2 * (lane & 3);
-            d[0] = o[j][2 * h]; d[1] = o[j][2 * h + 1];
-        }
+        for (int j = 0; j < HD / 8; ++j)
+            *reinterpret_cast<float2*>(os + (warp * 16 + row) * FINISH_LD + j * 8 + 2 * (lane & 3)) = make_float2(o[j][2 * h], o[j][2 * h + 1]);
     }
     sync_compute_warps();
     if (p.diff.lam && n_slices == 1) {
         finish_pairs(p, ms, ls, os, r, g, n_rows);
         return;
     }
-    for (int idx = threadIdx.x; idx < n_rows * HD; idx += THREADS) {
-        const int row = idx / HD, c = idx - row * HD;
+    for (int idx = threadIdx.x; idx < n_rows * (HD / 4); idx += THREADS) {      // four channels of a row
+        const int row = idx / (HD / 4), c = (idx - row * (HD / 4)) * 4;
         float M = -INFINITY;
 #pragma unroll
         for (int wv = 0; wv < NWARPS; ++wv) M = fmaxf(M, ms[wv * 16 + row]);
-        float acc = 0.f, L = 0.f;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        float L = 0.f;
 #pragma unroll
         for (int wv = 0; wv < NWARPS; ++wv) {
             const float mw = ms[wv * 16 + row];
             const float f = mw == -INFINITY ? 0.f : exp2f(mw - M);
-            acc += os[((size_t)(wv * 16 + row)) * HD + c] * f;
+            const float4 v = *reinterpret_cast<const float4*>(os + (wv * 16 + row) * FINISH_LD + c);
+            acc.x += v.x * f; acc.y += v.y * f; acc.z += v.z * f; acc.w += v.w * f;
             L += ls[wv * 16 + row] * f;
         }
-        const int tok = row / p.G, hg = row - tok * p.G;
         if (n_slices == 1) {
-            L += sink_term(p, g * p.G + hg, M);
-            p.out[((size_t)(p.cu_q[r] + tok) * p.nh + g * p.G + hg) * HD + c] =
-                __float2bfloat16_rn((L > 0.f ? acc / L : 0.f) *
-                                    bw::out_gate(p.gate, p.gate_ld, p.gate_dv, (size_t)(p.cu_q[r] + tok), g * p.G + hg, c));
+            const int tok = row / p.G, hg = row - tok * p.G, head = g * p.G + hg;
+            const size_t token = (size_t)(p.cu_q[r] + tok);
+            L += sink_term(p, head, M);
+            auto result = [&](float a, int ch) { return (L > 0.f ? a / L : 0.f) * bw::out_gate(p.gate, p.gate_ld, p.gate_dv, token, head, ch); };
+            *reinterpret_cast<uint2*>(p.out + (token * p.nh + head) * HD + c) =
+                make_uint2(pack_bf16(result(acc.x, c), result(acc.y, c + 1)), pack_bf16(result(acc.z, c + 2), result(acc.w, c + 3)));
         } else {
             // `item` counts the slices of all earlier items, so every (item, kv head, slice) has its own slot
             const size_t pr = ((size_t)item * p.nkv + (size_t)g * n_slices + slice) * 16 + row;
-            p.part_o[pr * HD + c] = acc;
-            if (c == 0) { p.part_ml[pr * 2] = M; p.part_ml[pr * 2 + 1] = L; }
+            *reinterpret_cast<float4*>(p.part_o + pr * HD + c) = acc;
+            if (c == 0) *reinterpret_cast<float2*>(p.part_ml + pr * 2) = make_float2(M, L);
         }
     }
 }
@@ -544,13 +571,12 @@ __device__ __forceinline__ void finish_keys(const Params& p, const RowState& st,
 __global__ void __launch_bounds__(THREADS)
 attn_keys_kernel(Params p) {
     BW_PDL_TRIGGER();
-    BW_PDL_WAIT();
     extern __shared__ __align__(16) uint8_t smem[];
     uint8_t* q_tile = smem;                       // 16 rows
     uint8_t* kv = smem + 16 * ROW_BYTES;          // [2 stages][K, V]
     const int4 w = reinterpret_cast<const int4*>(p.work)[blockIdx.x];
     const int r = w.x, slice = w.y, n_slices = w.z, item = w.w, g = blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
     const int q_len = p.cu_q[r + 1] - p.cu_q[r];
     const int kv_len = p.kv_len[r];
     const int n_rows = q_len * p.G;               // <= 16
@@ -558,12 +584,11 @@ attn_keys_kernel(Params p) {
     const int* bt = p.block_table + (size_t)r * p.max_blocks;
 
     const int last_pos = q_pos0 + q_len - 1;
-    const int first_key = bw::first_visible(q_pos0, p.window, p.chunk);
-    const int t_first = first_key / BN, t_end = last_pos / BN + 1;
-    const int kept = kept_tiles(p.keep_first, t_first);      // tiles of kept first keys that lie before the window's
-    const int n_walk = kept + t_end - t_first;               // the slices share the walk (walk_tile)
-    const int per = (n_walk + n_slices - 1) / n_slices;
-    const int v_lo = slice * per, v_hi = min(n_walk, v_lo + per) - 1;   // inclusive; may be empty
+    const Walk walk = walk_of(p, q_pos0, last_pos, n_slices);           // the slices share it (walk_tile)
+    if (slice >= walk.live) { leave(); return; }
+    const int t_first = walk.t_first, kept = walk.kept;
+    const int v_lo = slice * walk.per, v_hi = min(walk.n, v_lo + walk.per) - 1;   // inclusive
+    BW_PDL_WAIT();
 
     RowState st;
     init_rows(p, st, 0, n_rows, q_pos0, g);
@@ -571,7 +596,7 @@ attn_keys_kernel(Params p) {
 #pragma unroll
     for (int j = 0; j < HD / 8; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
 
-    if (v_lo <= v_hi) {
+    {
         load_q_rows(p, p.cu_q[r], g, 0, n_rows, q_tile, 16);
         cp_async_commit();
         load_kv_tile(p, bt, g, kv_len, walk_tile(v_lo, kept, t_first) * BN, kv, kv + TILE_BYTES);
@@ -773,12 +798,6 @@ attn_keys_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     uint64_t* bars = reinterpret_cast<uint64_t*>(q_tile + 16 * ROW_BYTES);
     bf16* kv_new = reinterpret_cast<bf16*>(q_tile + 16 * ROW_BYTES + 64);   // [2][HD]: the token's own key and value
     const uint32_t full0 = smem_u32(bars);
-    if (threadIdx.x == 0) {
-        bw::mbar_init(full0, 1); bw::mbar_init(full0 + 8, 1);
-        bw::fence_barrier_init();
-        bw::tma_prefetch_desc(&tmK); bw::tma_prefetch_desc(&tmV);
-    }
-    __syncthreads();
     // The step's lists (work items, lengths, block tables) were on the device before the step's first
     // kernel ran; only the queries, and the keys and values of this step's own tokens, come from the
     // kernels just before this one.  The wait for those kernels therefore comes late (below).
@@ -792,10 +811,16 @@ attn_keys_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     const int* bt = p.block_table + (size_t)r * p.max_blocks;
     const int last_pos = q_pos0 + q_len - 1;
     const int first_key = bw::first_visible(q_pos0, p.window, p.chunk);
-    const int t_first = first_key / BN, t_end = last_pos / BN + 1;
-    const int per = (t_end - t_first + n_slices - 1) / n_slices;
-    const int t_lo = t_first + slice * per, t_hi = min(t_end, t_lo + per) - 1;   // inclusive; may be empty
+    const Walk walk = walk_of(p, q_pos0, last_pos, n_slices);                      // (no kept keys here)
+    if (slice >= walk.live) { leave(); return; }
+    const int t_lo = walk.t_first + slice * walk.per, t_hi = min(last_pos / BN + 1, t_lo + walk.per) - 1;   // inclusive
     const int ppt = BN / p.page_size;
+    if (threadIdx.x == 0) {
+        bw::mbar_init(full0, 1); bw::mbar_init(full0 + 8, 1);
+        bw::fence_barrier_init();
+        bw::tma_prefetch_desc(&tmK); bw::tma_prefetch_desc(&tmV);
+    }
+    __syncthreads();
 
     // Warp 0 feeds the tiles: lane pg owns page pg of a tile.  Its page id is looked up one tile
     // before its boxes are issued, so the lookup's latency is off the path; pages that do not
@@ -831,14 +856,14 @@ attn_keys_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     for (int j = 0; j < HD / 8; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
 
     // a first tile that holds none of this step's tokens is requested before the wait
-    const bool early = t_lo <= t_hi && t_lo * BN + BN <= q_pos0;
+    const bool early = t_lo * BN + BN <= q_pos0;
     if (early && warp == 0) { lookup(t_lo); issue_tile(0); lookup(t_lo + 1); }
     BW_PDL_WAIT();
     // from the unsummed q/k/v product: the slice that holds the token's own position (one per request and
     // kv head, never empty) also makes the token's key and value and puts them into its tile below
     const int t_own = last_pos / BN;
     const bool own = p.qkv != nullptr && p.append && t_lo <= t_own && t_own <= t_hi;
-    if (t_lo <= t_hi) {
+    {
         if (!early && warp == 0) { lookup(t_lo); issue_tile(0); lookup(t_lo + 1); }
         if (p.qkv) {
             rows_from_qkv(p, p.cu_q[r], g, last_pos, bt, q_tile, kv_new, own);
@@ -867,20 +892,22 @@ attn_keys_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
                     *reinterpret_cast<uint4*>(tile + (ch >> 3) * SLICE_BYTES + rk * 128 + (((ch & 7) ^ (rk & 7)) << 4)) =
                         *reinterpret_cast<const uint4*>(kv_new + which * HD + ch * 8);
                 }
-                __syncthreads();
             }
             // Rows of keys that do not exist hold whatever was there: values times a probability of
-            // 0 must still be 0, so those rows of V are cleared (only in a request's last tile or at
-            // a window's edge).
-            if (t * BN + BN > kv_len || (t * BN < first_key)) {
-                for (int idx = threadIdx.x; idx < BN * NSL * 8; idx += THREADS) {
-                    const int rk = idx / (NSL * 8), rem = idx - rk * (NSL * 8);
-                    const int key = t * BN + rk;
-                    if (key >= kv_len || bt[key / p.page_size] < 0)
-                        *reinterpret_cast<uint4*>(v_tile + (rem >> 3) * SLICE_BYTES + rk * 128 + (rem & 7) * 16) = make_uint4(0, 0, 0, 0);
+            // 0 must still be 0, so those rows of V are cleared: behind a request's last key, and before a window pages that
+            // are gone (only there are pages looked up).
+            const int there = max(kv_len - t * BN, 0), gone = first_key - t * BN;
+            auto clear = [&](int rk, int rem) {
+                *reinterpret_cast<uint4*>(v_tile + (rem >> 3) * SLICE_BYTES + rk * 128 + (rem & 7) * 16) = make_uint4(0, 0, 0, 0);
+            };
+            if (there < BN)
+                for (int idx = threadIdx.x + there * (NSL * 8); idx < BN * NSL * 8; idx += THREADS) clear(idx / (NSL * 8), idx % (NSL * 8));
+            if (gone > 0)
+                for (int idx = threadIdx.x; idx < min(gone, BN) * NSL * 8; idx += THREADS) {
+                    const int rk = idx / (NSL * 8);
+                    if (bt[(t * BN + rk) / p.page_size] < 0) clear(rk, idx - rk * (NSL * 8));
                 }
-                __syncthreads();
-            }
+            if ((own && t == t_own) || there < BN || gone > 0) __syncthreads();
             const int k_off = warp * 16;
             if (ok && t * BN + k_off <= last_pos) {
                 const bool need_mask = (t * BN + BN - 1 > q_pos0) || (t * BN < bw::first_visible(last_pos, p.window, p.chunk));
@@ -895,7 +922,7 @@ attn_keys_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
 }
 #endif  // HEAD_DIM % 64 == 0
 
-// Sums the slices of every sliced item: grid (sliced items, nkv, 16 rows), one row of one head per
+// Sums the slices of every sliced item (the live ones): grid (sliced items, nkv, 16 rows), one row of one head per
 // CTA.  The threads form MERGE_GROUPS groups of HD / 4; group j takes slices j, j + MERGE_GROUPS, ...
 // with one float4 each, so all loads of a row are in flight together; shared memory adds the groups
 // (in slice order within a group, groups in order: the same sum whatever ran beside it).
@@ -908,13 +935,14 @@ __global__ void __launch_bounds__(MERGE_THREADS)
 attn_merge_kernel(Params p, const int* merge_items) {
     BW_PDL_TRIGGER();
     const int4 w = reinterpret_cast<const int4*>(merge_items)[blockIdx.x];   // written before the step's first kernel
-    const int r = w.x, n_slices = w.z, item = w.w, g = blockIdx.y, row = blockIdx.z;
-    BW_PDL_WAIT();
+    const int r = w.x, item = w.w, g = blockIdx.y, row = blockIdx.z;
     const int n_rows = (p.cu_q[r + 1] - p.cu_q[r]) * p.G;
-    if (row >= n_rows) return;
+    if (row >= n_rows) { leave(); return; }
+    const int n_slices = live_slices(p, r, w.z);
+    BW_PDL_WAIT();
     __shared__ float sm_m[MAX_SLICES], sm_f[MAX_SLICES], sm_lf[MAX_SLICES];
     __shared__ float4 red[MERGE_GROUPS][MERGE_QUADS];
-    const size_t base0 = ((size_t)item * p.nkv + (size_t)g * n_slices) * 16 + row;
+    const size_t base0 = ((size_t)item * p.nkv + (size_t)g * w.z) * 16 + row;
     const int tid = threadIdx.x, quad = tid % MERGE_QUADS, group = tid / MERGE_QUADS;
     // this thread's partial outputs: issued before anything that depends on the maxima
     float4 part[MERGE_PER];
@@ -988,12 +1016,12 @@ __global__ void __launch_bounds__(16 * MERGE_QUADS)
 attn_merge_few_kernel(Params p, const int* merge_items) {
     BW_PDL_TRIGGER();
     const int4 w = reinterpret_cast<const int4*>(merge_items)[blockIdx.x];
-    const int r = w.x, n_slices = w.z, item = w.w, g = blockIdx.y;
+    const int r = w.x, item = w.w, g = blockIdx.y;
     const int row = threadIdx.x / MERGE_QUADS, quad = threadIdx.x - row * MERGE_QUADS;
+    const int n_rows = (p.cu_q[r + 1] - p.cu_q[r]) * p.G, n_slices = live_slices(p, r, w.z);
     BW_PDL_WAIT();
-    const int n_rows = (p.cu_q[r + 1] - p.cu_q[r]) * p.G;
     if (row >= n_rows) return;
-    const size_t base0 = ((size_t)item * p.nkv + (size_t)g * n_slices) * 16 + row;
+    const size_t base0 = ((size_t)item * p.nkv + (size_t)g * w.z) * 16 + row;
     float4 part[MERGE_FEW];
     float2 ml[MERGE_FEW];
 #pragma unroll
@@ -1037,14 +1065,15 @@ __global__ void __launch_bounds__(2 * PAIR_THREADS)
 attn_merge_pairs_kernel(Params p, const int* merge_items) {
     BW_PDL_TRIGGER();
     const int4 w = reinterpret_cast<const int4*>(merge_items)[blockIdx.x];
-    const int r = w.x, n_slices = w.z, item = w.w, g = blockIdx.y, pair = blockIdx.z;
-    BW_PDL_WAIT();
+    const int r = w.x, item = w.w, g = blockIdx.y, pair = blockIdx.z;
     const int n_rows = (p.cu_q[r + 1] - p.cu_q[r]) * p.G;
-    if (2 * pair >= n_rows) return;
+    if (2 * pair >= n_rows) { leave(); return; }
+    const int n_slices = live_slices(p, r, w.z);
+    BW_PDL_WAIT();
     __shared__ float sm_m[2][MAX_SLICES], sm_l[2][MAX_SLICES];
     __shared__ float4 red[2][PAIR_GROUPS][MERGE_QUADS];
     const int which = threadIdx.x / PAIR_THREADS, tid = threadIdx.x % PAIR_THREADS;
-    const size_t base0 = ((size_t)item * p.nkv + (size_t)g * n_slices) * 16 + 2 * pair + which;
+    const size_t base0 = ((size_t)item * p.nkv + (size_t)g * w.z) * 16 + 2 * pair + which;
     const int quad = tid % MERGE_QUADS, group = tid / MERGE_QUADS;
     constexpr int AHEAD = 8;
     float4 part[AHEAD];       // the first loads do not wait for the maxima
