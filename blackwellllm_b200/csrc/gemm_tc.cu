@@ -79,6 +79,7 @@ struct Epilogue {
     // (after bias and activation), float32 or bfloat16
     int tma_add;
     int stream;           // the k-blocks of all tiles, laid end to end, are cut into one equal range per CTA
+                          // CTA pairs: this many ranges for each tile of tokens (0: rounds of whole tiles)
     int planes;           // split-K: the partial planes ARE the result (the bias in plane 0); whoever reads them adds them up
     // an activation of common.cuh on the finished sums.  With swiglu: the gated one that replaces silu(g) * u
     // (BW_ACT_SILU, BW_ACT_CLAMPED_SWISH with its limit and alpha); without: 0 = none, BW_ACT_RELU2 or BW_ACT_GELU on every value.
@@ -358,10 +359,10 @@ __device__ __forceinline__ void rope_direct(const Epilogue& ep, const uint32_t (
 // then one TMA operation per warp.  `width`: features from f0 to the tile's end (columns behind it go out as zeros; a result
 // that is written, not added, has tiles of whole chunks).  Rows and columns past the matrix are clipped.
 __device__ __forceinline__ void box_out(const Epilogue& ep, const CUtensorMap* map, uint32_t (&v)[32], uint8_t* box, int f0, int width,
-                                        int limit, int row0, int lane) {
+                                        int limit, int row0, int lane, bool with_bias = true) {
     if (lane == 0) bw::bulk_wait_group_read<1>();   // the box used two chunks ago has been read
     __syncwarp();
-    if (ep.bias) {
+    if (ep.bias && with_bias) {
         float b[32];
         load_bias32(ep, f0, limit, b);
 #pragma unroll
@@ -777,6 +778,64 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (warp == 1) bw::tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
+// The work items of a CTA pair: whole tiles (or K splits of them) in rounds, as above; or, with ep.stream = n, equal ranges: n pairs for
+// each tile of tokens share all k-blocks of its tiles of features, laid end to end.  The pairs of one range walk the same weights side by
+// side, so these come from memory once (ranges dealt out over all tiles in a row do not, and measured 112 us where the rounds took 82: down
+// of 3584 x 18944 at 800 tokens).  A tile that ranges share is ADDED into the result part by part, its last part first: that part is the
+// first thing its pair does, and the parts before it end when the kernel ends, so who has to wait seldom does.  Pairs wait for pairs behind
+// them only, and only for the first item of their ranges.
+struct PairItems {
+    int kb_total, kb_per_split, tiles, num_work, splits, sharers, w, stride, self, lo, hi, total, line, lines;
+    __host__ __device__ PairItems(int splits_, int sharers_, int kb_total_, int kb_per_split_, int tiles_, int num_work_, int tiles_a,
+                                  int pair, int n_pairs)
+        : kb_total(kb_total_), kb_per_split(kb_per_split_), tiles(tiles_), num_work(num_work_), splits(splits_), sharers(sharers_), w(pair),
+          stride(n_pairs), self(0), lo(0), hi(0), total(0), line(0), lines(tiles_a) {
+        if (sharers > 0) {
+            self = pair / lines;
+            line = pair - self * lines;
+            total = tiles / lines * kb_total;
+            lo = (int)((long long)self * total / sharers);
+            hi = (int)((long long)(self + 1) * total / sharers);
+        }
+    }
+    __host__ __device__ int owner(int kb) const { return (int)(((long long)(kb + 1) * sharers + total - 1) / total) - 1; }
+    __host__ __device__ bool next(Item& it) {
+        if (sharers == 0) {
+            if (w >= num_work) return false;
+            it.tile = w % tiles;
+            it.part = w / tiles;
+            it.nparts = splits;
+            it.kb0 = it.part * kb_per_split;
+            it.nkb = (kb_total < it.kb0 + kb_per_split ? kb_total : it.kb0 + kb_per_split) - it.kb0;
+            w += stride;
+            return true;
+        }
+        if (lo >= hi) return false;
+        const int t = lo / kb_total;
+        it.tile = t * lines + line;
+        it.kb0 = lo - t * kb_total;
+        it.nkb = kb_total - it.kb0 < hi - lo ? kb_total - it.kb0 : hi - lo;
+        lo += it.nkb;
+        const int first = owner(t * kb_total);
+        it.part = self - first;
+        it.nparts = owner((t + 1) * kb_total - 1) - first + 1;
+        return true;
+    }
+};
+
+// Waits until the later parts of a shared tile are in the result (lane 0's counter says how many are; bounded).
+__device__ __forceinline__ bool wait_for_parts(const int* counter, int want, int* status, int code) {
+    const uint64_t t0 = bw::global_timer_ns();
+    for (uint32_t i = 0; i < BW_SPIN_LIMIT; ++i) {
+        int seen;
+        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+        if (seen == want) return true;
+        if ((i & 63) == 63 && bw::global_timer_ns() - t0 > BW_WAIT_NS) break;
+    }
+    if (status) atomicExch(status, code);
+    return false;
+}
+
 // The same product for many tokens on CTA PAIRS (cta_group::2): a cluster of two CTAs takes a tile of
 // 256 tokens x BN features.  Each CTA loads its 128 rows of x and HALF of the BN weight rows (so a
 // k-block costs it 16 + BN / 8 KB instead of 16 + BN / 4: less traffic from L2 per flop, and room
@@ -836,7 +895,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (lane == 0) {
             uint32_t it = 0;
             bool ok = true;
-            Items items(ep, kb_total, kb_per_split, tiles, num_work, pair, n_pairs);
+            PairItems items(ep.splits, ep.stream, kb_total, kb_per_split, tiles, num_work, tiles_a, pair, n_pairs);
             Item im;
             BW_PDL_WAIT();
             while (ok && items.next(im)) {
@@ -858,7 +917,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             uint32_t it = 0, n = 0;
             bool ok = true;
             const uint32_t tmem0 = __shfl_sync(0xffffffffu, tmem_base, 0), smem0 = bw::smem_u32(smem);
-            Items items(ep, kb_total, kb_per_split, tiles, num_work, pair, n_pairs);
+            PairItems items(ep.splits, ep.stream, kb_total, kb_per_split, tiles, num_work, tiles_a, pair, n_pairs);
             Item im;
             for (; ok && items.next(im); ++n) {
                 const uint32_t acc = n & 1, accph = (n >> 1) & 1;
@@ -890,7 +949,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         float* stage = staging + (warp - 2) * (32 * 33);
         const int a_rows = ep.transposed ? ep.features : ep.tokens, b_rows = ep.transposed ? ep.tokens : ep.features;
         uint32_t n = 0;
-        Items items(ep, kb_total, kb_per_split, tiles, num_work, pair, n_pairs);
+        PairItems items(ep.splits, ep.stream, kb_total, kb_per_split, tiles, num_work, tiles_a, pair, n_pairs);
         Item im;
         for (; items.next(im); ++n) {
             const int tile_a = ep.transposed ? im.tile / tiles_b : im.tile % tiles_a, tile_b = ep.transposed ? im.tile % tiles_b : im.tile / tiles_a;
@@ -901,6 +960,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             const int row0 = tile_a * 2 * BM + (int)rank * BM + quarter * 32;   // first token of this warp
             float* part = (ep.partial && im.nparts > 1) ? ep.partial + (size_t)im.part * ((size_t)ep.tokens * ep.features) : nullptr;
             int rope_kv = -1;
+            // a tile that pairs share: added in a fixed order, so that the sum is the same whatever ran beside it
+            const bool shared = ep.stream > 0 && im.nparts > 1;
+            int* added = shared ? ep.counters + (im.tile * 2 + (int)rank) * 4 + quarter : nullptr;
+            if (shared && im.part < im.nparts - 1) {
+                int there = 1;
+                if (lane == 0) {
+                    there = wait_for_parts(added, im.nparts - 1 - im.part, &g_status, 35);
+                    asm volatile("fence.proxy.async;" ::: "memory");
+                }
+                if (!__shfl_sync(0xffffffffu, there, 0)) break;
+            }
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 32) {
                 uint32_t v[32];
@@ -937,7 +1007,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 } else if (ep.tma_add) {
                     if constexpr (!ROPE) {
                         uint8_t* box = (uint8_t*)staging + ((warp - 2) * 2 + ((c0 / 32) & 1)) * 4096;
-                        box_out(ep, &tmC, v, box, tile_b * BN + c0, BN - c0, b_rows, row0, lane);
+                        box_out(ep, &tmC, v, box, tile_b * BN + c0, BN - c0, b_rows, row0, lane, !shared || im.part == 0);
                     }
                 } else if (ROPE) {
                     if constexpr (ROPE) {
@@ -965,6 +1035,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             bw::tc_fence_before();
             __syncwarp();
             if (lane == 0) bw::mbar_arrive_cluster(bw::pair_leader_addr(tempty0 + 8 * acc));
+            if (shared && lane == 0) {
+                if (im.part == 0) *added = 0;          // (the others have counted; zero again for the next launch)
+                else {
+                    bw::bulk_wait_group<0>();          // the boxes have been added
+                    asm volatile("fence.proxy.async;" ::: "memory");
+                    __threadfence();
+                    atomicAdd(added, 1);
+                }
+            }
         }
         if (ep.tma_add && lane == 0) bw::bulk_wait_group<0>();
     }
@@ -1152,7 +1231,7 @@ int launch_pair(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c
     static bool attr_done[bw::MAX_DEVICES];
     if (cudaError_t e = bw::allow_dynamic_smem(gemm_pair_kernel<BN, ROPE>, smem, attr_done); e != cudaSuccess) return (int)e;
     const int NUM_SMS = bw::num_sms();
-    const int num_work = tiles_a * tiles_b * (ep.splits > 1 ? ep.splits : 1);
+    const int num_work = ep.stream > 0 ? ep.stream * tiles_a : tiles_a * tiles_b * (ep.splits > 1 ? ep.splits : 1);
     const int pairs = num_work < NUM_SMS / 2 ? num_work : NUM_SMS / 2;
     bw::launch_pairs((gemm_pair_kernel<BN, ROPE>), dim3(2 * pairs), dim3(THREADS), smem, s, a, b, c, ep, kb_total, kb_per_split,
                      tiles_a, tiles_b, num_work);
@@ -1297,8 +1376,32 @@ static double swiglu_pair_plan(int M, int N, int K, int* width) {
     return best;
 }
 
+// Pairs on equal ranges (PairItems), for sums that the TMA unit adds into float32: no planes, no second kernel, only the parts' turns.  As many
+// ranges for each tile of tokens as there are pairs for it, two a tile of features at most (three parts), of 16 k-blocks or more; tiles of 256
+// features.  Returns the ranges if they are to be taken in place of the pairs' plan (width, splits) with its estimate `cost`, else 0.
+// Measured, us, rounds / ranges: 3584 x 18944 at 512, 648 and 1,536 tokens 62.7 / 60.6, 81.1 / 72.9, 156.7 / 144.5; 4096 x 14336 at 512, 1,280
+// and 1,536 54.7 / 50.4, 119.7 / 99.5, 127.6 / 120.3; 5120 x 13824 at 300 and 1,024 62.1 / 52.8, 115.8 / 96.5; 5120 x 5120 at 1,024 49.4 /
+// 42.0; 4096 x 4096 at 1,280 39.9 / 35.2.  But 3584 x 18944 at 1,024 tokens 95.4 / 96.1 and 3584 x 3584 at 648 22.7 / 29.5: the ranges' time
+// is 0.38 us a k-block and 7 us; a round's is 0.40 us (256 columns), less in one that is partly empty, down to 0.85 of it (the chip as a
+// whole, not a pair, is the limit there).  Tokens of more than 60 MB, which each range reads at its own place, leave L2: at 2,048 tokens of
+// 18,944 188 / 195.
+static int shared_ranges(int M, int N, int K, int width, int splits, double cost) {
+    const int n_pairs = bw::num_sms() / 2, ta = ceil_div(M, 2 * BM), tb = ceil_div(N, 256), kb_total = ceil_div(K, BK);
+    int ranges = n_pairs / ta;
+    if (ranges > 2 * tb) ranges = 2 * tb;
+    if (ranges < 4 || (long long)tb * kb_total < 16LL * ranges || (long long)M * K * 2 > 60000000) return 0;
+    if (splits == 1 && width > 0) {
+        const long long t = (long long)ta * ceil_div(N, width);
+        const double columns = width == 256 ? 231.0 : width == 224 ? 213.0 : width == 192 ? 185.0 : 166.0;
+        const double last = (double)(t % n_pairs) / n_pairs;
+        cost = ((double)(t / n_pairs) + (last == 0.0 ? 0.0 : last < 0.85 ? 0.85 : last)) * kb_total * columns;
+    }
+    return (double)tb / ranges * kb_total * 220.0 + 4050.0 < 0.93 * cost ? ranges : 0;
+}
+
 // How a product runs, from bw_gemm_tc_plan's decision (transposed, bn, splits) and the pairs' estimate.  kind: 0 plain, 1 SwiGLU, 2 rotary,
-// 3 sums left open.  pair_mode: bw_gemm_tc_pair_mode's.  Returns 1 for CTA pairs (bn: a pair's features; transposed: its tokens), 0 for single CTAs.
+// 3 sums left open, 4 plain, added into float32 by TMA.  pair_mode: bw_gemm_tc_pair_mode's.  Returns 0 for single CTAs, 1 for CTA pairs (bn: a
+// pair's features; transposed: its tokens), 1 + n for n equal ranges a tile of tokens.
 BW_EXPORT int bw_gemm_tc_route(int M, int N, int K, int kind, int pair_mode, int force_splits, long long workspace_elems, int* transposed,
                                int* bn, int* splits) {
     const int NUM_SMS = bw::num_sms();
@@ -1320,7 +1423,7 @@ BW_EXPORT int bw_gemm_tc_route(int M, int N, int K, int kind, int pair_mode, int
         // 129 to 256 tokens on one pair tile of tokens, but for a long K, whose splits the 128-row tiles of features deal out better (us, as
         // they were / on pairs: gate/up of 28672 x 4096 at 160 and 256 tokens 77 / 54 and 92 / 56, q/k/v of 6144 x 4096 31 / 24 and 39 / 25,
         // o of 4096 at 160, 200 and 256 17.5 / 19.2, 20.7 / 19.4 and 21.4 / 19.4, its down projection 36 to 40 / 54)
-        if (pair_mode > 0 && M > BM && (kind != 0 || (kb_total < 128 && (M > 160 || *splits == 1)))) {
+        if (pair_mode > 0 && M > BM && ((kind != 0 && kind != 4) || (kb_total < 128 && (M > 160 || *splits == 1)))) {
             const double pair = pair_plan(M, N, K, 0, workspace_elems, true, &width, &ps);
             if (pair < 0.0) return 0;
             *transposed = 0; *bn = width; *splits = ps;
@@ -1342,7 +1445,12 @@ BW_EXPORT int bw_gemm_tc_route(int M, int N, int K, int kind, int pair_mode, int
         *transposed = 1; *bn = other; *splits = 1;
         return 1;
     }
-    if (pair < 0.0 || (pair_mode != 2 && pair > single)) return 0;
+    const bool use_single = pair < 0.0 || (pair_mode != 2 && pair > single);
+    if (kind == 4 && force_splits <= 0) {
+        const int ranges = shared_ranges(M, N, K, use_single ? 0 : width, use_single ? 1 : ps, use_single ? single : pair);
+        if (ranges > 0) { *bn = 256; *splits = 1; return 1 + ranges; }
+    }
+    if (use_single) return 0;
     *bn = width; *splits = ps;
     return 1;
 }
@@ -1391,8 +1499,13 @@ static int run_gemm_tc(const void* x, const void* w, const void* bias, int bias_
             return BW_ERR_BAD_ARG;
     }
     if (g_pair_mode < 0) { const char* e = getenv("BW_GEMM_PAIR"); g_pair_mode = (e && e[0] >= '0' && e[0] <= '2') ? e[0] - '0' : 1; }
-    const bool use_pairs = bw_gemm_tc_route(M, N, K, planes ? 3 : rope ? 2 : swiglu ? 1 : 0, g_pair_mode, force_splits,
-                                            can_split ? workspace_elems : 0, &tr, &bn, &splits) != 0;
+    const bool tma_out = ((uintptr_t)out & 15) == 0 && ldo % (out_type == BW_F32 ? 4 : 8) == 0;
+    // (a tile has eight counters: each of the two CTAs' four epilogue warps counts for itself)
+    const bool may_share = accumulate && tma_out && can_split && 8LL * ceil_div(M, 2 * BM) * ceil_div(N, 128) <= n_counters;
+    const int route = bw_gemm_tc_route(M, N, K, planes ? 3 : rope ? 2 : swiglu ? 1 : may_share ? 4 : 0, g_pair_mode, force_splits,
+                                       can_split ? workspace_elems : 0, &tr, &bn, &splits);
+    const bool use_pairs = route != 0;
+    const int sharers = route > 1 ? route - 1 : 0;
     const int kb_per_split = ceil_div(kb_total, splits);
     splits = ceil_div(kb_total, kb_per_split);   // no empty split
     const long long a_rows = tr ? N : M, b_rows = tr ? M : N;
@@ -1415,7 +1528,7 @@ static int run_gemm_tc(const void* x, const void* w, const void* bias, int bias_
     const bool stream_k = tr && fused_reduce && can_split && !planes && force_splits <= 0 && splits == 1 && n_tiles > NUM_SMS &&
                           n_tiles % NUM_SMS != 0 && 2LL * M * N <= workspace_elems && n_tiles * 4 <= n_counters;
     if (stream_k) splits = 2;   // at most two CTAs share a tile: two planes of partial sums
-    ep.out = out; ep.partial = splits > 1 ? workspace : nullptr; ep.counters = (fused_reduce && !planes) ? counters : nullptr;
+    ep.out = out; ep.partial = splits > 1 ? workspace : nullptr; ep.counters = ((fused_reduce && !planes) || sharers > 0) ? counters : nullptr;
     ep.planes = planes ? 1 : 0;
     if (planes) *planes_out = splits;
     ep.bias = bias; ep.ldo = ldo;
@@ -1423,13 +1536,13 @@ static int run_gemm_tc(const void* x, const void* w, const void* bias, int bias_
     ep.act = act; ep.act_limit = act_limit; ep.act_alpha = act_alpha;
     ep.swiglu = swiglu; ep.tokens = M; ep.features = N; ep.splits = splits;
     ep.rope_on = rope ? 1 : 0;
-    ep.stream = stream_k ? 1 : 0;
+    ep.stream = stream_k ? 1 : sharers;
     if (rope) ep.rope = *rope; else ep.rope = RopeOut{};
     // many tokens and no split: the epilogue hands 32 x 32 boxes to the TMA unit
     CUtensorMap tc;
     std::memset(&tc, 0, sizeof(tc));
     ep.tma_add = BOX_NONE;
-    if (!tr && splits == 1 && !rope && !swiglu && !planes && ((uintptr_t)out & 15) == 0 && ldo % (out_type == BW_F32 ? 4 : 8) == 0) {
+    if (!tr && splits == 1 && !rope && !swiglu && !planes && tma_out) {
         // (boxes that are written need tiles of whole boxes: 240 columns are seven and a half)
         if (accumulate) ep.tma_add = BOX_ADD;
         else if (bn % 32 == 0) ep.tma_add = out_type == BW_F32 ? BOX_F32 : BOX_BF16;

@@ -118,9 +118,10 @@ def test_pair_plan_splits_k_only_where_the_pairs_would_idle():
     assert plan(700, 520, 2240, force=3)[2] == 3                 # a forced split is taken as it is
 
 
-@pytest.mark.parametrize("kind", (0, 1, 2, 3))
+@pytest.mark.parametrize("kind", (0, 1, 2, 3, 4))
 def test_every_route_is_one_the_kernels_are_built_for(plan, kind):
-    """``bw_gemm_tc_route``: single CTAs in either orientation or CTA pairs (kind 0 plain, 1 SwiGLU, 2 rotary, 3 sums left open)."""
+    """``bw_gemm_tc_route``: single CTAs in either orientation or CTA pairs (kind 0 plain, 1 SwiGLU, 2 rotary, 3 sums left open, 4 added
+    into float32, in equal ranges of k-blocks where that is faster)."""
     from blackwellllm_b200.kernels.build import load_library
     fn = load_library("gemm_tc").bw_gemm_tc_route
     fn.argtypes = [ctypes.c_int] * 6 + [ctypes.c_longlong] + [ctypes.POINTER(ctypes.c_int)] * 3
@@ -140,5 +141,10 @@ def test_every_route_is_one_the_kernels_are_built_for(plan, kind):
                 else:
                     assert bn.value in (128, 192, 224, 256), what
                 assert not force or M > 256, what
+                if pairs > 1:       # ranges of half a tile of features or longer, and of 16 k-blocks; no planes
+                    ranges, tiles = pairs - 1, ceil_div(N, 256)
+                    assert kind == 4 and M > 256 and not force and (tr.value, bn.value, splits.value) == (0, 256, 1), what
+                    assert ranges * ceil_div(M, 2 * BM) <= NUM_SMS // 2 and ranges <= 2 * tiles, what
+                    assert tiles * ceil_div(K, BK) >= 16 * ranges, what
             elif (tr.value, bn.value, splits.value) != (tr0, bn0, planned):
                 assert kind == 1 and 64 < M <= 128 and tr.value == 0 and bn.value in (224, 256) and splits.value == 1, what

@@ -243,6 +243,35 @@ def test_gemm_tc_split_k_on_cta_pairs(ops, M, splits, mode):
         ops.gemm_pair_mode(before if before >= 0 else 1)
 
 
+@pytest.mark.parametrize("M,N,K,ldo", [(512, 4096, 14336, 4096), (300, 5120, 13824, 5120), (648, 3584, 18944, 3592), (1010, 5100, 5120, 5100),
+                                       (1280, 4090, 8200, 4096)])
+def test_gemm_tc_pairs_on_equal_ranges(ops, M, N, K, ldo):
+    """Sums added into float32 by CTA pairs in equal ranges of k-blocks: the parts of a tile are added one after another, the last range's
+    first: right (ragged rows and features, a wider row of the result), the bias added once, bit-equal when repeated, and the columns behind
+    the result untouched.  Tolerance: the tensor cores cut the running sum off at 24 bits after each 16 products, so K / 16 steps err by less
+    than K / 16 * 2^-23 of the largest sum."""
+    import ctypes
+    from blackwellllm_b200.kernels.build import load_library
+    fn = load_library("gemm_tc").bw_gemm_tc_route
+    fn.argtypes = [ctypes.c_int] * 6 + [ctypes.c_longlong] + [ctypes.POINTER(ctypes.c_int)] * 3
+    tr, bn, splits = ctypes.c_int(0), ctypes.c_int(256), ctypes.c_int(1)
+    assert fn(M, N, K, 4, 1, 0, 1 << 24, ctypes.byref(tr), ctypes.byref(bn), ctypes.byref(splits)) > 1
+    x = rand(M, K, dtype=torch.bfloat16, seed=5).to(DEV)
+    w = rand(N, K, dtype=torch.bfloat16, seed=6, scale=0.05).to(DEV)
+    b = rand(N, seed=7).to(DEV)
+    base = rand(M, ldo, seed=8).to(DEV)
+    ref = x.double() @ w.double().T + b.double() + base[:, :N].double()
+    outs = []
+    for _ in range(3):
+        out = base.clone()
+        ops.gemm_tc(x, w, b, out=out[:, :N], accumulate=True)
+        outs.append(out)
+    assert ops.gemm_tc_status() == 0
+    assert float((outs[0][:, :N].double() - ref).abs().max()) <= K / 16 * 2 ** -23 * float(ref.abs().max())
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    assert torch.equal(outs[0][:, N:], base[:, N:])
+
+
 def test_gemm_tc_split_k_on_a_tile_width_that_is_no_power_of_two(ops):
     M, N, K = 2048, 4096, 256     # 16 x 18 tiles of 240 columns: the last one of a row is cut at 4096
     x = rand(M, K, dtype=torch.bfloat16, seed=5).to(DEV)
