@@ -105,13 +105,14 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
     }
     // a portion's rows may differ in the size of their slices (it never shrinks, except where a block of positions begins)
     const bool same = !SLICES && slice_keys(p, end - 1) == keys && (p.chunk <= 0 || p.chunk <= SLICE * MOST);
-    int pages[KT / WARPS];                          // of the keys that are fetched next, looked up before
+    // Page and place in it of the warp's keys that are fetched next, looked up before: a lane a key (all lanes for every key were half of
+    // a decoding block's instructions)
+    constexpr int MINE = KT / WARPS;
+    int my_page = -1, my_slot = 0;
     auto look_up = [&](int tile) {
-#pragma unroll
-        for (int j = 0; j < KT / WARPS; ++j) {
-            const int kp = base + tile * KEYS + warp * (KT / WARPS) + j;
-            pages[j] = tile < last && kp < end ? bt[kp / p.page_size] : -1;
-        }
+        const int kp = base + tile * KEYS + warp * MINE + lane, block = kp / p.page_size;
+        my_slot = kp - block * p.page_size;
+        my_page = lane < MINE && tile < last && kp < end ? bt[block] : -1;
     };
     look_up(first);      // (block tables are on the device before the step's first kernel, as the work lists are)
     BW_PDL_WAIT();
@@ -121,17 +122,20 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
         for (int c = lane * 4; c < hd; c += 128) copy16(qs + i * ldk + c, src + c, i < rows);
     }
     auto fetch = [&](int tile, int st) {            // the KT keys from this tile on: a warp brings some and their values
+        const bool mine = my_page >= 0 && my_page < p.num_pages;
+        const long long mine_at = mine ? (((long long)my_page * p.nkv + kvh) * p.page_size + my_slot) * hd : -1;
 #pragma unroll
-        for (int j = 0; j < KT / WARPS; ++j) {
-            const int key = warp * (KT / WARPS) + j, kp = base + tile * KEYS + key, page = pages[j];
-            const bool ok = page >= 0 && page < p.num_pages;
-            const size_t at = ok ? (((size_t)page * p.nkv + kvh) * p.page_size + (kp % p.page_size)) * hd : 0;
+        for (int j = 0; j < MINE; ++j) {
+            const int key = warp * MINE + j;
+            const long long there = __shfl_sync(0xffffffffu, mine_at, j);
+            const bool ok = there >= 0;
+            const size_t at = ok ? there : 0;
             for (int c = lane * 4; c < hd; c += 128) {
                 copy16(ks + (st * KT + key) * ldk + c, p.k_pages + at + c, ok);
                 copy16(vs + (st * KT + key) * hd + c, p.v_pages + at + c, ok);
             }
-            if (lane == 0) known[st * KT + key] = ok;
         }
+        if (lane < MINE) known[st * KT + warp * MINE + lane] = mine;
         asm volatile("cp.async.commit_group;" ::: "memory");
         look_up(tile + PARTS);
     };
@@ -233,20 +237,21 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
             const int tile = from + part;
             if (tile >= last) break;
             float* pt = ps + part * KEYS;
-            if (ROWS == 64 || warp < rows) {
+            auto softmax_and_values = [&](auto taken) {
+                constexpr int N = decltype(taken)::value;     // of the warp's rows
                 // (a warp's rows side by side: one after another their shuffles and exponentials are the kernel's latency at few keys)
-                float sc[RW], m_new[RW], e[RW], sum[RW];
+                float sc[N], m_new[N], e[N], sum[N];
                 bool zero = false;
 #pragma unroll
-                for (int i = 0; i < RW; ++i) sc[i] = ROWS == 64 || row_of(i) < rows ? pt[row_of(i) * LDP + lane] : -INFINITY;
+                for (int i = 0; i < N; ++i) sc[i] = ROWS == 64 || row_of(i) < rows ? pt[row_of(i) * LDP + lane] : -INFINITY;
 #pragma unroll
-                for (int i = 0; i < RW; ++i) m_new[i] = fmaxf(m[i], bw::warp_max(sc[i]));
+                for (int i = 0; i < N; ++i) m_new[i] = fmaxf(m[i], bw::warp_max(sc[i]));
 #pragma unroll
-                for (int i = 0; i < RW; ++i) e[i] = sc[i] == -INFINITY ? 0.f : expf(sc[i] - m_new[i]);
+                for (int i = 0; i < N; ++i) e[i] = sc[i] == -INFINITY ? 0.f : expf(sc[i] - m_new[i]);
 #pragma unroll
-                for (int i = 0; i < RW; ++i) sum[i] = bw::warp_sum(e[i]);
+                for (int i = 0; i < N; ++i) sum[i] = bw::warp_sum(e[i]);
 #pragma unroll
-                for (int i = 0; i < RW; ++i) {
+                for (int i = 0; i < N; ++i) {
                     const float corr = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new[i]);
                     l[i] = l[i] * corr + sum[i];
                     m[i] = m_new[i];
@@ -262,9 +267,9 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
                 auto add_values = [&](auto skip) {
 #pragma unroll 2
                     for (int k4 = 0; k4 < KEYS; k4 += 4) {
-                        float4 w[RW];
+                        float4 w[N];
 #pragma unroll
-                        for (int i = 0; i < RW; ++i) w[i] = *reinterpret_cast<const float4*>(pt + row_of(i) * LDP + k4);
+                        for (int i = 0; i < N; ++i) w[i] = *reinterpret_cast<const float4*>(pt + row_of(i) * LDP + k4);
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
@@ -273,7 +278,7 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
                                 if (c >= hd) continue;
                                 const float4 v = *reinterpret_cast<const float4*>(vt + (k4 + kk) * hd + c);
 #pragma unroll
-                                for (int i = 0; i < RW; ++i) {
+                                for (int i = 0; i < N; ++i) {
                                     const float e = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
                                     if (decltype(skip)::value && e == 0.f) continue;
                                     o[i][4 * h] = fmaf(e, v.x, o[i][4 * h]);
@@ -286,7 +291,10 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
                 };
                 if (__any_sync(0xffffffffu, zero)) add_values(std::true_type{});
                 else add_values(std::false_type{});
-            }
+            };
+            if constexpr (ROWS == 64) softmax_and_values(std::integral_constant<int, RW>{});
+            else if (warp + WARPS < rows) softmax_and_values(std::integral_constant<int, 2>{});
+            else if (warp < rows) softmax_and_values(std::integral_constant<int, 1>{});
             if constexpr (SLICES) {
                 if (!whole && ((tile + 1) % per == 0 || tile + 1 == last)) {
                     const size_t at = part_row(p, item.w, tile / per, rows, kvh);
