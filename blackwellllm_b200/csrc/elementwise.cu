@@ -341,6 +341,44 @@ __global__ void swiglu_kernel(const IT* __restrict__ gu, OT* __restrict__ out, i
     }
 }
 
+// The same for I a multiple of four and rows that begin on four elements: a thread four channels of one token.  Bound by its bytes; the
+// element kernel is not, it divides for each of them (float32, 301 tokens of 14336: 15.8 us, 8.4 so).
+template <typename T> struct Four;
+template <> struct Four<float> {
+    static __device__ __forceinline__ void load(const float* p, float (&v)[4]) {
+        const float4 t = *reinterpret_cast<const float4*>(p);
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    }
+    static __device__ __forceinline__ void store(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+};
+template <> struct Four<bf16> {
+    static __device__ __forceinline__ void load(const bf16* p, float (&v)[4]) {
+        const uint2 t = *reinterpret_cast<const uint2*>(p);
+        const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&t.x), b = *reinterpret_cast<const __nv_bfloat162*>(&t.y);
+        v[0] = __bfloat162float(a.x); v[1] = __bfloat162float(a.y); v[2] = __bfloat162float(b.x); v[3] = __bfloat162float(b.y);
+    }
+    static __device__ __forceinline__ void store(bf16* p, const float (&v)[4]) {
+        __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+        *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+    }
+};
+template <typename IT, typename OT>
+__global__ void __launch_bounds__(256)
+swiglu_four_kernel(const IT* __restrict__ gu, OT* __restrict__ out, int I, int act, float limit, float alpha) {
+    BW_PDL_TRIGGER();
+    BW_PDL_WAIT();
+    const IT* row = gu + (size_t)blockIdx.x * 2 * I;
+    OT* to = out + (size_t)blockIdx.x * I;
+    for (int c = (blockIdx.y * 256 + threadIdx.x) * 4; c < I; c += gridDim.y * 1024) {
+        float g[4], u[4], y[4];
+        Four<IT>::load(row + c, g);
+        Four<IT>::load(row + I + c, u);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[i] = bw::glu(act, g[i], u[i], limit, alpha);
+        Four<OT>::store(to + c, y);
+    }
+}
+
 // An activation without a gate, element by element: BW_ACT_RELU2: max(x, 0)^2; BW_ACT_GELU: 0.5 x (1 + erf(x / sqrt(2))).
 template <typename IT, typename OT>
 __global__ void unary_act_kernel(const IT* __restrict__ x, OT* __restrict__ out, size_t total, int act) {
@@ -791,6 +829,15 @@ static int launch_glu(const void* gu, int in_type, void* out, int out_type, int 
     cudaStream_t s = (cudaStream_t)stream;
     const size_t total = (size_t)T * I;
     const int threads = 256;
+    if (I > 0 && I % 4 == 0 && (((uintptr_t)gu | (uintptr_t)out) & 15) == 0) {
+        const dim3 grid(T, (I + 1023) / 1024 < 64 ? (I + 1023) / 1024 : 64);
+        if (in_type == BW_F32 && out_type == BW_F32) bw::launch((swiglu_four_kernel<float, float>), grid, dim3(threads), 0, s, cp<float>(gu), mp<float>(out), I, act, limit, alpha);
+        else if (in_type == BW_BF16 && out_type == BW_BF16) bw::launch((swiglu_four_kernel<bf16, bf16>), grid, dim3(threads), 0, s, cp<bf16>(gu), mp<bf16>(out), I, act, limit, alpha);
+        else if (in_type == BW_F32 && out_type == BW_BF16) bw::launch((swiglu_four_kernel<float, bf16>), grid, dim3(threads), 0, s, cp<float>(gu), mp<bf16>(out), I, act, limit, alpha);
+        else return BW_ERR_BAD_ARG;
+        BW_LAUNCH_CHECK();
+        return 0;
+    }
     const int blocks = (int)((total + threads - 1) / threads < 148 * 16 ? (total + threads - 1) / threads : 148 * 16);
     if (in_type == BW_F32 && out_type == BW_F32) bw::launch((swiglu_kernel<float, float>), dim3(blocks), dim3(threads), 0, s, cp<float>(gu), mp<float>(out), I, total, act, limit, alpha);
     else if (in_type == BW_BF16 && out_type == BW_BF16) bw::launch((swiglu_kernel<bf16, bf16>), dim3(blocks), dim3(threads), 0, s, cp<bf16>(gu), mp<bf16>(out), I, total, act, limit, alpha);

@@ -507,6 +507,17 @@ def test_swiglu(ops, I, dt):
     assert float((out.double() - ref).abs().max()) <= tol * float(ref.abs().max())
 
 
+@pytest.mark.parametrize("T,I", [(1, 4), (3, 1020), (2, 1028), (300, 4100), (1, 65536 + 8)])
+@pytest.mark.parametrize("dt,out_dt", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16), (torch.float32, torch.bfloat16)])
+def test_swiglu_four_channels_a_thread(ops, T, I, dt, out_dt):
+    """Rows that begin on four elements take four channels a thread: bit for bit what the element kernel makes of the same rows
+    at an odd address (one formula, no sums)."""
+    odd = torch.empty(T * 2 * I + 1, dtype=dt, device=DEV)[1:].view(T, 2 * I)
+    gu = rand(T, 2 * I, dtype=dt, seed=1, scale=2.0).to(DEV)
+    odd.copy_(gu)
+    assert torch.equal(ops.swiglu(gu, out_dtype=out_dt), ops.swiglu(odd, out_dtype=out_dt))
+
+
 # ------------------------------------------------------------------ attention over pages
 
 class FakeBatch:
