@@ -13,8 +13,8 @@
 // partial results per kv head at any context: 64 requests of 8 kv heads and groups of 4 at 131,072 tokens 69 MB.)
 // What bounds it: decode, the bytes of keys and values; prompts, shared-memory reads (six 16-byte reads per 32 FMAs); few keys, latency.
 // Measured at head size 128, groups of 4, 8 kv heads, against attention_simt.cu (a block per token and head, a lane a key): 4 requests
-// at 1,000 keys 29 us with the merge against 167, 4 portions of 200 tokens 126 against 1,402, 9 tokens 6.1 against 9.5.  Slower than
-// that kernel is what keeps a tile's rows idle: 64 requests at 300 keys, groups of 1, 8 kv heads of 64: 92 us against 66.
+// at 1,000 keys 18 us with the merge against 167, 4 portions of 200 tokens 109 against 1,402, 64 requests at 300 keys, groups of 1, 8 kv
+// heads of 64, 54 against 66.
 #include <type_traits>
 #include "common.cuh"
 
@@ -39,8 +39,9 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool valid)
 // Tiles of keys in flight or at work: prompts work on a tile for longer than the next one takes to come; a decoding request's few rows do not.
 __host__ __device__ constexpr int stages(int rows) { return rows == 64 ? 2 : 3; }
 // Keys that a block fetches and scores at once (the softmax takes KEYS of them at a time).  Of a prompt's 64 rows a thread scores 4 x 4 with
-// 64 keys, eight 16-byte reads of shared memory per 64 FMAs; with 32 keys 2 x 4, six reads per 32, which the reads bound.
-__host__ __device__ constexpr int fetched(int rows, int ch, bool slices) { return rows == 64 && ch == 1 && !slices ? 64 : KEYS; }
+// 64 keys, eight 16-byte reads of shared memory per 64 FMAs; with 32 keys 2 x 4, six reads per 32, which the reads bound.  One such block an
+// SM, slices dealt out or not (two of 128 registers with 32 keys each took 56 us for a slice of 128 keys, one of this kind 30).
+__host__ __device__ constexpr int fetched(int rows, int ch) { return rows == 64 && ch == 1 ? 64 : KEYS; }
 __host__ __device__ constexpr int smem_floats(int rows, int hd, int kt) {
     return rows * (hd + 4) + stages(rows) * (kt * (hd + 4) + kt * hd + kt) + rows * (kt + 4);
 }
@@ -72,13 +73,13 @@ __device__ __forceinline__ size_t part_row(const Params& p, int where, int slice
 // the tile's slices, whose rows have slices of one size.  Of a single slice the block writes the tile's result (its fold is it).
 // CH: groups of four channels of a lane.
 template <int ROWS, int CH, bool SLICES>
-__global__ void __launch_bounds__(THREADS, !SLICES ? 1 : 2)
+__global__ void __launch_bounds__(THREADS, ROWS == 64 ? 1 : 2)
 attention_f32_kernel(Params p, const int4* __restrict__ work) {
     BW_PDL_TRIGGER();
     extern __shared__ float4 smem4[];
     const int hd = p.hd, ldk = hd + 4, G = p.nh / p.nkv;
     float* qs = reinterpret_cast<float*>(smem4);          // [ROWS][ldk]
-    constexpr int STAGES = stages(ROWS), KT = fetched(ROWS, CH, SLICES), PARTS = KT / KEYS, LDP = KT + 4;
+    constexpr int STAGES = stages(ROWS), KT = fetched(ROWS, CH), PARTS = KT / KEYS, LDP = KT + 4;
     float* ks = qs + ROWS * ldk;                          // [STAGES][KT][ldk]
     float* vs = ks + STAGES * KT * ldk;                   // [STAGES][KT][hd]
     float* ps = vs + STAGES * KT * hd;                    // [ROWS][LDP]
@@ -142,7 +143,7 @@ attention_f32_kernel(Params p, const int4* __restrict__ work) {
     // Rows that a warp takes through the softmax and the values: side by side in a tile of 64; of few rows one each for as many warps
     // as there are (with their neighbours, and all warps through the products of empty rows, two stages and a page looked up where it was
     // needed: 4 requests at 1,000 keys, groups of 4, 8 kv heads of 128, 30.4 us with the merge, 20.3 so; 16 at 1,500 155 and 105; 64 at
-    // 20 17.3 and 11.6)
+    // 20 17.3 and 11.6; with a key's look-up by one lane and no empty rows 18.0, 81 and 9.9)
     auto row_of = [&](int i) { return ROWS == 64 ? warp * (ROWS / WARPS) + i : warp + i * WARPS; };
 
     constexpr int RW = ROWS / WARPS;                // rows of a warp
@@ -387,7 +388,7 @@ attention_f32_merge_kernel(Params p, const int4* __restrict__ work) {
 template <int ROWS, int CH, bool SLICES>
 int go(const Params& p, const int* work, int n, cudaStream_t s) {
     static bool done[bw::MAX_DEVICES] = {};
-    constexpr int KT = fetched(ROWS, CH, SLICES);
+    constexpr int KT = fetched(ROWS, CH);
     const cudaError_t e = bw::allow_dynamic_smem(attention_f32_kernel<ROWS, CH, SLICES>, 4 * smem_floats(ROWS, CH * 128, KT), done);
     if (e != cudaSuccess) return (int)e;
     bw::launch(attention_f32_kernel<ROWS, CH, SLICES>, dim3(n, p.nkv), dim3(THREADS), 4 * (size_t)smem_floats(ROWS, p.hd, KT), s, p, (const int4*)work);

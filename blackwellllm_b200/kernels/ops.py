@@ -652,8 +652,18 @@ def plan_attention_f32(q_len, q_start, G: int, nkv: int, window: Optional[int], 
                 merge_rows = max(merge_rows, n * G)
     # blocks for eight rounds of two an SM: a block's slices follow one another, and a bound's slices that a short request does not have
     # cost their blocks' starts (64 requests of 20 tokens at a bound of 8,320, groups of 4, 8 kv heads of 128: 93 us
-    # with a block a slice, 21 so; groups of 1, 32 kv heads: 337 and 55)
+    # with a block a slice, 21 so; groups of 1, 32 kv heads: 337 and 55; since a lane looks up a key 15.6 and 32.5)
     share(few, keys, -(-8 * sms // max(1, len(few) * nkv)))
+    # A block an SM at a time.  Tiles by themselves end with the longest one, or with rounds that grow emptier; a block for each slice of
+    # every tile, of one length but the last, where those are a few rounds: about 0.4 of a slice more for the merge (us, unshared and so,
+    # groups of 4: 8 kv heads of 128, 200 tokens 51.8 / 32.8, 301 68.5 / 63.5, 400 118.5 / 94.5, 512 163.8 / 138.5, 4 x 200 108.9 / 110.6;
+    # 2 of 64, 301 tokens 58.7 / 28.0, 1,024 180 / 109; groups of 1, 8 of 256, 512 tokens 233 / 92)
+    counts = [slices(*t) for t in tiles] if len(tiles) * nkv <= 6 * sms else []
+    rounds = sum(counts) * nkv / sms
+    longest = max((q_start[r] + t0 + n - first(q_start[r] + t0) for r, t0, n in tiles), default=0) / slice_keys if counts else 0
+    if counts and min(counts) > 0 and max(counts) > 1 and rounds <= 6 and rounds + 0.5 < max(longest, rounds + 0.3 * longest) and small(tiles):
+        share(tiles, wide, most + 2)
+        tiles = []
     # tiles that leave half of the SMs idle share their slices, where they have some (40 tokens at 2,000,
     # groups of 64, one kv head of 8: 403 us unshared, 143 so; groups of 4, 8 kv heads of 128: 585 and 113)
     sliced = [t for t in tiles if slices(*t) >= 4] if 2 * len(tiles) * nkv <= sms else []
@@ -849,8 +859,9 @@ def _gemm_macros():
 
 
 def _workspace(device: torch.device):
-    """Scratch for split-K, one per device, made at first use: float32 partial sums and
-    int32 counters (zero between launches; the kernel returns them to zero)."""
+    """Scratch for split-K and shared tiles, one per device, made at first use: float32 partial sums and
+    int32 counters (zero between launches; the kernel returns them to zero).  So a device's products follow one
+    another in one stream's order."""
     ws = _workspaces.get(device)
     if ws is None:
         ws = (torch.empty(_WORKSPACE_BYTES // 4, dtype=torch.float32, device=device),

@@ -214,6 +214,22 @@ def test_slices_that_grow_with_the_context(ops, window, chunk):
                                                      chunk), out[rows])
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(8, 2, 64), (32, 8, 128), (6, 2, 132), (4, 4, 256)])
+@pytest.mark.parametrize("q_lens,kv_lens", [([385], [385]), ([257, 65], [257, 640]), ([512], [512])])
+def test_tiles_whose_slices_are_dealt_out(ops, monkeypatch, nh, nkv, hd, q_lens, kv_lens):
+    """A block for each slice of every tile: the bits of a block per tile (which slices there are does not depend on it), and float32's
+    distance from the general kernel (see test_tiled_attention)."""
+    q, kp, vp, table, _ = paged_case(q_lens, kv_lens, nh, nkv, hd, 16, torch.float32, seed=hd)
+    starts = [k - n for n, k in zip(q_lens, kv_lens)]
+    assert ops.plan_attention_f32(q_lens, starts, nh // nkv, nkv, None, None, 128, 64)[0][1]
+    batch = FakeBatch(q_lens, kv_lens)
+    out = ops.attention_f32(q, kp, vp, batch, table, nh, None, hd ** -0.5)
+    general = ops.attention_simt(q, kp, vp, batch.positions, batch.req_of_token, table, nh, None, hd ** -0.5)
+    assert float((out - general).abs().max()) <= 2e-5 * float(general.abs().max())
+    monkeypatch.setattr(ops, "num_sms", lambda device: 1)       # one SM: every tile is a block's
+    assert torch.equal(ops.attention_f32(q, kp, vp, FakeBatch(q_lens, kv_lens), table, nh, None, hd ** -0.5), out)
+
+
 @pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 16), (8, 2, 128), (3, 1, 132)])
 @pytest.mark.parametrize("window,chunk", [(None, None), (40, None), (None, 64)])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
