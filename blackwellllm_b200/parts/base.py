@@ -165,6 +165,9 @@ class Mixer(Part):
     #   input_projection()   the Linear that makes everything it reads of its input in one product (None: it has none),
     #   take_projection()    hands that Linear's weight over: a wider product makes its rows from now on,
     #   from_projection(proj, batch, cache, owns_cache)   from those rows (float32) to what its output projection ``o`` reads.
+    # True: from_projection launches no product (products share a device's scratch and counters) and neither makes nor reads what
+    # the step keeps for its layers (``batch.extras``), so it may run on a stream of its own beside another mixer's.
+    own_branch = False
 
     def borrower_request(self):
         """What a run that reads another run's cache (``ScheduleEntry.cache_of``) still keeps of its own; None: nothing.  With

@@ -38,6 +38,8 @@ UNIT_EPS = 1e-6   # under the root of a query's or key's sum of squares
 
 
 class GatedDeltaRule(Mixer):
+    own_branch = True
+
     def __init__(self, spec, hidden_size: int, ctx: BuildContext):
         self.heads, self.kv_heads = int(spec.num_heads), int(spec.num_kv_heads)
         self.dk, self.dv, self.taps = int(spec.key_dim), int(spec.value_dim), int(spec.conv_taps)

@@ -12,10 +12,10 @@ each of them once.  For a few tokens either product leaves its K splits to that 
 
 Between the joined projection and the output products neither child reads what the other makes, and in a step of single tokens each is
 a chain of kernels that is all latency.  Where a step is recorded into a graph, the second child's chain therefore goes to a stream
-of its own and the output products wait for both: two branches of the graph (eight requests, 2k wide, a layer's 85 us, 75 so).
+of its own, if the child declares that it can (``Mixer.own_branch``: no product, nothing shared through the step's batch), and
+the output products wait for both: two branches of the graph (eight requests, 2k wide, a layer's 85 us, 75 so).
 Whatever it allocates there is given back to that stream, whose next work waits for the first one's; what it reads, the projection's
-rows among it, is alive until the join is queued.  The children launch no product there, so the products' scratch stays with the one
-stream.  (Uncaptured prompts gain nothing: a recurrence's walk over its chunks fills the chip's issue slots; and a second stream's
+rows among it, is alive until the join is queued.  (Uncaptured prompts gain nothing: a recurrence's walk over its chunks fills the chip's issue slots; and a second stream's
 first blocks of memory cost 6 ms.)
 """
 from __future__ import annotations
@@ -81,7 +81,7 @@ class SideBySide(Mixer):
         rows = self.proj(x, out_dtype=torch.float32)
         (l0, l1), (r0, r1) = self.columns
         (left, right), (left_view, right_view) = self.children, self._views(cache)
-        if not torch.cuda.is_current_stream_capturing():
+        if not (getattr(right, "own_branch", False) and torch.cuda.is_current_stream_capturing()):
             return [left.from_projection(rows[:, l0:l1], batch, left_view, owns_cache),
                     right.from_projection(rows[:, r0:r1], batch, right_view, owns_cache)]
         main, side = torch.cuda.current_stream(rows.device), self.ctx.side_stream()

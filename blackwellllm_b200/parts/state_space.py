@@ -28,6 +28,8 @@ _DEFAULT_NAMES = {"in": "in_proj.weight", "conv": "conv1d.weight", "conv_bias": 
 
 
 class StateSpaceMixer(Mixer):
+    own_branch = True
+
     def __init__(self, spec, hidden_size: int, ctx: BuildContext):
         self.heads, self.dv, self.N = int(spec.num_heads), int(spec.value_dim), int(spec.state_dim)
         self.groups, self.taps, self.parts = int(spec.groups), int(spec.conv_taps), int(spec.norm_groups)

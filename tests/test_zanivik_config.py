@@ -145,6 +145,39 @@ def test_specs_that_do_not_go_together():
         build_mixer(SideBySideSpec(left=attn(), right=attn(), combine="product"), 32, ctx)
 
 
+@pytest.mark.parametrize("right", ["recurrence", "attention"])
+def test_only_a_mixer_that_shares_nothing_becomes_a_branch_of_a_recorded_step(monkeypatch, right):
+    """While a step is recorded, the second mixer goes to a stream of its own only if it declares that it launches no product and keeps
+    nothing in the step's batch: an attention, which makes rotation tables and cache slots for the other layers, does not."""
+    import contextlib
+    import types
+    from blackwellllm_b200.config.specs import AttentionSpec, RopeSpec, SideBySideSpec
+    from blackwellllm_b200.parts import BuildContext, build_mixer
+    ctx = BuildContext(torch.device("cpu"), torch.float32)
+    plain_attn = AttentionSpec(num_heads=2, num_kv_heads=1, head_dim=16, qkv_bias=False, position=RopeSpec(theta=100.0, rotary_dim=16))
+    specs = {"recurrence": parse_config(tz.MIXED).layers[0].mixer.right, "attention": plain_attn}
+    mixer = build_mixer(SideBySideSpec(left=plain_attn, right=specs[right], combine="sum"), 64, ctx)
+    on, where = ["main"], []
+
+    @contextlib.contextmanager
+    def stream(s):
+        on.append(s.name)
+        yield
+        on.pop()
+    main, side = (types.SimpleNamespace(name=n, wait_stream=lambda other: None) for n in ("main", "side"))
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: main)
+    monkeypatch.setattr(torch.cuda, "stream", stream)
+    object.__setattr__(ctx, "_side", side)
+    mixer.proj, mixer.columns = (lambda x, out_dtype: x), ((0, 4), (4, 8))
+    mixer._views = lambda cache: (None, None)
+    for k, child in enumerate(mixer.children):
+        child.from_projection = lambda rows, *a, k=k: where.append((k, on[-1])) or rows
+    a, b = mixer._read(torch.arange(16.0).view(2, 8), None, None, True)
+    assert sorted(where) == [(0, "main"), (1, "side" if right == "recurrence" else "main")]
+    assert a[0].tolist() == [0, 1, 2, 3] and b[0].tolist() == [4, 5, 6, 7]
+
+
 # ------------------------------------------------------------------ the plain implementation itself
 
 def test_plain_frequency_bands():
