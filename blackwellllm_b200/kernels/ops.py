@@ -8,6 +8,8 @@ from __future__ import annotations
 import ctypes
 import math
 import os
+import threading
+from collections import OrderedDict
 from typing import List, Optional, Tuple
 
 import numpy as np
@@ -859,15 +861,38 @@ def _gemm_macros():
 
 
 def _workspace(device: torch.device):
-    """Scratch for split-K and shared tiles, one per device, made at first use: float32 partial sums and
-    int32 counters (zero between launches; the kernel returns them to zero).  So a device's products follow one
-    another in one stream's order."""
+    """Scratch for split-K, one per device, made at first use: float32 partial sums and
+    int32 counters (zero between launches; the kernel returns them to zero).  So a device's split products follow one
+    another in one stream's order; products of more than 256 tokens that are not split touch neither."""
     ws = _workspaces.get(device)
     if ws is None:
         ws = (torch.empty(_WORKSPACE_BYTES // 4, dtype=torch.float32, device=device),
               torch.zeros(_COUNTERS, dtype=torch.int32, device=device))
         _workspaces[device] = ws
     return ws
+
+
+_TURN_STREAMS = 16
+_turns = OrderedDict()     # (device, stream) -> counters, the latest used last
+_turns_lock = threading.Lock()
+
+
+def _turn_counters(device: torch.device) -> torch.Tensor:
+    """The counters of a product that may add the parts of a tile in turns (more than 256 tokens, added into float32): zero between
+    launches, of the current stream alone, so that such products may run on several streams at once.  The last 16 streams' are kept; one
+    that goes was allocated on its stream, so its memory is next used in that stream's order.  While a graph is recorded: the graph's own."""
+    if torch.cuda.is_current_stream_capturing():
+        return torch.zeros(_COUNTERS, dtype=torch.int32, device=device)
+    key = (device, _stream())
+    with _turns_lock:
+        c = _turns.get(key)
+        if c is None:
+            c = _turns[key] = torch.zeros(_COUNTERS, dtype=torch.int32, device=device)
+            if len(_turns) > _TURN_STREAMS:
+                _turns.popitem(last=False)
+        else:
+            _turns.move_to_end(key)
+    return c
 
 
 def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
@@ -927,6 +952,8 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = Non
         if bias.numel() != N:
             raise KernelError("gemm: bias must have N entries")
     ws, counters = _workspace(x.device)
+    if accumulate and M > GEMM_PLANES_MAX_TOKENS:
+        counters = _turn_counters(x.device)
     if act is not None and not (swiglu and act == ACT_SILU):
         if accumulate:
             raise KernelError("gemm_tc: an activation goes with a result that is written, not added")

@@ -148,3 +148,27 @@ def test_every_route_is_one_the_kernels_are_built_for(plan, kind):
                     assert tiles * ceil_div(K, BK) >= 16 * ranges, what
             elif (tr.value, bn.value, splits.value) != (tr0, bn0, planned):
                 assert kind == 1 and 64 < M <= 128 and tr.value == 0 and bn.value in (224, 256) and splits.value == 1, what
+
+
+def test_each_stream_has_counters_of_its_own_for_products_that_add_in_turns(monkeypatch):
+    """Products of more than 256 tokens added into float32 may run on several streams at once: the parts of a tile are counted per stream,
+    the counters of the last streams are kept (a bounded number), a recorded graph has its own."""
+    import torch
+    from blackwellllm_b200.kernels import ops
+    at, capturing, device = [1], [False], torch.device("cpu")
+    monkeypatch.setattr(ops, "_stream", lambda: at[0])
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing[0])
+    monkeypatch.setattr(ops, "_turns", type(ops._turns)())
+    first = ops._turn_counters(device)
+    assert first.numel() == ops._COUNTERS and not bool(first.any())
+    at[0] = 2
+    second = ops._turn_counters(device)
+    assert second.data_ptr() != first.data_ptr()
+    at[0] = 1
+    assert ops._turn_counters(device) is first
+    capturing[0] = True
+    assert all(ops._turn_counters(device).data_ptr() not in (first.data_ptr(), second.data_ptr()) for _ in range(2))
+    capturing[0] = False
+    for at[0] in range(2, 40):      # the streams used longest ago go; stream 1's was used before the others
+        ops._turn_counters(device)
+    assert len(ops._turns) == ops._TURN_STREAMS and (device, 1) not in ops._turns and (device, 39) in ops._turns

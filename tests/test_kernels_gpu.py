@@ -272,6 +272,40 @@ def test_gemm_tc_pairs_on_equal_ranges(ops, M, N, K, ldo):
     assert torch.equal(outs[0][:, N:], base[:, N:])
 
 
+def test_gemm_tc_equal_ranges_on_two_streams_at_once(ops):
+    """Products whose parts are added in turns on two streams of a device, and in a graph replayed beside them: the bits of each alone."""
+    M, N, K = 512, 4096, 14336
+    w = rand(N, K, dtype=torch.bfloat16, seed=6, scale=0.05).to(DEV)
+    xs = [rand(M, K, dtype=torch.bfloat16, seed=i).to(DEV) for i in range(3)]
+    base = rand(M, N, seed=8).to(DEV)
+
+    def run(i, out):
+        out.copy_(base)
+        ops.gemm_tc(xs[i], w, None, out=out, accumulate=True)
+    outs = [torch.empty_like(base) for _ in xs]
+    alone = []
+    for i, out in enumerate(outs):
+        run(i, out)
+        alone.append(out.clone())
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in xs]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=streams[2]):
+        run(2, outs[2])
+    for out in outs:
+        out.zero_()
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for i in (0, 1):
+            with torch.cuda.stream(streams[i]):
+                run(i, outs[i])
+        with torch.cuda.stream(streams[2]):
+            graph.replay()
+    torch.cuda.synchronize()
+    assert ops.gemm_tc_status() == 0
+    assert all(torch.equal(out, a) for out, a in zip(outs, alone))
+
+
 def test_gemm_tc_split_k_on_a_tile_width_that_is_no_power_of_two(ops):
     M, N, K = 2048, 4096, 256     # 16 x 18 tiles of 240 columns: the last one of a row is cut at 4096
     x = rand(M, K, dtype=torch.bfloat16, seed=5).to(DEV)
