@@ -1643,10 +1643,15 @@ BW_EXPORT int bw_gemm_tc_pair_mode(int mode) {
     return old;
 }
 
-// Reads and clears the status word (synchronises the device).  0: no wait ever gave up.
+// Reads and clears the status word (synchronises the device).  0: no wait ever gave up.  After anything else the counters may have been
+// left in between: whoever owns them sets them to zero before the next product (BW_OWN_COUNTERS: this library does).
 BW_EXPORT int bw_gemm_tc_status() {
     int v = 0, zero = 0;
     if (cudaMemcpyFromSymbol(&v, g_status, sizeof(int)) != cudaSuccess) return -1;
-    if (v) cudaMemcpyToSymbol(g_status, &zero, sizeof(int));
+    if (!v) return 0;
+#ifdef BW_OWN_COUNTERS
+    if (!BW_OWN_COUNTERS()) return -1;
+#endif
+    cudaMemcpyToSymbol(g_status, &zero, sizeof(int));
     return v;
 }

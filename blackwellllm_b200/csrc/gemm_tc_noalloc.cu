@@ -2,6 +2,8 @@
 // gemm_tc_noalloc.h for who needs it and for its rules.  The kernels are those of
 // gemm_tc.cu, compiled into this library as well; only the home of the split-K
 // partial sums differs: a static device array instead of a caller's workspace.
+static bool zero_own_counters();
+#define BW_OWN_COUNTERS zero_own_counters
 #include "gemm_tc.cu"
 #include "gemm_tc_noalloc.h"
 
@@ -12,6 +14,13 @@ static __device__ __align__(256) float g_noalloc_scratch[BW_NOALLOC_SCRATCH_FLOA
 // Completion counters of the split-K tiles.  They must be zero when a call starts: static device
 // memory starts as zero, and the kernel sets every counter it used back to zero before it ends.
 static __device__ __align__(256) int g_noalloc_counters[BW_NOALLOC_COUNTERS];
+
+// Whether they are zero again after a product that gave up (bw_gemm_tc_status); waits for the device.
+static bool zero_own_counters() {
+    int* c = nullptr;
+    return cudaDeviceSynchronize() == cudaSuccess && cudaGetSymbolAddress((void**)&c, g_noalloc_counters) == cudaSuccess &&
+           cudaMemset(c, 0, sizeof(int) * BW_NOALLOC_COUNTERS) == cudaSuccess;
+}
 
 namespace {
 constexpr int MAX_DEVICES = 64;

@@ -1037,10 +1037,19 @@ def gemm_pair_mode(mode: int) -> int:
 
 
 def gemm_tc_status() -> int:
-    """0 if no bounded wait in the tensor-core kernels ever gave up (synchronises the device)."""
+    """0 if no bounded wait in the tensor-core kernels ever gave up (synchronises the device).  Clears the status, and the counters
+    that a product which gave up has left in between."""
     lib = load_library("gemm_tc", _gemm_macros())
     lib.bw_gemm_tc_status.restype = c_int
-    return int(lib.bw_gemm_tc_status())
+    status = int(lib.bw_gemm_tc_status())
+    if status:
+        torch.cuda.synchronize()
+        with _turns_lock:
+            for c in [ws[1] for ws in _workspaces.values()] + list(_turns.values()):
+                if c.device.index == torch.cuda.current_device():      # (the status word is this device's)
+                    c.zero_()
+        torch.cuda.synchronize()
+    return status
 
 
 ATTENTION_SIMT_MAX_HEAD_DIM = 1024   # the CUDA-core kernel's limit; the tensor-core kernels are built for head sizes up to 256

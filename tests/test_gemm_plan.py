@@ -172,3 +172,20 @@ def test_each_stream_has_counters_of_its_own_for_products_that_add_in_turns(monk
     for at[0] in range(2, 40):      # the streams used longest ago go; stream 1's was used before the others
         ops._turn_counters(device)
     assert len(ops._turns) == ops._TURN_STREAMS and (device, 1) not in ops._turns and (device, 39) in ops._turns
+
+
+@pytest.mark.parametrize("status", (0, 35))
+def test_counters_that_a_product_left_in_between_are_cleared_with_its_status(monkeypatch, status):
+    import types
+    import torch
+    from blackwellllm_b200.kernels import ops
+    mine = [types.SimpleNamespace(device=types.SimpleNamespace(index=i), zeroed=0) for i in (0, 0, 1)]
+    for m in mine:
+        m.zero_ = lambda m=m: setattr(m, "zeroed", m.zeroed + 1)
+    monkeypatch.setattr(ops, "_workspaces", {"cuda:0": (None, mine[0])})
+    monkeypatch.setattr(ops, "_turns", {("cuda:0", 7): mine[1], ("cuda:1", 7): mine[2]})
+    monkeypatch.setattr(ops, "load_library", lambda *a: types.SimpleNamespace(bw_gemm_tc_status=type("F", (), {"__call__": lambda self: status})()))
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a: None)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    assert ops.gemm_tc_status() == status
+    assert [m.zeroed for m in mine] == ([1, 1, 0] if status else [0, 0, 0])
