@@ -1323,7 +1323,7 @@ double gemm_single_cost(int M, int N, int K, int bn, long long tiles, int splits
 }
 }  // namespace
 
-// CTA pairs for out[M, N] = x[M, K] . w[N, K]^T with M > 128: the tile width (256 or 224, with `narrow` also 192 or 128) and the number
+// CTA pairs for out[M, N] = x[M, K] . w[N, K]^T with M > 128: the tile width (256, 224, 192 or 128) and the number
 // of K splits (1 to 4, each of 8 k-blocks or more, their planes within the scratch) with the lowest estimate, which is returned
 // (negative: pairs cannot take it).  force_splits > 0 fixes the splits.
 // A tile's cost in columns of a 256-wide one: a narrow tile draws nearly as many bytes per k-block (the tokens' half), and from 192
@@ -1332,13 +1332,13 @@ double gemm_single_cost(int M, int N, int K, int bn, long long tiles, int splits
 // were no faster than 256, 160 hardly faster than 192 where both fit a round.)  What the two narrow ones give: o of 3584 at 648 and 1,536
 // tokens 22.5 -> 20.3 and 37.4 -> 34.0, its down projection 87.4 -> 81.8 and 171 -> 161, q/k/v of 6144 x 4096 at 512 and 1,024 tokens
 // 31.9 -> 28.8 and 48.0 -> 44.5, o of 5120 at 2,048 82 -> 77, its down projection 217 -> 197.
-static double pair_plan(int M, int N, int K, int force_splits, long long workspace_elems, bool narrow, int* width, int* splits) {
+static double pair_plan(int M, int N, int K, int force_splits, long long workspace_elems, int* width, int* splits) {
     const int NUM_SMS = bw::num_sms();
     const int kb_total = ceil_div(K, BK), pa = ceil_div(M, 2 * BM);
     const int widths[4] = {256, 224, 192, 128};
-    const double columns[4] = {256.0, narrow ? 236.0 : 224.0, 205.0, 184.0};
+    const double columns[4] = {256.0, 236.0, 205.0, 184.0};
     double best = -1.0;
-    for (int i = 0; i < (narrow ? 4 : 2); ++i) {
+    for (int i = 0; i < 4; ++i) {
         const long long t = (long long)pa * ceil_div(N, widths[i]);
         for (int ps = 1; ps <= 4; ++ps) {
             if (force_splits > 0 && ps != (force_splits > kb_total ? kb_total : force_splits)) continue;
@@ -1354,21 +1354,17 @@ static double pair_plan(int M, int N, int K, int force_splits, long long workspa
     }
     return best;
 }
-// The same among the wide tiles.
-BW_EXPORT double bw_gemm_tc_pair_plan(int M, int N, int K, int force_splits, long long workspace_elems, int* width, int* splits) {
-    return pair_plan(M, N, K, force_splits, workspace_elems, false, width, splits);
-}
 
-// SwiGLU on CTA pairs in the other orientation, tiles of 256 features x 96 to 256 tokens: the tokens need no whole tiles of 256.  The
+// SwiGLU on CTA pairs in the other orientation, tiles of 256 features x 96 to 224 tokens: the tokens need no whole tiles of 256.  The
 // estimate as pair_plan makes it (columns of a tile as long as 256 of them would take; measured per k-block over many rounds 0.38 us at 256
-// tokens a tile, 0.33, 0.29, 0.27, 0.25, 0.22), *width set.  Against tiles of 256 tokens (us, 28672 x 4096: 300 tokens 86 -> 74, 550 120 -> 103,
+// tokens a tile, which the other orientation does as well, 0.33, 0.29, 0.27, 0.25, 0.22), *width set.  Against tiles of 256 tokens (us, 28672 x 4096: 300 tokens 86 -> 74, 550 120 -> 103,
 // 648 123 -> 115, 1,100 197 -> 176, 1,300 229 -> 213; 37888 x 3584: 648 136 -> 126, 1,300 302 -> 234); where the estimates differ by less than
 // 7 % either may be the faster one by 4 %.
 static double swiglu_pair_plan(int M, int N, int K, int* width) {
-    const int widths[6] = {256, 224, 192, 160, 128, 96};
-    const double columns[6] = {256.0, 222.0, 197.0, 182.0, 167.0, 148.0};
+    const int widths[5] = {224, 192, 160, 128, 96};
+    const double columns[5] = {222.0, 197.0, 182.0, 167.0, 148.0};
     double best = -1.0;
-    for (int i = 0; i < 6; ++i) {
+    for (int i = 0; i < 5; ++i) {
         const long long t = (long long)ceil_div(N, 2 * BM) * ceil_div(M, widths[i]);
         const double cost = (double)ceil_div(t, bw::num_sms() / 2) * ceil_div(K, BK) * columns[i];
         if (best < 0.0 || cost < best) { best = cost; *width = widths[i]; }
@@ -1424,7 +1420,7 @@ BW_EXPORT int bw_gemm_tc_route(int M, int N, int K, int kind, int pair_mode, int
         // they were / on pairs: gate/up of 28672 x 4096 at 160 and 256 tokens 77 / 54 and 92 / 56, q/k/v of 6144 x 4096 31 / 24 and 39 / 25,
         // o of 4096 at 160, 200 and 256 17.5 / 19.2, 20.7 / 19.4 and 21.4 / 19.4, its down projection 36 to 40 / 54)
         if (pair_mode > 0 && M > BM && ((kind != 0 && kind != 4) || (kb_total < 128 && (M > 160 || *splits == 1)))) {
-            const double pair = pair_plan(M, N, K, 0, workspace_elems, true, &width, &ps);
+            const double pair = pair_plan(M, N, K, 0, workspace_elems, &width, &ps);
             if (pair < 0.0) return 0;
             *transposed = 0; *bn = width; *splits = ps;
             if (kind == 1 && swiglu_pair_plan(M, N, K, &width) < 0.93 * pair) { *transposed = 1; *bn = width; *splits = 1; }
@@ -1438,7 +1434,7 @@ BW_EXPORT int bw_gemm_tc_route(int M, int N, int K, int kind, int pair_mode, int
     // products with few output features) the pairs split K as well; the partial sums are added in split
     // order by the second kernel.
     if (pair_mode <= 0 || M <= 2 * BM) return 0;
-    const double pair = pair_plan(M, N, K, force_splits, workspace_elems, true, &width, &ps);
+    const double pair = pair_plan(M, N, K, force_splits, workspace_elems, &width, &ps);
     const double single = gemm_single_cost(M, N, K, *bn, (long long)ceil_div(M, BM) * ceil_div(N, *bn), *splits);
     int other = 0;
     if (kind == 1 && force_splits <= 0 && swiglu_pair_plan(M, N, K, &other) < 0.93 * (pair >= 0.0 && (pair_mode == 2 || pair <= single) ? pair : single)) {
@@ -1635,7 +1631,7 @@ BW_EXPORT int bw_gemm_tc_rope(const void* x, const void* w, const void* bias, in
                        workspace_elems, counters, n_counters, force_splits, &ro, stream);
 }
 
-// When products of more than 256 tokens run on CTA pairs: 0 never, 1 when the estimate says they are
+// When products of more than 128 tokens run on CTA pairs: 0 never, 1 when the estimate says they are
 // faster (the default), 2 whenever the product allows it (tests).  Returns the mode before.
 BW_EXPORT int bw_gemm_tc_pair_mode(int mode) {
     const int old = g_pair_mode;

@@ -1030,7 +1030,7 @@ def gemm_tc_rope(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
 
 
 def gemm_pair_mode(mode: int) -> int:
-    """When products of more than 256 tokens run on CTA pairs: 0 never, 1 when estimated faster (the
+    """When products of more than 128 tokens run on CTA pairs: 0 never, 1 when estimated faster (the
     default), 2 whenever possible.  Returns the mode before (-1: not set yet, i.e. the default)."""
     fn = _fn("gemm_tc", "bw_gemm_tc_pair_mode", [c_int], macros=_gemm_macros())
     return fn(int(mode))

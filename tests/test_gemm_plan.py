@@ -88,34 +88,39 @@ def test_decode_shapes_fill_the_gpu(plan):
             assert NUM_SMS // 2 <= tiles * splits <= NUM_SMS, (M, N, K, splits)
 
 
-def test_pair_plan_splits_k_only_where_the_pairs_would_idle():
-    """CTA pairs for more than 256 tokens: K is split only where it was measured to pay: in two halves, a long K
-    (the down projection) at a few hundred tokens, when both halves of every tile fit one round of the 74 pairs."""
+@pytest.fixture(scope="module")
+def route(plan):
     from blackwellllm_b200.kernels.build import load_library
-    lib = load_library("gemm_tc")
-    fn = lib.bw_gemm_tc_pair_plan
-    fn.restype = ctypes.c_double
-    fn.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_longlong,
-                   ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]
+    fn = load_library("gemm_tc").bw_gemm_tc_route
+    fn.argtypes = [ctypes.c_int] * 6 + [ctypes.c_longlong] + [ctypes.POINTER(ctypes.c_int)] * 3
 
-    def plan(M, N, K, force=0, workspace=1 << 24):
-        wd, sp = ctypes.c_int(-1), ctypes.c_int(-1)
-        cost = fn(M, N, K, force, workspace, ctypes.byref(wd), ctypes.byref(sp))
-        return cost, wd.value, sp.value
+    def call(M, N, K, kind, mode=1, force=0, workspace=1 << 24):
+        planned, tr0, bn0 = plan(M, N, K, int(kind == 1), workspace)
+        tr, bn, splits = ctypes.c_int(tr0), ctypes.c_int(bn0), ctypes.c_int(planned)
+        pairs = fn(M, N, K, kind, mode, force, workspace, ctypes.byref(tr), ctypes.byref(bn), ctypes.byref(splits))
+        return pairs, tr.value, bn.value, splits.value
+    return call
 
-    for M in (300, 512, 1024, 2048, 8192):
+
+@pytest.mark.parametrize("kind", (0, 1, 2))
+def test_pair_plan_splits_k_only_where_the_pairs_would_idle(route, kind):
+    """CTA pairs split K only where it was measured to pay: in two halves, a long K (the down projection) at a few hundred tokens, when
+    both halves of every tile fit one round of the 74 pairs."""
+    for M in (200, 300, 512, 1024, 2048, 8192):
         for N, K in PRODUCTS[:14]:
-            cost, wd, sp = plan(M, N, K)
-            assert cost > 0 and wd in (224, 256) and 1 <= sp <= 4, (M, N, K)
+            pairs, tr, bn, sp = route(M, N, K, kind)
+            if not pairs:
+                continue
             kb = ceil_div(K, BK)
-            tiles = ceil_div(M, 2 * BM) * ceil_div(N, wd)
+            tiles = ceil_div(M, 2 * BM) * ceil_div(N, bn)
             if sp > 1:   # two halves of a long K whose items fit one round of the 74 pairs, planes within the scratch
-                assert sp == 2 and kb >= 128 and tiles * 2 <= NUM_SMS // 2 and sp * M * N <= 1 << 24
-            assert plan(M, N, K, workspace=0)[2] == 1            # no scratch, no split
-    assert plan(512, 4096, 14336)[2] == 2                        # down at 512 tokens: 32 tiles for 74 pairs
-    assert plan(512, 4096, 4096)[2] == 1 and plan(768, 4096, 14336)[2] == 1
-    assert plan(2048, 28672, 4096)[2] == 1                       # gate/up at 2,048 tokens: rounds of whole tiles
-    assert plan(700, 520, 2240, force=3)[2] == 3                 # a forced split is taken as it is
+                assert not tr and sp == 2 and kb >= 128 and tiles * 2 <= NUM_SMS // 2 and sp * M * N <= 1 << 24
+            assert route(M, N, K, kind, workspace=0)[3] == 1            # no scratch, no split
+    if kind != 1:
+        assert route(512, 4096, 14336, kind) == (1, 0, 256, 2)          # down at 512 tokens: 32 tiles for 74 pairs
+        assert route(700, 520, 2240, kind, force=3)[3] == 3             # a forced split is taken as it is
+    assert route(512, 4096, 4096, kind)[3] == 1 and route(768, 4096, 14336, kind)[3] == 1
+    assert route(2048, 28672, 4096, kind)[3] == 1                       # gate/up at 2,048 tokens: rounds of whole tiles
 
 
 @pytest.mark.parametrize("kind", (0, 1, 2, 3, 4))

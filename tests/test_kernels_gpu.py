@@ -384,12 +384,25 @@ def test_gemm_tc_rotary_epilogue(ops, M, splits, nh, nkv, hd, rd, page):
     assert ops.gemm_tc_status() == 0
 
 
-# the edges of the routes (64 | 65, 128 | 129, 256 | 257 tokens), tokens that leave a tile ragged, and products of fewer or more
-# tiles than SMs
-@pytest.mark.parametrize("M", [65, 93, 128, 129, 161, 200, 256, 257, 300, 550, 648])
-@pytest.mark.parametrize("I,K", [(176, 264), (528, 1000), (9616, 72)])
-def test_gemm_tc_swiglu_of_65_to_648_tokens(ops, M, I, K):
-    """Single CTAs on 128 tokens, CTA pairs in either orientation; biases; an output whose rows are further apart than they are long."""
+@pytest.fixture(scope="module")
+def route():
+    """``bw_gemm_tc_route`` of a product of M tokens (kind 1 SwiGLU, 2 rotary): pairs or not, other orientation, width, splits."""
+    import ctypes
+    from blackwellllm_b200.kernels.build import load_library
+    lib, ref = load_library("gemm_tc"), ctypes.byref
+    lib.bw_gemm_tc_plan.argtypes = [ctypes.c_int] * 4 + [ctypes.c_longlong] * 2 + [ctypes.POINTER(ctypes.c_int)] * 2
+    lib.bw_gemm_tc_route.argtypes = [ctypes.c_int] * 6 + [ctypes.c_longlong] + [ctypes.POINTER(ctypes.c_int)] * 3
+
+    def call(M, N, K, kind):
+        tr, bn = ctypes.c_int(), ctypes.c_int()
+        splits = ctypes.c_int(lib.bw_gemm_tc_plan(M, N, K, int(kind == 1), 1 << 24, 1 << 16, ref(tr), ref(bn)))
+        pairs = lib.bw_gemm_tc_route(M, N, K, kind, 1, 0, 1 << 24, ref(tr), ref(bn), ref(splits))
+        return pairs, tr.value, bn.value, splits.value
+    return call
+
+
+def swiglu_case(ops, M, I, K):
+    """Biases; an output whose rows are further apart than they are long."""
     x = rand(M, K, dtype=torch.bfloat16, seed=1).to(DEV)
     wg, wu = (rand(I, K, dtype=torch.bfloat16, seed=2 + i, scale=0.05).to(DEV) for i in range(2))
     bg, bu = (rand(I, seed=4 + i, scale=0.2).to(DEV) for i in range(2))
@@ -403,9 +416,37 @@ def test_gemm_tc_swiglu_of_65_to_648_tokens(ops, M, I, K):
     assert bool((wide[:, I:] == 7.0).all())
 
 
+# the edges of the routes (64 | 65, 128 | 129, 256 | 257 tokens), tokens that leave a tile ragged, and products of fewer or more
+# tiles than SMs
+@pytest.mark.parametrize("M", [65, 93, 128, 129, 161, 200, 256, 257, 300, 550, 648])
+@pytest.mark.parametrize("I,K", [(176, 264), (528, 1000), (9616, 72)])
+def test_gemm_tc_swiglu_of_65_to_648_tokens(ops, M, I, K):
+    """Single CTAs on 128 tokens, CTA pairs in either orientation; biases; an output whose rows are further apart than they are long."""
+    swiglu_case(ops, M, I, K)
+
+
+# a pair's tile of 256 features x 128, 192 and 224 tokens, ragged in both (96 and 160 are among the sizes above)
+@pytest.mark.parametrize("M,I,width", [(200, 4080, 128), (161, 14320, 192), (649, 18928, 224)])
+def test_gemm_tc_swiglu_on_pairs_of_every_width(ops, route, M, I, width):
+    K = 72
+    assert route(M, 2 * I, K, 1)[:3] == (1, 1, width)
+    swiglu_case(ops, M, I, K)
+
+
 @pytest.mark.parametrize("M", [17, 65, 128, 129, 200, 256, 257, 650])
 @pytest.mark.parametrize("nh,nkv,hd,rd,bias_dtype", [(28, 4, 128, 128, torch.bfloat16), (5, 1, 48, 32, torch.float32), (3, 1, 16, 6, None)])
 def test_gemm_tc_rotary_routes(ops, M, nh, nkv, hd, rd, bias_dtype):
+    rotary_case(ops, M, nh, nkv, hd, rd, bias_dtype)
+
+
+@pytest.mark.parametrize("M,nh,nkv,width", [(300, 52, 4, 224), (257, 64, 4, 256)])
+@pytest.mark.parametrize("bias_dtype", [torch.bfloat16, torch.float32])
+def test_gemm_tc_rotary_on_pairs_of_the_wide_tiles(ops, route, M, nh, nkv, width, bias_dtype):
+    assert route(M, (nh + 2 * nkv) * 128, 520, 2) == (1, 0, width, 1)
+    rotary_case(ops, M, nh, nkv, 128, 128, bias_dtype)
+
+
+def rotary_case(ops, M, nh, nkv, hd, rd, bias_dtype):
     """The rotation in each route's epilogue and in the second kernel, against the plain product and :func:`rope_append`."""
     K, page = 520, 16
     N = (nh + 2 * nkv) * hd
