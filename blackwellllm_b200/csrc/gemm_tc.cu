@@ -1395,6 +1395,29 @@ static int shared_ranges(int M, int N, int K, int width, int splits, double cost
     return (double)tb / ranges * kb_total * 220.0 + 4050.0 < 0.93 * cost ? ranges : 0;
 }
 
+// Products of 129 to 256 tokens, us: on single CTAs, tiles of 128 features x all tokens, in `splits` parts of K; and on CTA pairs, as
+// pair_plan or swiglu_pair_plan has it.  Lines fitted to 626 products of 256 to 28,672 features and 1,024 to 14,336 channels (about 5 % off
+// the measured times); for eight of them the slower of the two is taken, 3 to 10 % slower.  An unsplit tile's epilogue is what makes single
+// CTAs slow (a value a lane; the rotation), the whole K on a few pairs is what makes pairs slow.  (us, single CTAs / pairs: SwiGLU of 1024 x
+// 4096 at 161 tokens 15.0 / 20.3, of 11264 x 4096 47.1 / 28.9; rotary 768 x 4096 at 161 19.6 / 22.5, 1536 x 14336 24.0 / 33.9, 6144 x 8192 at 200
+// 45.0 / 36.6; plain 512 x 4096 at 161 14.2 / 18.0, 512 x 2048 at 200 27.1 / 11.0, 4096 x 4096 at 200 added 20.8 / 19.1.)
+static double single_wide_us(int M, int N, int K, int kind, int splits) {
+    const int rounds = (int)ceil_div((long long)ceil_div(N, BM) * splits, bw::num_sms());
+    const double t = 5.5 + (kind == 2 ? 0.45 : 0.40) * rounds * ceil_div(ceil_div(K, BK), splits);
+    const double planes = (splits + 2) * 4e-6 * M * N;      // MB
+    if (kind == 2) return t + (splits > 1 ? 2.0 + 0.65 * planes : rounds * (20.0 + 0.28 * M));
+    if (splits > 1) return t + (kind == 4 ? 0.35 : 0.42) * planes;
+    return t + rounds * (kind == 1 ? 3.0 + 0.067 * M : 5.0 + 0.033 * M);
+}
+static double pair_us(int M, int N, int K, int kind, int transposed, int width, int splits) {
+    const long long tiles = transposed ? (long long)ceil_div(N, 2 * BM) * ceil_div(M, width) : (long long)ceil_div(N, width);
+    const int rounds = (int)ceil_div(tiles * splits, bw::num_sms() / 2);
+    const double per_block = transposed ? (width == 96 ? 0.19 : width == 128 ? 0.25 : width == 160 ? 0.32 : width == 192 ? 0.37 : 0.42)
+                                        : (width == 128 ? 0.22 : width == 192 ? 0.345 : width == 224 ? 0.42 : 0.46);
+    return (kind == 0 || kind == 4 ? 2.8 : 4.8) * (1 + rounds) + rounds * per_block * ceil_div(ceil_div(K, BK), splits) +
+           (splits > 1 ? 0.42 * (splits + 2) * 4e-6 * M * N : 0.0);
+}
+
 // How a product runs, from bw_gemm_tc_plan's decision (transposed, bn, splits) and the pairs' estimate.  kind: 0 plain, 1 SwiGLU, 2 rotary,
 // 3 sums left open, 4 plain, added into float32 by TMA.  pair_mode: bw_gemm_tc_pair_mode's.  Returns 0 for single CTAs, 1 for CTA pairs (bn: a
 // pair's features; transposed: its tokens), 1 + n for n equal ranges a tile of tokens.
@@ -1402,7 +1425,7 @@ BW_EXPORT int bw_gemm_tc_route(int M, int N, int K, int kind, int pair_mode, int
                                int* bn, int* splits) {
     const int NUM_SMS = bw::num_sms();
     const int kb_total = ceil_div(K, BK);
-    int width = 0, ps = 1;
+    int width = 0, ps = 1, other = 0;
     if (*transposed) {
         if (force_splits > 0 || kind == 3) return 0;
         if (kind == 1 && M > 64 && M <= BM && ceil_div(N, BM) > NUM_SMS) {
@@ -1416,14 +1439,16 @@ BW_EXPORT int bw_gemm_tc_route(int M, int N, int K, int kind, int pair_mode, int
                 if (cost < least || (cost == least && *transposed)) { least = cost; *transposed = 0; *bn = wd; *splits = 1; }
             }
         }
-        // 129 to 256 tokens on one pair tile of tokens, but for a long K, whose splits the 128-row tiles of features deal out better (us, as
-        // they were / on pairs: gate/up of 28672 x 4096 at 160 and 256 tokens 77 / 54 and 92 / 56, q/k/v of 6144 x 4096 31 / 24 and 39 / 25,
-        // o of 4096 at 160, 200 and 256 17.5 / 19.2, 20.7 / 19.4 and 21.4 / 19.4, its down projection 36 to 40 / 54)
+        // 129 to 256 tokens on one pair tile of tokens where that is faster (mode 2: whenever they can).  Sums that are written or added as
+        // they are stay on single CTAs where K is long (8,192 and more), whose splits these deal out better, and up to 160 tokens where K is
+        // split (o of 4096 at 160 tokens 17.5 / 19.2, its down projection 36 to 40 / 54)
         if (pair_mode > 0 && M > BM && ((kind != 0 && kind != 4) || (kb_total < 128 && (M > 160 || *splits == 1)))) {
             const double pair = pair_plan(M, N, K, 0, workspace_elems, &width, &ps);
             if (pair < 0.0) return 0;
-            *transposed = 0; *bn = width; *splits = ps;
-            if (kind == 1 && swiglu_pair_plan(M, N, K, &width) < 0.93 * pair) { *transposed = 1; *bn = width; *splits = 1; }
+            int tr = 0;
+            if (kind == 1 && swiglu_pair_plan(M, N, K, &other) < 0.93 * pair) { tr = 1; width = other; ps = 1; }
+            if (pair_mode == 1 && single_wide_us(M, N, K, kind, *splits) < pair_us(M, N, K, kind, tr, width, ps)) return 0;
+            *transposed = tr; *bn = width; *splits = ps;
             return 1;
         }
         return 0;
@@ -1436,7 +1461,6 @@ BW_EXPORT int bw_gemm_tc_route(int M, int N, int K, int kind, int pair_mode, int
     if (pair_mode <= 0 || M <= 2 * BM) return 0;
     const double pair = pair_plan(M, N, K, force_splits, workspace_elems, &width, &ps);
     const double single = gemm_single_cost(M, N, K, *bn, (long long)ceil_div(M, BM) * ceil_div(N, *bn), *splits);
-    int other = 0;
     if (kind == 1 && force_splits <= 0 && swiglu_pair_plan(M, N, K, &other) < 0.93 * (pair >= 0.0 && (pair_mode == 2 || pair <= single) ? pair : single)) {
         *transposed = 1; *bn = other; *splits = 1;
         return 1;

@@ -123,6 +123,22 @@ def test_pair_plan_splits_k_only_where_the_pairs_would_idle(route, kind):
     assert route(2048, 28672, 4096, kind)[3] == 1                       # gate/up at 2,048 tokens: rounds of whole tiles
 
 
+def test_pairs_of_129_to_256_tokens_only_where_they_are_faster(route):
+    """Products measured on single CTAs and on CTA pairs: a weight of few features and a long K leaves most pairs idle."""
+    single = {0: [(161, 512, 4096), (161, 256, 4096), (160, 4096, 4096), (200, 4096, 14336)], 4: [(161, 512, 4096), (161, 4096, 4096), (129, 1024, 8192)],
+              1: [(161, 1024, 4096), (200, 1024, 8192), (129, 4096, 4096), (256, 512, 8192)],
+              2: [(161, 768, 4096), (161, 1536, 14336), (256, 768, 14336), (129, 1536, 8192)]}
+    pairs = {0: [(200, 512, 2048), (200, 4096, 4096), (256, 12288, 4096)], 4: [(200, 512, 2048), (256, 4096, 4096)],
+             1: [(161, 28672, 4096), (161, 11264, 4096), (256, 8192, 4096), (129, 512, 1024)],
+             2: [(161, 6144, 4096), (200, 6144, 8192), (129, 768, 2048), (256, 4608, 14336)]}
+    for kind in (0, 1, 2, 4):
+        for case in single[kind]:
+            assert route(*case, kind)[:2] == (0, 1), (kind, case)
+            assert kind in (0, 4) or route(*case, kind, mode=2)[0] == 1
+        for case in pairs[kind]:
+            assert route(*case, kind)[0] == 1, (kind, case)
+
+
 @pytest.mark.parametrize("kind", (0, 1, 2, 3, 4))
 def test_every_route_is_one_the_kernels_are_built_for(plan, kind):
     """``bw_gemm_tc_route``: single CTAs in either orientation or CTA pairs (kind 0 plain, 1 SwiGLU, 2 rotary, 3 sums left open, 4 added
