@@ -97,6 +97,14 @@ __device__ __forceinline__ void put4(bf16* p, float4 v) {
 __device__ __forceinline__ void put2(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
 __device__ __forceinline__ void put2(bf16* p, float a, float b) { *reinterpret_cast<uint32_t*>(p) = bw::pack_bf16x2(a, b); }
 
+// Two pairs of channels turned: x cos - y sin and y cos + x sin, the product with the cosine fused with the sum.  Written out, so that every
+// kernel of a token's heads makes the same bits of it (left to the compiler, the kernel for many tokens fused the other product).
+template <typename OT>
+__device__ __forceinline__ void turn2(OT* first, OT* second, float x0, float x1, float y0, float y1, float2 cs, float2 sn) {
+    put2(first, fmaf(x0, cs.x, -__fmul_rn(y0, sn.x)), fmaf(x1, cs.y, -__fmul_rn(y1, sn.y)));
+    put2(second, fmaf(y0, cs.x, __fmul_rn(x0, sn.x)), fmaf(y1, cs.y, __fmul_rn(x1, sn.y)));
+}
+
 // The same with the norm taken per HEAD: every query head of dq channels is divided by its own root mean
 // square and multiplied by q_gain [dq], one gain vector shared by all heads (k_gain [dq] for the key heads);
 // a null gain: no norm on that side.  After norm and rotation the queries of a token at position p are
@@ -202,8 +210,7 @@ head_norm_rope_kernel(const float* __restrict__ qkv, long long ld, const int* __
                 if (c < half) {
                     if (!FEW) scales(i);
                     const float x0 = a[i].x * r2 * ga[i].x, x1 = a[i].y * r2 * ga[i].y, y0 = b[i].x * r2 * gb[i].x, y1 = b[i].y * r2 * gb[i].y;
-                    put2(dst + c, x0 * cs[i].x - y0 * sn[i].x, x1 * cs[i].y - y1 * sn[i].y);
-                    put2(dst + half + c, y0 * cs[i].x + x0 * sn[i].x, y1 * cs[i].y + x1 * sn[i].y);
+                    turn2(dst + c, dst + half + c, x0, x1, y0, y1, cs[i], sn[i]);
                 }
             }
 #pragma unroll
@@ -295,7 +302,7 @@ head_norm_rope_kernel(const float* __restrict__ qkv, long long ld, const int* __
 // The same for many tokens whose heads rotate as a whole, in halves (rotary_dim == dq == dpad <= 128), and whose values pass as they are.
 // What bounds it is how many rows' loads are in flight: a warp asks for HEADS heads of a token at once, and for the token's angles and
 // the two gains, which all its heads share, once (1,777 tokens of 32 + 8 heads of 128: 45 us in head_norm_rope_kernel, 24 so).  Sums and
-// products are in that kernel's order.
+// products are that kernel's, bit for bit.
 constexpr int HEADS = 5;
 template <typename OT>
 __global__ void __launch_bounds__(256)
@@ -349,8 +356,7 @@ head_norm_rope_whole_kernel(const float* __restrict__ qkv, long long ld, const i
             const float2 ga = is_q ? gqa : gka, gb = is_q ? gqb : gkb;
             OT* dst = is_q ? q_out + ((size_t)t * nh + h) * dq : k_pages + (((size_t)page * nkv + (h - nh)) * page_size + slot) * dq;
             const float x0 = a[u].x * r2 * ga.x, x1 = a[u].y * r2 * ga.y, y0 = b[u].x * r2 * gb.x, y1 = b[u].y * r2 * gb.y;
-            put2(dst + c, x0 * cs.x - y0 * sn.x, x1 * cs.y - y1 * sn.y);
-            put2(dst + half + c, y0 * cs.x + x0 * sn.x, y1 * cs.y + x1 * sn.y);
+            turn2(dst + c, dst + half + c, x0, x1, y0, y1, cs, sn);
         }
     }
     if (page < 0) return;

@@ -472,7 +472,7 @@ def rotary_case(ops, M, nh, nkv, hd, rd, bias_dtype):
 @pytest.mark.parametrize("dq,dv,dtype", [(128, 128, torch.bfloat16), (64, 40, torch.float32), (36, 36, torch.bfloat16), (128, 64, torch.float32)])
 @pytest.mark.parametrize("shared,gains", [(False, True), (False, False), (True, True)])
 def test_heads_of_many_tokens_as_of_few(ops, dq, dv, dtype, shared, gains):
-    """More than two tokens an SM take a kernel of their own where whole heads rotate: what the one for few tokens makes."""
+    """More than two tokens an SM take a kernel of their own where whole heads rotate: the bits that the one for few tokens makes."""
     import types
     if shared and dv != dq:
         pytest.skip("values that are the keys have their size")
@@ -492,12 +492,8 @@ def test_heads_of_many_tokens_as_of_few(ops, dq, dv, dtype, shared, gains):
         q = [ops.head_norm_rope_append(qkv[a:b], types.SimpleNamespace(positions=positions[a:b], req_of_token=req[a:b]), table, cs[a:b].contiguous(),
                                        dq, False, gq, gk, 1e-5, k, v, nh, nkv, dq, dv, **kw) for a, b in pieces]
         return torch.cat(q), k, v
-    # the same products and sums, of which the compiler may contract others: two roundings of a sum of two terms, then one to the type
-    tol = 2 ** -22 if dtype == torch.float32 else 2 ** -8
     for a, b in zip(run([(0, T)]), run([(0, T // 2), (T // 2, T)])):
-        largest = float(b.float().abs().max())
-        assert largest > 0 and float((a.float() - b.float()).abs().max()) <= tol * largest
-        assert torch.equal(a == 0, b == 0)
+        assert bool(b.any()) and torch.equal(a, b)
 
 
 def test_gemm_tc_row_independent_of_batch(ops):
