@@ -80,8 +80,8 @@ __device__ __forceinline__ float level_cut(int l) { return __uint_as_float((unsi
 // cuts of which it has few enough, in index order, and the row's first block, with all lists and the row's mass, selects and draws
 // among them by itself: up to 32 tokens in one warp, more (up to four a thread) from histograms of its own.  Where they do not reach the
 // target mass (a flat row), or a weight is no number, the histograms over all blocks decide; both find the same token.
-// What bounds it: latency (three cluster barriers, with the histograms over all blocks five; 20 exponentials, masses and votes a thread); a
-// row of 128,256 is 0.5 MB.  Measured, temperature 0.6, top_p 0.9, logits as a language model gives them: a row of 128,256 in 14 us, 32 rows
+// What bounds it: latency (three cluster barriers without a nucleus, four with the list, eight with the histograms over all blocks; 20
+// exponentials, masses and votes a thread); a row of 128,256 is 0.5 MB.  Measured, temperature 0.6, top_p 0.9, logits as a language model gives them: a row of 128,256 in 14 us, 32 rows
 // of 152,064 in 32 us (25 and 61 with the histograms over all blocks alone; one block per row and a bisection: 728 and 1,162).
 template <int NV, bool IN_SMEM = false, int CLUSTER = ROW_BLOCKS>
 __global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(THREADS, IN_SMEM || (NV == 0 && CLUSTER == 1) ? 2 : 1)
@@ -553,7 +553,22 @@ BW_EXPORT int bw_log_prob(const float* logits, const int* target, float* out, in
     return 0;
 }
 
-static int sample(const float* logits, const Rows& rows, bool greedy, int* out, int R, int V, long long ld, void* stream) {
+// Whether rows that are not all greedy take a block each, not a cluster: a row that fits a block's registers, or so many rows that their
+// clusters take turns for longer than a block walks its row.  With a nucleus a block walks it several times, so the line depends on it.
+// Temperature alone, us, on clusters and in blocks, logits from memory: 32 rows of 9,000 10.5 and 11.0, 48 of them 16.6 and 11.3; 128 of
+// 32,000 39 and 42, 160 of them 48 and 43; 200 of 64,000 70 and 77, 256 of them 88 and 79; 512 of 100,000 214 and 228; 256 of 128,256
+// 120 and 166; rows that a cluster's registers do not hold: 128 of 170,000 173 and 182, 160 of them 213 and 201, 160 of 256,000 297 and
+// 314, 200 of them 376 and 323.  With a nucleus, likely tokens few: 32 of 9,000 15 and 16, 64 of them 25 and 17; 128 of 32,000 52 and 54, 256
+// of them 96 and 73; 256 of 64,000 120 and 181, 1,024 of them 448 and 367; 256 of 128,256 162 and 361; 128 of 200,000 286 and 517, 256
+// of them 559 and 594.
+BW_EXPORT int bw_sample_row_in_a_block(int R, int V, int nucleus) {
+    if (V <= 8 * THREADS) return 1;
+    if (V > 160 * 1024) return R > (nucleus ? 200 : V / 1300);
+    if (!nucleus) return V <= 80 * 1024 && R > V / 256;
+    return R > V / 200;
+}
+
+static int sample(const float* logits, const Rows& rows, bool greedy, bool nucleus, int* out, int R, int V, long long ld, void* stream) {
     int bits = 0;
     while ((1ll << bits) < V) ++bits;
     const float scale = (float)(1ull << (62 - bits < 45 ? 62 - bits : 45));
@@ -566,12 +581,7 @@ static int sample(const float* logits, const Rows& rows, bool greedy, int* out, 
         BW_LAUNCH_CHECK();
         return 0;
     }
-    // Else one block a row where that is faster: a row that fits a block's registers, or so many rows that their clusters take turns for
-    // longer than a block walks its row (temperature / nucleus, us, on clusters and in blocks: 64 rows of 9,000 19 / 25 and 12 / 17, 32 of
-    // them 11 / 15 and 11 / 16; 128 of 32,000 38 / 52 and 31 / 54, 256 of them 76 / 96 and 42 / 73; 256 of 64,000 90 / 120 and 79 / 181,
-    // 1,024 of them 342 / 448 and 264 / 367; 256 of 128,256 120 / 162 and 167 / 361; of 200,000, which a cluster's registers do not hold, 128
-    // 201 / 286 and 229 / 517, 256 390 / 559 and 261 / 594).
-    if (V <= 8 * THREADS || R > (V > 160 * 1024 ? 200 : V / 200)) {
+    if (bw_sample_row_in_a_block(R, V, nucleus)) {
         const auto kernel = V <= 8 * THREADS ? sample_kernel<8, false, 1> : sample_kernel<0, false, 1>;
         bw::launch(kernel, dim3((unsigned)R), block, 0, (cudaStream_t)stream, logits, rows, out, V, (size_t)ld, scale);
         BW_LAUNCH_CHECK();
@@ -611,7 +621,7 @@ BW_EXPORT int bw_sample(const float* logits, const float* temperature, const flo
     if (temperature && !u) return BW_ERR_BAD_ARG;
     Rows rows{};
     rows.temperature = temperature; rows.top_p = top_p; rows.u = u;
-    return sample(logits, rows, !temperature, out, R, V, ld, stream);
+    return sample(logits, rows, !temperature, top_p != nullptr, out, R, V, ld, stream);
 }
 
 // The same with the rows' parameters in the caller's memory: they travel with the launch, no copy and no buffer on the device.  All three
@@ -622,6 +632,10 @@ BW_EXPORT int bw_sample_values(const float* logits, const float* temperature, co
     if (V <= 0 || ld < V || !temperature || !top_p || !u || R > VALUE_ROWS) return BW_ERR_BAD_ARG;
     Rows rows{};
     rows.by_value = 1;
-    for (int r = 0; r < R; ++r) { rows.v[0][r] = temperature[r]; rows.v[1][r] = top_p[r]; rows.v[2][r] = u[r]; }
-    return sample(logits, rows, false, out, R, V, ld, stream);
+    bool nucleus = false;
+    for (int r = 0; r < R; ++r) {
+        rows.v[0][r] = temperature[r]; rows.v[1][r] = top_p[r]; rows.v[2][r] = u[r];
+        nucleus |= temperature[r] > 0.f && top_p[r] < 1.f;
+    }
+    return sample(logits, rows, false, nucleus, out, R, V, ld, stream);
 }

@@ -74,4 +74,5 @@ class Sampler:
         if few:
             return ops.sample(logits, *rows)
         dev = host.to(self.device, non_blocking=True)
-        return ops.sample(logits, dev[0], dev[1], dev[2])
+        nucleus = any(p.top_p < 1.0 for p in params if not p.greedy)     # (without one many rows take another form)
+        return ops.sample(logits, dev[0], dev[1] if nucleus else None, dev[2])

@@ -511,3 +511,41 @@ def test_sampler_uploads_what_the_kernels_expect(monkeypatch):
     assert seen == {"sample": (None, None, None)}
     with pytest.raises(ValueError, match="one SamplingParams per logits row"):
         sm.sample(logits, params[:2], seeds, draws)
+
+
+@pytest.mark.parametrize("top_p", [0.9, 1.0])
+def test_sampler_says_whether_many_rows_ask_for_a_nucleus(monkeypatch, top_p):
+    """More rows than travel with a launch: top_p goes to the device only where a row that is drawn has one (the form of the kernel follows
+    from it)."""
+    import types
+
+    from blackwellllm_b200 import SamplingParams
+    from blackwellllm_b200.sampling import sampler as S
+    seen = []
+    shim = types.SimpleNamespace(**{k: getattr(torch, k) for k in ("float32", "int32", "Tensor", "device", "tensor")},
+                                 empty=lambda *size, pin_memory=False, **kw: torch.empty(*size, **kw))
+    monkeypatch.setattr(S, "torch", shim)
+    monkeypatch.setattr(S.ops, "sample", lambda logits, t, p, u: seen.append((t, p, u)) or torch.zeros(logits.shape[0], dtype=torch.int32))
+    R = S.ops.SAMPLE_VALUE_ROWS + 6
+    params = [SamplingParams(temperature=0.0, top_p=0.5)] + [SamplingParams(temperature=0.7, top_p=top_p)] * (R - 1)
+    S.Sampler(torch.device("cpu")).sample(torch.zeros((R, 16)), params, list(range(R)), [0] * R, [[]] * R)
+    (t, p, u), = seen
+    assert t.shape == u.shape == (R,)
+    assert p is None if top_p == 1.0 else p.tolist() == pytest.approx([0.5] + [0.9] * (R - 1))
+
+
+def test_many_rows_without_a_nucleus_take_a_block_each_sooner():
+    import ctypes
+
+    from blackwellllm_b200.kernels.build import load_library
+    fn = load_library("sampling").bw_sample_row_in_a_block
+    fn.argtypes = [ctypes.c_int] * 3
+    for R, V in ((48, 9000), (128, 32000), (256, 64000), (160, 170000)):
+        assert fn(R, V, 0), (R, V)
+    for R, V in ((128, 64000), (1024, 100000), (256, 128256), (128, 170000), (160, 256000)):
+        assert not fn(R, V, 0), (R, V)
+    for R, V in ((64, 9000), (256, 32000), (1024, 64000), (256, 200000)):
+        assert fn(R, V, 1), (R, V)
+    for R, V in ((32, 9000), (128, 32000), (256, 64000), (256, 128256), (128, 200000)):
+        assert not fn(R, V, 1), (R, V)
+    assert all(fn(1, 8192, nucleus) and not fn(32, 152064, nucleus) for nucleus in (0, 1))
