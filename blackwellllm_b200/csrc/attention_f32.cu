@@ -3,15 +3,17 @@
 // CUDA cores, as there; a key and a value are read once for all query heads of their group and for all tokens of a tile.
 //
 // A block of eight warps takes a tile of ROWS stacked query rows (token-major, then the heads of the group) of one request and
-// kv head and walks 32 keys at a time (two stages, cp.async).  Scores: each thread a few rows times a few keys.  Softmax and
-// values: warp w owns rows w ROWS / 8 on, a lane four channels (twice that for heads above 128), so probabilities pass through
-// shared memory inside the warp only.  ROWS = 64 for prompt portions, 16 for the few rows of a decoding request.  The keys of a tile
-// are one block's, or dealt out by slices to several, whose results a second kernel adds up.
+// kv head and walks its keys (cp.async).  ROWS = 64 for prompt portions: 64 keys at a time (32 for heads above 128) in two stages, each
+// thread scores 4 rows times 4 keys (2 times 4), a warp owns eight neighbouring rows.  ROWS = 16 for the few rows of a decoding request: 32 keys at
+// a time in three stages, a warp owns a row or two, which share the key that a lane scores.  In the softmax, 32 keys at a time, and the
+// values a lane has four channels (twice that for heads above 128), so probabilities pass through shared memory inside the warp only.  The
+// keys of a tile are one block's, or dealt out by slices to several, whose results a second kernel adds up.
 // A row's result is the same bits whatever else is in the batch: both forms make a softmax per slice of keys, counted from position 0,
 // in the same order of operations, and fold the slices in their order (fold()).  A slice has SLICE keys, or as many times SLICE that a
 // row sees MOST slices or hardly more: what a row sees decides, and no batch.  (So a decoding request has at most MOST + 2 blocks and
 // partial results per kv head at any context: 64 requests of 8 kv heads and groups of 4 at 131,072 tokens 69 MB.)
-// What bounds it: decode, the bytes of keys and values; prompts, shared-memory reads (six 16-byte reads per 32 FMAs); few keys, latency.
+// What bounds it: decode, the bytes of keys and values; prompts, shared-memory reads (eight 16-byte reads per 64 FMAs, for
+// heads above 128 six per 32); few keys, latency.
 // Measured at head size 128, groups of 4, 8 kv heads, against attention_simt.cu (a block per token and head, a lane a key): 4 requests
 // at 1,000 keys 18 us with the merge against 167, 4 portions of 200 tokens 109 against 1,402, 64 requests at 300 keys, groups of 1, 8 kv
 // heads of 64, 54 against 66.
