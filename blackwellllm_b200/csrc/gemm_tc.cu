@@ -1056,13 +1056,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // Split-K with many tokens: out = epilogue(sum over splits of partial), one thread per (token,
 // feature), splits added in order.  SwiGLU: one thread per (token, output feature) reads its gate
 // and up sums from the interleaved layout.
-__global__ void splitk_reduce_kernel(Epilogue ep) {
+template <bool ROPE>      // (the rotation's registers would cost the plain sums warps in flight)
+__global__ void __launch_bounds__(256, 5) splitk_reduce_kernel(Epilogue ep) {
     BW_PDL_TRIGGER();
     BW_PDL_WAIT();
     const size_t plane = (size_t)ep.tokens * ep.features;
     const int width = ep.swiglu ? ep.features / 2 : ep.features;
     const size_t total = (size_t)ep.tokens * width;
-    if (!ep.swiglu && !ep.rope_on && ep.out_type == BW_F32 && (ep.features & 3) == 0 && (ep.ldo & 3) == 0 &&
+    if (!ep.swiglu && !ROPE && ep.out_type == BW_F32 && (ep.features & 3) == 0 && (ep.ldo & 3) == 0 &&
         ((uintptr_t)ep.out & 15) == 0) {
         // float32 result, four features a thread: 16-byte loads of every plane, one 16-byte store
         const size_t quads = total / 4;
@@ -1082,7 +1083,7 @@ __global__ void splitk_reduce_kernel(Epilogue ep) {
         }
         return;
     }
-    if (ep.rope_on && (ep.features & 3) == 0 && (ep.rope.hd & 3) == 0 && ((uintptr_t)ep.partial & 15) == 0 &&
+    if (ROPE && (ep.features & 3) == 0 && (ep.rope.hd & 3) == 0 && ((uintptr_t)ep.partial & 15) == 0 &&
         (((uintptr_t)ep.rope.q_out | (uintptr_t)ep.rope.k_pages | (uintptr_t)ep.rope.v_pages) & 3) == 0) {
         // rotary: two pairs a thread, 16-byte loads of every plane (a thread a feature, each pair's planes read twice: 93 tokens of
         // 6144 x 4096 with their product 21.9 us)
@@ -1103,11 +1104,17 @@ __global__ void splitk_reduce_kernel(Epilogue ep) {
                 sn[p] = rot[p] ? __ldg(tab + half) : 0.f;
             }
             const int kv = !is_q && ro.kv_slot ? __ldg(ro.kv_slot + token) : -1;
+            // (the loads of four planes together, and of the last ones too: one by one, 20 tokens of 768 x 4096, eight planes, 8.8 us with
+            // their product, 40 of 6144 x 4096, three planes, 15.8)
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-            for (int s = 0; s < ep.splits; ++s) {
-                const float4 t = *reinterpret_cast<const float4*>(ep.partial + (size_t)s * plane + 4 * q);
-                v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+            for (int s0 = 0; s0 < ep.splits; s0 += 4) {
+                float4 t[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (s0 + i < ep.splits) t[i] = *reinterpret_cast<const float4*>(ep.partial + (size_t)(s0 + i) * plane + 4 * q);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (s0 + i < ep.splits) { v.x += t[i].x; v.y += t[i].y; v.z += t[i].z; v.w += t[i].w; }
             }
             bf16* dst = ro.q_out + ((size_t)token * ro.nh + head) * ro.hd;
             if (!is_q) {
@@ -1150,7 +1157,7 @@ __global__ void splitk_reduce_kernel(Epilogue ep) {
             ((bf16*)ep.out)[(size_t)token * ep.ldo + j] = __float2bfloat16_rn(ep_glu(ep, g, u));
             continue;
         }
-        if (ep.rope_on) {
+        if (ROPE) {
             const RopeSlot sl = rope_slot(ep.rope, j);
             float x = 0.f, partner = 0.f;
             for (int s = 0; s < ep.splits; ++s) {
@@ -1595,7 +1602,7 @@ static int run_gemm_tc(const void* x, const void* w, const void* bias, int bias_
         const size_t total = (size_t)M * (swiglu ? N / 2 : N);
         const size_t want = (total + 255) / 256;
         const int blocks = (int)(want < (size_t)NUM_SMS * 8 ? want : (size_t)NUM_SMS * 8);
-        bw::launch((splitk_reduce_kernel), dim3(blocks), dim3(256), 0, s, ep);
+        bw::launch(rope ? splitk_reduce_kernel<true> : splitk_reduce_kernel<false>, dim3(blocks), dim3(256), 0, s, ep);
         BW_LAUNCH_CHECK();
     }
     return 0;
