@@ -1320,12 +1320,20 @@ namespace {
 double split_sum_cost(int M, int N, int s) {
     return s <= 1 ? 0.0 : (2.5e-6 + (double)(s + 2) * M * N * 4.0 / 5e12) / 1.73e-9;
 }
+// Below 2,048 channels what a round's epilogue takes counts: six k-blocks of its columns; and starting pairs takes 0.9 us longer.  (us, pairs on 192
+// or 128 columns and single CTAs on 128: 257 to 300 tokens x 5120 x 1024 13.6 and 12.1, 300 x 4096 x 512 7.7 and 6.7, 257 x 3072 x 512 7.0 and 6.2,
+// but 512 x 5120 x 1024 13.7 and 14.5.)  SwiGLU's epilogue runs behind the next tile's products and was not found to follow such a line.
+// A written result in tiles of 240 columns goes out value by value (boxes have 32): 17 us a round (1,024 tokens x 4096 x 1024 29.9, 12.4 on pairs).
+double epilogue_cost(int kb, int width, bool swiglu, bool written = false) {
+    return kb >= 32 || swiglu ? 0.0 : (written && width % 32 ? 40.0 : 6.0) * width;
+}
+double pair_start_cost(int kb, bool swiglu) { return kb >= 32 || swiglu ? 0.0 : 500.0; }
 // single CTAs on tiles of 128 tokens x bn features: measured 15-20 % slower per flop than pairs at 224 to 256
 // columns, and at 53-66 % of a pair's rate at 128 columns (steps of 512 tokens, o and down of the 8B shape)
-double gemm_single_cost(int M, int N, int K, int bn, long long tiles, int splits) {
+double gemm_single_cost(int M, int N, int K, int bn, long long tiles, int splits, int kind) {
     const int NUM_SMS = bw::num_sms();
-    const int kb_total = ceil_div(K, BK);
-    return (double)ceil_div(tiles * splits, NUM_SMS) * ceil_div(kb_total, splits) * bn * (bn == 128 ? 1.7 : 1.18) +
+    const int kb = ceil_div(ceil_div(K, BK), splits);
+    return (double)ceil_div(tiles * splits, NUM_SMS) * (kb * bn * (bn == 128 ? 1.7 : 1.18) + epilogue_cost(kb, bn, kind == 1, kind == 0)) +
            split_sum_cost(M, N, splits);
 }
 }  // namespace
@@ -1339,7 +1347,7 @@ double gemm_single_cost(int M, int N, int K, int bn, long long tiles, int splits
 // were no faster than 256, 160 hardly faster than 192 where both fit a round.)  What the two narrow ones give: o of 3584 at 648 and 1,536
 // tokens 22.5 -> 20.3 and 37.4 -> 34.0, its down projection 87.4 -> 81.8 and 171 -> 161, q/k/v of 6144 x 4096 at 512 and 1,024 tokens
 // 31.9 -> 28.8 and 48.0 -> 44.5, o of 5120 at 2,048 82 -> 77, its down projection 217 -> 197.
-static double pair_plan(int M, int N, int K, int force_splits, long long workspace_elems, int* width, int* splits) {
+static double pair_plan(int M, int N, int K, bool swiglu, int force_splits, long long workspace_elems, int* width, int* splits) {
     const int NUM_SMS = bw::num_sms();
     const int kb_total = ceil_div(K, BK), pa = ceil_div(M, 2 * BM);
     const int widths[4] = {256, 224, 192, 128};
@@ -1355,7 +1363,9 @@ static double pair_plan(int M, int N, int K, int force_splits, long long workspa
             // way through memory costs more than the idle pairs (o at 512 tokens: 38 against 26 us).
             if (ps > 1 && force_splits <= 0 && (ps != 2 || kb_total < 128 || t * ps > NUM_SMS / 2)) continue;
             if (ps > kb_total || (ps > 1 && (long long)ps * M * N > workspace_elems)) continue;
-            const double cost = (double)ceil_div(t * ps, NUM_SMS / 2) * ceil_div(kb_total, ps) * columns[i] + split_sum_cost(M, N, ps);
+            const int kb = ceil_div(kb_total, ps);
+            const double cost = (double)ceil_div(t * ps, NUM_SMS / 2) * (kb * columns[i] + epilogue_cost(kb, widths[i], swiglu)) +
+                                pair_start_cost(kb, swiglu) + split_sum_cost(M, N, ps);
             if (best < 0.0 || cost < best * 0.995) { best = cost; *width = widths[i]; *splits = ps; }
         }
     }
@@ -1450,7 +1460,7 @@ BW_EXPORT int bw_gemm_tc_route(int M, int N, int K, int kind, int pair_mode, int
         // they are stay on single CTAs where K is long (8,192 and more), whose splits these deal out better, and up to 160 tokens where K is
         // split (o of 4096 at 160 tokens 17.5 / 19.2, its down projection 36 to 40 / 54)
         if (pair_mode > 0 && M > BM && ((kind != 0 && kind != 4) || (kb_total < 128 && (M > 160 || *splits == 1)))) {
-            const double pair = pair_plan(M, N, K, 0, workspace_elems, &width, &ps);
+            const double pair = pair_plan(M, N, K, kind == 1, 0, workspace_elems, &width, &ps);
             if (pair < 0.0) return 0;
             int tr = 0;
             if (kind == 1 && swiglu_pair_plan(M, N, K, &other) < 0.93 * pair) { tr = 1; width = other; ps = 1; }
@@ -1466,8 +1476,8 @@ BW_EXPORT int bw_gemm_tc_route(int M, int N, int K, int kind, int pair_mode, int
     // products with few output features) the pairs split K as well; the partial sums are added in split
     // order by the second kernel.
     if (pair_mode <= 0 || M <= 2 * BM) return 0;
-    const double pair = pair_plan(M, N, K, force_splits, workspace_elems, &width, &ps);
-    const double single = gemm_single_cost(M, N, K, *bn, (long long)ceil_div(M, BM) * ceil_div(N, *bn), *splits);
+    const double pair = pair_plan(M, N, K, kind == 1, force_splits, workspace_elems, &width, &ps);
+    const double single = gemm_single_cost(M, N, K, *bn, (long long)ceil_div(M, BM) * ceil_div(N, *bn), *splits, kind);
     if (kind == 1 && force_splits <= 0 && swiglu_pair_plan(M, N, K, &other) < 0.93 * (pair >= 0.0 && (pair_mode == 2 || pair <= single) ? pair : single)) {
         *transposed = 1; *bn = other; *splits = 1;
         return 1;

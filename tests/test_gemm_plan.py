@@ -139,6 +139,16 @@ def test_pairs_of_129_to_256_tokens_only_where_they_are_faster(route):
             assert route(*case, kind)[0] == 1, (kind, case)
 
 
+def test_few_channels_on_pairs_only_where_they_are_faster(route):
+    """Below 2,048 channels a tile's epilogue and the pairs' start count; a written result on tiles of 240 columns goes out value by value."""
+    for kind in (0, 2, 4):
+        for case in ((300, 5120, 1024), (257, 6144, 1024), (257, 3072, 512), (300, 4096, 512)):
+            assert route(*case, kind)[0] == 0, (kind, case)
+        for case in ((512, 5120, 1024), (300, 5120, 4096), (400, 6144, 1024), (300, 3072, 1024)):
+            assert route(*case, kind)[0] == 1, (kind, case)
+    assert route(1024, 4096, 1024, 0)[0] == 1 and route(1024, 4096, 512, 0)[0] == 1
+
+
 @pytest.mark.parametrize("kind", (0, 1, 2, 3, 4))
 def test_every_route_is_one_the_kernels_are_built_for(plan, kind):
     """``bw_gemm_tc_route``: single CTAs in either orientation or CTA pairs (kind 0 plain, 1 SwiGLU, 2 rotary, 3 sums left open, 4 added

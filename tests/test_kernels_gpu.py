@@ -442,8 +442,9 @@ def test_gemm_tc_rotary_routes(ops, M, nh, nkv, hd, rd, bias_dtype):
 @pytest.mark.parametrize("M,nh,nkv,width", [(300, 52, 4, 224), (257, 64, 4, 256)])
 @pytest.mark.parametrize("bias_dtype", [torch.bfloat16, torch.float32])
 def test_gemm_tc_rotary_on_pairs_of_the_wide_tiles(ops, route, M, nh, nkv, width, bias_dtype):
-    assert route(M, (nh + 2 * nkv) * 128, 520, 2) == (1, 0, width, 1)
-    rotary_case(ops, M, nh, nkv, 128, 128, bias_dtype)
+    K = 2056                       # (of fewer channels single CTAs take these)
+    assert route(M, (nh + 2 * nkv) * 128, K, 2) == (1, 0, width, 1)
+    rotary_case(ops, M, nh, nkv, 128, 128, bias_dtype, K)
 
 
 @pytest.mark.parametrize("splits", [5, 8, 9, 17])
