@@ -1397,7 +1397,9 @@ static double swiglu_pair_plan(int M, int N, int K, int* width) {
 // 42.0; 4096 x 4096 at 1,280 39.9 / 35.2.  But 3584 x 18944 at 1,024 tokens 95.4 / 96.1 and 3584 x 3584 at 648 22.7 / 29.5: the ranges' time
 // is 0.38 us a k-block and 7 us; a round's is 0.40 us (256 columns), less in one that is partly empty, down to 0.85 of it (the chip as a
 // whole, not a pair, is the limit there).  Tokens of more than 60 MB, which each range reads at its own place, leave L2: at 2,048 tokens of
-// 18,944 188 / 195.
+// 18,944 188 / 195.  Error against 64 bits (2-norm, added into zeros), rounds / ranges: 648 tokens of 3584 x 18944 2.2e-5 / 1.0e-5, 1,280 of 4096 x 14336
+// 1.6e-5 / 1.2e-5, 1,024 of 5120 x 5120 5.6e-6 / 4.1e-6; into a stream thirty times as large as the sums 2.0e-6 / 9.6e-7, 1.3e-6 / 9.7e-7, 2.7e-7 / 2.0e-7:
+// shorter running sums lose less than the additions.
 static int shared_ranges(int M, int N, int K, int width, int splits, double cost) {
     const int n_pairs = bw::num_sms() / 2, ta = ceil_div(M, 2 * BM), tb = ceil_div(N, 256), kb_total = ceil_div(K, BK);
     int ranges = n_pairs / ta;
